@@ -1,62 +1,80 @@
-// Device format builder: CSR -> SR-BCRS 16x8 / ME-TCF, bit-identical to the reference host packers.
+// Device format builder: CSR -> SR-BCRS 16x8 / ME-TCF / MCO, bit-identical to the reference host packers.
 //
 // The reference condenses the columns of every 16-row window with a per-thread byte mask over
 // all K columns plus std::sort, then places every entry with a binary search
-// (examples/src_fp32/sr_bcrs/testbed/main_16x8.cu:209-318).  Here the same result is obtained
-// with flat, one-thread-per-entry kernels and two device-wide scans, so that hub windows with
-// millions of entries cost no more per entry than small ones:
+// (examples/src_fp32/sr_bcrs/testbed/main_16x8.cu:209-318).  Here:
 //
-//   1. row_of[e]       row of entry e (binary search in rowptr).
-//   2. rank            entry e = (row r, column c) gets its index p in the window's merged,
-//                      column-sorted multiset: its offset in its own row plus, for every other
-//                      row of the window, the number of entries < c (rows after r) or <= c (rows
-//                      before r).  Rows are sorted, so each count is a binary search.  The column
-//                      is scattered to merged[base + p]; rows that are not strictly ascending or
-//                      columns outside [0,K) raise an error flag.
-//   3. distinct scan   flag[q] = merged[q] starts a new column value inside its window;
-//                      D = inclusive scan(flag).  The condensed position of a slot is
-//                      D[q] - D[base]; a window holds D[last] - D[base] + 1 distinct columns.
-//   4. tiles per window = ceil(distinct/8), exclusive scan -> val_soff, total T.
-//   5. fill            column metadata from the flagged slots, values scattered by condensed
-//                      position (Swizzle<2,2,3> for SR-BCRS); ME-TCF orders the entries of a tile
-//                      by (row, CSR order) using a 16 x 4-bit per-tile row histogram.
+//   1. condense    every entry gets its condensed position (the rank of its column among the distinct
+//                  columns of its window), every window its number of distinct columns.  The entries of a
+//                  window are contiguous in the CSR.  Windows of up to 1024 entries: one warp sorts them in
+//                  registers (bitonic network over 1..32 keys a lane, key = column << 10 | entry) and
+//                  numbers the distinct ones.  Larger windows: one block marks the columns in a bitmap in
+//                  shared memory, 2^20 columns at a time, and ranks every entry by a prefix popcount, which
+//                  costs the same whatever the row lengths.  Rows that are not strictly ascending or columns
+//                  outside [0, K) raise an error flag.
+//   2. tiles       ceil(distinct / 8) per window, exclusive scan -> val_soff, total T; the scan also notes
+//                  the window in which every 128th tile lies.
+//   3. fill        one block per 128 consecutive tiles composes them 32 at a time in shared memory (a row of
+//                  the window is walked by 8 lanes from the entry where the tiles begin; positions ascend
+//                  along a row) and writes whole tiles, so a value array of 512 bytes a tile is written once,
+//                  coalesced, and never read.  ME-TCF and MCO count the entries per tile the same way first
+//                  (16 x 4-bit row histogram, 128-bit mask), scan the run lengths and place the entries.
+//
+// Measured on a power-law graph with 2^20 nodes (17.1 M entries, 1.97 M tiles; one read of the CSR and one
+// write of the packed arrays is 0.2 ms at copy speed): condense 0.45 ms, scan 0.02, SR-BCRS fill
+// 0.40; a binary search of every entry in its 15 sibling rows, two more scans and a scatter into cleared tiles took
+// 2.3 ms.
 #include <algorithm>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+#include "condense.cuh"
+#include "mem.h"
 
 namespace mask {
 
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 16;
 constexpr int kScanChunk = kScanThreads * kScanItems;
+constexpr int kSmallItems = 4;
+constexpr int kSmallScan = 8 * 1024 * kSmallItems;   // one block takes about as long for this many as three launches
+
+constexpr int kFillTiles = 128;   // tiles a block of the fill writes ...
+constexpr int kFillSub = 32;      // ... and composes at a time
 
 struct PackScratch {
-    int32_t* row_of;     // nnz
-    int32_t* pos;        // nnz: merged index, later condensed position
-    int32_t* merged;     // nnz
-    int32_t* dscan;      // nnz: inclusive scan of distinct flags
-    int64_t* spine;      // per scan chunk
-    int32_t* status;     // [0] error flag, [1..2] int64 total
+    int32_t* pos;           // nnz: condensed position of every entry
+    int32_t* cols;          // nnz: distinct columns of a window in ascending order, from the window's first entry on
+    int32_t* rows;          // 16 W + 1: rowptr, rows behind the last one empty
+    int32_t* distinct;      // W: distinct columns per window
+    int32_t* big_list;      // windows of condense_big_kernel
+    int32_t* hub_list;      // windows of condense_hub_kernel
+    int32_t* first_window;  // per kFillTiles tiles (at most nnz tiles)
+    int64_t* spine;         // per scan chunk
+    int32_t* status;        // [0] error flags, [2..3] int64 total, [4], [5] lengths of the lists
     size_t bytes;
 };
 
 static inline size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
 static PackScratch carve(void* base, int32_t M, int64_t nnz) {
-    (void)M;
     PackScratch s{};
     char* p = static_cast<char*>(base);
     size_t off = 0;
-    const size_t n = (size_t)std::max<int64_t>(nnz, 1);
+    const size_t n = (size_t)std::max<int64_t>(nnz, 1), W = (size_t)(M + kWinRows - 1) / kWinRows;
     auto take = [&](size_t bytes) { char* r = p ? p + off : nullptr; off += align_up(bytes); return r; };
-    s.row_of = reinterpret_cast<int32_t*>(take(n * 4));
     s.pos = reinterpret_cast<int32_t*>(take(n * 4));
-    s.merged = reinterpret_cast<int32_t*>(take(n * 4));
-    s.dscan = reinterpret_cast<int32_t*>(take(n * 4));
+    s.cols = reinterpret_cast<int32_t*>(take(n * 4));
+    s.rows = reinterpret_cast<int32_t*>(take((W * kWinRows + 1) * 4));
+    s.distinct = reinterpret_cast<int32_t*>(take(W * 4));
+    s.big_list = reinterpret_cast<int32_t*>(take((n / 1024 + 1) * 4));
+    s.hub_list = reinterpret_cast<int32_t*>(take((n / 8192 + 1) * 4));
+    s.first_window = reinterpret_cast<int32_t*>(take((n / kFillTiles + 1) * 4));
     const size_t chunks = (std::max<size_t>(n, (size_t)M + 1) + kScanChunk - 1) / kScanChunk + 1;
     s.spine = reinterpret_cast<int64_t*>(take(chunks * 8));
     s.status = reinterpret_cast<int32_t*>(take(64));
-    s.bytes = off;
+    s.bytes = std::max(off, 16 * n);   // hosts have sized it by 16 bytes an entry
     return s;
 }
 
@@ -147,8 +165,51 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(In in, Out out
     }
 }
 
+// The whole scan in one block, for counts that three launches would take longer for.
+template <typename In, typename Out>
+__global__ void __launch_bounds__(1024) scan_small_kernel(In in, Out out, int64_t n, int64_t* total) {
+    __shared__ int64_t warp_tot[32];
+    int64_t carry = 0;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (int64_t c = 0; c < n; c += 1024 * kSmallItems) {
+        const int64_t base = c + (int64_t)threadIdx.x * kSmallItems;
+        int32_t v[kSmallItems];
+        int64_t s = 0;
+#pragma unroll
+        for (int i = 0; i < kSmallItems; i++) {
+            v[i] = (base + i < n) ? in(base + i) : 0;
+            s += v[i];
+        }
+        int64_t x = s;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) warp_tot[wid] = x;
+        __syncthreads();
+        int64_t before = carry + x - s;
+        for (int i = 0; i < 32; i++) {
+            const int64_t t = warp_tot[i];
+            if (i < wid) before += t;
+            carry += t;
+        }
+#pragma unroll
+        for (int i = 0; i < kSmallItems; i++) {
+            if (base + i < n) out(base + i, before, v[i]);
+            before += v[i];
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0 && total) *total = carry;
+}
+
 template <typename In, typename Out>
 static int device_scan(In in, Out out, int64_t n, int64_t* spine, int64_t* d_total, cudaStream_t st) {
+    if (n <= kSmallScan) {
+        scan_small_kernel<<<1, 1024, 0, st>>>(in, out, n, d_total);
+        MASK_CUDA_TRY(cudaGetLastError());
+        return MASK_OK;
+    }
     const int64_t chunks = (n + kScanChunk - 1) / kScanChunk;
     if (chunks > 0) {
         scan_reduce_kernel<<<(unsigned)chunks, kScanThreads, 0, st>>>(in, n, spine);
@@ -163,130 +224,492 @@ static int device_scan(In in, Out out, int64_t n, int64_t* spine, int64_t* d_tot
     return MASK_OK;
 }
 
-// ---- analysis kernels ----------------------------------------------------------------------
-__global__ void row_of_kernel(const int32_t* __restrict__ rowptr, int32_t M, int64_t nnz, int32_t* __restrict__ row_of) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    int lo = 0, hi = M;  // last row with rowptr[row] <= e
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if ((int64_t)__ldg(rowptr + mid) <= e) lo = mid; else hi = mid;
+// ---- condensed positions ---------------------------------------------------------------------
+constexpr int kSortMax = 1024;                    // largest window a warp sorts in registers
+constexpr int kSortIdxBits = 10;
+constexpr int kHubMin = 8192;                     // larger windows are shared by the blocks of a cluster
+constexpr int kBigThreads = 512;
+constexpr int kBigKeep = kHubMin / kBigThreads;
+constexpr int kHubThreads = 1024;
+constexpr int kBigBits = 1 << 19;                 // columns marked at a time: two blocks per SM
+constexpr int kHubBlocks = 8;
+constexpr int kHubBits = kMarkMax;                // most columns marked at a time by one block of a cluster
+constexpr int kBitmapBits = 1 << 20;              // columns a block marks at a time
+constexpr int kBitmapWords = kBitmapBits / 32;
+constexpr int kBitmapRuns = kBitmapWords / 128;
+constexpr int kBitmapSmem = kBitmapWords * 4 + kBitmapWords * 2;
+
+// One window of n <= 32 E entries: sorts (column, entry), numbers the distinct columns, writes every entry's
+// number to pos and the distinct columns to cols; returns how many there are.
+template <int E, typename Key>
+__device__ __forceinline__ int condense_warp(const int32_t* __restrict__ col, int n, int lane, uint16_t* __restrict__ slot_pos,
+                                             int32_t* __restrict__ pos, int32_t* __restrict__ cols) {
+    Key key[E];
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+        const int e = i * 32 + lane;   // any order will do
+        key[i] = e < n ? ((Key)(uint32_t)__ldg(col + e) << kSortIdxBits) | (Key)e : ~(Key)0;
     }
-    row_of[e] = lo;
+    warp_sort<E, Key>(key, lane);
+    Key before = __shfl_up_sync(0xffffffffu, key[E - 1], 1);
+    int cnt = 0;
+    uint32_t first = 0;   // bit i: key i starts a new column
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+        const bool f = lane * E + i < n && ((lane == 0 && i == 0) || (key[i] >> kSortIdxBits) != (before >> kSortIdxBits));
+        before = key[i];
+        first |= (f ? 1u : 0u) << i;
+        cnt += f;
+    }
+    int x = cnt;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    int at = x - cnt - 1;
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+        at += (first >> i) & 1u;
+        if (lane * E + i < n) slot_pos[(uint32_t)key[i] & (kSortMax - 1)] = (uint16_t)at;
+    }
+    __syncwarp();
+    for (int e = lane; e < n; e += 32) {
+        const int q = slot_pos[e];
+        pos[e] = q;
+        if (q < n) cols[q] = __ldg(col + e);   // entries of one column write the same word
+    }
+    return __shfl_sync(0xffffffffu, x, 31);
 }
 
-__device__ __forceinline__ int count_below(const int32_t* __restrict__ col, int lo, int hi, int key, bool inclusive) {
-    // number of entries in col[lo,hi) that are < key (or <= key)
-    const int start = lo;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const int v = __ldg(col + mid);
-        if (inclusive ? (v <= key) : (v < key)) lo = mid + 1; else hi = mid;
-    }
-    return lo - start;
+// Is column c of entry e acceptable: inside [0, K), and above its left neighbour unless e begins a row?
+__device__ __forceinline__ int entry_faults(const int32_t* __restrict__ colind, int e, int c, int32_t K, bool row_start) {
+    int bad = (c < 0 || c >= K) ? 2 : 0;
+    if (!row_start && __ldg(colind + e - 1) >= c) bad |= 1;
+    return bad;
 }
 
-__global__ void rank_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M, int32_t K,
-                            int64_t nnz, const int32_t* __restrict__ row_of, int32_t* __restrict__ pos,
-                            int32_t* __restrict__ merged, int32_t* __restrict__ status) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    const int r = row_of[e];
-    const int c = __ldg(colind + e);
-    const int rs = __ldg(rowptr + r);
-    if (c < 0 || c >= K) { atomicOr(status, 2); }
-    if (e > rs && __ldg(colind + e - 1) >= c) { atomicOr(status, 1); }
-    const int r0 = (r / kWinRows) * kWinRows;
-    const int r1 = min(r0 + kWinRows, M);
-    int p = (int)(e - rs);
-    int lo = __ldg(rowptr + r0);
-    const int base = lo;
-    for (int i = r0; i < r1; i++) {
-        const int hi = __ldg(rowptr + i + 1);
-        if (i != r) p += count_below(colind, lo, hi, c, i < r);
-        lo = hi;
+// One warp per window; windows above kSortMax entries go to the list of the bitmap kernel.
+template <typename Key>
+__global__ void __launch_bounds__(128) condense_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
+                                                       int32_t M, int32_t K, int32_t W, int32_t* __restrict__ pos,
+                                                       int32_t* __restrict__ cols, int32_t* __restrict__ rows,
+                                                       int32_t* __restrict__ distinct, int32_t* __restrict__ big_list,
+                                                       int32_t* __restrict__ hub_list, int32_t* __restrict__ status) {
+    __shared__ uint16_t slot_pos[4][kSortMax];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int w = blockIdx.x * 4 + warp;
+    if (w >= W) return;
+    const int r0 = w * kWinRows;
+    const int bound = __ldg(rowptr + min(r0 + min(lane, kWinRows), M));   // lane i: where row i of the window begins
+    const int base = __shfl_sync(0xffffffffu, bound, 0), n = __shfl_sync(0xffffffffu, bound, kWinRows) - base;
+    if (lane <= kWinRows) rows[r0 + lane] = bound;   // entry 16 is the next window's entry 0
+    if (n > kSortMax) {
+        if (lane == 0) {
+            if (n > kHubMin) hub_list[atomicAdd(status + 5, 1)] = w;
+            else big_list[atomicAdd(status + 4, 1)] = w;
+        }
+        return;
     }
-    pos[e] = p;
-    merged[base + p] = c;
+    int bad = 0;
+    for (int j = 0; j < n; j += 32) {
+        const int e = base + j + lane;
+        bool start = false;
+#pragma unroll
+        for (int i = 0; i < kWinRows; i++) start |= e == __shfl_sync(0xffffffffu, bound, i);
+        if (j + lane < n) bad |= entry_faults(colind, e, __ldg(colind + e), K, start);
+    }
+    if (bad) atomicOr(status, bad);
+    int d = 0;
+    if (n > 512) d = condense_warp<32, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
+    else if (n > 256) d = condense_warp<16, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
+    else if (n > 128) d = condense_warp<8, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
+    else if (n > 64) d = condense_warp<4, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
+    else if (n > 32) d = condense_warp<2, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
+    else if (n > 0) d = condense_warp<1, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
+    if (lane == 0) distinct[w] = d;
 }
 
-struct FlagIn {
-    const int32_t* rowptr;
-    const int32_t* row_of;
-    const int32_t* merged;
-    __device__ int32_t operator()(int64_t q) const {
-        const int w0 = (row_of[q] / kWinRows) * kWinRows;
-        if (q == (int64_t)__ldg(rowptr + w0)) return 1;
-        return merged[q] != merged[q - 1];
+// Windows of kSortMax + 1 to kHubMin entries, dealt to the blocks round-robin: the entries stay in registers,
+// kBigBits columns are marked, counted, ranked and unmarked at a time.
+__global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
+                                                                   int32_t M, int32_t K, int32_t* __restrict__ pos,
+                                                                   int32_t* __restrict__ cols, int32_t* __restrict__ distinct,
+                                                                   const int32_t* __restrict__ big_list, int32_t* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int run_before[kBigBits / 4096];
+    __shared__ int bound[kWinRows + 1];
+    __shared__ int warp_sum[32];
+    const int tid = threadIdx.x;
+    const int n_big = status[4];
+    if ((int)blockIdx.x >= n_big) return;
+    MarkSet marks{reinterpret_cast<uint32_t*>(smem), reinterpret_cast<uint16_t*>(smem + kBigBits / 8), run_before,
+                  (min(K, kBigBits) + 4095) / 4096};
+    for (int i = tid; i < marks.n_runs * 128; i += kBigThreads) marks.bits[i] = 0;
+    for (int b = blockIdx.x; b < n_big; b += gridDim.x) {
+        const int w = big_list[b];
+        __syncthreads();
+        if (tid <= kWinRows) bound[tid] = rowptr[min(w * kWinRows + tid, M)];
+        __syncthreads();
+        const int e0 = bound[0], n = bound[kWinRows] - e0;
+        int total = 0, bad = 0;
+        int c[kBigKeep];
+#pragma unroll
+        for (int i = 0; i < kBigKeep; i++) {
+            const int j = i * kBigThreads + tid;
+            c[i] = j < n ? __ldg(colind + e0 + j) : -1;
+        }
+#pragma unroll
+        for (int i = 0; i < kBigKeep; i++) {
+            const int e = e0 + i * kBigThreads + tid;
+            bool start = false;
+#pragma unroll
+            for (int r = 0; r < kWinRows; r++) start |= e == bound[r];
+            if (e - e0 < n) bad |= entry_faults(colind, e, c[i], K, start);
+        }
+        for (int c0 = 0; c0 < K; c0 += kBigBits) {
+            const int span = min(kBigBits, K - c0);
+#pragma unroll
+            for (int i = 0; i < kBigKeep; i++)
+                if (c[i] >= c0 && c[i] - c0 < span) marks.mark(c[i] - c0);
+            const int all = marks.count<kBigThreads>(warp_sum);
+#pragma unroll
+            for (int i = 0; i < kBigKeep; i++)
+                if (c[i] >= c0 && c[i] - c0 < span) {
+                    const int q = total + marks.rank(c[i] - c0);
+                    pos[e0 + i * kBigThreads + tid] = q;
+                    cols[e0 + q] = c[i];
+                }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < kBigKeep; i++)
+                if (c[i] >= c0 && c[i] - c0 < span) marks.unmark(c[i] - c0);
+            total += all;
+            __syncthreads();
+        }
+        if (bad) atomicOr(status, bad);
+        if (tid == 0) distinct[w] = total;
     }
-};
-struct InclusiveOut {
-    int32_t* d;
-    __device__ void operator()(int64_t i, int64_t before, int32_t v) const { d[i] = (int32_t)(before + v); }
-};
+}
 
-// tiles per window from the distinct-column scan
+// Windows of more than kHubMin entries, dealt to clusters of kHubBlocks blocks.  Every block takes a range of
+// columns -- cut at the eighths of the window's longest row, so that the ranges hold about as many entries each --
+// which is a run of entries in each of the 16 rows, found by a 32-way search; the blocks exchange their counts
+// through distributed shared memory and rank what they marked themselves.  A range wider than kHubBits is taken in
+// parts (marked once to count, once more to rank).  With one block per window the 150 000 entries of the largest
+// window of a power-law graph with 2^20 nodes took 0.3 ms while the rest of the GPU had finished.
+__global__ void __cluster_dims__(kHubBlocks, 1, 1) __launch_bounds__(kHubThreads, 1)
+condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M, int32_t K, int32_t span,
+                    int32_t* __restrict__ pos, int32_t* __restrict__ cols, int32_t* __restrict__ distinct,
+                    const int32_t* __restrict__ hub_list, int32_t* __restrict__ status) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int run_before[kHubBits / 4096];
+    __shared__ int bound[kWinRows + 1];
+    __shared__ int cut[2][kWinRows];           // first entry of the row in this block's columns, first behind them
+    __shared__ int first[kWinRows + 1];        // list index of the row's first entry
+    __shared__ int warp_sum[32];
+    __shared__ int range_marks[2][kHubBlocks]; // two windows: a block may be one ahead of another
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int me = (int)cluster.block_rank();
+    const int n_hub = status[5], n_clusters = gridDim.x / kHubBlocks;
+    MarkSet marks{reinterpret_cast<uint32_t*>(smem), reinterpret_cast<uint16_t*>(smem + span / 8), run_before, span / 4096};
+    for (int i = tid; i < span / 128; i += kHubThreads) reinterpret_cast<uint4*>(marks.bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+    int turn = 0;
+    for (int b = blockIdx.x / kHubBlocks; b < n_hub; b += n_clusters, turn ^= 1) {
+        const int w = hub_list[b];
+        __syncthreads();
+        if (tid <= kWinRows) bound[tid] = rowptr[min(w * kWinRows + tid, M)];
+        __syncthreads();
+        const int e0 = bound[0], n = bound[kWinRows] - e0;
+        int bad = 0;
+        for (int j = me * kHubThreads + tid; j < n; j += kHubBlocks * kHubThreads) {
+            const int e = e0 + j;
+            bool start = false;
+#pragma unroll
+            for (int r = 0; r < kWinRows; r++) start |= e == bound[r];
+            bad |= entry_faults(colind, e, __ldg(colind + e), K, start);
+        }
+        if (bad) atomicOr(status, bad);
+        int longest = 0;
+        for (int r = 1; r < kWinRows; r++)
+            if (bound[r + 1] - bound[r] > bound[longest + 1] - bound[longest]) longest = r;
+        const int at = bound[longest], len = bound[longest + 1] - at;   // len >= 512: the window has more than 8192 entries
+        auto splitter = [&](int i) {
+            const int c = i == 0 ? 0 : (i == kHubBlocks ? K : __ldg(colind + at + (int)((int64_t)len * i / kHubBlocks)));
+            return max(0, min(K, c));
+        };
+        const int c_lo = splitter(me), c_hi = max(c_lo, splitter(me + 1));
+        {   // warp: row warp % 16, lower or upper end
+            const int r = warp & (kWinRows - 1), hi = warp >> 4, key = hi ? c_hi : c_lo;
+            int p = bound[r], left = bound[r + 1] - p;
+            while (left > 0) {
+                const int stride = (left + 31) >> 5, probe = min((lane + 1) * stride, left);
+                const bool below = __ldg(colind + p + probe - 1) < key;
+                const int hits = __popc(__ballot_sync(0xffffffffu, below));   // the probes that hit come first
+                const int step = hits == 32 ? left : min(hits * stride, left);
+                p += step;
+                left = hits == 32 ? 0 : min(stride - 1, left - step);
+            }
+            if (lane == 0) cut[hi][r] = p;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            int x = 0;
+            for (int r = 0; r < kWinRows; r++) {
+                first[r] = x;
+                x += max(cut[1][r] - cut[0][r], 0);
+            }
+            first[kWinRows] = x;
+        }
+        __syncthreads();
+        const int m = first[kWinRows];
+        auto entry = [&](int i) {   // entry of list index i
+            int r = 0;
+#pragma unroll
+            for (int half = kWinRows / 2; half > 0; half >>= 1)
+                if (first[r + half] <= i) r += half;
+            return cut[0][r] + i - first[r];
+        };
+        // columns of [c0, c0 + part); others only occur in the list when rows are not ascending, which is an error anyway
+        auto mark_part = [&](int c0, int part) {
+            marks.n_runs = (part + 4095) / 4096;
+            for (int i0 = 0; i0 < m; i0 += kHubThreads) {
+                const int i = i0 + tid, d = i < m ? __ldg(colind + entry(i)) - c0 : -1;
+                marks.mark_ascending(d < part ? d : -1);
+            }
+        };
+        auto unmark_part = [&](int c0, int part) {
+            __syncthreads();
+            for (int i = tid; i < m; i += kHubThreads) {
+                const int d = __ldg(colind + entry(i)) - c0;
+                if (d >= 0 && d < part) marks.unmark(d);
+            }
+            __syncthreads();
+        };
+        const bool whole = c_hi - c_lo <= span;
+        int mine = 0;
+        for (int c0 = c_lo; c0 < c_hi; c0 += span) {
+            mark_part(c0, min(span, c_hi - c0));
+            mine += marks.count<kHubThreads>(warp_sum);
+            if (!whole) unmark_part(c0, min(span, c_hi - c0));
+        }
+        if (tid < kHubBlocks) cluster.map_shared_rank(range_marks[turn], tid)[me] = mine;
+        cluster.sync();
+        int ahead = 0, total = 0;
+        for (int i = 0; i < kHubBlocks; i++) {
+            const int v = range_marks[turn][i];
+            total += v;
+            if (i < me) ahead += v;
+        }
+        for (int c0 = c_lo; c0 < c_hi; c0 += span) {
+            const int part = min(span, c_hi - c0);
+            int here = mine;
+            if (!whole) {
+                mark_part(c0, part);
+                here = marks.count<kHubThreads>(warp_sum);
+            }
+#pragma unroll 2
+            for (int i = tid; i < m; i += kHubThreads) {
+                const int e = entry(i), c = __ldg(colind + e), d = c - c0;
+                if (d >= 0 && d < part) {
+                    const int q = ahead + marks.rank(d);
+                    pos[e] = q;
+                    cols[e0 + q] = c;
+                }
+            }
+            unmark_part(c0, part);
+            ahead += here;
+        }
+        if (me == 0 && tid == 0) distinct[w] = total;
+    }
+    cluster.sync();   // nobody leaves while another block may still write its counts here
+}
+
+// tiles per window, and their exclusive scan
 struct WindowTilesIn {
-    const int32_t* rowptr;
-    const int32_t* dscan;
-    int32_t M, W;
-    __device__ int32_t operator()(int64_t w) const {
-        if (w >= W) return 0;
-        const int r0 = (int)w * kWinRows, r1 = min(r0 + kWinRows, M);
-        const int b = __ldg(rowptr + r0), e = __ldg(rowptr + r1);
-        if (e <= b) return 0;
-        const int distinct = dscan[e - 1] - dscan[b] + 1;
-        return (distinct + kTileCols - 1) / kTileCols;
+    const int32_t* distinct;
+    int32_t W;
+    __device__ int32_t operator()(int64_t w) const { return w < W ? (distinct[w] + kTileCols - 1) / kTileCols : 0; }
+};
+// first_window[c]: the window that holds tile c * kFillTiles (where the fill's block c begins)
+struct SoffOut {
+    int32_t* soff;
+    int32_t* first_window;
+    __device__ void operator()(int64_t w, int64_t before, int32_t tiles) const {
+        soff[w] = (int32_t)before;
+        for (int64_t c = (before + kFillTiles - 1) / kFillTiles; c * kFillTiles < before + tiles; c++) first_window[c] = (int32_t)w;
     }
 };
-struct ExclusiveOut {
-    int32_t* d;
-    __device__ void operator()(int64_t i, int64_t before, int32_t) const { d[i] = (int32_t)before; }
+
+// ---- fill ------------------------------------------------------------------------------------
+// nibble r of a tile's row word: stored entries of window row r in the tile (at most 8)
+__device__ __forceinline__ int nibble_sum(unsigned long long x) {
+    x = (x & 0x0f0f0f0f0f0f0f0full) + ((x >> 4) & 0x0f0f0f0f0f0f0f0full);
+    return (int)((x * 0x0101010101010101ull) >> 56);
+}
+
+enum FillMode { kFillSrbcrs, kCountMetcf, kFillMetcf, kMaskMco, kFillMco };
+
+struct FillArgs {
+    const int32_t* rows;
+    const int32_t* cols;
+    const int32_t* distinct;
+    const float* values;       // NULL: every entry is 1.0 (ME-TCF, MCO)
+    const int32_t* pos;
+    const int32_t* soff;
+    const int32_t* first_window;
+    int64_t T;
+    int32_t skip_zero;         // MCO: entries with value 0 are not stored
+    int32_t* sidx;
+    float* block_val;          // SR-BCRS
+    int32_t* edge_to_col;
+    int32_t* edge_to_row;
+    unsigned long long* tile_rows;   // ME-TCF: entries per row of a tile, 16 nibbles
+    unsigned long long* masks;       // MCO
+    const int32_t* off;        // ME-TCF: [begin, end) per tile; MCO: begin per tile
+    int32_t* coo_idx;
+    float* out_val;
 };
 
-__global__ void condensed_pos_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ row_of,
-                                     const int32_t* __restrict__ dscan, int64_t nnz, int32_t* __restrict__ pos) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    const int base = __ldg(rowptr + (row_of[e] / kWinRows) * kWinRows);
-    pos[e] = dscan[base + pos[e]] - dscan[base];
-}
-
-// ---- fill kernels --------------------------------------------------------------------------
-// Column metadata: one thread per merged slot.  PAD_LAST: tail slots of a window's last tile
-// repeat its last real column (SR-BCRS); otherwise they stay 0 (ME-TCF).
-template <bool PAD_LAST>
-__global__ void sidx_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ row_of,
-                            const int32_t* __restrict__ merged, const int32_t* __restrict__ dscan,
-                            const int32_t* __restrict__ val_soff, int32_t M, int64_t nnz, int32_t* __restrict__ val_sidx) {
-    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nnz) return;
-    const int w = row_of[q] / kWinRows;
-    const int r0 = w * kWinRows, r1 = min(r0 + kWinRows, M);
-    const int base = __ldg(rowptr + r0), end = __ldg(rowptr + r1);
-    const int c = merged[q];
-    const bool first = (q == base) || (merged[q - 1] != c);
-    const int rank = dscan[q] - dscan[base];
-    int32_t* out = val_sidx + (int64_t)__ldg(val_soff + w) * kTileCols;
-    if (first) out[rank] = c;
-    if (PAD_LAST && q == end - 1) {
-        const int slots = (__ldg(val_soff + w + 1) - __ldg(val_soff + w)) * kTileCols;
-        for (int j = rank + 1; j < slots; j++) out[j] = c;
+// One block per kFillTiles consecutive tiles, kFillSub at a time.  The entries of a row that fall into the
+// tiles are consecutive (positions ascend along a row): the 8 lanes of group tid / 8 find their number with an
+// 8-way search, then all threads take the entries of the 16 rows as one list -- a hub row with most of the
+// entries is not left to 8 lanes.  What bounds it is writing the tiles (SR-BCRS); several blocks per SM
+// cover the chain first_window -> val_soff -> rows -> positions -> values.
+template <int MODE>
+__global__ void __launch_bounds__(128) fill_kernel(const FillArgs p) {
+    constexpr bool kIds = MODE == kFillSrbcrs || MODE == kFillMetcf || MODE == kFillMco;
+    constexpr bool kMco = MODE == kMaskMco || MODE == kFillMco;
+    __shared__ __align__(16) float tile[MODE == kFillSrbcrs ? kFillSub * kTileElems : 4];
+    __shared__ unsigned long long words[MODE == kFillSrbcrs ? 1 : (kMco ? 2 * kFillSub : kFillSub)];
+    __shared__ int32_t begin[kFillSub];
+    __shared__ int row_entry[kWinRows], row_first[kWinRows + 1], row_begin[kWinRows];
+    const int tid = threadIdx.x, r = tid >> 3, l = tid & 7, group = (tid & 31) & ~7;
+    const int64_t block_end = min(p.T, ((int64_t)blockIdx.x + 1) * kFillTiles);
+    int64_t t = (int64_t)blockIdx.x * kFillTiles;
+    int w = p.first_window[blockIdx.x];
+    int64_t s0 = p.soff[w], s1 = p.soff[w + 1];
+    while (t < block_end) {
+        const int row = w * kWinRows + r;
+        const int beg = __ldg(p.rows + row), end = __ldg(p.rows + row + 1);
+        const int base = kIds ? __ldg(p.rows + w * kWinRows) : 0, n_cols = kIds ? __ldg(p.distinct + w) : 0;
+        const int64_t te = s1 < block_end ? s1 : block_end;
+        const int64_t next_s1 = te < block_end ? p.soff[w + 2] : 0;
+        int e = beg;
+        if (t > s0) {   // the block begins inside this window: first entry of the row at or after tile t
+            const int first = (int)(t - s0) * kTileCols;
+            int hi = end;
+            while (e < hi) {
+                const int mid = (e + hi) >> 1;
+                if (__ldg(p.pos + mid) < first) e = mid + 1; else hi = mid;
+            }
+        }
+        for (int64_t c = t; c < te; c += kFillSub) {
+            const int nt = (int)min((int64_t)kFillSub, te - c);
+            const int p0 = (int)(c - s0) * kTileCols, limit = p0 + nt * kTileCols;
+            if (MODE == kFillSrbcrs) {
+                for (int i = tid; i < nt * 32; i += 128) reinterpret_cast<float4*>(tile)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            } else if (MODE == kCountMetcf) {
+                if (tid < nt) words[tid] = 0ull;
+            } else if (MODE == kMaskMco) {
+                if (tid < 2 * nt) words[tid] = 0ull;
+            } else if (MODE == kFillMetcf) {
+                if (tid < nt) { words[tid] = p.tile_rows[c + tid]; begin[tid] = p.off[2 * (c + tid)]; }
+            } else {
+                if (tid < 2 * nt) words[tid] = p.masks[2 * c + tid];
+                if (tid < nt) begin[tid] = p.off[c + tid];
+            }
+            if (kIds) {   // tail slots of a window repeat its last column, or are 0 (ME-TCF)
+                for (int i = tid; i < nt * kTileCols; i += 128) {
+                    const int q = p0 + i;
+                    p.sidx[c * kTileCols + i] = (MODE == kFillMetcf && q >= n_cols) ? 0 : __ldg(p.cols + base + min(q, n_cols - 1));
+                }
+            }
+            // entries of this row that lie in the tiles: [e, e + cnt)
+            int cnt = 0;
+            for (int left = min(end - e, nt * kTileCols);;) {
+                const int stride = (left + 7) >> 3, probe = min((l + 1) * stride, left);
+                const bool below = left > 0 && __ldg(p.pos + e + cnt + probe - 1) < limit;
+                const int hits = __popc((__ballot_sync(0xffffffffu, below) >> group) & 0xffu);   // the probes that hit come first
+                const int step = hits == 8 ? left : hits * stride;
+                cnt += step;
+                left = hits == 8 ? 0 : min(stride - 1, left - step);
+                if (!__any_sync(0xffffffffu, left > 0)) break;
+            }
+            if (l == 0) { row_entry[r] = e; row_begin[r] = beg; row_first[r + 1] = cnt; }
+            e += cnt;
+            __syncthreads();
+            if (tid < 32) {
+                int x = tid < kWinRows ? row_first[tid + 1] : 0;
+                for (int o = 1; o < kWinRows; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (tid >= o) x += y;
+                }
+                if (tid < kWinRows) row_first[tid + 1] = x;
+                if (tid == 0) row_first[0] = 0;
+            }
+            __syncthreads();
+            for (int i = tid; i < row_first[kWinRows]; i += 128) {
+                int rr = 0;   // last row whose first list index is <= i
+#pragma unroll
+                for (int half = kWinRows / 2; half > 0; half >>= 1)
+                    if (row_first[rr + half] <= i) rr += half;
+                const int ee = row_entry[rr] + i - row_first[rr];
+                const int q = __ldg(p.pos + ee), lt = (q - p0) >> 3, cc = q & 7;
+                if (MODE == kFillSrbcrs) {
+                    tile[lt * kTileElems + sw223(rr * kTileCols + cc)] = __ldg(p.values + ee);
+                    if (p.edge_to_col) p.edge_to_col[ee] = q;
+                    if (p.edge_to_row) p.edge_to_row[ee] = w * kWinRows + rr;
+                } else if (MODE == kCountMetcf) {
+                    atomicAdd(words + lt, 1ull << (4 * rr));
+                } else if (MODE == kFillMetcf) {   // entries of earlier rows, then earlier entries of this row
+                    int at = begin[lt] + (rr == 0 ? 0 : nibble_sum(words[lt] & ((1ull << (4 * rr)) - 1ull)));
+                    for (int j = ee - 1; j >= row_begin[rr] && (__ldg(p.pos + j) >> 3) == (q >> 3); j--) at++;
+                    p.coo_idx[at] = sw123(rr * kTileCols + cc);
+                    p.out_val[at] = p.values ? __ldg(p.values + ee) : 1.0f;
+                } else {
+                    const float v = p.values ? __ldg(p.values + ee) : 1.0f;
+                    if (!(p.skip_zero && p.values && v == 0.0f)) {
+                        const int phys = sw123(rr * kTileCols + cc), upper = phys >> 6;
+                        if (MODE == kMaskMco) {
+                            atomicOr(words + 2 * lt + upper, 1ull << (phys & 63));
+                        } else {   // values in ascending bit order: the slot is the number of bits below
+                            const int below = __popcll(words[2 * lt + upper] & ((1ull << (phys & 63)) - 1ull));
+                            p.out_val[begin[lt] + below + (upper ? __popcll(words[2 * lt]) : 0)] = v;
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            if (MODE == kFillSrbcrs) {
+                float4* out = reinterpret_cast<float4*>(p.block_val + c * kTileElems);
+                for (int i = tid; i < nt * 32; i += 128) out[i] = reinterpret_cast<const float4*>(tile)[i];
+            } else if (MODE == kCountMetcf) {
+                if (tid < nt) p.tile_rows[c + tid] = words[tid];
+            } else if (MODE == kMaskMco) {
+                if (tid < 2 * nt) p.masks[2 * c + tid] = words[tid];
+            } else if (tid < nt) {   // the padding at the end of the tile's run
+                const int cnt = MODE == kFillMetcf ? nibble_sum(words[tid]) : __popcll(words[2 * tid]) + __popcll(words[2 * tid + 1]);
+                const int pad = MODE == kFillMetcf ? (cnt + 7) & ~7 : (cnt + 3) & ~3;
+                for (int i = cnt; i < pad; i++) {
+                    if (MODE == kFillMetcf) p.coo_idx[begin[tid] + i] = 0;
+                    p.out_val[begin[tid] + i] = 0.f;
+                }
+            }
+            __syncthreads();
+        }
+        t = te;
+        if (t == s1 && t < block_end) {   // on to the next window with tiles
+            w++;
+            s0 = s1;
+            s1 = next_s1;
+            while (s1 == s0) {
+                w++;
+                s1 = p.soff[w + 1];
+            }
+        }
     }
-}
-
-__global__ void srbcrs_values_kernel(const int32_t* __restrict__ row_of, const int32_t* __restrict__ pos,
-                                     const float* __restrict__ values, const int32_t* __restrict__ val_soff, int64_t nnz,
-                                     float* __restrict__ val_block_val, int32_t* __restrict__ edge_to_col,
-                                     int32_t* __restrict__ edge_to_row) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    const int r = row_of[e], p = pos[e];
-    const int w = r / kWinRows;
-    const int64_t tile = (int64_t)__ldg(val_soff + w) + p / kTileCols;
-    val_block_val[tile * kTileElems + sw223((r - w * kWinRows) * kTileCols + p % kTileCols)] = values[e];
-    if (edge_to_col) edge_to_col[e] = p;
-    if (edge_to_row) edge_to_row[e] = r;
 }
 
 __global__ void block_partition_kernel(const int32_t* __restrict__ val_soff, int32_t W, int32_t* __restrict__ bp) {
@@ -294,98 +717,66 @@ __global__ void block_partition_kernel(const int32_t* __restrict__ val_soff, int
     if (w < W) bp[w] = val_soff[w + 1] - val_soff[w];
 }
 
-// ME-TCF: per tile, a 64-bit word with one 4-bit counter per window row (a row holds at most 8
-// entries of a tile, so the counters cannot carry).
-__global__ void metcf_histogram_kernel(const int32_t* __restrict__ row_of, const int32_t* __restrict__ pos,
-                                       const int32_t* __restrict__ val_soff, int64_t nnz,
-                                       unsigned long long* __restrict__ tile_rows) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    const int r = row_of[e];
-    const int w = r / kWinRows;
-    const int64_t tile = (int64_t)__ldg(val_soff + w) + pos[e] / kTileCols;
-    atomicAdd(tile_rows + tile, 1ull << (4 * (r - w * kWinRows)));
-}
-
-__device__ __forceinline__ int nibble_sum(unsigned long long x) {
-    // sum of sixteen 4-bit fields (each <= 8)
-    x = (x & 0x0f0f0f0f0f0f0f0full) + ((x >> 4) & 0x0f0f0f0f0f0f0f0full);
-    return (int)((x * 0x0101010101010101ull) >> 56);
-}
-
 struct TilePadIn {
     const unsigned long long* tile_rows;
     __device__ int32_t operator()(int64_t t) const { return (nibble_sum(tile_rows[t]) + 7) & ~7; }
 };
+// also the closing entry, behind the last tile
 struct CooOffOut {
     const unsigned long long* tile_rows;
     int32_t* off;
-    __device__ void operator()(int64_t t, int64_t before, int32_t) const {
+    int64_t T;
+    __device__ void operator()(int64_t t, int64_t before, int32_t v) const {
         off[2 * t] = (int32_t)before;
         off[2 * t + 1] = (int32_t)before + nibble_sum(tile_rows[t]);
+        if (t == T - 1) off[2 * T] = (int32_t)(before + v);
     }
 };
-
-__global__ void metcf_values_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ row_of,
-                                    const int32_t* __restrict__ pos, const float* __restrict__ values,
-                                    const int32_t* __restrict__ val_soff, const int32_t* __restrict__ coo_off,
-                                    const unsigned long long* __restrict__ tile_rows, int64_t nnz,
-                                    int32_t* __restrict__ coo_idx, float* __restrict__ coo_val) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    const int r = row_of[e], p = pos[e];
-    const int w = r / kWinRows, rr = r - w * kWinRows, b = p / kTileCols;
-    const int64_t tile = (int64_t)__ldg(val_soff + w) + b;
-    // entries of earlier rows in this tile, then earlier entries of this row in this tile
-    const unsigned long long below = rr == 0 ? 0ull : (tile_rows[tile] & ((1ull << (4 * rr)) - 1ull));
-    int slot = __ldg(coo_off + 2 * tile) + nibble_sum(below);
-    const int64_t rs = __ldg(rowptr + r);
-    for (int64_t j = e - 1; j >= rs && pos[j] / kTileCols == b; j--) slot++;
-    coo_idx[slot] = sw123(rr * kTileCols + p % kTileCols);
-    coo_val[slot] = values ? values[e] : 1.0f;
-}
-
-// MCO (bitmap leaf): bit Swizzle<1,2,3>(8r+c) of the tile's two 64-bit words marks a stored entry.
-__global__ void mco_mask_kernel(const int32_t* __restrict__ row_of, const int32_t* __restrict__ pos,
-                                const float* __restrict__ values, const int32_t* __restrict__ val_soff, int64_t nnz,
-                                int skip_zero_values, unsigned long long* __restrict__ masks) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    if (skip_zero_values && values && values[e] == 0.0f) return;
-    const int r = row_of[e], p = pos[e];
-    const int w = r / kWinRows;
-    const int64_t tile = (int64_t)__ldg(val_soff + w) + p / kTileCols;
-    const int phys = sw123((r - w * kWinRows) * kTileCols + p % kTileCols);
-    atomicOr(masks + 2 * tile + (phys >> 6), 1ull << (phys & 63));
-}
-
 struct McoCountIn {
     const unsigned long long* masks;
     __device__ int32_t operator()(int64_t t) const { return (__popcll(masks[2 * t]) + __popcll(masks[2 * t + 1]) + 3) & ~3; }
 };
 struct McoOffOut {
     int32_t* off;
-    __device__ void operator()(int64_t t, int64_t before, int32_t) const { off[t] = (int32_t)before; }
+    int64_t T;
+    __device__ void operator()(int64_t t, int64_t before, int32_t v) const {
+        off[t] = (int32_t)before;
+        if (t == T - 1) off[T] = (int32_t)(before + v);
+    }
 };
 
-// Values in ascending bit order: an entry's slot is the number of mask bits below its own.
-__global__ void mco_values_kernel(const int32_t* __restrict__ row_of, const int32_t* __restrict__ pos,
-                                  const float* __restrict__ values, const int32_t* __restrict__ val_soff,
-                                  const int32_t* __restrict__ mco_off, const unsigned long long* __restrict__ masks,
-                                  int64_t nnz, int skip_zero_values, float* __restrict__ mco_val) {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    if (skip_zero_values && values && values[e] == 0.0f) return;
-    const int r = row_of[e], p = pos[e];
-    const int w = r / kWinRows;
-    const int64_t tile = (int64_t)__ldg(val_soff + w) + p / kTileCols;
-    const int phys = sw123((r - w * kWinRows) * kTileCols + p % kTileCols);
-    const unsigned long long m0 = masks[2 * tile], m1 = masks[2 * tile + 1];
-    const int below = phys < 64 ? __popcll(m0 & ((1ull << phys) - 1ull)) : __popcll(m0) + __popcll(m1 & ((1ull << (phys - 64)) - 1ull));
-    mco_val[__ldg(mco_off + tile) + below] = values ? values[e] : 1.0f;
+static inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
+
+template <int MODE>
+static int launch_fill(const FillArgs& a, cudaStream_t st) {
+    fill_kernel<MODE><<<blocks_for(a.T, kFillTiles), 128, 0, st>>>(a);
+    MASK_CUDA_TRY(cudaGetLastError());
+    return MASK_OK;
 }
 
-static inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
+static FillArgs fill_args(const PackScratch& s, const float* d_values, const int32_t* d_val_soff, int64_t T) {
+    FillArgs a{};
+    a.rows = s.rows;
+    a.cols = s.cols;
+    a.distinct = s.distinct;
+    a.values = d_values;
+    a.pos = s.pos;
+    a.soff = d_val_soff;
+    a.first_window = s.first_window;
+    a.T = T;
+    return a;
+}
+
+// Copies n int32 words at d_src to the host and waits for them.
+static int read_words(const int32_t* d_src, int32_t* out, int n, cudaStream_t st) {
+    HostStage stage;
+    int rc = stage.get((size_t)n * 4);
+    if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(cudaMemcpyAsync(stage.as<int32_t>(), d_src, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
+    MASK_CUDA_TRY(cudaStreamSynchronize(st));
+    memcpy(out, stage.as<int32_t>(), (size_t)n * 4);
+    return MASK_OK;
+}
 
 }  // namespace mask
 
@@ -408,24 +799,35 @@ extern "C" int mask_pack_analyze(const int32_t* d_rowptr, const int32_t* d_colin
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int W = (M + kWinRows - 1) / kWinRows;
     MASK_CUDA_TRY(cudaMemsetAsync(s.status, 0, 64, st));
-    if (nnz > 0) {
-        row_of_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(d_rowptr, M, nnz, s.row_of);
+    // a key is the column and the entry's index within the window
+    if (K <= (1 << (32 - kSortIdxBits)))
+        condense_kernel<uint32_t><<<blocks_for(W, 4), 128, 0, st>>>(d_rowptr, d_colind, M, K, W, s.pos, s.cols, s.rows, s.distinct, s.big_list, s.hub_list, s.status);
+    else
+        condense_kernel<unsigned long long><<<blocks_for(W, 4), 128, 0, st>>>(d_rowptr, d_colind, M, K, W, s.pos, s.cols, s.rows, s.distinct, s.big_list, s.hub_list, s.status);
+    MASK_CUDA_TRY(cudaGetLastError());
+    if (nnz > kSortMax) {
+        constexpr int kSmem = kBigBits / 8 + kBigBits / 16;
+        MASK_CUDA_TRY(cudaFuncSetAttribute(condense_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        const int64_t most = std::min<int64_t>(W, nnz / kSortMax);
+        condense_big_kernel<<<(unsigned)std::min<int64_t>(most, 2 * sm_count()), kBigThreads, kSmem, st>>>(
+            d_rowptr, d_colind, M, K, s.pos, s.cols, s.distinct, s.big_list, s.status);
         MASK_CUDA_TRY(cudaGetLastError());
-        rank_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(d_rowptr, d_colind, M, K, nnz, s.row_of, s.pos, s.merged, s.status);
-        MASK_CUDA_TRY(cudaGetLastError());
-        int rc = device_scan(FlagIn{d_rowptr, s.row_of, s.merged}, InclusiveOut{s.dscan}, nnz, s.spine, nullptr, st);
-        if (rc != MASK_OK) return rc;
     }
-    int rc = device_scan(WindowTilesIn{d_rowptr, s.dscan, M, W}, ExclusiveOut{d_val_soff}, (int64_t)W + 1, s.spine,
+    if (nnz > kHubMin) {
+        const int span = (int)std::min<int64_t>(((int64_t)K + 4095) / 4096 * 4096, kHubBits);   // columns a block marks at a time
+        const int smem = span / 8 + span / 16;
+        MASK_CUDA_TRY(cudaFuncSetAttribute(condense_hub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHubBits / 8 + kHubBits / 16));
+        const int64_t most = std::min<int64_t>(W, nnz / kHubMin);
+        condense_hub_kernel<<<(unsigned)(kHubBlocks * std::min<int64_t>(most, std::max(1, sm_count() / kHubBlocks))), kHubThreads, smem, st>>>(
+            d_rowptr, d_colind, M, K, span, s.pos, s.cols, s.distinct, s.hub_list, s.status);
+        MASK_CUDA_TRY(cudaGetLastError());
+    }
+    int rc = device_scan(WindowTilesIn{s.distinct, W}, SoffOut{d_val_soff, s.first_window}, (int64_t)W + 1, s.spine,
                          reinterpret_cast<int64_t*>(s.status + 2), st);
     if (rc != MASK_OK) return rc;
-    if (nnz > 0) {
-        condensed_pos_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(d_rowptr, s.row_of, s.dscan, nnz, s.pos);
-        MASK_CUDA_TRY(cudaGetLastError());
-    }
     int32_t host_status[4] = {0, 0, 0, 0};
-    MASK_CUDA_TRY(cudaMemcpyAsync(host_status, s.status, 16, cudaMemcpyDeviceToHost, st));
-    MASK_CUDA_TRY(cudaStreamSynchronize(st));
+    rc = read_words(s.status, host_status, 4, st);
+    if (rc != MASK_OK) return rc;
     if (host_status[0] & 2) return fail(MASK_ERR_COLUMN_RANGE, "a column id is outside [0, K)");
     if (host_status[0] & 1) return fail(MASK_ERR_UNSORTED_ROWS, "CSR rows must hold strictly ascending column ids");
     int64_t T;
@@ -448,13 +850,14 @@ extern "C" int mask_srbcrs_fill(const int32_t* d_rowptr, const int32_t* d_colind
     PackScratch s = carve(const_cast<void*>(d_scratch), M, nnz);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int W = (M + kWinRows - 1) / kWinRows;
-    if (T > 0) MASK_CUDA_TRY(cudaMemsetAsync(d_val_block_val, 0, (size_t)T * kTileElems * sizeof(float), st));
-    if (nnz > 0) {
-        sidx_kernel<true><<<blocks_for(nnz, 256), 256, 0, st>>>(d_rowptr, s.row_of, s.merged, s.dscan, d_val_soff, M, nnz, d_val_sidx);
-        MASK_CUDA_TRY(cudaGetLastError());
-        srbcrs_values_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(s.row_of, s.pos, d_values, d_val_soff, nnz,
-                                                                   d_val_block_val, d_edge_to_col, d_edge_to_row);
-        MASK_CUDA_TRY(cudaGetLastError());
+    if (T > 0) {
+        FillArgs a = fill_args(s, d_values, d_val_soff, T);
+        a.sidx = d_val_sidx;
+        a.block_val = d_val_block_val;
+        a.edge_to_col = d_edge_to_col;
+        a.edge_to_row = d_edge_to_row;
+        int rc = launch_fill<kFillSrbcrs>(a, st);
+        if (rc != MASK_OK) return rc;
     }
     if (d_block_partition) {
         block_partition_kernel<<<blocks_for(W, 256), 256, 0, st>>>(d_val_soff, W, d_block_partition);
@@ -474,22 +877,22 @@ extern "C" int mask_metcf_offsets(const int32_t* d_rowptr, int32_t M, int64_t nn
     PackScratch s = carve(const_cast<void*>(d_scratch), M, nnz);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto* rows = reinterpret_cast<unsigned long long*>(d_tile_rows);
-    if (T > 0) MASK_CUDA_TRY(cudaMemsetAsync(rows, 0, (size_t)T * 8, st));
-    if (nnz > 0) {
-        metcf_histogram_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(s.row_of, s.pos, d_val_soff, nnz, rows);
-        MASK_CUDA_TRY(cudaGetLastError());
+    *h_nnz_pad = 0;
+    if (T == 0) {
+        MASK_CUDA_TRY(cudaMemsetAsync(d_val_coo_off, 0, 4, st));
+        return MASK_OK;
     }
+    FillArgs a = fill_args(s, nullptr, d_val_soff, T);
+    a.tile_rows = rows;
+    int rc = launch_fill<kCountMetcf>(a, st);
+    if (rc != MASK_OK) return rc;
     // the spine is sized for max(nnz, W+1) items and T <= nnz
-    int rc = device_scan(TilePadIn{rows}, CooOffOut{rows, d_val_coo_off}, T, s.spine,
-                         reinterpret_cast<int64_t*>(s.status + 2), st);
+    rc = device_scan(TilePadIn{rows}, CooOffOut{rows, d_val_coo_off, T}, T, s.spine, reinterpret_cast<int64_t*>(s.status + 2), st);
     if (rc != MASK_OK) return rc;
     int64_t total = 0;
-    MASK_CUDA_TRY(cudaMemcpyAsync(&total, s.status + 2, 8, cudaMemcpyDeviceToHost, st));
-    MASK_CUDA_TRY(cudaStreamSynchronize(st));
+    rc = read_words(s.status + 2, reinterpret_cast<int32_t*>(&total), 2, st);
+    if (rc != MASK_OK) return rc;
     if (total >= (int64_t)1 << 31) return fail(MASK_ERR_INDEX_OVERFLOW, "nnz_pad does not fit int32");
-    const int32_t closing = (int32_t)total;
-    MASK_CUDA_TRY(cudaMemcpyAsync(d_val_coo_off + 2 * T, &closing, 4, cudaMemcpyHostToDevice, st));
-    MASK_CUDA_TRY(cudaStreamSynchronize(st));
     *h_nnz_pad = total;
     return MASK_OK;
 }
@@ -506,20 +909,14 @@ extern "C" int mask_metcf_fill(const int32_t* d_rowptr, const int32_t* d_colind,
     MASK_REQUIRE(nnz_pad == 0 || (d_val_coo_idx && d_val_coo_val), "output arrays are NULL");
     PackScratch s = carve(const_cast<void*>(d_scratch), M, nnz);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (T > 0) MASK_CUDA_TRY(cudaMemsetAsync(d_val_sidx, 0, (size_t)T * kTileCols * 4, st));
-    if (nnz_pad > 0) {
-        MASK_CUDA_TRY(cudaMemsetAsync(d_val_coo_idx, 0, (size_t)nnz_pad * 4, st));
-        MASK_CUDA_TRY(cudaMemsetAsync(d_val_coo_val, 0, (size_t)nnz_pad * 4, st));
-    }
-    if (nnz > 0) {
-        sidx_kernel<false><<<blocks_for(nnz, 256), 256, 0, st>>>(d_rowptr, s.row_of, s.merged, s.dscan, d_val_soff, M, nnz, d_val_sidx);
-        MASK_CUDA_TRY(cudaGetLastError());
-        metcf_values_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(d_rowptr, s.row_of, s.pos, d_values, d_val_soff, d_val_coo_off,
-                                                                  reinterpret_cast<const unsigned long long*>(d_tile_rows),
-                                                                  nnz, d_val_coo_idx, d_val_coo_val);
-        MASK_CUDA_TRY(cudaGetLastError());
-    }
-    return MASK_OK;
+    if (T == 0) return MASK_OK;
+    FillArgs a = fill_args(s, d_values, d_val_soff, T);
+    a.sidx = d_val_sidx;
+    a.tile_rows = const_cast<unsigned long long*>(reinterpret_cast<const unsigned long long*>(d_tile_rows));
+    a.off = d_val_coo_off;
+    a.coo_idx = d_val_coo_idx;
+    a.out_val = d_val_coo_val;
+    return launch_fill<kFillMetcf>(a, st);
 }
 
 extern "C" int mask_mco_offsets(const float* d_values, int32_t M, int64_t nnz, const void* d_scratch, const int32_t* d_val_soff,
@@ -532,20 +929,22 @@ extern "C" int mask_mco_offsets(const float* d_values, int32_t M, int64_t nnz, c
     PackScratch s = carve(const_cast<void*>(d_scratch), M, nnz);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     auto* masks = reinterpret_cast<unsigned long long*>(d_val_mco_mask);
-    if (T > 0) MASK_CUDA_TRY(cudaMemsetAsync(masks, 0, (size_t)T * 16, st));
-    if (nnz > 0) {
-        mco_mask_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(s.row_of, s.pos, d_values, d_val_soff, nnz, skip_zero_values, masks);
-        MASK_CUDA_TRY(cudaGetLastError());
+    *h_nval = 0;
+    if (T == 0) {
+        MASK_CUDA_TRY(cudaMemsetAsync(d_val_mco_off, 0, 4, st));
+        return MASK_OK;
     }
-    int rc = device_scan(McoCountIn{masks}, McoOffOut{d_val_mco_off}, T, s.spine, reinterpret_cast<int64_t*>(s.status + 2), st);
+    FillArgs a = fill_args(s, d_values, d_val_soff, T);
+    a.skip_zero = skip_zero_values;
+    a.masks = masks;
+    int rc = launch_fill<kMaskMco>(a, st);
+    if (rc != MASK_OK) return rc;
+    rc = device_scan(McoCountIn{masks}, McoOffOut{d_val_mco_off, T}, T, s.spine, reinterpret_cast<int64_t*>(s.status + 2), st);
     if (rc != MASK_OK) return rc;
     int64_t total = 0;
-    MASK_CUDA_TRY(cudaMemcpyAsync(&total, s.status + 2, 8, cudaMemcpyDeviceToHost, st));
-    MASK_CUDA_TRY(cudaStreamSynchronize(st));
+    rc = read_words(s.status + 2, reinterpret_cast<int32_t*>(&total), 2, st);
+    if (rc != MASK_OK) return rc;
     if (total >= (int64_t)1 << 31) return fail(MASK_ERR_INDEX_OVERFLOW, "value count does not fit int32");
-    const int32_t closing = (int32_t)total;
-    MASK_CUDA_TRY(cudaMemcpyAsync(d_val_mco_off + T, &closing, 4, cudaMemcpyHostToDevice, st));
-    MASK_CUDA_TRY(cudaStreamSynchronize(st));
     *h_nval = total;
     return MASK_OK;
 }
@@ -561,14 +960,12 @@ extern "C" int mask_mco_fill(const int32_t* d_rowptr, const float* d_values, int
     MASK_REQUIRE(nval == 0 || d_val_mco_val, "val_mco_val is NULL");
     PackScratch s = carve(const_cast<void*>(d_scratch), M, nnz);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (nval > 0) MASK_CUDA_TRY(cudaMemsetAsync(d_val_mco_val, 0, (size_t)nval * 4, st));
-    if (nnz > 0) {
-        sidx_kernel<true><<<blocks_for(nnz, 256), 256, 0, st>>>(d_rowptr, s.row_of, s.merged, s.dscan, d_val_soff, M, nnz, d_val_sidx);
-        MASK_CUDA_TRY(cudaGetLastError());
-        mco_values_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(s.row_of, s.pos, d_values, d_val_soff, d_val_mco_off,
-                                                                reinterpret_cast<const unsigned long long*>(d_val_mco_mask), nnz,
-                                                                skip_zero_values, d_val_mco_val);
-        MASK_CUDA_TRY(cudaGetLastError());
-    }
-    return MASK_OK;
+    if (T == 0) return MASK_OK;
+    FillArgs a = fill_args(s, d_values, d_val_soff, T);
+    a.skip_zero = skip_zero_values;
+    a.masks = const_cast<unsigned long long*>(reinterpret_cast<const unsigned long long*>(d_val_mco_mask));
+    a.off = d_val_mco_off;
+    a.sidx = d_val_sidx;
+    a.out_val = d_val_mco_val;
+    return launch_fill<kFillMco>(a, st);
 }
