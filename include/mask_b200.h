@@ -270,6 +270,10 @@ int mask_peer_free(void* d_ptr);
  * 414-528).  Without this call a plan uses the widest block N fills.  Synchronises the stream.
  * mask_plan_column_features returns what was measured and chosen. */
 int mask_plan_autotune(mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t K, void* stream);
+/* mask_plan_create and mask_plan_autotune in one call: the device measures the columns while the host
+ * builds the tables, and the stream is synchronised once less. */
+int mask_plan_create_tuned(const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t M, int32_t K, int64_t T,
+                           int policy, int32_t group_tiles, void* stream, mask_plan** out);
 int mask_plan_column_features(const mask_plan* plan, mask_column_features* out, int32_t* nslab_wide);
 /* Prepares the plan for the TMA-fed SpMM kernel: keeps a copy of val_block_val (128 T floats, owned
  * by the plan) with every value rounded to TF32 -- nearest, ties away, the reference kernels'

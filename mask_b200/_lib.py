@@ -42,6 +42,7 @@ SIGNATURES = {
     "mask_plan_strict_lb": (C.c_int, [vp, i32, i32, vp, vp, vp, C.POINTER(i64), C.POINTER(i64)]),
     "mask_plan_multi_bind": (C.c_int, [vp, i32, vp, vp, vp, C.POINTER(i64)]),
     "mask_plan_create": (C.c_int, [vp, i32, i64, C.c_int, i32, vp, C.POINTER(vp)]),
+    "mask_plan_create_tuned": (C.c_int, [vp, vp, i32, i32, i64, C.c_int, i32, vp, C.POINTER(vp)]),
     "mask_plan_destroy": (None, [vp]),
     "mask_plan_scratch_bytes": (sz, [vp, i32]),
     "mask_plan_info": (C.c_int, [vp, C.POINTER(i64), C.POINTER(i64), C.POINTER(i64), C.POINTER(i32)]),

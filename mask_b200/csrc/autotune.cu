@@ -15,69 +15,168 @@
 //     that fraction is what L2 can serve; where a narrower row raises it markedly, sweeping the matrix
 //     once per 256 columns instead of once per 512 saves more DRAM traffic (rows of B) than it costs
 //     (tile values and ids read twice).
-#include <cub/cub.cuh>
-
 #include <algorithm>
+#include <functional>
+#include <vector>
 
 #include "common.cuh"
-#include "plan.h"
+#include "column_stats.h"
 
 namespace mask {
 
 namespace {
 
-struct Scratch {
-    void* p = nullptr;
-    ~Scratch() { if (p) cudaFree(p); }
-    int alloc(size_t bytes) {
-        MASK_CUDA_TRY(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
-        return MASK_OK;
-    }
-    template <typename T> T* as() const { return static_cast<T*>(p); }
+constexpr int kBandBuckets = 33;   // bucket b: distances in [2^(b-1), 2^b), bucket 0: distance 0
+constexpr int kCountBins = 8192;   // columns gathered fewer times than this are counted by that number, the others listed
+
+struct StatsHead {                 // what goes back to the host in one copy, followed by the list
+    unsigned long long band[kBandBuckets + 1];   // last entry: gathers within local_rows of the diagonal
+    uint32_t bins[kCountBins];     // columns by number of gathers
+    uint32_t listed;
+    uint32_t pad[3];
 };
 
-constexpr int kBandBuckets = 33;   // bucket b: distances in [2^(b-1), 2^b), bucket 0: distance 0
-
-// one thread per tile: window by binary search in val_soff, then its 8 ids
-__global__ void column_stats_kernel(const int32_t* __restrict__ soff, const int32_t* __restrict__ sidx, int32_t W, int64_t T,
-                                    int32_t M, int32_t K, int64_t local_rows, uint32_t* __restrict__ counts,
-                                    unsigned long long* __restrict__ band_hist) {
-    __shared__ unsigned int hist[kBandBuckets + 1];   // last entry: gathers within local_rows of the diagonal
+// One thread per tile: its window, then its 8 ids.  A block's 256 tiles lie in few windows, so the search runs
+// between the windows of its first and last tile.  Ids of a warp fall into the same few distance buckets: the lanes
+// that share the first one's are counted together.
+__global__ void __launch_bounds__(256) column_stats_kernel(const int32_t* __restrict__ soff, const int32_t* __restrict__ sidx, int32_t W,
+                                                           int64_t T, int32_t M, int32_t K, int64_t local_rows,
+                                                           uint32_t* __restrict__ counts, StatsHead* __restrict__ head) {
+    __shared__ unsigned int hist[kBandBuckets + 1];
+    __shared__ int range[2];
+    const int lane = threadIdx.x & 31;
     if (threadIdx.x <= kBandBuckets) hist[threadIdx.x] = 0;
+    const int64_t t0 = (int64_t)blockIdx.x * 256, t = t0 + threadIdx.x;
+    if (threadIdx.x < 2) {
+        const int64_t key = threadIdx.x == 0 ? t0 : (t0 + 255 < T ? t0 + 255 : T - 1);
+        int lo = 0, hi = W;   // last window whose first tile is <= key
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if ((int64_t)soff[mid] <= key) lo = mid; else hi = mid;
+        }
+        range[threadIdx.x] = lo;
+    }
     __syncthreads();
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < T) {
-        int lo = 0, hi = W;   // last window whose first tile is <= t
+    int lo = range[0], hi = range[1] + 1;
+    int64_t diag = 0;
+    const bool live = t < T;
+    if (live) {
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if ((int64_t)soff[mid] <= t) lo = mid; else hi = mid;
         }
-        const int64_t diag = (int64_t)lo * kWinRows * K / M;
-        for (int j = 0; j < kTileCols; j++) {
-            const int id = sidx[t * kTileCols + j];
-            if (id < 0 || id >= K) continue;
-            atomicAdd(&counts[id], 1u);
-            const int64_t d = id > diag ? id - diag : diag - id;
-            atomicAdd(&hist[d == 0 ? 0 : 64 - __clzll((unsigned long long)d)], 1u);
-            if (d <= local_rows) atomicAdd(&hist[kBandBuckets], 1u);
-        }
+        diag = (int64_t)lo * kWinRows * K / M;
+    }
+    int local = 0;
+#pragma unroll
+    for (int j = 0; j < kTileCols; j++) {
+        const int id = live ? __ldg(sidx + t * kTileCols + j) : -1;
+        const bool ok = id >= 0 && id < K;
+        if (ok) atomicAdd(&counts[id], 1u);
+        const int64_t d = id > diag ? id - diag : diag - id;
+        const int bucket = !ok ? -1 : (d == 0 ? 0 : 64 - __clzll((unsigned long long)d));
+        const int lead = __shfl_sync(0xffffffffu, bucket, 0);
+        const unsigned same = __ballot_sync(0xffffffffu, bucket == lead);
+        if (lane == 0) { if (ok) atomicAdd(&hist[bucket], (unsigned)__popc(same)); }
+        else if (ok && bucket != lead) atomicAdd(&hist[bucket], 1u);
+        local += ok && d <= local_rows;
+    }
+    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
+    if (lane == 0 && local) atomicAdd(&hist[kBandBuckets], (unsigned)local);
+    __syncthreads();
+    if (threadIdx.x <= kBandBuckets && hist[threadIdx.x]) atomicAdd(&head->band[threadIdx.x], (unsigned long long)hist[threadIdx.x]);
+}
+
+// columns by number of gathers; those with kCountBins and more, one by one
+__global__ void __launch_bounds__(512) count_bins_kernel(const uint32_t* __restrict__ counts, int32_t K, StatsHead* __restrict__ head,
+                                                         uint32_t* __restrict__ list) {
+    __shared__ uint32_t bins[kCountBins];
+    for (int i = threadIdx.x; i < kCountBins; i += 512) bins[i] = 0;
+    __syncthreads();
+    for (int i = blockIdx.x * 512 + threadIdx.x; i < K; i += gridDim.x * 512) {
+        const uint32_t c = counts[i];
+        if (c < (uint32_t)kCountBins) atomicAdd(&bins[c], 1u);
+        else list[atomicAdd(&head->listed, 1u)] = c;
     }
     __syncthreads();
-    if (threadIdx.x <= kBandBuckets && hist[threadIdx.x]) atomicAdd(&band_hist[threadIdx.x], (unsigned long long)hist[threadIdx.x]);
+    for (int i = threadIdx.x; i < kCountBins; i += 512)
+        if (bins[i]) atomicAdd(&head->bins[i], bins[i]);
 }
-
-__global__ void count_nonzero_kernel(const uint32_t* __restrict__ counts, int32_t K, int32_t* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool nz = i < K && counts[i] != 0;
-    const unsigned b = __ballot_sync(0xffffffffu, nz);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(out, __popc(b));
-}
-
-struct ToU64 {
-    __host__ __device__ unsigned long long operator()(uint32_t v) const { return v; }
-};
 
 }  // namespace
+
+int ColumnStatsJob::enqueue(const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t M, int32_t K, int64_t T, int32_t N, cudaStream_t st) {
+    int dev = 0;
+    MASK_CUDA_TRY(cudaGetDevice(&dev));
+    MASK_CUDA_TRY(cudaDeviceGetAttribute(&l2_, cudaDevAttrL2CacheSize, dev));
+    K_ = K;
+    N_ = N;
+    T_ = T;
+    if (T == 0) return MASK_OK;
+    const int32_t W = (M + kWinRows - 1) / kWinRows;
+    // one allocation: what goes back to the host (with room for every column that can be listed), then counts
+    const int64_t most_listed = std::min<int64_t>(K, T * kTileCols / kCountBins) + 1;
+    const size_t counts_at = (sizeof(StatsHead) + (size_t)most_listed * 4 + 15) & ~(size_t)15;
+    const size_t bytes = counts_at + (size_t)K * 4;
+    int rc = buf_.alloc(bytes, st);
+    if (rc == MASK_OK) rc = host_.get(counts_at);
+    if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(cudaMemsetAsync(buf_.p, 0, bytes, st));
+    // "local": a band of windows keeps rows of B alive that take at most half the L2 at this row width
+    const int width0 = std::min(N, 512);
+    local_rows_ = (int32_t)std::min<int64_t>(K, std::max<int64_t>(0, ((int64_t)(l2_ / 2) / ((int64_t)width0 * 4) - kWinRows) / 2));
+    uint32_t* counts = buf_.as<uint32_t>(counts_at);
+    column_stats_kernel<<<(unsigned)((T + 255) / 256), 256, 0, st>>>(d_val_soff, d_val_sidx, W, T, M, K, (int64_t)local_rows_, counts,
+                                                                    buf_.as<StatsHead>());
+    MASK_CUDA_TRY(cudaGetLastError());
+    const unsigned bin_blocks = (unsigned)std::min<int64_t>(((int64_t)K + 4095) / 4096, sm_count());
+    count_bins_kernel<<<bin_blocks, 512, 0, st>>>(counts, K, buf_.as<StatsHead>(), buf_.as<uint32_t>(sizeof(StatsHead)));
+    MASK_CUDA_TRY(cudaGetLastError());
+    MASK_CUDA_TRY(cudaMemcpyAsync(host_.as<void>(), buf_.p, counts_at, cudaMemcpyDeviceToHost, st));
+    return MASK_OK;
+}
+
+void ColumnStatsJob::finish(mask_column_features* out) const {
+    *out = mask_column_features{};
+    out->l2_bytes = l2_;
+    out->gathers = T_ * kTileCols;
+    if (T_ == 0) return;
+    out->local_rows = local_rows_;
+    const StatsHead& head = *host_.as<StatsHead>();
+    const unsigned long long* h = head.band;
+    const uint32_t* list = reinterpret_cast<const uint32_t*>(&head + 1);
+    out->distinct_columns = (int32_t)(K_ - (int64_t)head.bins[0]);
+    // gathers that go to the most gathered columns: the listed ones first, then bin by bin
+    std::vector<uint32_t> top(list, list + head.listed);
+    std::sort(top.begin(), top.end(), std::greater<uint32_t>());
+    unsigned long long reach[3] = {0, 0, 0};
+    for (int i = 0; i < 3; i++) {
+        const int width = std::min(N_, 512 >> i);                               // columns of one gathered row at 4, 2, 1 slabs
+        const int64_t rows = std::max<int64_t>(1, (int64_t)(l2_ / 2) / ((int64_t)width * 4));
+        out->hub_columns[i] = (int32_t)std::min<int64_t>(rows, K_);
+        int64_t left = out->hub_columns[i];
+        for (size_t j = 0; j < top.size() && left > 0; j++, left--) reach[i] += top[j];
+        for (int b = kCountBins - 1; b > 0 && left > 0; b--) {
+            const int64_t take = std::min<int64_t>(left, head.bins[b]);
+            reach[i] += (unsigned long long)take * (unsigned)b;
+            left -= take;
+        }
+    }
+    unsigned long long total = 0;
+    for (int b = 0; b < kBandBuckets; b++) total += h[b];
+    for (int i = 0; i < 3; i++) out->hub_share[i] = total ? (double)reach[i] / (double)total : 0.0;
+    out->local_share = total ? (double)h[kBandBuckets] / (double)total : 1.0;
+    auto percentile = [&](double q) -> int32_t {
+        unsigned long long run = 0;
+        for (int b = 0; b < kBandBuckets; b++) {
+            run += h[b];
+            if ((double)run >= q * (double)total) return b == 0 ? 0 : (int32_t)std::min<int64_t>((int64_t)1 << b, (int64_t)K_);
+        }
+        return K_;
+    };
+    out->band_p50 = percentile(0.50);
+    out->band_p90 = percentile(0.90);
+}
 
 }  // namespace mask
 
@@ -87,67 +186,16 @@ extern "C" int mask_features_columns(const int32_t* d_val_soff, const int32_t* d
     MASK_REQUIRE(out != nullptr && d_val_soff != nullptr && M >= 1 && K >= 1 && T >= 0 && N >= 1, "bad arguments");
     MASK_REQUIRE(T == 0 || d_val_sidx != nullptr, "val_sidx is NULL");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    *out = mask_column_features{};
-    int dev = 0, l2 = 0;
-    MASK_CUDA_TRY(cudaGetDevice(&dev));
-    MASK_CUDA_TRY(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev));
-    out->l2_bytes = l2;
-    out->gathers = T * kTileCols;
-    if (T == 0) return MASK_OK;
-    const int32_t W = (M + kWinRows - 1) / kWinRows;
-    Scratch counts, sorted, prefix, hist, nz, tmp;
-    int rc = counts.alloc((size_t)K * 4);
-    if (rc == MASK_OK) rc = sorted.alloc((size_t)K * 4);
-    if (rc == MASK_OK) rc = prefix.alloc((size_t)K * 8);
-    if (rc == MASK_OK) rc = hist.alloc((kBandBuckets + 1) * 8);
-    if (rc == MASK_OK) rc = nz.alloc(16);
+    ColumnStatsJob job;
+    int rc = job.enqueue(d_val_soff, d_val_sidx, M, K, T, N, st);
+    const cudaError_t e = cudaStreamSynchronize(st);   // also after a failure: the copy may be in flight
     if (rc != MASK_OK) return rc;
-    MASK_CUDA_TRY(cudaMemsetAsync(counts.p, 0, (size_t)K * 4, st));
-    MASK_CUDA_TRY(cudaMemsetAsync(hist.p, 0, (kBandBuckets + 1) * 8, st));
-    MASK_CUDA_TRY(cudaMemsetAsync(nz.p, 0, 16, st));
-    // "local": a band of windows keeps rows of B alive that take at most half the L2 at this row width
-    const int width0 = std::min(N, 512);
-    out->local_rows = (int32_t)std::min<int64_t>(K, std::max<int64_t>(0, ((int64_t)(l2 / 2) / ((int64_t)width0 * 4) - kWinRows) / 2));
-    column_stats_kernel<<<(unsigned)((T + 255) / 256), 256, 0, st>>>(d_val_soff, d_val_sidx, W, T, M, K, (int64_t)out->local_rows,
-                                                                    counts.as<uint32_t>(), hist.as<unsigned long long>());
-    count_nonzero_kernel<<<(unsigned)((K + 255) / 256), 256, 0, st>>>(counts.as<uint32_t>(), K, nz.as<int32_t>());
-    MASK_CUDA_TRY(cudaGetLastError());
-    // gathers per column, most gathered first, and their running sum
-    size_t b1 = 0, b2 = 0;
-    cub::TransformInputIterator<unsigned long long, ToU64, const uint32_t*> as64(sorted.as<uint32_t>(), ToU64());
-    MASK_CUDA_TRY(cub::DeviceRadixSort::SortKeysDescending(nullptr, b1, counts.as<uint32_t>(), sorted.as<uint32_t>(), K, 0, 32, st));
-    MASK_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, b2, as64, prefix.as<unsigned long long>(), K, st));
-    rc = tmp.alloc(std::max(b1, b2));
-    if (rc != MASK_OK) return rc;
-    MASK_CUDA_TRY(cub::DeviceRadixSort::SortKeysDescending(tmp.p, b1, counts.as<uint32_t>(), sorted.as<uint32_t>(), K, 0, 32, st));
-    MASK_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp.p, b2, as64, prefix.as<unsigned long long>(), K, st));
-    unsigned long long h[kBandBuckets + 1];
-    MASK_CUDA_TRY(cudaMemcpyAsync(h, hist.p, sizeof(h), cudaMemcpyDeviceToHost, st));
-    MASK_CUDA_TRY(cudaMemcpyAsync(&out->distinct_columns, nz.p, 4, cudaMemcpyDeviceToHost, st));
-    unsigned long long reach[3] = {0, 0, 0};
-    for (int i = 0; i < 3; i++) {
-        const int width = std::min(N, 512 >> i);                               // columns of one gathered row at 4, 2, 1 slabs
-        const int64_t rows = std::max<int64_t>(1, (int64_t)(l2 / 2) / ((int64_t)width * 4));
-        out->hub_columns[i] = (int32_t)std::min<int64_t>(rows, K);
-        MASK_CUDA_TRY(cudaMemcpyAsync(&reach[i], prefix.as<unsigned long long>() + (out->hub_columns[i] - 1), 8, cudaMemcpyDeviceToHost, st));
-    }
-    MASK_CUDA_TRY(cudaStreamSynchronize(st));
-    unsigned long long total = 0;
-    for (int b = 0; b < kBandBuckets; b++) total += h[b];
-    for (int i = 0; i < 3; i++) out->hub_share[i] = total ? (double)reach[i] / (double)total : 0.0;
-    out->local_share = total ? (double)h[kBandBuckets] / (double)total : 1.0;
-    auto percentile = [&](double q) -> int32_t {
-        unsigned long long run = 0;
-        for (int b = 0; b < kBandBuckets; b++) {
-            run += h[b];
-            if ((double)run >= q * (double)total) return b == 0 ? 0 : (int32_t)std::min<int64_t>((int64_t)1 << b, (int64_t)K);
-        }
-        return K;
-    };
-    out->band_p50 = percentile(0.50);
-    out->band_p90 = percentile(0.90);
+    MASK_CUDA_TRY(e);
+    job.finish(out);
     return MASK_OK;
 }
+
+namespace mask {
 
 // The plan table.  Keyed on: does the matrix keep its gathers local (band), and if not, how much more
 // of them L2 can serve when a gathered row is half as wide (hub shares).  Chooses the number of
@@ -155,12 +203,7 @@ extern "C" int mask_features_columns(const int32_t* d_val_soff, const int32_t* d
 // products have one slab.  Thresholds fitted on the five benchmark configurations (27-point stencil
 // and uniform-random: 4 slabs; power-law graphs with 2^21 and 2^22 nodes: 2 slabs, 3-5 % faster than
 // 4; 2^20 nodes: a tie).
-extern "C" int mask_plan_autotune(mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t K, void* stream) {
-    using namespace mask;
-    MASK_REQUIRE(plan != nullptr, "plan is NULL");
-    mask_column_features f;
-    int rc = mask_features_columns(d_val_soff, d_val_sidx, plan->M, K, plan->T, 512, &f, stream);
-    if (rc != MASK_OK) return rc;
+void choose_plan_parameters(mask_plan* plan, const mask_column_features& f) {
     plan->col_features = f;
     plan->has_col_features = 1;
     const double half_l2 = 0.5 * (double)f.l2_bytes;
@@ -169,6 +212,17 @@ extern "C" int mask_plan_autotune(mask_plan* plan, const int32_t* d_val_soff, co
     // hub-heavy (a quarter of the gathers already fit at full width) and markedly more fits at half width
     const bool narrower_rows_pay = !local && b_bytes > 8.0 * half_l2 && f.hub_share[0] >= 0.25 && f.hub_share[1] - f.hub_share[0] >= 0.02;
     plan->nslab = narrower_rows_pay ? 2 : 4;
+}
+
+}  // namespace mask
+
+extern "C" int mask_plan_autotune(mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t K, void* stream) {
+    using namespace mask;
+    MASK_REQUIRE(plan != nullptr, "plan is NULL");
+    mask_column_features f;
+    int rc = mask_features_columns(d_val_soff, d_val_sidx, plan->M, K, plan->T, 512, &f, stream);
+    if (rc != MASK_OK) return rc;
+    choose_plan_parameters(plan, f);
     return MASK_OK;
 }
 

@@ -6,6 +6,7 @@
 #include <cstring>
 
 #include "common.cuh"
+#include "column_stats.h"
 
 namespace mask {
 
@@ -59,6 +60,20 @@ static void multi_bind(const int32_t* soff, int32_t W, std::vector<int32_t>& tas
             task_soff.push_back(task_soff.back() + base + (i < rem ? 1 : 0));
         }
     }
+}
+
+// Tiles in one piece of a split window, and in one group of the warp-level kernel, when nobody asked for a
+// size.  That kernel has 15 one-warp blocks per SM, each of which takes about half a microsecond per tile:
+// with fewer than 128 tiles for every resident warp the pieces get shorter, so that all of them have work and
+// no long chain of tiles is left at the end.  Not below kMinPiece, where filling a block's pipeline costs more
+// than the balance gains, and not below the mean window: cutting every window adds a partial tile and a fix-up
+// for each (uniform 4096-node matrix, 42 tiles a window, N = 512: 23 us whole, 29 us in three pieces).
+constexpr int32_t kMinPiece = 16;
+constexpr int32_t kWarpBlocksPerSm = 15;
+static int32_t default_piece_tiles(int64_t T, int32_t W) {
+    const int64_t resident = (int64_t)sm_count() * kWarpBlocksPerSm;
+    const int64_t piece = std::max<int64_t>((T + resident - 1) / resident, (T + W - 1) / W);
+    return (int32_t)std::max<int64_t>(kMinPiece, std::min<int64_t>(128, piece));
 }
 
 static int32_t default_group_tiles(int64_t T) {
@@ -117,68 +132,125 @@ static void build_tables(mask_plan& p, const int32_t* soff) {
         }
         if (go.back() != (int32_t)fw.size()) go.push_back((int32_t)fw.size());
     } else {
-        // Groups are closed on window boundaries once their cost (tiles plus a fixed share per window
-        // for the rows of C it writes) reaches G; a window of more than 5/4 G tiles is cut into
-        // near-equal pieces of at most G tiles, one group each (each piece costs one partial tile in
-        // scratch and the fix-up pass sums them in tile order).
+        // Groups are closed on fragment boundaries once their cost (tiles plus a fixed share per fragment
+        // for the rows of C it writes) reaches G; a window of more than 5/4 of a piece is cut into near-equal
+        // pieces (each piece costs one partial tile in scratch and the fix-up pass sums them in tile order).
         constexpr int32_t kWindowCost = 4;
-        const int32_t split_above = G + G / 4;
-        int32_t load = 0;
+        const int32_t piece = p.piece_tiles;
+        const int32_t split_above = piece + piece / 4;
+        const size_t most = (size_t)W + (size_t)(p.T / std::max(piece, 1)) + 1;   // fragments
+        fo.resize(most + 1);
+        fw.resize(most);
+        go.resize(most + 1);
+        int32_t *fo_at = fo.data(), *fw_at = fw.data(), *go_at = go.data() + 1;
+        int32_t load = 0, n_frag = 0, closed = 0;
+        auto add = [&](int32_t tile, int32_t w) { *fo_at++ = tile; *fw_at++ = w; n_frag++; };
         auto close = [&]() {
-            if (go.back() != (int32_t)fw.size()) go.push_back((int32_t)fw.size());
+            if (closed != n_frag) *go_at++ = closed = n_frag;
             load = 0;
         };
         for (int32_t w = 0; w < W; w++) {
             const int32_t s = soff[w], x = soff[w + 1] - s;
             if (p.policy == MASK_POLICY_ROW) {
-                fo.push_back(s); fw.push_back(w); close();
+                add(s, w); close();
                 continue;
             }
-            if (x > split_above) {  // split into near-equal parts, one group each
-                close();
-                const int32_t parts = (x + G - 1) / G, base = x / parts, rem = x % parts;
+            if (x > split_above) {
+                const int32_t parts = (x + piece - 1) / piece, base = x / parts, rem = x % parts;
                 int32_t at = s;
+                if (piece >= G) close();
                 for (int32_t i = 0; i < parts; i++) {
-                    fo.push_back(at); fw.push_back(w); close();
+                    add(at, w);
                     at += base + (i < rem ? 1 : 0);
+                    load += base + kWindowCost;
+                    if (load >= G || piece >= G) close();
                 }
                 continue;
             }
             if (load > 0 && load + x + kWindowCost > G + G / 8) close();
-            fo.push_back(s); fw.push_back(w);
+            add(s, w);
             load += x + kWindowCost;
             if (load >= G) close();
         }
         close();
+        fo.resize(n_frag);
+        fw.resize(n_frag);
+        go.resize(go_at - go.data());
     }
     fo.push_back(soff[W]);
 
     p.F = (int64_t)fw.size();
     p.G = (int64_t)go.size() - 1;
-    p.h_frag_slot.assign((size_t)p.F, -1);
-    p.h_head_frag.clear();
-    p.P = 0;
-    for (int64_t f = 0; f < p.F; f++) {
-        const int32_t w = fw[f];
-        const bool whole = fo[f] == soff[w] && fo[f + 1] == soff[w + 1];
-        if (!whole) {
-            if (f == 0 || fw[f - 1] != w) p.h_head_frag.push_back((int32_t)f);
-            p.h_frag_slot[f] = (int32_t)p.P++;
+
+    // groups of the warp-level kernel: the same fragments, dealt out in shorter runs where the plan's own
+    // groups are longer than a piece
+    p.h_warp_off.clear();
+    if (p.policy == MASK_POLICY_AUTO && p.piece_tiles < G) {
+        constexpr int32_t kFragCost = 4;
+        int32_t load = 0;
+        p.h_warp_off.push_back(0);
+        for (int64_t f = 0; f < p.F; f++) {
+            const int32_t cost = fo[f + 1] - fo[f] + kFragCost;
+            if (load > 0 && load + cost > p.piece_tiles + p.piece_tiles / 4) {
+                p.h_warp_off.push_back((int32_t)f);
+                load = 0;
+            }
+            load += cost;
         }
+        if (p.F > 0) p.h_warp_off.push_back((int32_t)p.F);
     }
-    p.H = (int64_t)p.h_head_frag.size();
-    p.max_group_tiles = 0;
-    p.h_group_tile.resize((size_t)p.G + 1);
-    for (int64_t g = 0; g <= p.G; g++) p.h_group_tile[(size_t)g] = fo[go[g]];
-    for (int64_t g = 0; g < p.G; g++)
-        p.max_group_tiles = std::max<int32_t>(p.max_group_tiles, fo[go[g + 1]] - fo[go[g]]);
 }
 
-template <typename T>
-static int upload(const std::vector<T>& h, T** d, cudaStream_t st) {
-    const size_t n = std::max<size_t>(h.size(), 1);
-    MASK_CUDA_TRY(cudaMalloc(reinterpret_cast<void**>(d), n * sizeof(T)));
-    if (!h.empty()) MASK_CUDA_TRY(cudaMemcpyAsync(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+// One device array for all tables, filled by one copy: sections start on 16-byte boundaries.
+static int upload_tables(mask_plan& p, const int32_t* soff, cudaStream_t st) {
+    const auto& fo = p.h_frag_off; const auto& fw = p.h_frag_win; const auto& go = p.h_group_off;
+    const auto& wo = p.h_warp_off.empty() ? p.h_group_off : p.h_warp_off;
+    p.Gw = (int64_t)wo.size() - 1;
+    // split windows: first fragment and number of pieces; pieces are numbered in fragment order
+    std::vector<int32_t> heads;
+    p.P = 0;
+    auto whole = [&](int64_t f) { return fo[f] == soff[fw[f]] && fo[f + 1] == soff[fw[f] + 1]; };
+    for (int64_t f = 0; f < p.F; f++) {
+        if (whole(f)) continue;
+        if (f == 0 || fw[f - 1] != fw[f]) { heads.push_back((int32_t)f); heads.push_back(0); }
+        heads.back()++;
+        p.P++;
+    }
+    p.H = (int64_t)heads.size() / 2;
+    size_t at = 0;
+    auto section = [&](size_t n) { const size_t o = at; at += (n + 3) & ~(size_t)3; return o; };
+    const size_t o_fo = section(fo.size()), o_fw = section(fw.size()), o_fs = section(fw.size()), o_go = section(go.size()),
+                 o_gt = section(go.size()), o_wo = section(wo.size()), o_wt = section(wo.size()), o_hd = section(heads.size()),
+                 o_st = section(4);
+    HostStage stage;
+    int rc = stage.get(at * sizeof(int32_t));
+    if (rc != MASK_OK) return rc;
+    int32_t* h = stage.as<int32_t>();
+    std::copy(fo.begin(), fo.end(), h + o_fo);
+    std::copy(fw.begin(), fw.end(), h + o_fw);
+    std::copy(go.begin(), go.end(), h + o_go);
+    std::copy(wo.begin(), wo.end(), h + o_wo);
+    std::copy(heads.begin(), heads.end(), h + o_hd);
+    std::fill(h + o_st, h + o_st + 4, 0);
+    int32_t slot = 0;
+    for (int64_t f = 0; f < p.F; f++) h[o_fs + f] = whole(f) ? -1 : slot++;
+    for (size_t g = 0; g < go.size(); g++) h[o_gt + g] = fo[go[g]];
+    for (size_t g = 0; g < wo.size(); g++) h[o_wt + g] = fo[wo[g]];
+    rc = device_alloc(reinterpret_cast<void**>(&p.d_tables), at * sizeof(int32_t), st);
+    if (rc != MASK_OK) return rc;
+    p.d_frag_off = p.d_tables + o_fo;
+    p.d_frag_win = p.d_tables + o_fw;
+    p.d_frag_slot = p.d_tables + o_fs;
+    p.d_group_off = p.d_tables + o_go;
+    p.d_group_tile = p.d_tables + o_gt;
+    p.d_warp_off = p.d_tables + o_wo;
+    p.d_warp_tile = p.d_tables + o_wt;
+    p.d_heads = reinterpret_cast<const int2*>(p.d_tables + o_hd);
+    p.d_status = p.d_tables + o_st;
+    cudaError_t e = cudaMemcpyAsync(p.d_tables, h, at * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+    const cudaError_t e2 = cudaStreamSynchronize(st);   // the plan may be used on any stream from here on
+    MASK_CUDA_TRY(e);
+    MASK_CUDA_TRY(e2);
     return MASK_OK;
 }
 
@@ -212,48 +284,57 @@ extern "C" int mask_plan_multi_bind(const int32_t* h_val_soff, int32_t M, int32_
     return MASK_OK;
 }
 
-extern "C" int mask_plan_create(const int32_t* d_val_soff, int32_t M, int64_t T, int policy, int32_t group_tiles,
-                                void* stream, mask_plan** out) {
-    using namespace mask;
-    MASK_REQUIRE(out != nullptr, "out is NULL");
-    *out = nullptr;
-    MASK_REQUIRE(d_val_soff != nullptr && M >= 1 && T >= 0, "bad arguments");
-    MASK_REQUIRE(policy >= MASK_POLICY_AUTO && policy <= MASK_POLICY_REF_AUTO, "unknown policy");
-    if (T >= (int64_t)1 << 31) return fail(MASK_ERR_INDEX_OVERFLOW, "T does not fit int32");
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
+namespace mask {
+
+// With d_val_sidx the column features are measured and the plan table is applied as well: the kernels that
+// measure run while the host builds the tables (both take 0.15 to 0.2 ms on a graph with 2^20 nodes).
+static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t M, int32_t K, int64_t T, int policy,
+                       int32_t group_tiles, cudaStream_t st, mask_plan** out) {
     mask_plan* p = new mask_plan();
     p->M = M;
     p->W = (M + kWinRows - 1) / kWinRows;
     p->T = T;
     p->policy = policy;
     p->group_tiles = group_tiles > 0 ? group_tiles : (policy == MASK_POLICY_STRICT_LB ? 64 : default_group_tiles(T));
-    std::vector<int32_t> soff((size_t)p->W + 1);
-    cudaError_t e = cudaMemcpyAsync(soff.data(), d_val_soff, soff.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-        delete p;
-        set_error("copying val_soff to the host failed: %s", cudaGetErrorString(e));
-        return MASK_ERR_CUDA;
+    p->piece_tiles = (group_tiles > 0 || policy != MASK_POLICY_AUTO) ? p->group_tiles : std::min(p->group_tiles, default_piece_tiles(T, p->W));
+    HostStage stage;
+    ColumnStatsJob job;
+    cudaEvent_t have_soff = nullptr;
+    auto body = [&]() -> int {
+        MASK_CUDA_TRY(cudaGetDevice(&p->device));
+        const size_t bytes = ((size_t)p->W + 1) * sizeof(int32_t);
+        int rc = stage.get(bytes);
+        if (rc != MASK_OK) return rc;
+        const int32_t* soff = stage.as<int32_t>();
+        MASK_CUDA_TRY(cudaMemcpyAsync(stage.as<int32_t>(), d_val_soff, bytes, cudaMemcpyDeviceToHost, st));
+        if (d_val_sidx) {
+            MASK_CUDA_TRY(cudaEventCreateWithFlags(&have_soff, cudaEventDisableTiming));
+            MASK_CUDA_TRY(cudaEventRecord(have_soff, st));
+            rc = job.enqueue(d_val_soff, d_val_sidx, M, K, T, 512, st);
+            if (rc != MASK_OK) return rc;
+            MASK_CUDA_TRY(cudaEventSynchronize(have_soff));
+        } else {
+            MASK_CUDA_TRY(cudaStreamSynchronize(st));
+        }
+        if (soff[0] != 0 || (int64_t)soff[p->W] != T) return fail(MASK_ERR_INVALID_ARGUMENT, "val_soff does not start at 0 / end at T");
+        if (policy == MASK_POLICY_REF_AUTO) {  // the bridge's automatic choice between its own two mappings
+            mask_features f;
+            mask_features_from_soff(soff, M, 0, &f);
+            p->policy = f.heavy_tail ? MASK_POLICY_STRICT_LB : MASK_POLICY_ROW;
+            if (group_tiles <= 0) p->group_tiles = 64;
+        }
+        build_tables(*p, soff);
+        return upload_tables(*p, soff, st);
+    };
+    const int rc = body();
+    if (rc != MASK_OK) {
+        cudaStreamSynchronize(st);   // copies into the staging buffers may be in flight
+    } else if (d_val_sidx) {
+        mask_column_features f;
+        job.finish(&f);
+        choose_plan_parameters(p, f);
     }
-    if (soff[0] != 0 || (int64_t)soff[p->W] != T) {
-        delete p;
-        return fail(MASK_ERR_INVALID_ARGUMENT, "val_soff does not start at 0 / end at T");
-    }
-    if (policy == MASK_POLICY_REF_AUTO) {  // the bridge's automatic choice between its own two mappings
-        mask_features f;
-        mask_features_from_soff(soff.data(), M, 0, &f);
-        p->policy = f.heavy_tail ? MASK_POLICY_STRICT_LB : MASK_POLICY_ROW;
-        if (group_tiles <= 0) p->group_tiles = 64;
-    }
-    build_tables(*p, soff.data());
-    int rc = upload(p->h_frag_off, &p->d_frag_off, st);
-    if (rc == MASK_OK) rc = upload(p->h_frag_win, &p->d_frag_win, st);
-    if (rc == MASK_OK) rc = upload(p->h_frag_slot, &p->d_frag_slot, st);
-    if (rc == MASK_OK) rc = upload(p->h_group_off, &p->d_group_off, st);
-    if (rc == MASK_OK) rc = upload(p->h_head_frag, &p->d_head_frag, st);
-    if (rc == MASK_OK) rc = upload(p->h_group_tile, &p->d_group_tile, st);
-    if (rc == MASK_OK) rc = upload(std::vector<int32_t>(4, 0), &p->d_status, st);
-    if (rc == MASK_OK && cudaStreamSynchronize(st) != cudaSuccess) rc = fail(MASK_ERR_CUDA, "plan upload failed");
+    if (have_soff) cudaEventDestroy(have_soff);
     if (rc != MASK_OK) {
         mask_plan_destroy(p);
         return rc;
@@ -262,16 +343,43 @@ extern "C" int mask_plan_create(const int32_t* d_val_soff, int32_t M, int64_t T,
     return MASK_OK;
 }
 
+}  // namespace mask
+
+extern "C" int mask_plan_create(const int32_t* d_val_soff, int32_t M, int64_t T, int policy, int32_t group_tiles,
+                                void* stream, mask_plan** out) {
+    using namespace mask;
+    MASK_REQUIRE(out != nullptr, "out is NULL");
+    *out = nullptr;
+    MASK_REQUIRE(d_val_soff != nullptr && M >= 1 && T >= 0, "bad arguments");
+    MASK_REQUIRE(policy >= MASK_POLICY_AUTO && policy <= MASK_POLICY_REF_AUTO, "unknown policy");
+    if (T >= (int64_t)1 << 31) return fail(MASK_ERR_INDEX_OVERFLOW, "T does not fit int32");
+    return create_plan(d_val_soff, nullptr, M, 0, T, policy, group_tiles, static_cast<cudaStream_t>(stream), out);
+}
+
+extern "C" int mask_plan_create_tuned(const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t M, int32_t K, int64_t T, int policy,
+                                      int32_t group_tiles, void* stream, mask_plan** out) {
+    using namespace mask;
+    MASK_REQUIRE(out != nullptr, "out is NULL");
+    *out = nullptr;
+    MASK_REQUIRE(d_val_soff != nullptr && M >= 1 && K >= 1 && T >= 0, "bad arguments");
+    MASK_REQUIRE(T == 0 || d_val_sidx != nullptr, "val_sidx is NULL");
+    MASK_REQUIRE(policy >= MASK_POLICY_AUTO && policy <= MASK_POLICY_REF_AUTO, "unknown policy");
+    if (T >= (int64_t)1 << 31) return fail(MASK_ERR_INDEX_OVERFLOW, "T does not fit int32");
+    return create_plan(d_val_soff, T > 0 ? d_val_sidx : nullptr, M, K, T, policy, group_tiles, static_cast<cudaStream_t>(stream), out);
+}
+
 extern "C" void mask_plan_destroy(mask_plan* p) {
     if (!p) return;
-    cudaFree(p->d_frag_off);
-    cudaFree(p->d_frag_win);
-    cudaFree(p->d_frag_slot);
-    cudaFree(p->d_group_off);
-    cudaFree(p->d_head_frag);
-    cudaFree(p->d_group_tile);
+    // kernels that read the tables may still be running on any stream
+    int cur = -1;
+    const bool elsewhere = p->d_tables && cudaGetDevice(&cur) == cudaSuccess && cur != p->device;
+    if (elsewhere) cudaSetDevice(p->device);
+    if (p->d_tables) {
+        cudaDeviceSynchronize();
+        mask::device_free(p->d_tables, nullptr);
+    }
     cudaFree(p->d_vals_tf32);
-    cudaFree(p->d_status);
+    if (elsewhere) cudaSetDevice(cur);
     delete p;
 }
 

@@ -269,23 +269,34 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, MIN_BLOCKS) spmm_mma_kern
     }
 }
 
-// Sums the partial tiles of every split window in fragment (= tile) order and writes C.
-__global__ void __launch_bounds__(256) spmm_fixup_kernel(const int32_t* head_frag, const int32_t* frag_win,
-                                                        const int32_t* frag_slot, int64_t n_frag,
+// Sums the partial tiles of every split window in fragment (= tile) order and writes C.  heads: first
+// fragment and number of pieces of each split window; the pieces' partial tiles lie one behind the other, so
+// the reads of a thread are independent and eight of them are in flight at a time (walking the fragment
+// tables piece by piece instead was a chain of dependent loads: 0.78 ms for 85 000 pieces at N = 512, now 0.57).
+__global__ void __launch_bounds__(256) spmm_fixup_kernel(const int2* heads, const int32_t* frag_win, const int32_t* frag_slot,
                                                         const float* scratch, float* C, int64_t ldc, int32_t M,
                                                         int32_t N, int32_t relu, const int32_t* row_map,
                                                         float* const* peer_out, int32_t n_peer_out) {
-    const int64_t f0 = head_frag[blockIdx.x];
-    const int w = frag_win[f0];
-    int64_t f1 = f0;
-    while (f1 < n_frag && frag_win[f1] == w && frag_slot[f1] >= 0) f1++;
+    const int2 head = heads[blockIdx.x];
+    const int w = frag_win[head.x];
     const int nvec = N >> 2;
+    const int64_t tile_vecs = (int64_t)kWinRows * nvec;
+    const float4* first = reinterpret_cast<const float4*>(scratch) + (int64_t)frag_slot[head.x] * tile_vecs;
     for (int v = blockIdx.y * blockDim.x + threadIdx.x; v < kWinRows * nvec; v += gridDim.y * blockDim.x) {
         const int r = v / nvec, c = (v - r * nvec) << 2;
         if (w * kWinRows + r >= M) continue;
+        const float4* at = first + v;
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int64_t ff = f0; ff < f1; ff++) {
-            const float4 x = *reinterpret_cast<const float4*>(scratch + ((int64_t)frag_slot[ff] * kWinRows + r) * N + c);
+        int i = 0;
+        for (; i + 8 <= head.y; i += 8, at += 8 * tile_vecs) {
+            float4 x[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) x[j] = at[j * tile_vecs];
+#pragma unroll
+            for (int j = 0; j < 8; j++) { s.x += x[j].x; s.y += x[j].y; s.z += x[j].z; s.w += x[j].w; }
+        }
+        for (; i < head.y; i++, at += tile_vecs) {
+            const float4 x = *at;
             s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
         }
         if (relu) { s.x = fmaxf(s.x, 0.f); s.y = fmaxf(s.y, 0.f); s.z = fmaxf(s.z, 0.f); s.w = fmaxf(s.w, 0.f); }
@@ -298,8 +309,8 @@ __global__ void __launch_bounds__(256) spmm_fixup_kernel(const int32_t* head_fra
 static int launch_fixup(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st) {
     if (plan->H > 0) {
         dim3 fgrid((unsigned)plan->H, (unsigned)((kWinRows * (a.N >> 2) + 255) / 256));
-        spmm_fixup_kernel<<<fgrid, 256, 0, st>>>(plan->d_head_frag, plan->d_frag_win, plan->d_frag_slot, plan->F,
-                                                 a.scratch, a.C, a.ldc, a.M, a.N, a.relu, a.row_map, a.peer_out, a.n_peer_out);
+        spmm_fixup_kernel<<<fgrid, 256, 0, st>>>(plan->d_heads, plan->d_frag_win, plan->d_frag_slot, a.scratch, a.C, a.ldc, a.M,
+                                                 a.N, a.relu, a.row_map, a.peer_out, a.n_peer_out);
         MASK_CUDA_TRY(cudaGetLastError());
     }
     return MASK_OK;

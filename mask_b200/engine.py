@@ -34,11 +34,17 @@ def _req(t, dtype, name):
 class Plan:
     """How tiles are dealt to thread blocks (``mask_plan``)."""
 
-    def __init__(self, val_soff: torch.Tensor, M: int, T: int, policy: str = "auto", group_tiles: int = 0):
+    def __init__(self, val_soff: torch.Tensor, M: int, T: int, policy: str = "auto", group_tiles: int = 0,
+                 val_sidx: torch.Tensor | None = None, K: int = 0):
+        """With ``val_sidx`` and ``K`` the plan is tuned from the matrix's column features as well."""
         _req(val_soff, torch.int32, "val_soff")
         h = C.c_void_p()
-        check(lib().mask_plan_create(_ptr(val_soff), M, T, _lib.POLICY[policy], group_tiles, _stream(), C.byref(h)),
-              "mask_plan_create")
+        if val_sidx is not None:
+            check(lib().mask_plan_create_tuned(_ptr(val_soff), _ptr(val_sidx), M, K, T, _lib.POLICY[policy], group_tiles, _stream(),
+                                               C.byref(h)), "mask_plan_create_tuned")
+        else:
+            check(lib().mask_plan_create(_ptr(val_soff), M, T, _lib.POLICY[policy], group_tiles, _stream(), C.byref(h)),
+                  "mask_plan_create")
         self._h = h
         self.policy = policy
         self.M, self.T = M, T
@@ -135,9 +141,8 @@ class PackedSRBCRS:
         """A plan for this matrix: tuned from the matrix's column features (``autotune``), carrying the
         row map when the rows were reordered and, on request, the rounded copy of the tile values that
         the TMA-fed kernel reads (``prepare``; as much device memory as val_block_val again)."""
-        p = Plan(self.val_soff, self.M, self.T, policy, group_tiles)
-        if autotune and self.T > 0:
-            check(lib().mask_plan_autotune(p._h, _ptr(self.val_soff), _ptr(self.val_sidx), self.K, _stream()), "mask_plan_autotune")
+        tuned = autotune and self.T > 0
+        p = Plan(self.val_soff, self.M, self.T, policy, group_tiles, self.val_sidx if tuned else None, self.K)
         if prepare and isinstance(self, PackedSRBCRS) and self.T > 0:
             check(lib().mask_plan_prepare_values(p._h, _ptr(self.val_block_val), _stream()), "mask_plan_prepare_values")
         if self.row_order is not None:
