@@ -12,11 +12,13 @@
 //                   similarity a warp-wide intersection count by binary search.
 //   row_rcm         reverse Cuthill-McKee.  The sequential queue order is reproduced level by level:
 //                   a node's parent is the EARLIEST queue position among its visited neighbours
-//                   (atomicMin), a level is its nodes sorted by (parent position, degree, id), and all
+//                   (atomicMin), the children of a parent follow each other in (degree, id) order, and all
 //                   connected components advance together; components are then laid out by the rank of
 //                   their start node (the unvisited node of least (degree, id)) and each is reversed.
-//                   One round of kernels per breadth-first level: the cost grows with the graph's
-//                   diameter (tens of levels for graphs, hundreds for 3-D meshes).
+//                   The traversal is one cooperative launch; a level costs about 10 us, which for meshes
+//                   and other graphs with tens to hundreds of levels is most of the time (64 000-node shuffled
+//                   27-point mesh, 40 levels: 0.44 of 0.8 ms; a launch
+//                   sequence with three radix sorts and a host read per level took 13 ms).
 // Applying an order -- gathering the rows of a device CSR matrix -- and undoing it are device work
 // too: the SpMM kernels take the order as a row map and write output row order[new_row] directly,
 // which replaces the bridge's host-side unpack_output (:1083-1100).
@@ -27,22 +29,15 @@
 #include <algorithm>
 #include <cstring>
 
+#include <cooperative_groups.h>
+
 #include "common.cuh"
+#include "condense.cuh"
+#include "mem.h"
 
 namespace mask {
 
 namespace {
-
-// Device scratch that frees itself; sized once per call (these are format-conversion passes).
-struct DevBuf {
-    void* p = nullptr;
-    ~DevBuf() { if (p) cudaFree(p); }
-    int alloc(size_t bytes) {
-        MASK_CUDA_TRY(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
-        return MASK_OK;
-    }
-    template <typename T> T* as() const { return static_cast<T*>(p); }
-};
 
 __global__ void iota_kernel(int32_t* a, int32_t n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -88,17 +83,18 @@ __global__ void gather_keys_kernel(const KeyT* __restrict__ key_of_row, const in
 template <typename KeyT>
 int sort_rows_by(const KeyT* key_of_row, int32_t* rows_in, int32_t* rows_out, int32_t n, int end_bit, cudaStream_t st) {
     if (n == 0) return MASK_OK;
-    DevBuf kin, kout, tmp;
-    int rc = kin.alloc((size_t)n * sizeof(KeyT));
-    if (rc == MASK_OK) rc = kout.alloc((size_t)n * sizeof(KeyT));
+    DevScratch keys, tmp;
+    const size_t half = ((size_t)n * sizeof(KeyT) + 255) & ~(size_t)255;
+    int rc = keys.alloc(2 * half, st);
     if (rc != MASK_OK) return rc;
-    gather_keys_kernel<KeyT><<<(n + 255) / 256, 256, 0, st>>>(key_of_row, rows_in, n, kin.as<KeyT>());
+    KeyT *kin = keys.as<KeyT>(), *kout = keys.as<KeyT>(half);
+    gather_keys_kernel<KeyT><<<(n + 255) / 256, 256, 0, st>>>(key_of_row, rows_in, n, kin);
+    MASK_CUDA_TRY(cudaGetLastError());
     size_t bytes = 0;
-    MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kin.as<KeyT>(), kout.as<KeyT>(), rows_in, rows_out, n, 0, end_bit, st));
-    rc = tmp.alloc(bytes);
+    MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kin, kout, rows_in, rows_out, n, 0, end_bit, st));
+    rc = tmp.alloc(bytes, st);
     if (rc != MASK_OK) return rc;
-    MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, bytes, kin.as<KeyT>(), kout.as<KeyT>(), rows_in, rows_out, n, 0, end_bit, st));
-    MASK_CUDA_TRY(cudaStreamSynchronize(st));   // the scratch goes away with this frame
+    MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, bytes, kin, kout, rows_in, rows_out, n, 0, end_bit, st));
     return MASK_OK;
 }
 
@@ -171,6 +167,10 @@ __global__ void __launch_bounds__(256) jaccard_chain_kernel(const int32_t* __res
 }
 
 // ---- reverse Cuthill-McKee ------------------------------------------------------------------------
+// Nodes are renamed by their rank in (degree, id) order, and every node's neighbours are listed in ascending
+// rank: the children a node contributes to the queue are then its new neighbours as they stand in its list,
+// and no level has to be sorted.
+
 __global__ void sym_edge_keys_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M,
                                      uint64_t* __restrict__ keys) {
     // one warp per row; every stored (r, c) with c != r in range gives (r, c) and (c, r); others give a sentinel
@@ -191,201 +191,539 @@ __global__ void split_targets_kernel(const uint64_t* __restrict__ keys, int64_t 
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) adj[i] = (int32_t)(keys[i] & 0xffffffffu);
 }
-__global__ void scatter_rank_kernel(const int32_t* __restrict__ starts, int32_t M, int32_t* __restrict__ rank) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < M) rank[starts[i]] = i;
+// one thread per entry of a CSR matrix: its row, searched between the rows of the block's first and last entry
+__device__ __forceinline__ int row_of_entry(const int32_t* __restrict__ ptr, int32_t M, int64_t first, int64_t last, int64_t e, int* range) {
+    if (threadIdx.x < 2) {
+        const int64_t key = threadIdx.x == 0 ? first : last;
+        int lo = 0, hi = M;   // last row with ptr[row] <= key
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if ((int64_t)ptr[mid] <= key) lo = mid; else hi = mid;
+        }
+        range[threadIdx.x] = lo;
+    }
+    __syncthreads();
+    int lo = range[0], hi = range[1] + 1;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if ((int64_t)ptr[mid] <= e) lo = mid; else hi = mid;
+    }
+    __syncthreads();
+    return lo;
 }
-// label[v] = min(label[v], labels of its neighbours), then one shortcut through the node that label names
-// (labels are ranks, starts[label] is a node of the same component), so chains collapse in a logarithmic
-// number of rounds; flag set when anything moved
-__global__ void propagate_labels_kernel(const int64_t* __restrict__ beg, const int32_t* __restrict__ adj,
-                                        const int32_t* __restrict__ starts, int32_t M, int32_t* __restrict__ label,
-                                        int32_t* __restrict__ changed) {
-    const int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (v >= M) return;
-    int best = label[v];
-    for (int64_t q = beg[v] + lane; q < beg[v + 1]; q += 32) best = min(best, label[adj[q]]);
-    for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (lane == 0) {
-        best = min(best, label[starts[best]]);
-        if (best < label[v]) { label[v] = best; *changed = 1; }
+
+__global__ void row_lengths_kernel(const int32_t* __restrict__ ptr, int32_t M, int32_t* __restrict__ len) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < M) len[i] = ptr[i + 1] - ptr[i];
+}
+
+// Takes diagonal and out-of-range entries off the degrees; *asymmetric is set if some other entry (r, c) has no
+// counterpart (c, r).
+__global__ void __launch_bounds__(256) check_symmetry_kernel(const int32_t* __restrict__ ptr, const int32_t* __restrict__ col, int32_t M,
+                                                             int64_t nnz, int32_t* __restrict__ deg, int32_t* __restrict__ asymmetric) {
+    __shared__ int range[2];
+    const int64_t first = (int64_t)blockIdx.x * 256, e = first + threadIdx.x;
+    const int64_t last = first + 255 < nnz ? first + 255 : nnz - 1;
+    const int r = row_of_entry(ptr, M, first, last, e < nnz ? e : last, range);
+    if (e >= nnz) return;
+    const int c = col[e];
+    if (c < 0 || c >= M || c == r) {
+        atomicSub(&deg[r], 1);
+        return;
+    }
+    int lo = ptr[c], hi = ptr[c + 1];
+    const int end = hi;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (__ldg(col + mid) < r) lo = mid + 1; else hi = mid;
+    }
+    if (lo == end || col[lo] != r) *asymmetric = 1;
+}
+
+__global__ void scatter_rank_kernel(const int32_t* __restrict__ starts, int32_t M, int32_t* __restrict__ rank, int32_t* __restrict__ label) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < M) {
+        rank[starts[i]] = i;
+        label[i] = i;
     }
 }
-__global__ void seed_frontier_kernel(const int32_t* __restrict__ label, const int32_t* __restrict__ rank, int32_t M,
-                                     int32_t* __restrict__ frontier, int32_t* __restrict__ count, int32_t* __restrict__ pos) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= M) return;
-    pos[v] = -1;
-    if (label[v] == rank[v]) frontier[atomicAdd(count, 1)] = v;   // the component's node of least (degree, id)
+
+constexpr int kAdjSortMax = 1024;   // longest neighbour list a warp sorts
+
+// neighbours of node starts[i] by rank; lists of more than 32 E entries are not for this E
+template <int E>
+__device__ __forceinline__ void sort_neighbours(const int32_t* __restrict__ col, int n, int self, int32_t M, const int32_t* __restrict__ rank,
+                                                int32_t* __restrict__ out, int n_out, int lane) {
+    uint32_t key[E];
+#pragma unroll
+    for (int i = 0; i < E; i++) {
+        const int e = i * 32 + lane;
+        const int c = e < n ? __ldg(col + e) : -1;
+        key[i] = (c >= 0 && c < M && c != self) ? (uint32_t)rank[c] : ~0u;
+    }
+    warp_sort<E, uint32_t>(key, lane);
+#pragma unroll
+    for (int i = 0; i < E; i++)
+        if (lane * E + i < n_out) out[lane * E + i] = (int32_t)key[i];
 }
-__global__ void assign_positions_kernel(const int32_t* __restrict__ frontier, int32_t n, int32_t base, int32_t* __restrict__ pos) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) pos[frontier[i]] = base + i;
-}
-// every unvisited neighbour of a frontier node records the earliest queue position that reaches it and
-// is appended to the next level once
-__global__ void expand_frontier_kernel(const int64_t* __restrict__ beg, const int32_t* __restrict__ adj,
-                                       const int32_t* __restrict__ frontier, int32_t n, int32_t base, const int32_t* __restrict__ pos,
-                                       int32_t* __restrict__ parent, int32_t* __restrict__ claimed, int32_t* __restrict__ next,
-                                       int32_t* __restrict__ next_count) {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= n) return;
-    const int v = frontier[i];
-    for (int64_t q = beg[v] + lane; q < beg[v + 1]; q += 32) {
-        const int nb = adj[q];
-        if (pos[nb] >= 0) continue;
-        atomicMin(&parent[nb], base + i);
-        if (atomicExch(&claimed[nb], 1) == 0) next[atomicAdd(next_count, 1)] = nb;
+
+__global__ void __launch_bounds__(128) sort_adjacency_kernel(const int32_t* __restrict__ ptr, const int32_t* __restrict__ col, int32_t M,
+                                                             const int32_t* __restrict__ starts, const int32_t* __restrict__ rank,
+                                                             const int32_t* __restrict__ out_ptr, int32_t* __restrict__ out,
+                                                             int32_t* __restrict__ long_list, int32_t* __restrict__ n_long) {
+    const int i = (blockIdx.x * 128 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i >= M) return;
+    const int v = starts[i], b = ptr[v], n = ptr[v + 1] - b, o = out_ptr[i], n_out = out_ptr[i + 1] - o;
+    if (n > kAdjSortMax) {
+        if (lane == 0) long_list[atomicAdd(n_long, 1)] = i;
+    } else if (n > 512) {
+        sort_neighbours<32>(col + b, n, v, M, rank, out + o, n_out, lane);
+    } else if (n > 128) {
+        sort_neighbours<16>(col + b, n, v, M, rank, out + o, n_out, lane);
+    } else if (n > 32) {
+        sort_neighbours<4>(col + b, n, v, M, rank, out + o, n_out, lane);
+    } else if (n > 0) {
+        sort_neighbours<1>(col + b, n, v, M, rank, out + o, n_out, lane);
     }
 }
-__global__ void final_keys_kernel(const int32_t* __restrict__ label, const int32_t* __restrict__ pos, int32_t M,
-                                  uint64_t* __restrict__ keys, int32_t* __restrict__ ids) {
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= M) return;
-    keys[v] = ((uint64_t)(uint32_t)label[v] << 32) | (uint32_t)(0x7fffffff - pos[v]);   // component by start rank, queue order reversed
-    ids[v] = v;
+
+constexpr int kLongBits = 1 << 19;
+// the same for long lists: one block marks the ranks and places every one by the number of marks below it
+__global__ void __launch_bounds__(512) sort_long_adjacency_kernel(const int32_t* __restrict__ ptr, const int32_t* __restrict__ col, int32_t M,
+                                                                  const int32_t* __restrict__ starts, const int32_t* __restrict__ rank,
+                                                                  const int32_t* __restrict__ out_ptr, int32_t* __restrict__ out,
+                                                                  const int32_t* __restrict__ long_list, const int32_t* __restrict__ n_long) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int run_before[kLongBits / 4096];
+    __shared__ int warp_sum[32];
+    const int total = *n_long;
+    MarkSet marks{reinterpret_cast<uint32_t*>(smem), reinterpret_cast<uint16_t*>(smem + kLongBits / 8), run_before,
+                  (min(M, kLongBits) + 4095) / 4096};
+    for (int j = blockIdx.x; j < total; j += gridDim.x) {
+        const int i = long_list[j], v = starts[i], b = ptr[v], n = ptr[v + 1] - b, o = out_ptr[i];
+        int placed = 0;
+        for (int r0 = 0; r0 < M; r0 += kLongBits) {
+            const int span = min(kLongBits, M - r0);
+            __syncthreads();
+            for (int k = threadIdx.x; k < marks.n_runs * 128; k += 512) marks.bits[k] = 0;
+            __syncthreads();
+            auto each = [&](auto f) {
+#pragma unroll 4
+                for (int e = threadIdx.x; e < n; e += 512) {
+                    const int c = __ldg(col + b + e);
+                    if (c < 0 || c >= M || c == v) continue;
+                    const int d = rank[c] - r0;
+                    if (d >= 0 && d < span) f(d);
+                }
+            };
+            each([&](int d) { marks.mark(d); });
+            const int here = marks.count<512>(warp_sum);
+            each([&](int d) { out[o + placed + marks.rank(d)] = r0 + d; });
+            placed += here;
+        }
+    }
+}
+
+// Connected components by hooking: the root of a tree is its least node, so labels end as the component's least rank.
+__device__ __forceinline__ int find_root(int32_t* label, int i) {
+    int cur = __ldcg(label + i);
+    if (cur != i) {
+        int prev = i, next;
+        while (cur > (next = __ldcg(label + cur))) {   // halve the path on the way
+            label[prev] = next;
+            prev = cur;
+            cur = next;
+        }
+    }
+    return cur;
+}
+__global__ void __launch_bounds__(256) hook_kernel(const int32_t* __restrict__ ptr, const int32_t* __restrict__ adj, int32_t M, int32_t* __restrict__ label) {
+    __shared__ int range[2];
+    const int64_t n = ptr[M];
+    const int64_t first = (int64_t)blockIdx.x * 256, e = first + threadIdx.x;
+    if (first >= n) return;
+    const int64_t last = first + 255 < n ? first + 255 : n - 1;
+    const int i = row_of_entry(ptr, M, first, last, e < n ? e : last, range);
+    if (e >= n) return;
+    const int j = adj[e];
+    if (j >= i) return;   // every edge is listed from both ends
+    int a = find_root(label, i), b = find_root(label, j);
+    while (a != b) {      // the larger root joins the smaller; a failed exchange returns a smaller label
+        if (a < b) { const int t = a; a = b; b = t; }
+        const int was = atomicCAS(label + a, a, b);
+        if (was == a) break;
+        a = was;
+    }
+}
+__global__ void flatten_labels_kernel(int32_t* __restrict__ label, int32_t M) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= M) return;
+    int cur = __ldcg(label + i), next;
+    while (cur > (next = __ldcg(label + cur))) cur = next;
+    label[i] = cur;
+}
+struct IsRoot {
+    const int32_t* label;
+    __device__ bool operator()(int i) const { return label[i] == i; }
+};
+
+// Breadth-first levels of all components at once, in Cuthill-McKee queue order, as one cooperative launch.
+// Per level: (1) every unvisited neighbour records the earliest queue position that reaches it, (2) every queue
+// node counts the neighbours that recorded it, (3) the counts are scanned and the children written behind the
+// queue.  A block takes a run of consecutive queue nodes, a warp a node (nodes with long lists: the block).
+// Levels of at most kSmallLevel nodes are walked by one block alone, without grid-wide barriers.
+struct BfsArgs {
+    const int32_t* ptr;
+    const int32_t* adj;
+    int32_t* queue;
+    int32_t* pos;        // queue position, -1 before
+    int32_t* parent;     // earliest queue position that reaches the node
+    int32_t* children;   // per node of the level
+    int32_t* block_sum;  // per block
+    int32_t* state;      // [0] base of the level, [1] its size
+    const int32_t* n_start;
+    int32_t M;
+};
+constexpr int kBfsThreads = 512, kBfsWarps = kBfsThreads / 32;
+constexpr int kBlockList = 1024;   // lists longer than this are walked by the whole block
+constexpr int kSmallLevel = 64;
+
+constexpr int kMaxLong = 256;
+
+struct BfsShared {
+    int warp_sum[kBfsWarps];
+    int n_long;            // nodes of the block's share with long lists; too many of them: every node to a warp
+    int long_at[kMaxLong];
+    __device__ __forceinline__ bool by_block(int len) const { return len > kBlockList && n_long <= kMaxLong; }
+};
+
+// `width` lanes (a warp or the block) record queue position qpos with the unvisited neighbours of its node.
+__device__ __forceinline__ void bfs_mark(const BfsArgs& p, int qpos, int lane, int width) {
+    const int v = __ldcg(p.queue + qpos), b = p.ptr[v], e = p.ptr[v + 1];
+    for (int q = b + lane; q < e; q += width) {
+        const int nb = p.adj[q];
+        if (__ldcg(p.pos + nb) < 0 && __ldcg(p.parent + nb) > qpos) atomicMin(p.parent + nb, qpos);
+    }
+}
+__device__ __forceinline__ int warp_total(int x) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+__device__ __forceinline__ int block_exclusive(int x, BfsShared& s, int* total) {   // all threads
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int y = x;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int z = __shfl_up_sync(0xffffffffu, y, o);
+        if (lane >= o) y += z;
+    }
+    __syncthreads();
+    if (lane == 31) s.warp_sum[warp] = y;
+    __syncthreads();
+    int before = 0, all = 0;
+    for (int i = 0; i < kBfsWarps; i++) {
+        const int v = s.warp_sum[i];
+        all += v;
+        if (i < warp) before += v;
+    }
+    *total = all;
+    return before + y - x;
+}
+
+// The queue nodes [lo, hi) of the level that begins at `base`: marks.
+__device__ void bfs_mark_range(const BfsArgs& p, int base, int lo, int hi, BfsShared& s) {
+    if (threadIdx.x == 0) s.n_long = 0;
+    __syncthreads();
+    for (int i = lo + threadIdx.x; i < hi; i += kBfsThreads) {
+        const int v = __ldcg(p.queue + base + i);
+        if (p.ptr[v + 1] - p.ptr[v] > kBlockList) {
+            const int k = atomicAdd(&s.n_long, 1);
+            if (k < kMaxLong) s.long_at[k] = i;
+        }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int i = lo + warp; i < hi; i += kBfsWarps) {
+        const int v = __ldcg(p.queue + base + i);
+        if (!s.by_block(p.ptr[v + 1] - p.ptr[v])) bfs_mark(p, base + i, lane, 32);
+    }
+    if (s.n_long <= kMaxLong)
+        for (int k = 0; k < s.n_long; k++) bfs_mark(p, base + s.long_at[k], threadIdx.x, kBfsThreads);
+}
+// Counts children per node; returns the sum over the range (to every thread).
+__device__ int bfs_count_range(const BfsArgs& p, int base, int lo, int hi, BfsShared& s) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int sum = 0;
+    for (int i = lo + warp; i < hi; i += kBfsWarps) {
+        const int v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
+        if (s.by_block(e - b)) continue;
+        int c = 0;
+        for (int q = b + lane; q < e; q += 32) c += __ldcg(p.parent + p.adj[q]) == base + i;
+        c = warp_total(c);
+        if (lane == 0) { p.children[i] = c; sum += c; }
+    }
+    for (int k = 0; k < s.n_long && s.n_long <= kMaxLong; k++) {
+        const int i = s.long_at[k], v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
+        int c = 0, all = 0;
+        for (int q = b + threadIdx.x; q < e; q += kBfsThreads) c += __ldcg(p.parent + p.adj[q]) == base + i;
+        block_exclusive(c, s, &all);
+        if (threadIdx.x == 0) { p.children[i] = all; sum += all; }
+    }
+    int total = 0;
+    block_exclusive(sum, s, &total);
+    return total;
+}
+// Writes the children of the range behind queue position `at` and numbers them.
+__device__ void bfs_place_range(const BfsArgs& p, int base, int lo, int hi, int at, BfsShared& s) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();   // children[] of the range has been written by this block
+    for (int c0 = lo; c0 < hi; c0 += kBfsThreads) {
+        const int mine = c0 + (int)threadIdx.x < hi ? __ldcg(p.children + c0 + threadIdx.x) : 0;
+        int all = 0;
+        const int before = block_exclusive(mine, s, &all);
+        if (c0 + (int)threadIdx.x < hi) p.children[c0 + threadIdx.x] = at + before;   // now: where they go
+        at += all;
+    }
+    __syncthreads();
+    for (int i = lo + warp; i < hi; i += kBfsWarps) {
+        const int v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
+        if (s.by_block(e - b)) continue;
+        int to = __ldcg(p.children + i);
+        for (int q0 = b; q0 < e; q0 += 32) {
+            const int nb = q0 + lane < e ? p.adj[q0 + lane] : -1;
+            const bool child = nb >= 0 && __ldcg(p.parent + nb) == base + i;
+            const unsigned m = __ballot_sync(0xffffffffu, child);
+            if (child) {
+                const int o = to + __popc(m & ((1u << lane) - 1u));
+                p.queue[o] = nb;
+                p.pos[nb] = o;
+            }
+            to += __popc(m);
+        }
+    }
+    for (int k = 0; k < s.n_long && s.n_long <= kMaxLong; k++) {
+        const int i = s.long_at[k], v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
+        int to = __ldcg(p.children + i);
+        for (int q0 = b; q0 < e; q0 += kBfsThreads) {
+            const int nb = q0 + (int)threadIdx.x < e ? p.adj[q0 + threadIdx.x] : -1;
+            const bool child = nb >= 0 && __ldcg(p.parent + nb) == base + i;
+            int all = 0;
+            const int before = block_exclusive(child, s, &all);
+            if (child) {
+                p.queue[to + before] = nb;
+                p.pos[nb] = to + before;
+            }
+            to += all;
+        }
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kBfsThreads) bfs_kernel(const BfsArgs p) {
+    namespace cg = cooperative_groups;
+    cg::grid_group grid = cg::this_grid();
+    __shared__ BfsShared s;
+    int base = 0, n = *p.n_start;
+    for (int i = blockIdx.x * kBfsThreads + threadIdx.x; i < n; i += gridDim.x * kBfsThreads) p.pos[__ldcg(p.queue + i)] = i;
+    grid.sync();
+    while (n > 0) {
+        if (n <= kSmallLevel) {
+            if (blockIdx.x == 0) {
+                while (n > 0 && n <= kSmallLevel) {
+                    bfs_mark_range(p, base, 0, n, s);
+                    __syncthreads();
+                    const int next = bfs_count_range(p, base, 0, n, s);
+                    bfs_place_range(p, base, 0, n, base + n, s);
+                    base += n;
+                    n = next;
+                }
+                if (threadIdx.x == 0) { p.state[0] = base; p.state[1] = n; }
+            }
+            grid.sync();
+            base = __ldcg(p.state);
+            n = __ldcg(p.state + 1);
+            grid.sync();   // everybody has read the state
+            continue;
+        }
+        const int share = (n + gridDim.x - 1) / gridDim.x;
+        const int lo = min(n, (int)blockIdx.x * share), hi = min(n, lo + share);
+        bfs_mark_range(p, base, lo, hi, s);
+        grid.sync();
+        const int sum = bfs_count_range(p, base, lo, hi, s);
+        if (threadIdx.x == 0) p.block_sum[blockIdx.x] = sum;
+        grid.sync();
+        int x = 0, all = 0, before = 0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += kBfsThreads) {
+            const int v = __ldcg(p.block_sum + i);
+            all += v;
+            if (i < (int)blockIdx.x) x += v;
+        }
+        block_exclusive(x, s, &before);
+        int next = 0;
+        block_exclusive(all, s, &next);
+        bfs_place_range(p, base, lo, hi, base + n + before, s);
+        base += n;
+        n = next;
+        grid.sync();
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) p.state[0] = base;
+}
+
+// item i of the final order before it is sorted by component: the queue from its end
+__global__ void reversed_queue_kernel(const int32_t* __restrict__ queue, const int32_t* __restrict__ label, const int32_t* __restrict__ starts,
+                                      int32_t M, uint32_t* __restrict__ key, int32_t* __restrict__ row) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= M) return;
+    const int v = queue[M - 1 - i];
+    key[i] = (uint32_t)label[v];
+    row[i] = starts[v];
+}
+
+inline int bits_for(int64_t n) {   // bits of the numbers below n
+    int b = 1;
+    while (((int64_t)1 << b) < n) b++;
+    return b;
+}
+
+// Both directions of every off-diagonal entry, deduplicated, as a CSR matrix: for patterns that are not symmetric.
+int symmetrised_pattern(const int32_t* rowptr, const int32_t* colind, int32_t M, int64_t nnz, DevScratch& ptr_b, DevScratch& adj_b,
+                        int64_t* n_edges_out, cudaStream_t st) {
+    DevScratch keys, keys_sorted, tmp, n_unique_d, deg_b;
+    const int64_t n_keys = 2 * nnz;
+    if (n_keys >= ((int64_t)1 << 31)) return fail(MASK_ERR_INDEX_OVERFLOW, "too many entries for the device reorder");
+    int rc = keys.alloc((size_t)n_keys * 8, st);
+    if (rc == MASK_OK) rc = keys_sorted.alloc((size_t)n_keys * 8, st);
+    if (rc == MASK_OK) rc = n_unique_d.alloc(8, st);
+    if (rc == MASK_OK) rc = deg_b.alloc(((size_t)M + 1) * 4, st);
+    if (rc == MASK_OK) rc = ptr_b.alloc(((size_t)M + 1) * 4, st);
+    if (rc != MASK_OK) return rc;
+    const unsigned row_blocks = (unsigned)(((int64_t)M * 32 + 255) / 256);
+    sym_edge_keys_kernel<<<row_blocks, 256, 0, st>>>(rowptr, colind, M, keys.as<uint64_t>());
+    MASK_CUDA_TRY(cudaGetLastError());
+    uint64_t *k0 = keys.as<uint64_t>(), *k1 = keys_sorted.as<uint64_t>();
+    size_t b1 = 0, b2 = 0, b3 = 0;
+    MASK_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, b1, k0, k1, (int)n_keys, 0, 64, st));
+    MASK_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, b2, k1, k0, n_unique_d.as<int64_t>(), (int)n_keys, st));
+    MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, b3, deg_b.as<int32_t>(), ptr_b.as<int32_t>(), M + 1, st));
+    rc = tmp.alloc(std::max(b1, std::max(b2, b3)), st);
+    if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tmp.p, b1, k0, k1, (int)n_keys, 0, 64, st));
+    MASK_CUDA_TRY(cub::DeviceSelect::Unique(tmp.p, b2, k1, k0, n_unique_d.as<int64_t>(), (int)n_keys, st));
+    HostStage host;
+    rc = host.get(8);
+    if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(cudaMemcpyAsync(host.as<int64_t>(), n_unique_d.p, 8, cudaMemcpyDeviceToHost, st));
+    MASK_CUDA_TRY(cudaStreamSynchronize(st));
+    int64_t n_edges = *host.as<int64_t>();
+    if (n_edges > 0) {   // the sentinel (all ones) sorts last and, if present, is one unique key: drop it
+        MASK_CUDA_TRY(cudaMemcpyAsync(host.as<int64_t>(), k0 + (n_edges - 1), 8, cudaMemcpyDeviceToHost, st));
+        MASK_CUDA_TRY(cudaStreamSynchronize(st));
+        if (*host.as<uint64_t>() == ~0ULL) n_edges--;
+    }
+    rc = adj_b.alloc((size_t)std::max<int64_t>(n_edges, 1) * 4, st);
+    if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(cudaMemsetAsync(deg_b.p, 0, ((size_t)M + 1) * 4, st));
+    if (n_edges > 0) {
+        const unsigned eb = (unsigned)((n_edges + 255) / 256);
+        count_sources_kernel<<<eb, 256, 0, st>>>(k0, n_edges, deg_b.as<int32_t>());
+        split_targets_kernel<<<eb, 256, 0, st>>>(k0, n_edges, adj_b.as<int32_t>());
+        MASK_CUDA_TRY(cudaGetLastError());
+    }
+    MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, b3, deg_b.as<int32_t>(), ptr_b.as<int32_t>(), M + 1, st));
+    *n_edges_out = n_edges;
+    return MASK_OK;
 }
 
 int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, int64_t nnz, int32_t* order, cudaStream_t st) {
-    const unsigned row_blocks = (unsigned)(((int64_t)M * 32 + 255) / 256), node_blocks = (unsigned)((M + 255) / 256);
-    // symmetrised, deduplicated adjacency
-    DevBuf keys, keys_sorted, keys_unique, n_unique_d, tmp, deg_b, beg_b, adj_b;
-    const int64_t n_keys = 2 * nnz;
-    int rc = keys.alloc((size_t)n_keys * 8);
-    if (rc == MASK_OK) rc = keys_sorted.alloc((size_t)n_keys * 8);
-    if (rc == MASK_OK) rc = keys_unique.alloc((size_t)n_keys * 8);
-    if (rc == MASK_OK) rc = n_unique_d.alloc(8);
-    if (rc == MASK_OK) rc = deg_b.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = beg_b.alloc(((size_t)M + 1) * 8);
+    const unsigned node_blocks = (unsigned)((M + 255) / 256);
+    const int32_t *ptr = rowptr, *col = colind;
+    int64_t n_edges = nnz;
+    DevScratch deg_b, flag_b, sym_ptr, sym_adj;
+    HostStage host;
+    int rc = deg_b.alloc(((size_t)M + 1) * 4, st);
+    if (rc == MASK_OK) rc = flag_b.alloc(64, st);
+    if (rc == MASK_OK) rc = host.get(64);
     if (rc != MASK_OK) return rc;
-    int64_t n_edges = 0;
-    if (n_keys > 0) {
-        if (n_keys >= ((int64_t)1 << 31)) return fail(MASK_ERR_INDEX_OVERFLOW, "too many entries for the device reorder");
-        sym_edge_keys_kernel<<<row_blocks, 256, 0, st>>>(rowptr, colind, M, keys.as<uint64_t>());
-        size_t bytes = 0, bytes2 = 0;
-        MASK_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, bytes, keys.as<uint64_t>(), keys_sorted.as<uint64_t>(), (int)n_keys, 0, 64, st));
-        MASK_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, bytes2, keys_sorted.as<uint64_t>(), keys_unique.as<uint64_t>(), n_unique_d.as<int64_t>(), (int)n_keys, st));
-        rc = tmp.alloc(std::max(bytes, bytes2));
-        if (rc != MASK_OK) return rc;
-        MASK_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tmp.p, bytes, keys.as<uint64_t>(), keys_sorted.as<uint64_t>(), (int)n_keys, 0, 64, st));
-        MASK_CUDA_TRY(cub::DeviceSelect::Unique(tmp.p, bytes2, keys_sorted.as<uint64_t>(), keys_unique.as<uint64_t>(), n_unique_d.as<int64_t>(), (int)n_keys, st));
-        MASK_CUDA_TRY(cudaMemcpyAsync(&n_edges, n_unique_d.p, 8, cudaMemcpyDeviceToHost, st));
-        MASK_CUDA_TRY(cudaStreamSynchronize(st));
-        // the sentinel (all ones) sorts last and, if present, is one unique key: drop it
-        if (n_edges > 0) {
-            uint64_t last = 0;
-            MASK_CUDA_TRY(cudaMemcpy(&last, keys_unique.as<uint64_t>() + (n_edges - 1), 8, cudaMemcpyDeviceToHost));
-            if (last == ~0ULL) n_edges--;
-        }
-    }
-    MASK_CUDA_TRY(cudaMemsetAsync(deg_b.p, 0, (size_t)M * 4, st));
-    rc = adj_b.alloc((size_t)std::max<int64_t>(n_edges, 1) * 4);
-    if (rc != MASK_OK) return rc;
-    if (n_edges > 0) {
-        const unsigned eb = (unsigned)((n_edges + 255) / 256);
-        count_sources_kernel<<<eb, 256, 0, st>>>(keys_unique.as<uint64_t>(), n_edges, deg_b.as<int32_t>());
-        split_targets_kernel<<<eb, 256, 0, st>>>(keys_unique.as<uint64_t>(), n_edges, adj_b.as<int32_t>());
-    }
-    {   // beg = exclusive scan of the degrees (64-bit), closing entry = n_edges
-        size_t bytes = 0;
-        DevBuf t2;
-        auto deg64 = cub::TransformInputIterator<int64_t, cub::CastOp<int64_t>, const int32_t*>(deg_b.as<int32_t>(), cub::CastOp<int64_t>());
-        MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, deg64, beg_b.as<int64_t>(), M, st));
-        rc = t2.alloc(bytes);
-        if (rc != MASK_OK) return rc;
-        MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(t2.p, bytes, deg64, beg_b.as<int64_t>(), M, st));
-        MASK_CUDA_TRY(cudaMemcpyAsync(beg_b.as<int64_t>() + M, &n_edges, 8, cudaMemcpyHostToDevice, st));
-        MASK_CUDA_TRY(cudaStreamSynchronize(st));
-    }
-    // rank of every node in (degree, id) order
-    DevBuf ids, starts, rank, label, flag;
-    rc = ids.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = starts.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = rank.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = label.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = flag.alloc(16);
-    if (rc != MASK_OK) return rc;
-    iota_kernel<<<node_blocks, 256, 0, st>>>(ids.as<int32_t>(), M);
-    rc = sort_rows_by<uint32_t>(deg_b.as<uint32_t>(), ids.as<int32_t>(), starts.as<int32_t>(), M, 32, st);
-    if (rc != MASK_OK) return rc;
-    scatter_rank_kernel<<<node_blocks, 256, 0, st>>>(starts.as<int32_t>(), M, rank.as<int32_t>());
-    // connected components: label = least rank in the component
-    MASK_CUDA_TRY(cudaMemcpyAsync(label.p, rank.p, (size_t)M * 4, cudaMemcpyDeviceToDevice, st));
-    for (int it = 0; it < M + 1; it++) {
-        int32_t changed = 0;
-        MASK_CUDA_TRY(cudaMemsetAsync(flag.p, 0, 4, st));
-        propagate_labels_kernel<<<row_blocks, 256, 0, st>>>(beg_b.as<int64_t>(), adj_b.as<int32_t>(), starts.as<int32_t>(), M, label.as<int32_t>(), flag.as<int32_t>());
-        MASK_CUDA_TRY(cudaMemcpyAsync(&changed, flag.p, 4, cudaMemcpyDeviceToHost, st));
-        MASK_CUDA_TRY(cudaStreamSynchronize(st));
-        if (!changed) break;
-    }
-    // breadth-first levels of all components at once, in queue order
-    DevBuf pos, parent, claimed, fa, fb, fs, counter;
-    rc = pos.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = parent.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = claimed.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = fa.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = fb.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = fs.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = counter.alloc(16);
-    if (rc != MASK_OK) return rc;
-    MASK_CUDA_TRY(cudaMemsetAsync(parent.p, 0x7f, (size_t)M * 4, st));
-    MASK_CUDA_TRY(cudaMemsetAsync(claimed.p, 0, (size_t)M * 4, st));
-    MASK_CUDA_TRY(cudaMemsetAsync(counter.p, 0, 16, st));
-    seed_frontier_kernel<<<node_blocks, 256, 0, st>>>(label.as<int32_t>(), rank.as<int32_t>(), M, fa.as<int32_t>(), counter.as<int32_t>(), pos.as<int32_t>());
-    int32_t n_front = 0;
-    MASK_CUDA_TRY(cudaMemcpyAsync(&n_front, counter.p, 4, cudaMemcpyDeviceToHost, st));
+    int32_t* deg = deg_b.as<int32_t>();
+    int32_t* flags = flag_b.as<int32_t>();   // [0] asymmetric, [1] long lists, [2] start nodes, [4..5] state of the traversal
+    MASK_CUDA_TRY(cudaMemsetAsync(flags, 0, 64, st));
+    row_lengths_kernel<<<node_blocks, 256, 0, st>>>(ptr, M, deg);
+    if (nnz > 0) check_symmetry_kernel<<<(unsigned)((nnz + 255) / 256), 256, 0, st>>>(ptr, col, M, nnz, deg, flags);
+    MASK_CUDA_TRY(cudaGetLastError());
+    MASK_CUDA_TRY(cudaMemcpyAsync(host.as<int32_t>(), flags, 4, cudaMemcpyDeviceToHost, st));
     MASK_CUDA_TRY(cudaStreamSynchronize(st));
-    // the start nodes in component order (by their rank)
-    rc = sort_rows_by<uint32_t>(rank.as<uint32_t>(), fa.as<int32_t>(), fb.as<int32_t>(), n_front, 32, st);
-    if (rc != MASK_OK) return rc;
-    int32_t* cur = fb.as<int32_t>();
-    int32_t* nxt = fa.as<int32_t>();
-    int32_t base = 0;
-    while (n_front > 0) {
-        assign_positions_kernel<<<(n_front + 255) / 256, 256, 0, st>>>(cur, n_front, base, pos.as<int32_t>());
-        MASK_CUDA_TRY(cudaMemsetAsync(counter.p, 0, 4, st));
-        expand_frontier_kernel<<<(unsigned)(((int64_t)n_front * 32 + 255) / 256), 256, 0, st>>>(
-            beg_b.as<int64_t>(), adj_b.as<int32_t>(), cur, n_front, base, pos.as<int32_t>(), parent.as<int32_t>(), claimed.as<int32_t>(), nxt,
-            counter.as<int32_t>());
-        int32_t n_next = 0;
-        MASK_CUDA_TRY(cudaMemcpyAsync(&n_next, counter.p, 4, cudaMemcpyDeviceToHost, st));
-        MASK_CUDA_TRY(cudaStreamSynchronize(st));
-        base += n_front;
-        if (n_next > 0) {   // next level in (parent position, degree, id) order: three stable passes, least significant key first
-            rc = sort_rows_by<uint32_t>(ids.as<uint32_t>(), nxt, fs.as<int32_t>(), n_next, 32, st);          // key = the id itself
-            if (rc == MASK_OK) rc = sort_rows_by<uint32_t>(deg_b.as<uint32_t>(), fs.as<int32_t>(), nxt, n_next, 32, st);
-            if (rc == MASK_OK) rc = sort_rows_by<uint32_t>(parent.as<uint32_t>(), nxt, fs.as<int32_t>(), n_next, 32, st);
-            if (rc != MASK_OK) return rc;
-            MASK_CUDA_TRY(cudaMemcpyAsync(cur == fb.as<int32_t>() ? fa.p : fb.p, fs.p, (size_t)n_next * 4, cudaMemcpyDeviceToDevice, st));
-        }
-        std::swap(cur, nxt);
-        n_front = n_next;
+    if (*host.as<int32_t>()) {
+        rc = symmetrised_pattern(rowptr, colind, M, nnz, sym_ptr, sym_adj, &n_edges, st);
+        if (rc != MASK_OK) return rc;
+        ptr = sym_ptr.as<int32_t>();
+        col = sym_adj.as<int32_t>();
+        row_lengths_kernel<<<node_blocks, 256, 0, st>>>(ptr, M, deg);
+        MASK_CUDA_TRY(cudaGetLastError());
     }
-    if (base != M) return fail(MASK_ERR_INVALID_ARGUMENT, "row_rcm: the traversal did not reach every row");
+    // node arrays, one allocation
+    const size_t row_words = ((size_t)M + 1 + 63) & ~(size_t)63;
+    enum { kIds, kStarts, kSortedDeg, kOutPtr, kRank, kLabel, kQueue, kPos, kParent, kChildren, kKey, kKeyOut, kRow, kLong, kArrays };
+    DevScratch nodes, adj_b, tmp;
+    rc = nodes.alloc(row_words * kArrays * 4, st);
+    if (rc == MASK_OK) rc = adj_b.alloc((size_t)std::max<int64_t>(n_edges, 1) * 4, st);
+    if (rc != MASK_OK) return rc;
+    auto arr = [&](int which) { return nodes.as<int32_t>(row_words * which * 4); };
+    uint32_t *udeg = reinterpret_cast<uint32_t*>(deg), *usorted = reinterpret_cast<uint32_t*>(arr(kSortedDeg));
+    uint32_t *key = reinterpret_cast<uint32_t*>(arr(kKey)), *key_out = reinterpret_cast<uint32_t*>(arr(kKeyOut));
+    const int bits = bits_for((int64_t)M + 1);
+    cub::CountingInputIterator<int> counting(0);
+    size_t b1 = 0, b2 = 0, b3 = 0;
+    MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, b1, udeg, usorted, arr(kIds), arr(kStarts), M, 0, bits, st));
+    MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, b2, arr(kSortedDeg), arr(kOutPtr), M + 1, st));
+    MASK_CUDA_TRY(cub::DeviceSelect::If(nullptr, b3, counting, arr(kQueue), flags + 2, M, IsRoot{arr(kLabel)}, st));
+    rc = tmp.alloc(std::max(b1, std::max(b2, b3)), st);
+    if (rc != MASK_OK) return rc;
+    // ranks in (degree, id) order, adjacency in ranks
+    iota_kernel<<<node_blocks, 256, 0, st>>>(arr(kIds), M);
+    MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, b1, udeg, usorted, arr(kIds), arr(kStarts), M, 0, bits, st));
+    scatter_rank_kernel<<<node_blocks, 256, 0, st>>>(arr(kStarts), M, arr(kRank), arr(kLabel));
+    MASK_CUDA_TRY(cudaMemsetAsync(arr(kSortedDeg) + M, 0, 4, st));
+    MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, b2, arr(kSortedDeg), arr(kOutPtr), M + 1, st));
+    int32_t* adj = adj_b.as<int32_t>();
+    sort_adjacency_kernel<<<(unsigned)(((int64_t)M * 32 + 127) / 128), 128, 0, st>>>(ptr, col, M, arr(kStarts), arr(kRank), arr(kOutPtr), adj,
+                                                                                  arr(kLong), flags + 1);
+    MASK_CUDA_TRY(cudaGetLastError());
+    if (n_edges > kAdjSortMax) {
+        constexpr int kSmem = kLongBits / 8 + kLongBits / 16;
+        MASK_CUDA_TRY(cudaFuncSetAttribute(sort_long_adjacency_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        const int64_t most = std::min<int64_t>(n_edges / kAdjSortMax, 2 * sm_count());
+        sort_long_adjacency_kernel<<<(unsigned)most, 512, kSmem, st>>>(ptr, col, M, arr(kStarts), arr(kRank), arr(kOutPtr), adj, arr(kLong), flags + 1);
+        MASK_CUDA_TRY(cudaGetLastError());
+    }
+    // components; their least ranks, ascending, begin the queue
+    if (n_edges > 0) hook_kernel<<<(unsigned)((n_edges + 255) / 256), 256, 0, st>>>(arr(kOutPtr), adj, M, arr(kLabel));
+    flatten_labels_kernel<<<node_blocks, 256, 0, st>>>(arr(kLabel), M);
+    MASK_CUDA_TRY(cudaGetLastError());
+    MASK_CUDA_TRY(cub::DeviceSelect::If(tmp.p, b3, counting, arr(kQueue), flags + 2, M, IsRoot{arr(kLabel)}, st));
+    MASK_CUDA_TRY(cudaMemsetAsync(arr(kPos), 0xff, (size_t)M * 4, st));
+    MASK_CUDA_TRY(cudaMemsetAsync(arr(kParent), 0x7f, (size_t)M * 4, st));
+    BfsArgs a{arr(kOutPtr), adj, arr(kQueue), arr(kPos), arr(kParent), arr(kChildren), arr(kRow), flags + 4, flags + 2, M};
+    // block sums: one word per block, in an array that is not used yet
+    const unsigned blocks = (unsigned)std::min<int64_t>(sm_count(), ((int64_t)M + kBfsWarps - 1) / kBfsWarps);
+    void* args[] = {&a};
+    MASK_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(bfs_kernel), dim3(blocks), dim3(kBfsThreads), args, 0, st));
+    MASK_CUDA_TRY(cudaMemcpyAsync(host.as<int32_t>(), flags + 4, 4, cudaMemcpyDeviceToHost, st));
     // components by the rank of their start, each in reversed queue order
-    DevBuf fk, fk2, tmp2;
-    rc = fk.alloc((size_t)M * 8);
-    if (rc == MASK_OK) rc = fk2.alloc((size_t)M * 8);
-    if (rc != MASK_OK) return rc;
-    final_keys_kernel<<<node_blocks, 256, 0, st>>>(label.as<int32_t>(), pos.as<int32_t>(), M, fk.as<uint64_t>(), ids.as<int32_t>());
-    size_t bytes = 0;
-    MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, bytes, fk.as<uint64_t>(), fk2.as<uint64_t>(), ids.as<int32_t>(), order, M, 0, 64, st));
-    rc = tmp2.alloc(bytes);
-    if (rc != MASK_OK) return rc;
-    MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp2.p, bytes, fk.as<uint64_t>(), fk2.as<uint64_t>(), ids.as<int32_t>(), order, M, 0, 64, st));
+    reversed_queue_kernel<<<node_blocks, 256, 0, st>>>(arr(kQueue), arr(kLabel), arr(kStarts), M, key, arr(kRow));
+    MASK_CUDA_TRY(cudaGetLastError());
+    MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, b1, key, key_out, arr(kRow), order, M, 0, bits, st));
     MASK_CUDA_TRY(cudaStreamSynchronize(st));
+    if (*host.as<int32_t>() != M) return fail(MASK_ERR_INVALID_ARGUMENT, "row_rcm: the traversal did not reach every row");
     return MASK_OK;
 }
 
 }  // namespace
 
 // ---- device: gather the rows of a CSR matrix in a given order ------------------------------------
-__global__ void permuted_row_lengths_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ order, int32_t M,
-                                            int32_t* __restrict__ len) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < M) { const int r = order[i]; len[i] = rowptr[r + 1] - rowptr[r]; }
-}
+struct PermutedLength {
+    const int32_t* rowptr;
+    const int32_t* order;
+    __device__ int32_t operator()(int32_t i) const { const int r = order[i]; return rowptr[r + 1] - rowptr[r]; }
+};
 // one warp per new row copies its entries
 __global__ void gather_rows_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
                                    const float* __restrict__ values, const int32_t* __restrict__ order,
@@ -399,35 +737,6 @@ __global__ void gather_rows_kernel(const int32_t* __restrict__ rowptr, const int
         colind_out[dst + j] = colind[src + j];
         values_out[dst + j] = values[src + j];
     }
-}
-// single-block exclusive scan of M lengths (row counts are small next to the entry counts the
-// format builder scans; 4 M rows take well under a millisecond)
-__global__ void __launch_bounds__(1024) scan_lengths_kernel(const int32_t* __restrict__ len, int32_t M, int32_t* __restrict__ rowptr_out) {
-    __shared__ int64_t warp_tot[32];
-    __shared__ int64_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int base = 0; base < M; base += 1024) {
-        const int idx = base + threadIdx.x;
-        const int64_t v = idx < M ? len[idx] : 0;
-        int64_t x = v;
-        for (int o = 1; o < 32; o <<= 1) { const int64_t y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
-        if (lane == 31) warp_tot[wid] = x;
-        __syncthreads();
-        if (wid == 0) {
-            int64_t w = warp_tot[lane];
-            for (int o = 1; o < 32; o <<= 1) { const int64_t y = __shfl_up_sync(0xffffffffu, w, o); if (lane >= o) w += y; }
-            warp_tot[lane] = w;
-        }
-        __syncthreads();
-        const int64_t before = carry + (wid > 0 ? warp_tot[wid - 1] : 0);
-        if (idx < M) rowptr_out[idx] = (int32_t)(before + x - v);
-        __syncthreads();
-        if (threadIdx.x == 0) carry += warp_tot[31];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) rowptr_out[M] = (int32_t)carry;
 }
 
 }  // namespace mask
@@ -445,31 +754,34 @@ extern "C" int mask_reorder_rows(int kind, const int32_t* d_rowptr, const int32_
     }
     MASK_REQUIRE(kind == MASK_REORDER_ROW_RCM || kind == MASK_REORDER_FIRST_COL_SORT || kind == MASK_REORDER_JACCARD_GREEDY,
                  "unknown reorder kind");
-    int32_t nnz32 = 0;
-    MASK_CUDA_TRY(cudaMemcpyAsync(&nnz32, d_rowptr + M, 4, cudaMemcpyDeviceToHost, st));
+    HostStage host;
+    int rc = host.get(4);
+    if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(cudaMemcpyAsync(host.as<int32_t>(), d_rowptr + M, 4, cudaMemcpyDeviceToHost, st));
     MASK_CUDA_TRY(cudaStreamSynchronize(st));
+    const int32_t nnz32 = *host.as<int32_t>();
     MASK_REQUIRE(nnz32 == 0 || d_colind, "colind is NULL");
     if (kind == MASK_REORDER_ROW_RCM) {
         if (M != K) return fail(MASK_ERR_INVALID_ARGUMENT, "row_rcm needs a square matrix");
         return order_rcm_device(d_rowptr, d_colind, M, nnz32, d_row_order, st);
     }
-    DevBuf first, sig, ids, by_first;
-    int rc = first.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = sig.alloc((size_t)M * 8);
-    if (rc == MASK_OK) rc = ids.alloc((size_t)M * 4);
-    if (rc == MASK_OK) rc = by_first.alloc((size_t)M * 4);
+    DevScratch first, sig, ids, by_first;
+    rc = first.alloc((size_t)M * 4, st);
+    if (rc == MASK_OK) rc = sig.alloc((size_t)M * 8, st);
+    if (rc == MASK_OK) rc = ids.alloc((size_t)M * 4, st);
+    if (rc == MASK_OK) rc = by_first.alloc((size_t)M * 4, st);
     if (rc != MASK_OK) return rc;
     row_keys_kernel<<<row_blocks, 256, 0, st>>>(d_rowptr, d_colind, M, K, first.as<uint32_t>(), sig.as<uint64_t>());
     iota_kernel<<<node_blocks, 256, 0, st>>>(ids.as<int32_t>(), M);
     MASK_CUDA_TRY(cudaGetLastError());
-    if (kind == MASK_REORDER_FIRST_COL_SORT) return sort_rows_by<uint32_t>(first.as<uint32_t>(), ids.as<int32_t>(), d_row_order, M, 32, st);
+    const int col_bits = bits_for((int64_t)K + 1);   // K stands for "no column"
+    if (kind == MASK_REORDER_FIRST_COL_SORT) return sort_rows_by<uint32_t>(first.as<uint32_t>(), ids.as<int32_t>(), d_row_order, M, col_bits, st);
     // (signature, first column, id): stable by first column, then stable by signature
-    rc = sort_rows_by<uint32_t>(first.as<uint32_t>(), ids.as<int32_t>(), by_first.as<int32_t>(), M, 32, st);
+    rc = sort_rows_by<uint32_t>(first.as<uint32_t>(), ids.as<int32_t>(), by_first.as<int32_t>(), M, col_bits, st);
     if (rc == MASK_OK) rc = sort_rows_by<uint64_t>(sig.as<uint64_t>(), by_first.as<int32_t>(), ids.as<int32_t>(), M, 64, st);
     if (rc != MASK_OK) return rc;
     jaccard_chain_kernel<<<(unsigned)((M + 63) / 64), 256, 0, st>>>(d_rowptr, d_colind, ids.as<int32_t>(), M, d_row_order);
     MASK_CUDA_TRY(cudaGetLastError());
-    MASK_CUDA_TRY(cudaStreamSynchronize(st));   // the scratch goes away with this frame
     return MASK_OK;
 }
 
@@ -479,13 +791,15 @@ extern "C" int mask_csr_permute_rows(const int32_t* d_rowptr, const int32_t* d_c
     using namespace mask;
     MASK_REQUIRE(d_rowptr && d_row_order && d_rowptr_out && M >= 1, "bad arguments");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // row lengths in the new order go to rowptr_out[1..M] first, then are scanned in place
-    permuted_row_lengths_kernel<<<(M + 255) / 256, 256, 0, st>>>(d_rowptr, d_row_order, M, d_rowptr_out + 1);
-    MASK_CUDA_TRY(cudaGetLastError());
-    // in place: the scan reads len[i] = rowptr_out[i+1] into registers before a block barrier and
-    // writes rowptr_out[i] after it; later chunks only read positions no earlier chunk has written
-    scan_lengths_kernel<<<1, 1024, 0, st>>>(d_rowptr_out + 1, M, d_rowptr_out);
-    MASK_CUDA_TRY(cudaGetLastError());
+    cub::TransformInputIterator<int32_t, PermutedLength, cub::CountingInputIterator<int32_t>> lengths(
+        cub::CountingInputIterator<int32_t>(0), PermutedLength{d_rowptr, d_row_order});
+    size_t bytes = 0;
+    MASK_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, bytes, lengths, d_rowptr_out + 1, M, st));
+    DevScratch tmp;
+    int rc = tmp.alloc(bytes, st);
+    if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp.p, bytes, lengths, d_rowptr_out + 1, M, st));
+    MASK_CUDA_TRY(cudaMemsetAsync(d_rowptr_out, 0, 4, st));
     if (d_colind && d_values && d_colind_out && d_values_out) {
         gather_rows_kernel<<<(unsigned)(((int64_t)M * 32 + 255) / 256), 256, 0, st>>>(d_rowptr, d_colind, d_values, d_row_order,
                                                                                    d_rowptr_out, M, d_colind_out, d_values_out);
