@@ -68,11 +68,15 @@ static void multi_bind(const int32_t* soff, int32_t W, std::vector<int32_t>& tas
 // no long chain of tiles is left at the end.  Not below kMinPiece, where filling a block's pipeline costs more
 // than the balance gains, and not below the mean window: cutting every window adds a partial tile and a fix-up
 // for each (uniform 4096-node matrix, 42 tiles a window, N = 512: 23 us whole, 29 us in three pieces).
+// With very many tiles the pieces get longer again: the partial tiles are then what counts (2^22-node power-law
+// graph, 15 M tiles, N = 512: pieces of 128 tiles write and read 5.6 GB of them, pieces of 512 0.6 GB).
 constexpr int32_t kMinPiece = 16;
 constexpr int32_t kWarpBlocksPerSm = 15;
+constexpr int64_t kManyTiles = 30000;
 static int32_t default_piece_tiles(int64_t T, int32_t W) {
     const int64_t resident = (int64_t)sm_count() * kWarpBlocksPerSm;
     const int64_t piece = std::max<int64_t>((T + resident - 1) / resident, (T + W - 1) / W);
+    if (T > 128 * kManyTiles) return (int32_t)std::min<int64_t>(512, T / kManyTiles);
     return (int32_t)std::max<int64_t>(kMinPiece, std::min<int64_t>(128, piece));
 }
 
@@ -182,23 +186,35 @@ static void build_tables(mask_plan& p, const int32_t* soff) {
     p.F = (int64_t)fw.size();
     p.G = (int64_t)go.size() - 1;
 
-    // groups of the warp-level kernel: the same fragments, dealt out in shorter runs where the plan's own
-    // groups are longer than a piece
+}
+
+// Groups of the warp-level kernel: the same fragments in shorter runs, closed before their cost passes 5/4 of a
+// target.  Two reasons to keep them short.  Balance: 15 x 148 blocks are resident, and with 1.4 times as many
+// groups the second round is half empty; a target of half a resident warp's share leaves more and smaller ones
+// (100 000 rows, 20 tiles a window, N = 64: one window a group 35 us, two 41 us).  Locality: what the resident
+// warps touch together should stay in L2; where windows share rows of B with their neighbours, a window a
+// group keeps the band narrow (27-point stencil with 10^6 rows, N = 128: 517 us, with 128 tiles a group 585 us).
+// Not shorter than that: on a power-law graph half the windows hold a few tiles, and a block's start costs
+// about three tiles' time (130 000 nodes, N = 48: 16 tiles a group 78 us, 64 tiles 72 us).
+static void build_warp_groups(mask_plan& p) {
     p.h_warp_off.clear();
-    if (p.policy == MASK_POLICY_AUTO && p.piece_tiles < G) {
-        constexpr int32_t kFragCost = 4;
-        int32_t load = 0;
-        p.h_warp_off.push_back(0);
-        for (int64_t f = 0; f < p.F; f++) {
-            const int32_t cost = fo[f + 1] - fo[f] + kFragCost;
-            if (load > 0 && load + cost > p.piece_tiles + p.piece_tiles / 4) {
-                p.h_warp_off.push_back((int32_t)f);
-                load = 0;
-            }
-            load += cost;
+    if (p.policy != MASK_POLICY_AUTO || !p.auto_groups) return;   // the plan's own groups
+    const int64_t share = p.T / ((int64_t)sm_count() * kWarpBlocksPerSm * 2);
+    const int32_t target = p.local ? kMinPiece : (int32_t)std::max<int64_t>(kMinPiece, std::min<int64_t>(128, share));
+    constexpr int32_t kFragCost = 4;
+    const auto& fo = p.h_frag_off;
+    int32_t load = 0;
+    p.h_warp_off.reserve((size_t)p.F + 1);
+    p.h_warp_off.push_back(0);
+    for (int64_t f = 0; f < p.F; f++) {
+        const int32_t cost = fo[f + 1] - fo[f] + kFragCost;
+        if (load > 0 && load + cost > target + target / 4) {
+            p.h_warp_off.push_back((int32_t)f);
+            load = 0;
         }
-        if (p.F > 0) p.h_warp_off.push_back((int32_t)p.F);
+        load += cost;
     }
+    if (p.F > 0) p.h_warp_off.push_back((int32_t)p.F);
 }
 
 // One device array for all tables, filled by one copy: sections start on 16-byte boundaries.
@@ -296,7 +312,9 @@ static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int
     p->T = T;
     p->policy = policy;
     p->group_tiles = group_tiles > 0 ? group_tiles : (policy == MASK_POLICY_STRICT_LB ? 64 : default_group_tiles(T));
-    p->piece_tiles = (group_tiles > 0 || policy != MASK_POLICY_AUTO) ? p->group_tiles : std::min(p->group_tiles, default_piece_tiles(T, p->W));
+    p->auto_groups = group_tiles <= 0;
+    // a piece may be longer than a group: it then is a group of its own
+    p->piece_tiles = (group_tiles > 0 || policy != MASK_POLICY_AUTO) ? p->group_tiles : default_piece_tiles(T, p->W);
     HostStage stage;
     ColumnStatsJob job;
     cudaEvent_t have_soff = nullptr;
@@ -324,16 +342,17 @@ static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int
             if (group_tiles <= 0) p->group_tiles = 64;
         }
         build_tables(*p, soff);
+        if (d_val_sidx) {
+            MASK_CUDA_TRY(cudaStreamSynchronize(st));
+            mask_column_features f;
+            job.finish(&f);
+            choose_plan_parameters(p, f);
+        }
+        build_warp_groups(*p);
         return upload_tables(*p, soff, st);
     };
     const int rc = body();
-    if (rc != MASK_OK) {
-        cudaStreamSynchronize(st);   // copies into the staging buffers may be in flight
-    } else if (d_val_sidx) {
-        mask_column_features f;
-        job.finish(&f);
-        choose_plan_parameters(p, f);
-    }
+    if (rc != MASK_OK) cudaStreamSynchronize(st);   // copies into the staging buffers may be in flight
     if (have_soff) cudaEventDestroy(have_soff);
     if (rc != MASK_OK) {
         mask_plan_destroy(p);

@@ -150,7 +150,8 @@ int launch_spmm_sweep(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st,
 bool spmm_tma_applies(const mask_plan* plan, const SpmmArgs& a);
 int launch_spmm_tma(const mask_plan* plan, const SpmmArgs& a, int64_t K, cudaStream_t st, int nslab);
 
-// spmm_async.cu: shared-memory ring variant (SR-BCRS).  nq / stages 0 = defaults.
-int launch_spmm_async(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st, int nq, int stages);
+// spmm_warp.cu: one warp per block, every encoding.  nq = 32-column groups per warp (1..4; 0 = by N).
+template <int FMT>
+int launch_spmm_warp(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st, int nq);
 
 }  // namespace mask

@@ -38,10 +38,8 @@ namespace mask {
 // Development knobs (mask_tune): 0 = library default.
 static int g_tune_nq = 0;
 static int g_tune_min_blocks = 0;
-static int g_tune_async = 1;   // 1 = shared-memory ring fed by cp.async (SR-BCRS), 0 = register pipeline
-static int g_tune_stages = 0;
+static int g_tune_async = 1;   // 1 = warp-level kernel of spmm_warp.cu, 0 = register pipeline (below)
 extern int g_session_chunk_cols;      // api.cu: column chunks of the host-buffer pipeline
-constexpr int kNarrowN = 80;   // below: the warp-level ring kernel (see launch_spmm)
 static int g_tune_sweep = 1;   // 1 = persistent tcgen05 kernel except where the warp-level one measures faster, 2 = always, 0 = warp-level kernels only
 static int g_tune_nslab = 0;   // persistent kernel: 128-column slabs per column block (0 = the plan's choice)
 static int g_tune_tma = 0;     // 1 = the TMA-fed kernel where the plan holds rounded tile values (spmm_tma.cu); measured slower, off by default
@@ -316,6 +314,45 @@ static int launch_fixup(const mask_plan* plan, const SpmmArgs& a, cudaStream_t s
     return MASK_OK;
 }
 
+// 128-column slabs per column block of the persistent kernel for an N-column product
+static int sweep_slabs(const mask_plan* plan, int N) {
+    int nslab = g_tune_nslab != 0 ? g_tune_nslab : plan->nslab;
+    const int fills = N > 256 ? 4 : (N > 128 ? 2 : 1);
+    if (nslab != 1 && nslab != 2 && nslab != 4) nslab = fills;
+    return nslab < fills ? nslab : fills;
+}
+
+// Which kernel: one warp per block (spmm_warp.cu) or the persistent tcgen05 kernel (spmm_sweep.cu).  The tcgen05
+// kernel takes up to 512 columns of a tile at once: tile values and ids are read once and every gathered byte goes
+// through shared memory once to and once from, so it wins where full-width rows are gathered at the L2's or
+// shared memory's rate.  The warp kernel takes 128 columns at a time, has no minimum width, spreads small
+// matrices over 2220 blocks instead of 296, and re-reads the tiles once per 128 columns.  Measured (us, tcgen05 /
+// warp; power-law graphs of 20 000 / 300 000 / 2^20 / 2^22 nodes, stencils of 40^3 / 100^3, uniform 10^5 / 2 10^5 rows):
+//   N = 16     39 / 18,   172 / 98,   -,           -,               41 / 18,   -,           45 / 25,   -
+//   N = 128    41 / 23,   283 / 216,  1020 / 870,  -,               48 / 37,   586 / 517,   64 / 60,   132 / 136
+//   N = 192    47 / 31,   -,          1498 / 1362, -,               68 / 57,   880 / 929,   94 / 95,   206 / 209
+//   N = 256    47 / 36,   416 / 424,  1688 / 1681, -,               67 / 70,   945 / 1145,  108 / 116, 266 / 265
+//   N = 512    70 / 59,   798 / 813,  3363 / 3338, 28 500 / 26 900, 115 / 131, 1800 / 2050, 253 / 221, 599 / 512
+static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, bool sidx_aligned) {
+    if (tf32x3) return true;                    // compensated products: the warp kernel only
+    if (!sidx_aligned || g_tune_sweep == 2) return false;
+    if (g_tune_async == 0) return false;
+    if (g_tune_sweep == 0) return true;
+    if (g_tune_tma != 0 && fmt == kFmtSrbcrs && plan->d_vals_tf32 != nullptr) return false;
+    // a handful of long groups: one warp takes half a microsecond per tile, a tcgen05 block a quarter of that
+    if (plan->Gw < 4 * sm_count() && plan->T > 24 * plan->Gw) return false;
+    const int64_t slabs = (N + 127) / 128;
+    if (N <= 128)   // a bitmap tile costs the warp kernel more to expand, and unaligned rows two passes a quarter-warp
+        return !(fmt == kFmtMco && N > 96 && N < 128 && !plan->hub_heavy && !plan->local);
+    if (plan->T * slabs <= (fmt == kFmtMco ? 100000 : 150000)) return true;   // too little work for long-lived blocks
+    if (fmt == kFmtMco) return false;
+    if (plan->far_beyond_l2 && fmt == kFmtSrbcrs) return true;   // narrower rows of B: more of the hubs stay in L2
+    if (plan->slab_fits && N > 256) return true;
+    // columns that the tcgen05 kernel's blocks would only pad: a quarter of N and more
+    const int64_t block = 128 * sweep_slabs(plan, N), padded = (N + block - 1) / block * block;
+    return !plan->local && 4 * padded >= 5 * (int64_t)N;
+}
+
 template <int FMT>
 static int launch_spmm(const mask_plan* plan, SpmmArgs a, cudaStream_t st) {
     if (plan->G == 0) return MASK_OK;
@@ -326,38 +363,22 @@ static int launch_spmm(const mask_plan* plan, SpmmArgs a, cudaStream_t st) {
     a.row_map = plan->d_row_map;
     a.peer_out = plan->d_peer_out;
     a.n_peer_out = plan->n_peer_out;
-    // columns per warp: wide slabs (fewer re-reads of the tile values per column) when N fills
-    // four warps of them, else narrower slabs so that small N still spreads over a block
     const int N = a.N;
-    constexpr bool METCF = FMT != kFmtSrbcrs;   // the COO and bitmap leaves take the same routes
-    if (FMT == kFmtSrbcrs && a.tf32x3) {   // compensated products: mma.sync ring kernel
-        int rc = launch_spmm_async(plan, a, st, 0, 0);
-        if (rc != MASK_OK) return rc;
-        return launch_fixup(plan, a, st);
-    }
-    // Narrow products: below about 80 columns a tile's one mostly empty 128-column MMA costs more than
-    // the warp-level MMAs of the shared-memory ring kernel (measured on a 2^22-node power-law graph:
-    // N = 64 5.33 against 6.33 ms, N = 80 6.57 against 6.48 ms, N = 128 6.8 ms for the tcgen05 kernel).
-    if (FMT == kFmtSrbcrs && g_tune_sweep == 1 && N < kNarrowN && g_tune_async != 0) {
-        int rc = launch_spmm_async(plan, a, st, g_tune_nq, g_tune_stages);
-        if (rc != MASK_OK) return rc;
-        return launch_fixup(plan, a, st);
+    int rc;
+    if (use_warp_kernel(plan, FMT, N, a.tf32x3, (reinterpret_cast<uintptr_t>(a.val_sidx) & 15) == 0)) {
+        rc = launch_spmm_warp<FMT>(plan, a, st, g_tune_nq);
+        return rc != MASK_OK ? rc : launch_fixup(plan, a, st);
     }
     if (g_tune_sweep != 0 && g_tune_tma != 0 && FMT == kFmtSrbcrs && spmm_tma_applies(plan, a)) {
-        int rc = launch_spmm_tma(plan, a, a.K, st, g_tune_nslab != 0 ? g_tune_nslab : plan->nslab);
-        if (rc != MASK_OK) return rc;
-        return launch_fixup(plan, a, st);
+        rc = launch_spmm_tma(plan, a, a.K, st, g_tune_nslab != 0 ? g_tune_nslab : plan->nslab);
+        return rc != MASK_OK ? rc : launch_fixup(plan, a, st);
     }
     if (g_tune_sweep != 0) {
-        int rc = launch_spmm_sweep(plan, a, st, g_tune_nslab != 0 ? g_tune_nslab : plan->nslab);
-        if (rc != MASK_OK) return rc;
-        return launch_fixup(plan, a, st);
+        rc = launch_spmm_sweep(plan, a, st, g_tune_nslab != 0 ? g_tune_nslab : plan->nslab);
+        return rc != MASK_OK ? rc : launch_fixup(plan, a, st);
     }
-    if (!METCF && g_tune_async != 0) {
-        int rc = launch_spmm_async(plan, a, st, g_tune_nq, g_tune_stages);
-        if (rc != MASK_OK) return rc;
-        return launch_fixup(plan, a, st);
-    }
+    // columns per warp: wide slabs (fewer re-reads of the tile values per column) when N fills
+    // four warps of them, else narrower slabs so that small N still spreads over a block
     int nq = N > 256 ? 4 : (N > 128 ? 2 : 1);
     if (g_tune_nq == 1 || g_tune_nq == 2 || g_tune_nq == 4) nq = g_tune_nq;
     const int cols_per_block = 32 * nq * kWarpsPerBlock;
@@ -401,24 +422,19 @@ static int check_common(const mask_plan* plan, int32_t M, int32_t K, int32_t N, 
 
 }  // namespace mask
 
-extern "C" int mask_kernel_revision(void) { return 4; }
+extern "C" int mask_kernel_revision(void) { return 5; }
 
 extern "C" int mask_spmm_kernel_name(const mask_plan* plan, int format, int32_t N, int epilogue, char* out, size_t capacity) {
     using namespace mask;
     MASK_REQUIRE(plan != nullptr && out != nullptr && capacity > 0, "NULL argument");
     MASK_REQUIRE(format >= kFmtSrbcrs && format <= kFmtMco && N > 0, "bad format or N");
     static const char* const fmt_name[] = {"srbcrs", "metcf", "mco"};
-    if (format == kFmtSrbcrs && (epilogue & MASK_NUMERICS_TF32X3)) {
-        snprintf(out, capacity, "spmm_async_kernel<tf32x3>");
-    } else if (format == kFmtSrbcrs && g_tune_sweep == 1 && N < kNarrowN && g_tune_async != 0) {
-        snprintf(out, capacity, "spmm_async_kernel<%s>", fmt_name[format]);
+    const bool tf32x3 = format == kFmtSrbcrs && (epilogue & MASK_NUMERICS_TF32X3);
+    if (use_warp_kernel(plan, format, N, tf32x3, true)) {
+        snprintf(out, capacity, "spmm_warp_kernel<%s>", tf32x3 ? "tf32x3" : fmt_name[format]);
     } else if (g_tune_sweep != 0) {
-        int nslab = g_tune_nslab != 0 ? g_tune_nslab : plan->nslab;
-        const int fills = N > 256 ? 4 : (N > 128 ? 2 : 1);
-        if (nslab != 1 && nslab != 2 && nslab != 4) nslab = fills;
-        nslab = nslab < fills ? nslab : fills;
         const bool tma = g_tune_tma != 0 && format == kFmtSrbcrs && plan->d_vals_tf32 != nullptr;
-        snprintf(out, capacity, "%s<nslab=%d,%s>", tma ? "spmm_tma_kernel" : "spmm_sweep_kernel", nslab, fmt_name[format]);
+        snprintf(out, capacity, "%s<nslab=%d,%s>", tma ? "spmm_tma_kernel" : "spmm_sweep_kernel", sweep_slabs(plan, N), fmt_name[format]);
     } else {
         snprintf(out, capacity, "legacy routing (mask_tune sweep=0), %s", fmt_name[format]);
     }
@@ -431,7 +447,7 @@ extern "C" int mask_tune(const char* name, int value) {
     if (!strcmp(name, "nq")) g_tune_nq = value;
     else if (!strcmp(name, "min_blocks")) g_tune_min_blocks = value;
     else if (!strcmp(name, "async")) g_tune_async = value;
-    else if (!strcmp(name, "stages")) g_tune_stages = value;
+    else if (!strcmp(name, "stages")) {}   // the ring depth is fixed
     else if (!strcmp(name, "sweep")) g_tune_sweep = value;
     else if (!strcmp(name, "nslab")) g_tune_nslab = value;
     else if (!strcmp(name, "tma")) g_tune_tma = value;
