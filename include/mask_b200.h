@@ -334,6 +334,25 @@ int mask_spmm_mco(const mask_plan* plan, const int32_t* d_val_soff, const int32_
                   int64_t ldb, float* d_C, int64_t ldc, void* d_scratch, size_t scratch_bytes,
                   int epilogue, void* stream);
 
+/* A packed matrix as one argument: format 0 SR-BCRS (values = val_block_val), 1 ME-TCF (offsets =
+ * val_coo_off, index = val_coo_idx, values = val_coo_val), 2 MCO (offsets = val_mco_off, index =
+ * val_mco_mask, values = val_mco_val).  The arrays are the caller's. */
+typedef struct mask_matrix {
+    int32_t format, M, K, reserved;
+    const int32_t* val_sidx;
+    const int32_t* offsets;
+    const void* index;
+    const void* values;
+} mask_matrix;
+
+/* The product of any of the encodings, for any n, ldb >= n, ldc >= n and alignment of B and C (of float).
+ * Where n % 4, ldb % 4 or the alignment of B rules out 16-byte rows, B is first copied to d_pad
+ * (K * (n rounded up to 4) floats, 16-byte aligned; otherwise it may be NULL).  Scratch as for n rounded
+ * up to 4 columns (mask_plan_scratch_bytes).  C is written in place, whatever its row length. */
+int mask_spmm(const mask_plan* plan, const mask_matrix* matrix, int32_t n, const float* d_B, int64_t ldb,
+              float* d_C, int64_t ldc, float* d_pad, void* d_scratch, size_t scratch_bytes, int epilogue,
+              void* stream);
+
 /* SR-BCRS SpMM for callers that are not allowed to allocate device memory -- a process whose
  * whole device heap belongs to an arena of its own (an inference server, an engine that loads this
  * library as a plug-in) or a loop that cannot afford the device-wide synchronisation of

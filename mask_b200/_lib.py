@@ -55,6 +55,7 @@ SIGNATURES = {
     "mask_spmm_srbcrs": (C.c_int, [vp, vp, vp, vp, i32, i32, i32, vp, i64, vp, i64, vp, sz, C.c_int, vp]),
     "mask_spmm_metcf": (C.c_int, [vp, vp, vp, vp, vp, vp, i32, i32, i32, vp, i64, vp, i64, vp, sz, C.c_int, vp]),
     "mask_spmm_mco": (C.c_int, [vp, vp, vp, vp, vp, vp, i32, i32, i32, vp, i64, vp, i64, vp, sz, C.c_int, vp]),
+    "mask_spmm": (C.c_int, [vp, vp, i32, vp, i64, vp, i64, vp, vp, sz, C.c_int, vp]),
     "mask_static_scratch_capacity": (sz, []),
     "mask_spmm_srbcrs_static_scratch": (C.c_int, [vp, vp, vp, vp, i32, i32, i32, vp, i64, vp, i64, C.c_int, vp]),
     "mask_tune": (C.c_int, [C.c_char_p, C.c_int]),
@@ -70,6 +71,11 @@ SIGNATURES = {
 
 REORDER = {"none": 0, "row_rcm": 1, "first_col_sort": 2, "jaccard_greedy": 3}
 POLICY = {"auto": 0, "row": 1, "strict_lb": 2, "multi_bind": 3, "ref_auto": 4}
+
+
+class Matrix(C.Structure):
+    """mask_matrix"""
+    _fields_ = [("format", i32), ("M", i32), ("K", i32), ("reserved", i32), ("val_sidx", vp), ("offsets", vp), ("index", vp), ("values", vp)]
 
 
 class Features(C.Structure):

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
@@ -43,12 +44,30 @@ __host__ __device__ inline int sw223(int i) { return i ^ (((i >> 5) & 3) << 2); 
 // Swizzle<1,2,3> over the same tile (ME-TCF COO index).
 __host__ __device__ inline int sw123(int i) { return i ^ (((i >> 5) & 1) << 2); }
 
+constexpr int kMaxDevices = 64;
+
 inline int sm_count() {
+    static std::atomic<int> known[kMaxDevices];   // asked for once per device
     int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (dev >= 0 && dev < kMaxDevices && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
         return 148;
+    if (dev >= 0 && dev < kMaxDevices) known[dev].store(n, std::memory_order_relaxed);
     return n;
+}
+
+// Opts a kernel in to `bytes` of dynamic shared memory and the largest carveout, once per device.  `done` is the
+// caller's, one bit per device and kernel (setting an attribute again does no harm).
+inline int opt_in_shared_memory(const void* kernel, int bytes, std::atomic<uint64_t>& done) {
+    int dev = 0;
+    MASK_CUDA_TRY(cudaGetDevice(&dev));
+    const uint64_t bit = dev >= 0 && dev < 64 ? (uint64_t)1 << dev : 0;
+    if (done.load(std::memory_order_acquire) & bit) return MASK_OK;
+    MASK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    MASK_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    done.fetch_or(bit, std::memory_order_release);
+    return MASK_OK;
 }
 
 }  // namespace mask

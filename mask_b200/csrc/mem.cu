@@ -10,7 +10,6 @@ namespace mask {
 
 namespace {
 
-constexpr int kMaxDevices = 64;
 std::mutex g_pool_mu;
 cudaMemPool_t g_pool[kMaxDevices] = {};
 

@@ -31,7 +31,9 @@ struct SpmmArgs {
     float* scratch;
     int32_t M;
     int32_t K;
-    int32_t N;
+    int32_t N;               // columns that are multiplied (a multiple of 4); B and the scratch tiles have them all
+    int32_t n_out;           // columns of C that are written: N, or up to 3 fewer
+    int32_t vec_out;         // rows of C can be written 16 bytes at a time
     int32_t relu;
     int32_t tf32x3;  // compensated products (MASK_NUMERICS_TF32X3)
 };
@@ -122,6 +124,13 @@ __device__ __forceinline__ void flush_fragment(const SpmmArgs& p, int ff, int co
             }
             if (r < rows_ok) {
                 float* row = (slot < 0 && p.row_map) ? p.C + (int64_t)p.row_map[w * kWinRows + r] * p.ldc : dst + (int64_t)r * ld;
+                if (slot < 0 && !p.vec_out) {   // C with an odd row length (never together with peers' copies)
+                    const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        if (c0 + i < p.n_out) row[c0 + i] = v[i];
+                    continue;
+                }
                 if (c0 < p.N) *reinterpret_cast<float4*>(row + c0) = v0;
                 if (c0 + 4 < p.N) *reinterpret_cast<float4*>(row + c0 + 4) = v1;
                 if (slot < 0) {  // the same row into every peer's copy of C (plain stores over NVLink)

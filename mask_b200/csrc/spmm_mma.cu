@@ -26,6 +26,7 @@
 //
 // Windows split across blocks write their partial 16xN tiles to scratch; a second kernel sums
 // them in fragment order, so no atomics and no zero-fill of C are needed.
+#include <algorithm>
 #include <cstring>
 
 #include "common.cuh"
@@ -273,7 +274,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, MIN_BLOCKS) spmm_mma_kern
 // tables piece by piece instead was a chain of dependent loads: 0.78 ms for 85 000 pieces at N = 512, now 0.57).
 __global__ void __launch_bounds__(256) spmm_fixup_kernel(const int2* heads, const int32_t* frag_win, const int32_t* frag_slot,
                                                         const float* scratch, float* C, int64_t ldc, int32_t M,
-                                                        int32_t N, int32_t relu, const int32_t* row_map,
+                                                        int32_t N, int32_t n_out, int32_t vec_out, int32_t relu, const int32_t* row_map,
                                                         float* const* peer_out, int32_t n_peer_out) {
     const int2 head = heads[blockIdx.x];
     const int w = frag_win[head.x];
@@ -299,6 +300,11 @@ __global__ void __launch_bounds__(256) spmm_fixup_kernel(const int2* heads, cons
         }
         if (relu) { s.x = fmaxf(s.x, 0.f); s.y = fmaxf(s.y, 0.f); s.z = fmaxf(s.z, 0.f); s.w = fmaxf(s.w, 0.f); }
         const int out_row = row_map ? row_map[w * kWinRows + r] : w * kWinRows + r;
+        if (!vec_out) {
+            const float x[4] = {s.x, s.y, s.z, s.w};
+            for (int j = 0; j < 4 && c + j < n_out; j++) C[(int64_t)out_row * ldc + c + j] = x[j];
+            continue;
+        }
         *reinterpret_cast<float4*>(C + (int64_t)out_row * ldc + c) = s;
         for (int j = 0; j < n_peer_out; j++) *reinterpret_cast<float4*>(peer_out[j] + (int64_t)out_row * ldc + c) = s;
     }
@@ -308,7 +314,7 @@ static int launch_fixup(const mask_plan* plan, const SpmmArgs& a, cudaStream_t s
     if (plan->H > 0) {
         dim3 fgrid((unsigned)plan->H, (unsigned)((kWinRows * (a.N >> 2) + 255) / 256));
         spmm_fixup_kernel<<<fgrid, 256, 0, st>>>(plan->d_heads, plan->d_frag_win, plan->d_frag_slot, a.scratch, a.C, a.ldc, a.M,
-                                                 a.N, a.relu, a.row_map, a.peer_out, a.n_peer_out);
+                                                 a.N, a.n_out, a.vec_out, a.relu, a.row_map, a.peer_out, a.n_peer_out);
         MASK_CUDA_TRY(cudaGetLastError());
     }
     return MASK_OK;
@@ -456,65 +462,129 @@ extern "C" int mask_tune(const char* name, int value) {
     return MASK_OK;
 }
 
+namespace mask {
+
+// Rows of n floats, any alignment -> rows of n4 floats (n4 = n rounded up to 4, at most 3 zeros at the end).  One
+// warp per run of rows; writes are 16 bytes a lane.
+__global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ src, int64_t ld, int32_t rows, int32_t n, int32_t n4,
+                                                       float4* __restrict__ dst) {
+    const int vecs = n4 >> 2;
+    const int64_t total = (int64_t)rows * vecs;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
+        const int64_t r = i / vecs;
+        const int c = (int)(i - r * vecs) << 2;
+        const float* at = src + r * ld + c;
+        float4 v;
+        v.x = __ldg(at);
+        v.y = c + 1 < n ? __ldg(at + 1) : 0.f;
+        v.z = c + 2 < n ? __ldg(at + 2) : 0.f;
+        v.w = c + 3 < n ? __ldg(at + 3) : 0.f;
+        dst[i] = v;
+    }
+}
+
+static bool whole_vectors(const void* p, int64_t ld, int32_t n) {
+    return n % 4 == 0 && ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+}
+
+static int fill_matrix_args(const mask_plan* plan, const mask_matrix* m, SpmmArgs& a) {
+    const bool some = plan->T > 0;
+    a.val_sidx = m->val_sidx;
+    switch (m->format) {
+        case kFmtSrbcrs:
+            MASK_REQUIRE(!some || (m->val_sidx && m->values), "packed arrays are NULL");
+            a.val_blk = static_cast<const float*>(m->values);
+            return MASK_OK;
+        case kFmtMetcf:
+            MASK_REQUIRE(!some || (m->val_sidx && m->offsets && m->index && m->values), "packed arrays are NULL");
+            a.coo_off = m->offsets;
+            a.coo_idx = static_cast<const int32_t*>(m->index);
+            a.coo_val = static_cast<const float*>(m->values);
+            return MASK_OK;
+        case kFmtMco:
+            MASK_REQUIRE(!some || (m->val_sidx && m->offsets && m->index), "packed arrays are NULL");
+            MASK_REQUIRE((reinterpret_cast<uintptr_t>(m->index) & 15) == 0 && (reinterpret_cast<uintptr_t>(m->values) & 15) == 0,
+                         "val_mco_mask and val_mco_val must be 16-byte aligned");
+            a.coo_off = m->offsets;
+            a.coo_val = static_cast<const float*>(m->values);
+            a.mco_mask = static_cast<const unsigned long long*>(m->index);
+            return MASK_OK;
+        default: return fail(MASK_ERR_INVALID_ARGUMENT, "unknown format");
+    }
+}
+
+}  // namespace mask
+
+extern "C" int mask_spmm(const mask_plan* plan, const mask_matrix* m, int32_t n, const float* d_B, int64_t ldb, float* d_C, int64_t ldc,
+                         float* d_pad, void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
+    using namespace mask;
+    MASK_REQUIRE(plan != nullptr && m != nullptr, "plan or matrix is NULL");
+    MASK_REQUIRE(n >= 0 && n <= 0x7fffffff - 3, "bad column count");
+    if (n == 0) return MASK_OK;
+    MASK_REQUIRE(d_B != nullptr && d_C != nullptr && ldb >= n && ldc >= n, "B or C is NULL, or a leading dimension is too small");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int32_t n4 = (n + 3) & ~3;
+    const bool pad = !whole_vectors(d_B, ldb, n), vec_out = whole_vectors(d_C, ldc, n);
+    MASK_REQUIRE(!pad || d_pad != nullptr, "B needs padding and the padding buffer is NULL");
+    MASK_REQUIRE(vec_out || plan->n_peer_out == 0, "peer outputs need N % 4 == 0, ldc % 4 == 0 and 16-byte aligned C");
+    const float* B = pad ? d_pad : d_B;
+    const int64_t ld = pad ? n4 : ldb;
+    int rc = check_common(plan, m->M, m->K, n4, B, ld, vec_out ? d_C : const_cast<float*>(B), vec_out ? ldc : n4, d_scratch, scratch_bytes);
+    if (rc != MASK_OK) return rc;
+    SpmmArgs a{};
+    rc = fill_matrix_args(plan, m, a);
+    if (rc != MASK_OK) return rc;
+    a.B = B; a.ldb = ld; a.C = d_C; a.ldc = ldc;
+    a.scratch = static_cast<float*>(d_scratch);
+    a.M = m->M; a.K = m->K; a.N = n4; a.n_out = n; a.vec_out = vec_out;
+    a.relu = ((epilogue & 0xff) == MASK_EPILOGUE_RELU);
+    a.tf32x3 = (epilogue & MASK_NUMERICS_TF32X3) ? 1 : 0;
+    MASK_REQUIRE(!a.tf32x3 || m->format == kFmtSrbcrs, "compensated products are implemented for SR-BCRS only");
+    if (pad && plan->T > 0) {
+        const int64_t blocks = ((int64_t)m->K * (n4 / 4) + 1023) / 1024;
+        pad_rows_kernel<<<(unsigned)std::min<int64_t>(blocks, 8 * sm_count()), 256, 0, st>>>(d_B, ldb, m->K, n, n4, reinterpret_cast<float4*>(d_pad));
+        MASK_CUDA_TRY(cudaGetLastError());
+    }
+    switch (m->format) {
+        case kFmtSrbcrs: return launch_spmm<kFmtSrbcrs>(plan, a, st);
+        case kFmtMetcf: return launch_spmm<kFmtMetcf>(plan, a, st);
+        default: return launch_spmm<kFmtMco>(plan, a, st);
+    }
+}
+
+// The entry points that take a matrix array by array.
+namespace mask {
+static int spmm_arrays(const mask_plan* plan, const mask_matrix& m, int32_t N, const float* d_B, int64_t ldb, float* d_C, int64_t ldc,
+                       void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
+    const int rc = check_common(plan, m.M, m.K, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes);
+    if (rc != MASK_OK || N == 0) return rc;
+    return mask_spmm(plan, &m, N, d_B, ldb, d_C, ldc, nullptr, d_scratch, scratch_bytes, epilogue, stream);
+}
+}  // namespace mask
+
 extern "C" int mask_spmm_srbcrs(const mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx,
                                 const float* d_val_block_val, int32_t M, int32_t K, int32_t N, const float* d_B,
                                 int64_t ldb, float* d_C, int64_t ldc, void* d_scratch, size_t scratch_bytes,
                                 int epilogue, void* stream) {
-    using namespace mask;
     (void)d_val_soff;
-    int rc = check_common(plan, M, K, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes);
-    if (rc != MASK_OK || N == 0) return rc;
-    MASK_REQUIRE(plan->T == 0 || (d_val_sidx != nullptr && d_val_block_val != nullptr), "packed arrays are NULL");
-    SpmmArgs a{};
-    a.val_sidx = d_val_sidx;
-    a.val_blk = d_val_block_val;
-    a.B = d_B; a.ldb = ldb; a.C = d_C; a.ldc = ldc;
-    a.scratch = static_cast<float*>(d_scratch);
-    a.M = M; a.K = K; a.N = N; a.relu = ((epilogue & 0xff) == MASK_EPILOGUE_RELU);
-    a.tf32x3 = (epilogue & MASK_NUMERICS_TF32X3) ? 1 : 0;
-    return launch_spmm<kFmtSrbcrs>(plan, a, static_cast<cudaStream_t>(stream));
+    const mask_matrix m{mask::kFmtSrbcrs, M, K, 0, d_val_sidx, nullptr, nullptr, d_val_block_val};
+    return mask::spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, epilogue, stream);
 }
 
 extern "C" int mask_spmm_metcf(const mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx,
                                const int32_t* d_val_coo_off, const int32_t* d_val_coo_idx, const float* d_val_coo_val,
                                int32_t M, int32_t K, int32_t N, const float* d_B, int64_t ldb, float* d_C, int64_t ldc,
                                void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
-    using namespace mask;
     (void)d_val_soff;
-    int rc = check_common(plan, M, K, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes);
-    if (rc != MASK_OK || N == 0) return rc;
-    MASK_REQUIRE(plan->T == 0 || (d_val_sidx != nullptr && d_val_coo_off != nullptr && d_val_coo_idx != nullptr &&
-                                  d_val_coo_val != nullptr), "packed arrays are NULL");
-    SpmmArgs a{};
-    a.val_sidx = d_val_sidx;
-    a.coo_off = d_val_coo_off; a.coo_idx = d_val_coo_idx; a.coo_val = d_val_coo_val;
-    a.B = d_B; a.ldb = ldb; a.C = d_C; a.ldc = ldc;
-    a.scratch = static_cast<float*>(d_scratch);
-    a.M = M; a.K = K; a.N = N; a.relu = ((epilogue & 0xff) == MASK_EPILOGUE_RELU);
-    MASK_REQUIRE(!(epilogue & MASK_NUMERICS_TF32X3), "compensated products are implemented for SR-BCRS only");
-    return launch_spmm<kFmtMetcf>(plan, a, static_cast<cudaStream_t>(stream));
+    const mask_matrix m{mask::kFmtMetcf, M, K, 0, d_val_sidx, d_val_coo_off, d_val_coo_idx, d_val_coo_val};
+    return mask::spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, epilogue, stream);
 }
 
 extern "C" int mask_spmm_mco(const mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx,
                              const int32_t* d_val_mco_off, const uint64_t* d_val_mco_mask, const float* d_val_mco_val,
                              int32_t M, int32_t K, int32_t N, const float* d_B, int64_t ldb, float* d_C, int64_t ldc,
                              void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
-    using namespace mask;
     (void)d_val_soff;
-    int rc = check_common(plan, M, K, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes);
-    if (rc != MASK_OK || N == 0) return rc;
-    MASK_REQUIRE(plan->T == 0 || (d_val_sidx != nullptr && d_val_mco_off != nullptr && d_val_mco_mask != nullptr),
-                 "packed arrays are NULL");
-    MASK_REQUIRE((reinterpret_cast<uintptr_t>(d_val_mco_mask) & 15) == 0 && (reinterpret_cast<uintptr_t>(d_val_mco_val) & 15) == 0,
-                 "val_mco_mask and val_mco_val must be 16-byte aligned");
-    SpmmArgs a{};
-    a.val_sidx = d_val_sidx;
-    a.coo_off = d_val_mco_off;
-    a.coo_val = d_val_mco_val;
-    a.mco_mask = reinterpret_cast<const unsigned long long*>(d_val_mco_mask);
-    a.B = d_B; a.ldb = ldb; a.C = d_C; a.ldc = ldc;
-    a.scratch = static_cast<float*>(d_scratch);
-    a.M = M; a.K = K; a.N = N; a.relu = ((epilogue & 0xff) == MASK_EPILOGUE_RELU);
-    MASK_REQUIRE(!(epilogue & MASK_NUMERICS_TF32X3), "compensated products are implemented for SR-BCRS only");
-    return launch_spmm<kFmtMco>(plan, a, static_cast<cudaStream_t>(stream));
+    const mask_matrix m{mask::kFmtMco, M, K, 0, d_val_sidx, d_val_mco_off, d_val_mco_mask, d_val_mco_val};
+    return mask::spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, epilogue, stream);
 }

@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(kSweepThreads, 2) spmm_sweep_kernel(const Spmm
                 }
                 bool colok[NSLAB];
 #pragma unroll
-                for (int sl = 0; sl < NSLAB; sl++) colok[sl] = col + 128 * sl < p.N;
+                for (int sl = 0; sl < NSLAB; sl++) colok[sl] = col + 128 * sl < (slot < 0 ? p.n_out : p.N);
                 // destination 0 is C (or the partial-tile scratch); 1.. are the peers' copies of C, which
                 // get the finished rows with plain stores over NVLink
                 const int n_dst = slot < 0 ? 1 + p.n_peer_out : 1;
@@ -461,8 +461,9 @@ static int launch_sweep_variant(const mask_plan* plan, SpmmArgs a, cudaStream_t 
     using L = SweepLayout<NSLAB, FMT>;
     static_assert(2 * (L::kDynamicBytes + 1024) <= 228 * 1024, "two blocks per SM");
     auto kern = spmm_sweep_kernel<NSLAB, FMT>;
-    MASK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamicBytes));   // per device
-    MASK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    static std::atomic<uint64_t> opted_in;
+    const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(kern), L::kDynamicBytes, opted_in);
+    if (rc != MASK_OK) return rc;
     // Two blocks per SM by construction: shared memory (asserted above), registers (launch bounds) and
     // tensor memory (at most 256 of the SM's 512 columns per block) all fit twice.  The occupancy
     // calculator is not asked: it answered 1 here because it assumes the default carveout.

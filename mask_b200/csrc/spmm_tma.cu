@@ -404,7 +404,7 @@ static int launch_tma_variant(const mask_plan* plan, SpmmArgs a, const CUtensorM
 // True when this plan and operand can take the TMA kernel: rounded tile values prepared from exactly
 // these values, and a row pitch the tensor map can express.
 bool spmm_tma_applies(const mask_plan* plan, const SpmmArgs& a) {
-    return plan->d_vals_tf32 != nullptr && plan->vals_src == a.val_blk && a.coo_off == nullptr && a.mco_mask == nullptr &&
+    return plan->d_vals_tf32 != nullptr && a.n_out == a.N && plan->vals_src == a.val_blk && a.coo_off == nullptr && a.mco_mask == nullptr &&
            a.N >= 32 && a.ldb % 4 == 0 && (reinterpret_cast<uintptr_t>(a.B) & 15) == 0 && encode_tiled_fn() != nullptr;
 }
 

@@ -255,8 +255,9 @@ template <int NQ, int KT, int S, int MINB, int FMT, bool GUARD, bool COMP>
 static int launch_warp_variant(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st) {
     using L = WarpLayout<NQ, KT, S, FMT>;
     auto kern = spmm_warp_kernel<NQ, KT, S, MINB, FMT, GUARD, COMP>;
-    MASK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
-    MASK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    static std::atomic<uint64_t> opted_in;
+    const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(kern), L::kBytes, opted_in);
+    if (rc != MASK_OK) return rc;
     dim3 grid((unsigned)plan->Gw, (unsigned)((a.N + 32 * NQ - 1) / (32 * NQ)));
     if (grid.y > 65535) return fail(MASK_ERR_INVALID_ARGUMENT, "N too large");
     kern<<<grid, 32, L::kBytes, st>>>(a);

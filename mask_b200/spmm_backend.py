@@ -67,15 +67,11 @@ def _run(fmt, variant, rowptr, colind, values, dense, num_rows):
         raise RuntimeError(f"unknown {fmt} variant '{variant}'")
     packed = _prep(fmt, rowptr, colind, values, num_rows, variant)
     d = dense if (dense.dtype == torch.float32 and dense.is_contiguous()) else dense.to(torch.float32).contiguous()
-    n = int(d.shape[1])
-    if n % 4:  # the kernels take any multiple of 4; pad like the reference pads to its tile width
-        d = torch.nn.functional.pad(d, (0, 4 - n % 4))
     if packed.K > d.shape[0]:
         raise RuntimeError(f"dense has {d.shape[0]} rows but the matrix references column {packed.K - 1}")
     if packed.K < d.shape[0]:
         d = d[: packed.K]
-    out = engine.spmm(packed, d, policy=policy)
-    return out if out.shape[1] == n else out[:, :n].contiguous()
+    return engine.spmm_any_width(packed, d, policy=policy)
 
 
 def srbcrs_spmm(rowptr, colind, values, dense, num_rows, feat_dim, num_nodes_ori):

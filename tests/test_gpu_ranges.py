@@ -1,0 +1,185 @@
+"""GPU tests at the sizes where a kernel's range ends: window sizes at which the format builder changes
+method, column counts around the warp-level kernel's groups, odd row lengths, neighbour lists and traversals
+of unusual shape in the row reorders.  Everything against the CPU oracle."""
+import numpy as np
+import pytest
+
+from mask_b200 import generators as G
+from tests.test_gpu_pack import _check_mco, _check_metcf, _check_srbcrs, _dev
+from tests.test_gpu_spmm import _assert_close
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows_to_csr(rows, K, seed):
+    rowptr = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    colind = np.concatenate(rows).astype(np.int32) if rowptr[-1] else np.zeros(0, np.int32)
+    values = np.random.Generator(np.random.PCG64(seed)).uniform(-1, 1, colind.size).astype(np.float32)
+    return G.CSR(len(rows), K, rowptr, colind, values)
+
+
+def _window(n, K, hub, seed):
+    """16 rows with n entries in all, most of them in one row if `hub`."""
+    rng = np.random.Generator(np.random.PCG64(seed))
+    share = np.full(16, n // 16) if not hub else np.full(16, n // 64)
+    share[3] += n - share.sum()
+    return [np.sort(rng.choice(K, int(c), replace=False)) for c in share]
+
+
+# sizes at which a window is sorted with more registers, ranked in one block's bitmap, shared by a cluster; key
+# width changes at 2^22 columns, bitmaps cover 2^19 (block) and 2^20 (block of a cluster) columns at a time
+@pytest.mark.parametrize("K", [3000, 600_000, 2_200_000, 4_300_000])
+@pytest.mark.parametrize("hub", [False, True])
+def test_pack_window_sizes(oracle_mod, K, hub):
+    from mask_b200 import engine
+    sizes = [0, 1, 32, 33, 64, 65, 128, 129, 256, 257, 512, 513, 1023, 1024, 1025, 8191, 8192, 8193, 20000]
+    sizes = [n for n in sizes if n < 0.7 * K]
+    rows = []
+    for i, n in enumerate(sizes):
+        rows += _window(n, K, hub, 100 + i)
+    m = _rows_to_csr(rows[:-5], K, 7)   # the last window is ragged
+    rp, ci, va = _dev(m)
+    _check_srbcrs(engine.pack_srbcrs(rp, ci, va, m.M, m.K), oracle_mod.pack_srbcrs(m.M, m.rowptr, m.colind, m.values))
+    _check_metcf(engine.pack_metcf(rp, ci, va, m.M, m.K), oracle_mod.pack_metcf(m.M, m.rowptr, m.colind, m.values))
+    _check_mco(engine.pack_mco(rp, ci, va, m.M, m.K), oracle_mod.pack_mco(m.M, m.rowptr, m.colind, m.values))
+
+
+@pytest.mark.parametrize("n", [40, 1030, 9000])
+@pytest.mark.parametrize("fault", ["order", "range"])
+def test_pack_finds_faults_in_every_kind_of_window(n, fault):
+    from mask_b200 import _lib, engine
+    K = 40_000
+    m = _rows_to_csr(_window(n, K, True, 3), K, 7)
+    e = int(m.rowptr[4]) - 2            # near the end of the longest row
+    if fault == "order":
+        m.colind[e], m.colind[e + 1] = m.colind[e + 1], m.colind[e]
+    else:
+        m.colind[e + 1] = K
+    with pytest.raises(_lib.MaskError) as err:
+        engine.pack_srbcrs(*_dev(m), m.M, m.K)
+    assert err.value.status == (3 if fault == "order" else 6)
+
+
+def _mixed_matrix():
+    """Power-law rows, an empty window, a window long enough to be split, a ragged end."""
+    a = G.rmat_gcn_normalised(scale=10, samples_per_node=8, seed=5)
+    rows = [a.colind[a.rowptr[i]:a.rowptr[i + 1]] for i in range(700)]
+    rows[64:80] = [np.zeros(0, np.int32)] * 16
+    rng = np.random.Generator(np.random.PCG64(2))
+    rows[100] = np.sort(rng.choice(a.K, 900, replace=False)).astype(np.int32)
+    return _rows_to_csr(rows[:-3], a.K, 9)
+
+
+@pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
+@pytest.mark.parametrize("N", [4, 28, 32, 36, 64, 68, 96, 100, 128, 132, 192, 260])
+def test_warp_kernel_column_counts(oracle_mod, fmt, N):
+    import torch
+    from mask_b200 import engine
+    m = _mixed_matrix()
+    p = {"srbcrs": engine.pack_srbcrs, "metcf": engine.pack_metcf, "mco": engine.pack_mco}[fmt](*_dev(m), m.M, m.K)
+    B = np.random.Generator(np.random.PCG64(N)).standard_normal((m.K, N), dtype=np.float32)
+    Bd = torch.from_numpy(B).cuda()
+    engine.tune("sweep", 0)
+    try:
+        plan = p.new_plan("auto")
+        assert engine.kernel_signature(p, N, plan)[0] == f"spmm_warp_kernel<{fmt}>"
+        for gt in (0, 5):               # whole windows and split ones
+            out = torch.full((m.M, N), float("nan"), device="cuda")
+            engine.spmm(p, Bd, out=out, plan=p.new_plan("auto", gt), relu=gt == 5)
+            _assert_close(oracle_mod, m, B, out.cpu().numpy(), relu=gt == 5)
+        if fmt == "srbcrs":
+            out = engine.spmm(p, Bd, plan=plan, tf32x3=True).cpu().numpy()
+            ref = oracle_mod.spmm_f32(m.M, m.rowptr, m.colind, m.values, B)
+            absp = oracle_mod.spmm_abs_f64(m.M, m.rowptr, m.colind, m.values, B)
+            bad, worst = oracle_mod.check_tolerance(out, ref, absp, 2e-5, 1e-6)
+            assert bad == 0, worst
+    finally:
+        engine.tune("sweep", 1)
+
+
+@pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
+@pytest.mark.parametrize("N,offset,sweep", [(1, 0, 1), (3, 0, 1), (47, 0, 1), (47, 1, 2), (64, 3, 1), (129, 2, 1), (515, 0, 2)])
+def test_rows_that_are_not_whole_vectors(oracle_mod, fmt, N, offset, sweep):
+    """Any column count, B and C at any multiple of 4 bytes, whole and split windows, both kernels, and a row map."""
+    import torch
+    from mask_b200 import engine
+    m = _mixed_matrix()
+    dev = _dev(m)
+    p = {"srbcrs": engine.pack_srbcrs, "metcf": engine.pack_metcf, "mco": engine.pack_mco}[fmt](*dev, m.M, m.K)
+    packed = [(p, None), (p, 5)]
+    if fmt == "srbcrs":
+        packed.append((engine.pack_srbcrs(*dev, m.M, m.K, reorder="first_col_sort"), None))
+    B = np.random.Generator(np.random.PCG64(N)).standard_normal((m.K, N), dtype=np.float32)
+    Bd = torch.empty(m.K * N + offset, device="cuda")[offset:].view(m.K, N)
+    Bd.copy_(torch.from_numpy(B))
+    engine.tune("sweep", sweep)
+    try:
+        for q, gt in packed:
+            whole = torch.full((m.M * N + offset + 64,), 7.0, device="cuda")
+            out = whole[offset:offset + m.M * N].view(m.M, N)
+            engine.spmm_any_width(q, Bd, out=out, plan=q.new_plan("auto", gt or 0))
+            _assert_close(oracle_mod, m, B, out.cpu().numpy())
+            assert bool((whole[:offset] == 7).all()) and bool((whole[offset + m.M * N:] == 7).all())   # nothing beside C was written
+    finally:
+        engine.tune("sweep", 1)
+
+
+def _graph(edges, n, extra=()):
+    e = np.array(sorted(set(edges) | set(extra)), dtype=np.int64)
+    order = np.lexsort((e[:, 1], e[:, 0])) if len(e) else np.zeros(0, np.int64)
+    rows = np.split(e[order, 1], np.cumsum(np.bincount(e[:, 0], minlength=n))[:-1]) if len(e) else [np.zeros(0)] * n
+    return _rows_to_csr([r.astype(np.int32) for r in rows], n, 1)
+
+
+def _both(pairs):
+    return {(a, b) for a, b in pairs} | {(b, a) for a, b in pairs}
+
+
+GRAPHS = {
+    # one node a level: the part of the traversal that one block does alone, thousands of levels
+    "path": lambda: _graph(_both((i, i + 1) for i in range(2999)), 3000),
+    # lists longer than a warp sorts (1024) and longer than a block walks at once, and a level of 5000 nodes
+    "stars": lambda: _graph(_both([(0, i) for i in range(1, 5001)] + [(7000, i) for i in range(5001, 6100)]), 7001),
+    # not symmetric: a one-way ring with chords, and entries on the diagonal
+    "one_way": lambda: _graph({(i, (i + 1) % 500) for i in range(500)} | {(i, (7 * i) % 500) for i in range(500)} | {(i, i) for i in range(0, 500, 3)}, 500),
+    # hundreds of components of different sizes, isolated nodes between them
+    "components": lambda: _graph(_both((10 * c + i, 10 * c + i + 1) for c in range(300) for i in range(c % 8)), 3000),
+    "no_edges": lambda: _graph({(3, 3)}, 50),
+    "single": lambda: _graph({(0, 0)}, 1),
+}
+
+
+@pytest.mark.parametrize("name", sorted(GRAPHS))
+@pytest.mark.parametrize("kind", ["row_rcm", "first_col_sort", "jaccard_greedy"])
+def test_reorders_of_unusual_graphs(oracle_mod, name, kind):
+    from mask_b200 import engine
+    m = GRAPHS[name]()
+    rp, ci, va = _dev(m)
+    order = engine.reorder_rows(rp, ci, m.M, m.K, kind)
+    want = oracle_mod.reorder_rows(kind, m.M, m.K, m.rowptr, m.colind)
+    assert np.array_equal(order.cpu().numpy(), want)
+    got = engine.permute_rows(rp, ci, va, m.M, order)
+    for a, b in zip(got, oracle_mod.permute_csr(m.M, m.rowptr, m.colind, m.values, want)):
+        assert np.array_equal(a.cpu().numpy(), b)
+
+
+def test_column_features_with_very_hot_columns():
+    """More than 8192 gathers of a column: the counts that are listed instead of binned."""
+    import ctypes as C
+    import torch
+    from mask_b200 import _lib, engine
+    M, K = 16 * 9000, 70_000
+    rows = [np.array([0, 5, 100 + (i * 37) % 60_000], dtype=np.int32) if i % 16 == 0 else np.zeros(0, np.int32) for i in range(M)]
+    m = _rows_to_csr(rows, K, 3)
+    rp, ci, va = _dev(m)
+    p = engine.pack_srbcrs(rp, ci, va, m.M, m.K)
+    f = _lib.ColumnFeatures()
+    _lib.check(_lib.lib().mask_features_columns(p.val_soff.data_ptr(), p.val_sidx.data_ptr(), m.M, m.K, p.T, 512, C.byref(f),
+                                                C.c_void_p(torch.cuda.current_stream().cuda_stream)), "mask_features_columns")
+    counts = np.bincount(p.val_sidx.cpu().numpy(), minlength=K)
+    top = np.sort(counts)[::-1].cumsum()
+    assert (counts >= 8192).sum() >= 2 and f.distinct_columns == int((counts > 0).sum())
+    for i in range(3):
+        assert abs(f.hub_share[i] - top[f.hub_columns[i] - 1] / counts.sum()) < 1e-12
+    tuned, plain = p.new_plan(), p.new_plan(autotune=False)
+    assert tuned.column_features()["distinct_columns"] == f.distinct_columns and plain.column_features() is None
