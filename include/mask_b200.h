@@ -422,10 +422,11 @@ int mask_session_create_csr(int32_t M, int32_t K, int64_t nnz, const int32_t* h_
                             const int32_t* h_colind, const float* h_values, int policy,
                             mask_session** out);
 /* C_host[M,N] = A * B_host[K,N]; pinned host buffers make the copies asynchronous.  kernel_ms,
- * if not NULL, receives the device time of the SpMM kernels alone.  When N is a multiple of 128
- * and at least 256 the product is cut into column chunks (independent products) whose upload,
- * multiplication and download overlap on three streams, so both directions of the host link are
- * busy at once; mask_tune("session_chunk", columns | 0 = off | -1 = automatic) overrides. */
+ * if not NULL, receives the device time of the SpMM kernels alone.  A product of more than a few
+ * megabytes with N a multiple of 32 is cut into column chunks (independent products of 64 or 128
+ * columns) whose upload, multiplication and download overlap on three streams, so both directions of
+ * the host link are busy at once; mask_tune("session_chunk", columns | 0 = off | -1 = automatic)
+ * overrides. */
 int mask_session_spmm_host(mask_session* s, const float* h_B, float* h_C, int32_t N,
                            float* kernel_ms);
 int64_t mask_session_tiles(const mask_session* s);

@@ -1,8 +1,10 @@
 // Status reporting and the host-buffer session seam of the C ABI.
 #include <cstdarg>
+#include <algorithm>
 #include <cstring>
 
 #include "common.cuh"
+#include "mem.h"
 #include "plan.h"
 
 namespace mask {
@@ -67,12 +69,13 @@ struct mask_session {
     // column-chunk pipeline of mask_session_spmm_host: upload, multiply and download on three streams
     static constexpr int kMaxChunks = 16;
     cudaStream_t up = nullptr, down = nullptr;
-    cudaEvent_t uploaded[kMaxChunks] = {}, k0[kMaxChunks] = {}, k1[kMaxChunks] = {}, downloaded = nullptr;
+    cudaEvent_t uploaded[kMaxChunks] = {}, k0[kMaxChunks] = {}, k1[kMaxChunks] = {};
+    mask::HostStage status;              // the kernels' status word after a call
 };
 
 namespace mask {
 
-// -1 = automatic (128-column chunks), 0 = no chunking, else columns per chunk (mask_tune "session_chunk")
+// -1 = automatic, 0 = no chunking, else columns per chunk (mask_tune "session_chunk")
 int g_session_chunk_cols = -1;
 
 static int session_common_init(mask_session* s) {
@@ -86,26 +89,32 @@ static int session_common_init(mask_session* s) {
         MASK_CUDA_TRY(cudaEventCreate(&s->k0[i]));
         MASK_CUDA_TRY(cudaEventCreate(&s->k1[i]));
     }
-    MASK_CUDA_TRY(cudaEventCreateWithFlags(&s->downloaded, cudaEventDisableTiming));
+    return s->status.get(sizeof(int32_t));
+}
+
+// Columns per chunk of the host-buffer pipeline, or 0 for one piece.  With equal chunks a call costs (1 + 1/chunks) of
+// one direction of the link, so more chunks are better, until the copies of narrow pieces of rows fall behind: alone,
+// 256 bytes a row run at the link's rate, but with copies the other way at the same time 256-byte pieces of 2 KB rows
+// cost more than the shorter tail gains (200 000 rows, N = 512: 128 columns 10.5 ms, 64 columns 11.6 ms; N = 320: 7.6
+// and 6.9; N = 256: 6.3 and 5.5; N = 128: one piece 4.1, 64 columns 3.3), 128-byte pieces always do, and so do
+// pieces that do not start on 128-byte lines (N = 100: one piece 3.3 ms, two 3.7).  At least 2 MB a chunk and
+// direction (40 us of link time).
+static int session_chunk_cols(int32_t N, int64_t rows) {
+    if (g_session_chunk_cols == 0 || N % 32 != 0) return 0;
+    int w = g_session_chunk_cols > 0 ? (g_session_chunk_cols + 31) / 32 * 32 : (N < 512 ? 64 : 128);
+    while (w < N && ((N + w - 1) / w > mask_session::kMaxChunks || (int64_t)w * 4 * rows < ((int64_t)2 << 20))) w += 32;
+    return w < N ? w : 0;
+}
+
+// Enqueued behind the last product of a call: the status word to the host, and cleared.
+static int session_fetch_status(mask_session* s) {
+    MASK_CUDA_TRY(cudaMemcpyAsync(s->status.as<int32_t>(), s->plan->d_status, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
+    MASK_CUDA_TRY(cudaMemsetAsync(s->plan->d_status, 0, sizeof(int32_t), s->stream));
     return MASK_OK;
 }
-
-// Columns per chunk of the host-buffer pipeline: a multiple of 128 that gives 2..kMaxChunks chunks,
-// or 0 when N is too narrow or ragged to be worth cutting.
-static int session_chunk_cols(int32_t N) {
-    if (g_session_chunk_cols == 0 || N % 128 != 0 || N < 256) return 0;
-    int w = g_session_chunk_cols > 0 ? g_session_chunk_cols : 128;
-    if (w % 32 != 0 || N % w != 0) w = 128;
-    while (N / w > mask_session::kMaxChunks) w *= 2;
-    return (N % w == 0 && N / w >= 2) ? w : 0;
-}
-
 // After the session's streams are idle: has a kernel of this call given up on a bounded wait?
 static int session_kernel_status(mask_session* s) {
-    int32_t st = 0;
-    int rc = mask_plan_status(s->plan, &st, s->stream);
-    if (rc != MASK_OK) return rc;
-    if (st != 0) return fail(MASK_ERR_KERNEL_TIMEOUT, "a kernel gave up on a bounded wait; the product is invalid");
+    if (*s->status.as<int32_t>() != 0) return fail(MASK_ERR_KERNEL_TIMEOUT, "a kernel gave up on a bounded wait; the product is invalid");
     return MASK_OK;
 }
 
@@ -140,7 +149,6 @@ extern "C" void mask_session_destroy(mask_session* s) {
         if (s->k0[i]) cudaEventDestroy(s->k0[i]);
         if (s->k1[i]) cudaEventDestroy(s->k1[i]);
     }
-    if (s->downloaded) cudaEventDestroy(s->downloaded);
     if (s->stream) cudaStreamDestroy(s->stream);
     delete s;
 }
@@ -186,23 +194,24 @@ extern "C" int mask_session_create_csr(int32_t M, int32_t K, int64_t nnz, const 
     mask_session* s = new mask_session();
     s->M = M; s->K = K;
     const size_t W = (size_t)(M + kWinRows - 1) / kWinRows;
-    int32_t *d_rowptr = nullptr, *d_colind = nullptr;
-    float* d_values = nullptr;
-    void* d_ws = nullptr;
+    DevScratch rowptr_b, colind_b, values_b, work_b;
     auto body = [&]() -> int {
         int rc = session_common_init(s);
         if (rc != MASK_OK) return rc;
-        const size_t n = (size_t)std::max<int64_t>(nnz, 1);
-        MASK_CUDA_TRY(cudaMalloc((void**)&d_rowptr, ((size_t)M + 1) * 4));
-        MASK_CUDA_TRY(cudaMalloc((void**)&d_colind, n * 4));
-        MASK_CUDA_TRY(cudaMalloc((void**)&d_values, n * 4));
+        const size_t n = (size_t)std::max<int64_t>(nnz, 1), ws = mask_pack_scratch_bytes(M, nnz);
+        rc = rowptr_b.alloc(((size_t)M + 1) * 4, s->stream);
+        if (rc == MASK_OK) rc = colind_b.alloc(n * 4, s->stream);
+        if (rc == MASK_OK) rc = values_b.alloc(n * 4, s->stream);
+        if (rc == MASK_OK) rc = work_b.alloc(ws, s->stream);
+        if (rc != MASK_OK) return rc;
+        int32_t *d_rowptr = rowptr_b.as<int32_t>(), *d_colind = colind_b.as<int32_t>();
+        float* d_values = values_b.as<float>();
+        void* d_ws = work_b.p;
         MASK_CUDA_TRY(cudaMemcpyAsync(d_rowptr, h_rowptr, ((size_t)M + 1) * 4, cudaMemcpyHostToDevice, s->stream));
         if (nnz > 0) {
             MASK_CUDA_TRY(cudaMemcpyAsync(d_colind, h_colind, (size_t)nnz * 4, cudaMemcpyHostToDevice, s->stream));
             MASK_CUDA_TRY(cudaMemcpyAsync(d_values, h_values, (size_t)nnz * 4, cudaMemcpyHostToDevice, s->stream));
         }
-        const size_t ws = mask_pack_scratch_bytes(M, nnz);
-        MASK_CUDA_TRY(cudaMalloc(&d_ws, ws));
         MASK_CUDA_TRY(cudaMalloc((void**)&s->d_soff, (W + 1) * 4));
         rc = mask_pack_analyze(d_rowptr, d_colind, M, K, nnz, d_ws, ws, s->d_soff, &s->T, s->stream);
         if (rc != MASK_OK) return rc;
@@ -214,11 +223,8 @@ extern "C" int mask_session_create_csr(int32_t M, int32_t K, int64_t nnz, const 
         return mask_plan_create_tuned(s->d_soff, s->d_sidx, M, K, s->T, policy, 0, s->stream, &s->plan);
     };
     int rc = body();
+    for (DevScratch* b : {&rowptr_b, &colind_b, &values_b, &work_b}) b->release();   // before the session's stream may go
     if (s->stream) cudaStreamSynchronize(s->stream);
-    cudaFree(d_rowptr);
-    cudaFree(d_colind);
-    cudaFree(d_values);
-    cudaFree(d_ws);
     if (rc != MASK_OK) { mask_session_destroy(s); return rc; }
     *out = s;
     return MASK_OK;
@@ -241,25 +247,27 @@ extern "C" int mask_session_spmm_host(mask_session* s, const float* h_B, float* 
     // Column chunks are independent products, so the upload of chunk i+1, the SpMM of chunk i and the
     // download of chunk i-1 overlap: the link carries both directions at once and the call costs
     // about (1 + 1/chunks) of one direction instead of both in sequence.
-    const int w = session_chunk_cols(N);
+    const int w = session_chunk_cols(N, std::min(s->M, s->K));
     if (w > 0) {
-        const int chunks = N / w;
-        const size_t pitch = (size_t)N * 4, width = (size_t)w * 4;
+        const int chunks = (N + w - 1) / w;
+        const size_t pitch = (size_t)N * 4;
         auto enqueue = [&]() -> int {
             for (int i = 0; i < chunks; i++) {
                 const size_t c0 = (size_t)i * w;
+                const int32_t n = std::min<int32_t>(w, N - i * w);
+                const size_t width = (size_t)n * 4;
                 MASK_CUDA_TRY(cudaMemcpy2DAsync(s->d_B + c0, pitch, h_B + c0, pitch, width, (size_t)s->K, cudaMemcpyHostToDevice, s->up));
                 MASK_CUDA_TRY(cudaEventRecord(s->uploaded[i], s->up));
                 MASK_CUDA_TRY(cudaStreamWaitEvent(s->stream, s->uploaded[i], 0));
                 MASK_CUDA_TRY(cudaEventRecord(s->k0[i], s->stream));
-                int r = mask_spmm_srbcrs(s->plan, s->d_soff, s->d_sidx, s->d_blk, s->M, s->K, w, s->d_B + c0, N, s->d_C + c0, N,
+                int r = mask_spmm_srbcrs(s->plan, s->d_soff, s->d_sidx, s->d_blk, s->M, s->K, n, s->d_B + c0, N, s->d_C + c0, N,
                                          s->d_scratch, s->scratch_bytes, MASK_EPILOGUE_NONE, s->stream);
                 if (r != MASK_OK) return r;
                 MASK_CUDA_TRY(cudaEventRecord(s->k1[i], s->stream));
                 MASK_CUDA_TRY(cudaStreamWaitEvent(s->down, s->k1[i], 0));
                 MASK_CUDA_TRY(cudaMemcpy2DAsync(h_C + c0, pitch, s->d_C + c0, pitch, width, (size_t)s->M, cudaMemcpyDeviceToHost, s->down));
             }
-            return MASK_OK;
+            return session_fetch_status(s);
         };
         rc = enqueue();
         // whatever was enqueued -- also when enqueueing failed half way -- must finish before the caller's
@@ -288,7 +296,7 @@ extern "C" int mask_session_spmm_host(mask_session* s, const float* h_B, float* 
         if (r != MASK_OK) return r;
         MASK_CUDA_TRY(cudaEventRecord(s->ev1, s->stream));
         MASK_CUDA_TRY(cudaMemcpyAsync(h_C, s->d_C, cb, cudaMemcpyDeviceToHost, s->stream));
-        return MASK_OK;
+        return session_fetch_status(s);
     };
     rc = enqueue();
     cudaError_t es = cudaStreamSynchronize(s->stream);   // also after a failed enqueue: the upload may be in flight

@@ -27,7 +27,11 @@ struct DevScratch {
     DevScratch() = default;
     DevScratch(const DevScratch&) = delete;
     DevScratch& operator=(const DevScratch&) = delete;
-    ~DevScratch() { if (p) device_free(p, st); }
+    ~DevScratch() { release(); }
+    void release() {
+        if (p) device_free(p, st);
+        p = nullptr;
+    }
     int alloc(size_t bytes, cudaStream_t stream) {
         st = stream;
         return device_alloc(&p, bytes, stream);

@@ -189,28 +189,31 @@ static void build_tables(mask_plan& p, const int32_t* soff) {
 }
 
 // Groups of the warp-level kernel: the same fragments in shorter runs, closed before their cost passes 5/4 of a
-// target.  Two reasons to keep them short.  Balance: 15 x 148 blocks are resident, and with 1.4 times as many
-// groups the second round is half empty; a target of half a resident warp's share leaves more and smaller ones
-// (100 000 rows, 20 tiles a window, N = 64: one window a group 35 us, two 41 us).  Locality: what the resident
-// warps touch together should stay in L2; where windows share rows of B with their neighbours, a window a
-// group keeps the band narrow (27-point stencil with 10^6 rows, N = 128: 517 us, with 128 tiles a group 585 us).
-// Not shorter than that: on a power-law graph half the windows hold a few tiles, and a block's start costs
-// about three tiles' time (130 000 nodes, N = 48: 16 tiles a group 78 us, 64 tiles 72 us).
+// target.  Two reasons to keep them short.  Balance: 15 x 148 blocks are resident and take groups in order as they
+// come free, so the target is a resident block's share of what is still left: long groups first, short ones at
+// the end.  Twice the share leaves a second round half empty (100 000 rows, 20 tiles a window, N = 64: 67 us
+// against 44), half of it starts more blocks for nothing (a start costs about three tiles' time; power-law graph
+// with 130 000 nodes, N = 48: 82 us against 80).  Locality: what the resident warps touch together should stay
+// in L2; where windows share rows of B with their neighbours, a window a group keeps the band narrow
+// (27-point stencil with 10^6 rows, N = 128: 517 us, with 128 tiles a group 585 us).
 static void build_warp_groups(mask_plan& p) {
     p.h_warp_off.clear();
     if (p.policy != MASK_POLICY_AUTO || !p.auto_groups) return;   // the plan's own groups
-    const int64_t share = p.T / ((int64_t)sm_count() * kWarpBlocksPerSm * 2);
-    const int32_t target = p.local ? kMinPiece : (int32_t)std::max<int64_t>(kMinPiece, std::min<int64_t>(128, share));
-    constexpr int32_t kFragCost = 4;
+    constexpr int32_t kFragCost = 4, kMaxTarget = 128;
+    const int64_t takers = (int64_t)sm_count() * kWarpBlocksPerSm;
     const auto& fo = p.h_frag_off;
-    int32_t load = 0;
+    int64_t left = p.T + kFragCost * p.F;   // cost of the fragments not dealt yet
+    auto target_now = [&]() { return p.local ? (int64_t)kMinPiece : std::max<int64_t>(kMinPiece, std::min<int64_t>(kMaxTarget, left / takers)); };
+    int64_t load = 0, limit = target_now() * 5 / 4;
     p.h_warp_off.reserve((size_t)p.F + 1);
     p.h_warp_off.push_back(0);
     for (int64_t f = 0; f < p.F; f++) {
-        const int32_t cost = fo[f + 1] - fo[f] + kFragCost;
-        if (load > 0 && load + cost > target + target / 4) {
+        const int64_t cost = fo[f + 1] - fo[f] + kFragCost;
+        if (load > 0 && load + cost > limit) {
             p.h_warp_off.push_back((int32_t)f);
+            left -= load;
             load = 0;
+            limit = target_now() * 5 / 4;
         }
         load += cost;
     }

@@ -183,3 +183,23 @@ def test_column_features_with_very_hot_columns():
         assert abs(f.hub_share[i] - top[f.hub_columns[i] - 1] / counts.sum()) < 1e-12
     tuned, plain = p.new_plan(), p.new_plan(autotune=False)
     assert tuned.column_features()["distinct_columns"] == f.distinct_columns and plain.column_features() is None
+
+
+@pytest.mark.parametrize("rows,N", [(17, 64), (9000, 96), (20_000, 160), (20_000, 100), (5000, 512)])
+def test_session_column_chunks(oracle_mod, rows, N):
+    """Host-buffer products that are cut into chunks (also with a narrower last one) and that are not."""
+    import ctypes as C
+    from mask_b200 import _lib
+    L = _lib.lib()
+    m = _rows_to_csr([np.array([i % 300, 300 + i % 41], dtype=np.int32) for i in range(rows)], max(rows, 400), 5)
+    h, ms = C.c_void_p(), C.c_float()
+    _lib.check(L.mask_session_create_csr(m.M, m.K, m.nnz, m.rowptr.ctypes.data, m.colind.ctypes.data, m.values.ctypes.data, 0, C.byref(h)), "create")
+    B = np.random.Generator(np.random.PCG64(N)).standard_normal((m.K, N), dtype=np.float32)
+    try:
+        for _ in range(2):
+            out = np.full((m.M, N), np.nan, dtype=np.float32)
+            _lib.check(L.mask_session_spmm_host(h, B.ctypes.data, out.ctypes.data, N, C.byref(ms)), "spmm_host")
+            assert ms.value > 0
+            _assert_close(oracle_mod, m, B, out)
+    finally:
+        L.mask_session_destroy(h)
