@@ -131,6 +131,23 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_binding = None
+
+
+def binding():
+    """The extension module behind the products (``csrc/torch_binding.cpp``)."""
+    global _binding
+    if _binding is None:
+        lib()
+        path = os.path.join(_HERE, "_binding.so")
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing: build it with `make -C mask_b200/csrc`. There is no fallback path.")
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        from . import _binding as module
+        _binding = module
+    return _binding
+
+
 def check(status: int, where: str) -> None:
     if status != 0:
         L = lib()

@@ -22,11 +22,6 @@ def _stream():
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-# Handle of the current stream without building a Stream object (the products' host path takes a few
-# microseconds in all).
-_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda device: torch.cuda.current_stream(device).cuda_stream)
-
-
 def _req(t, dtype, name):
     if not (isinstance(t, torch.Tensor) and t.is_cuda):
         raise RuntimeError(f"{name} must be a CUDA tensor")
@@ -51,11 +46,10 @@ class Plan:
             check(lib().mask_plan_create(_ptr(val_soff), M, T, _lib.POLICY[policy], group_tiles, _stream(), C.byref(h)),
                   "mask_plan_create")
         self._h = h
-        self._address = h.value
+        self._address = h.value or 0
         self.policy = policy
         self.M, self.T = M, T
         self._scratch = {}
-        self._scratch_per_column = int(lib().mask_plan_scratch_bytes(h, 4)) // 4
         self._row_order = None
 
     def __del__(self):
@@ -111,26 +105,14 @@ class Plan:
     def scratch(self, N: int, device) -> torch.Tensor | None:
         """Partial-tile buffer for the current stream: products on different streams may overlap on
         the GPU, so each stream gets its own buffer (products on one stream run in order and share it)."""
-        return self._scratch_for(N, torch.cuda.current_stream().cuda_stream, device)
-
-    def _scratch_for(self, N: int, stream: int, device):
-        need = self._scratch_per_column * N
+        need = self.scratch_bytes(N)
         if need == 0:
             return None
-        buf = self._scratch.get((stream, device))
+        key = (torch.cuda.current_stream().cuda_stream, device)
+        buf = self._scratch.get(key)
         if buf is None or buf.numel() < need:
-            buf = self._scratch[(stream, device)] = torch.empty(need, dtype=torch.uint8, device=device)
+            buf = self._scratch[key] = torch.empty(need, dtype=torch.uint8, device=device)
         return buf
-
-
-def _matrix_address(packed) -> int:
-    """Address of the matrix's ``mask_matrix``, rebuilt when its arrays have moved."""
-    ptrs = packed._pointers()
-    known = packed.__dict__.get("_matrix")
-    if known is None or known[0] != ptrs:
-        m = _lib.Matrix(packed._FORMAT, packed.M, packed.K, 0, *ptrs)
-        known = packed.__dict__["_matrix"] = (ptrs, m, C.addressof(m))
-    return known[2]
 
 
 @dataclass
@@ -149,10 +131,9 @@ class PackedSRBCRS:
     row_order: torch.Tensor | None = None   # set when the rows were reordered: packed row i = original row row_order[i]
     plans: dict = field(default_factory=dict)
 
-    _FORMAT = 0
-
-    def _pointers(self):
-        return self.val_sidx.data_ptr(), None, None, self.val_block_val.data_ptr()
+    def _arrays(self):
+        """What the C ABI's ``mask_matrix`` holds: format, offsets, index, values."""
+        return 0, None, None, self.val_block_val
 
     def plan(self, policy: str = "auto", group_tiles: int = 0) -> Plan:
         key = (policy, group_tiles)
@@ -192,10 +173,9 @@ class PackedMETCF:
 
     plan = PackedSRBCRS.plan
     new_plan = PackedSRBCRS.new_plan
-    _FORMAT = 1
 
-    def _pointers(self):
-        return self.val_sidx.data_ptr(), self.val_coo_off.data_ptr(), self.val_coo_idx.data_ptr(), self.val_coo_val.data_ptr()
+    def _arrays(self):
+        return 1, self.val_coo_off, self.val_coo_idx, self.val_coo_val
 
 
 @dataclass
@@ -217,10 +197,9 @@ class PackedMCO:
 
     plan = PackedSRBCRS.plan
     new_plan = PackedSRBCRS.new_plan
-    _FORMAT = 2
 
-    def _pointers(self):
-        return self.val_sidx.data_ptr(), self.val_mco_off.data_ptr(), self.val_mco_mask.data_ptr(), self.val_mco_val.data_ptr()
+    def _arrays(self):
+        return 2, self.val_mco_off, self.val_mco_mask, self.val_mco_val
 
 
 def _analyze(rowptr, colind, M, K):
@@ -339,49 +318,30 @@ def spmm(packed, dense: torch.Tensor, out: torch.Tensor | None = None, policy: s
          plan: Plan | None = None, tf32x3: bool = False) -> torch.Tensor:
     """out[M,N] = A @ dense[K,N] on the current stream.  ``out`` is fully overwritten.
     ``tf32x3`` (SR-BCRS): compensated products, FP32-level accuracy at about 1.7x the time."""
-    if isinstance(dense, torch.Tensor) and dense.dim() == 2 and dense.shape[0] == packed.K and dense.shape[1]:
-        if dense.shape[1] % 4:
-            raise _lib.MaskError(1, "mask_spmm", "N must be a multiple of 4")
-        if (dense.data_ptr() | (0 if out is None else out.data_ptr())) & 15:
-            raise _lib.MaskError(1, "mask_spmm", "B and C must be 16-byte aligned")
-    return spmm_any_width(packed, dense, out, policy, relu, plan, tf32x3)
+    return _product(packed, dense, out, policy, relu, plan, tf32x3, True)
 
 
 def spmm_any_width(packed, dense: torch.Tensor, out: torch.Tensor | None = None, policy: str = "auto", relu: bool = False,
                    plan: Plan | None = None, tf32x3: bool = False) -> torch.Tensor:
     """``spmm`` for any number of columns.  Rows of ``dense`` that are not whole 16-byte vectors are copied to
     padded rows first; ``out`` is written in place whatever its row length."""
-    if not (isinstance(dense, torch.Tensor) and dense.is_cuda and dense.dtype is torch.float32 and dense.is_contiguous()):
-        _req(dense, torch.float32, "dense")
-    if dense.dim() != 2:
-        raise RuntimeError("dense must be 2-D")
-    K, N = dense.shape
-    if K != packed.K:
-        raise RuntimeError(f"dense has {K} rows, the matrix has {packed.K} columns")
-    device = dense.device
-    if out is None:
-        out = torch.empty((packed.M, N), dtype=torch.float32, device=device)
-    else:
-        _req(out, torch.float32, "out")
-        if tuple(out.shape) != (packed.M, N):
-            raise RuntimeError("out has the wrong shape")
-    if N == 0:
-        return out
+    return _product(packed, dense, out, policy, relu, plan, tf32x3, False)
+
+
+def _product(packed, dense, out, policy, relu, plan, tf32x3, whole_vectors):
     if plan is None:
         plan = packed.plan(policy)
     if packed.row_order is not None and plan._row_order is not packed.row_order:
         raise RuntimeError("this matrix was packed from reordered rows: use packed.plan() / packed.new_plan()")
-    stream = _raw_stream(torch._C._cuda_getDevice())
-    n4 = (N + 3) & ~3
-    b = dense.data_ptr()
-    pad = torch.empty(K * n4, dtype=torch.float32, device=device) if n4 != N or b & 15 else None
-    scratch = plan._scratch_for(n4, stream, device)
-    epi = (_lib.EPILOGUE_RELU if relu else _lib.EPILOGUE_NONE) | (_lib.NUMERICS_TF32X3 if tf32x3 else 0)
-    rc = lib().mask_spmm(plan._address, _matrix_address(packed), N, b, N, out.data_ptr(), N, None if pad is None else pad.data_ptr(),
-                         None if scratch is None else scratch.data_ptr(), 0 if scratch is None else scratch.numel(), epi, stream)
-    if rc != 0:
-        check(rc, "mask_spmm")
-    return out
+    fmt, offsets, index, values = packed._arrays()
+    got = (_lib._binding or _lib.binding()).spmm(fmt, packed.M, packed.K, packed.val_sidx, offsets, index, values, plan._address, dense, out,
+                                                 (_lib.EPILOGUE_RELU if relu else _lib.EPILOGUE_NONE) | (_lib.NUMERICS_TF32X3 if tf32x3 else 0),
+                                                 whole_vectors)
+    if type(got) is int:
+        if got < 0:
+            raise _lib.MaskError(1, "mask_spmm", "N must be a multiple of 4" if got == -1 else "B and C must be 16-byte aligned")
+        check(got, "mask_spmm")
+    return got
 
 
 def kernel_signature(packed, N: int, plan: Plan, tf32x3: bool = False) -> tuple[str, int]:
