@@ -276,10 +276,12 @@ __global__ void __launch_bounds__(256) spmm_fixup_kernel(const int2* heads, cons
                                                         const float* scratch, float* C, int64_t ldc, int32_t M,
                                                         int32_t N, int32_t n_out, int32_t vec_out, int32_t relu, const int32_t* row_map,
                                                         float* const* peer_out, int32_t n_peer_out) {
+    let_next_kernel_start();
     const int2 head = heads[blockIdx.x];
     const int w = frag_win[head.x];
     const int nvec = N >> 2;
     const int64_t tile_vecs = (int64_t)kWinRows * nvec;
+    wait_for_previous_kernel();
     const float4* first = reinterpret_cast<const float4*>(scratch) + (int64_t)frag_slot[head.x] * tile_vecs;
     for (int v = blockIdx.y * blockDim.x + threadIdx.x; v < kWinRows * nvec; v += gridDim.y * blockDim.x) {
         const int r = v / nvec, c = (v - r * nvec) << 2;
@@ -313,9 +315,8 @@ __global__ void __launch_bounds__(256) spmm_fixup_kernel(const int2* heads, cons
 static int launch_fixup(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st) {
     if (plan->H > 0) {
         dim3 fgrid((unsigned)plan->H, (unsigned)((kWinRows * (a.N >> 2) + 255) / 256));
-        spmm_fixup_kernel<<<fgrid, 256, 0, st>>>(plan->d_heads, plan->d_frag_win, plan->d_frag_slot, a.scratch, a.C, a.ldc, a.M,
-                                                 a.N, a.n_out, a.vec_out, a.relu, a.row_map, a.peer_out, a.n_peer_out);
-        MASK_CUDA_TRY(cudaGetLastError());
+        return launch_overlapped(spmm_fixup_kernel, fgrid, 256, 0, st, plan->d_heads, plan->d_frag_win, plan->d_frag_slot, a.scratch, a.C,
+                                 a.ldc, a.M, a.N, a.n_out, a.vec_out, a.relu, a.row_map, a.peer_out, a.n_peer_out);
     }
     return MASK_OK;
 }
@@ -468,6 +469,8 @@ namespace mask {
 // warp per run of rows; writes are 16 bytes a lane.
 __global__ void __launch_bounds__(256) pad_rows_kernel(const float* __restrict__ src, int64_t ld, int32_t rows, int32_t n, int32_t n4,
                                                        float4* __restrict__ dst) {
+    let_next_kernel_start();
+    wait_for_previous_kernel();
     const int vecs = n4 >> 2;
     const int64_t total = (int64_t)rows * vecs;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < total; i += (int64_t)gridDim.x * 256) {
@@ -542,8 +545,9 @@ extern "C" int mask_spmm(const mask_plan* plan, const mask_matrix* m, int32_t n,
     MASK_REQUIRE(!a.tf32x3 || m->format == kFmtSrbcrs, "compensated products are implemented for SR-BCRS only");
     if (pad && plan->T > 0) {
         const int64_t blocks = ((int64_t)m->K * (n4 / 4) + 1023) / 1024;
-        pad_rows_kernel<<<(unsigned)std::min<int64_t>(blocks, 8 * sm_count()), 256, 0, st>>>(d_B, ldb, m->K, n, n4, reinterpret_cast<float4*>(d_pad));
-        MASK_CUDA_TRY(cudaGetLastError());
+        rc = launch_overlapped(pad_rows_kernel, dim3((unsigned)std::min<int64_t>(blocks, 8 * sm_count())), 256, 0, st, d_B, ldb, m->K, n, n4,
+                               reinterpret_cast<float4*>(d_pad));
+        if (rc != MASK_OK) return rc;
     }
     switch (m->format) {
         case kFmtSrbcrs: return launch_spmm<kFmtSrbcrs>(plan, a, st);

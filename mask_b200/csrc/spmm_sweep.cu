@@ -135,6 +135,8 @@ __global__ void __launch_bounds__(kSweepThreads, 2) spmm_sweep_kernel(const Spmm
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    let_next_kernel_start();
+    wait_for_previous_kernel();
 
     // item -> (column block, group): column blocks slowest, odd ones walk the groups backwards
     auto item_cb = [&](int item) { return item / G; };
@@ -473,6 +475,10 @@ static int launch_sweep_variant(const mask_plan* plan, SpmmArgs a, cudaStream_t 
     if (items >= ((int64_t)1 << 31)) return fail(MASK_ERR_INVALID_ARGUMENT, "too many work items");
     const int64_t resident = (int64_t)blocks_per_sm * sm_count();
     const unsigned grid = (unsigned)(items < resident ? items : resident);
+    // Overlapping the start with the previous kernel's end pays where a block has a few items (4096-node matrix, N = 512:
+    // 19.4 -> 16.8 us).  A long run of blocks that took their places one by one as the previous ones left keeps
+    // a ragged front over the matrix and loses reuse in L2 (27-point stencil with 10^6 rows: 1.82 -> 1.91 ms).
+    if (items <= 4 * resident) return launch_overlapped(kern, dim3(grid), kSweepThreads, L::kDynamicBytes, st, a, plan->d_status);
     kern<<<grid, kSweepThreads, L::kDynamicBytes, st>>>(a, plan->d_status);
     MASK_CUDA_TRY(cudaGetLastError());
     return MASK_OK;

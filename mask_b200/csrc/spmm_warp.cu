@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
     constexpr bool METCF = FMT == kFmtMetcf, MCO = FMT == kFmtMco;
     extern __shared__ __align__(128) unsigned char smem[];
 
+    let_next_kernel_start();
     const int lane = threadIdx.x;
     const int g = lane >> 2, k = lane & 3;
     const int col_base = blockIdx.y * (32 * NQ);
@@ -68,6 +69,8 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
     if (f >= f_end) return;
     int f_tend = p.frag_off[f + 1] - t0;
     int f_next = p.frag_off[min((int64_t)f + 2, p.n_frag)] - t0;   // end of the following fragment, loaded ahead
+
+    wait_for_previous_kernel();
 
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem);
 
@@ -260,9 +263,7 @@ static int launch_warp_variant(const mask_plan* plan, const SpmmArgs& a, cudaStr
     if (rc != MASK_OK) return rc;
     dim3 grid((unsigned)plan->Gw, (unsigned)((a.N + 32 * NQ - 1) / (32 * NQ)));
     if (grid.y > 65535) return fail(MASK_ERR_INVALID_ARGUMENT, "N too large");
-    kern<<<grid, 32, L::kBytes, st>>>(a);
-    MASK_CUDA_TRY(cudaGetLastError());
-    return MASK_OK;
+    return launch_overlapped(kern, grid, 32, L::kBytes, st, a);
 }
 
 template <int FMT>
