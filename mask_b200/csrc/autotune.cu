@@ -33,8 +33,10 @@ struct StatsHead {                 // what goes back to the host in one copy, fo
     unsigned long long band[kBandBuckets + 1];   // last entry: gathers within local_rows of the diagonal
     uint32_t bins[kCountBins];     // columns by number of gathers
     uint32_t listed;
-    uint32_t pad[3];
+    int32_t local;                 // local_share >= kLocalShare, for the kernels that group the tiles
+    uint32_t pad[2];
 };
+constexpr double kLocalShare = 0.9;
 
 // One thread per tile: its window, then its 8 ids.  A block's 256 tiles lie in few windows, so the search runs
 // between the windows of its first and last tile.  Ids of a warp fall into the same few distance buckets: the lanes
@@ -91,6 +93,11 @@ __global__ void __launch_bounds__(256) column_stats_kernel(const int32_t* __rest
 __global__ void __launch_bounds__(512) count_bins_kernel(const uint32_t* __restrict__ counts, int32_t K, StatsHead* __restrict__ head,
                                                          uint32_t* __restrict__ list) {
     __shared__ uint32_t bins[kCountBins];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned long long total = 0;
+        for (int b = 0; b < kBandBuckets; b++) total += head->band[b];
+        head->local = total && (double)head->band[kBandBuckets] / (double)total >= kLocalShare;
+    }
     for (int i = threadIdx.x; i < kCountBins; i += 512) bins[i] = 0;
     __syncthreads();
     for (int i = blockIdx.x * 512 + threadIdx.x; i < K; i += gridDim.x * 512) {
@@ -126,6 +133,7 @@ int ColumnStatsJob::enqueue(const int32_t* d_val_soff, const int32_t* d_val_sidx
     const int width0 = std::min(N, 512);
     local_rows_ = (int32_t)std::min<int64_t>(K, std::max<int64_t>(0, ((int64_t)(l2_ / 2) / ((int64_t)width0 * 4) - kWinRows) / 2));
     uint32_t* counts = buf_.as<uint32_t>(counts_at);
+    d_local_ = &buf_.as<StatsHead>()->local;
     column_stats_kernel<<<(unsigned)((T + 255) / 256), 256, 0, st>>>(d_val_soff, d_val_sidx, W, T, M, K, (int64_t)local_rows_, counts,
                                                                     buf_.as<StatsHead>());
     MASK_CUDA_TRY(cudaGetLastError());
@@ -208,12 +216,12 @@ void choose_plan_parameters(mask_plan* plan, const mask_column_features& f) {
     plan->has_col_features = 1;
     const double half_l2 = 0.5 * (double)f.l2_bytes;
     const double b_bytes = (double)f.distinct_columns * 4.0 * 512.0;
-    const bool local = f.local_share >= 0.9 || b_bytes <= half_l2;   // the gathers stay near the diagonal, or all of B fits
+    const bool local = f.local_share >= kLocalShare || b_bytes <= half_l2;   // the gathers stay near the diagonal, or all of B fits
     // hub-heavy (a quarter of the gathers already fit at full width) and markedly more fits at half width
     const bool narrower_rows_pay = !local && b_bytes > 8.0 * half_l2 && f.hub_share[0] >= 0.25 && f.hub_share[1] - f.hub_share[0] >= 0.02;
     plan->nslab = narrower_rows_pay ? 2 : 4;
     const double even_share = f.distinct_columns ? (double)std::min(f.hub_columns[0], f.distinct_columns) / f.distinct_columns : 1.0;
-    plan->local = f.local_share >= 0.9;
+    plan->local = f.local_share >= kLocalShare;
     plan->hub_heavy = f.hub_share[0] >= 1.5 * even_share;
     plan->slab_fits = !plan->local && !plan->hub_heavy && b_bytes > f.l2_bytes && b_bytes / 4 <= f.l2_bytes;
     plan->far_beyond_l2 = plan->nslab == 2 && b_bytes >= 24.0 * f.l2_bytes;

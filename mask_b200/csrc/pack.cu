@@ -31,14 +31,10 @@
 #include "common.cuh"
 #include "condense.cuh"
 #include "mem.h"
+#include "scan.cuh"
+#include "launch.cuh"
 
 namespace mask {
-
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 16;
-constexpr int kScanChunk = kScanThreads * kScanItems;
-constexpr int kSmallItems = 4;
-constexpr int kSmallScan = 8 * 1024 * kSmallItems;   // one block takes about as long for this many as three launches
 
 constexpr int kFillTiles = 128;   // tiles a block of the fill writes ...
 constexpr int kFillSub = 32;      // ... and composes at a time
@@ -76,152 +72,6 @@ static PackScratch carve(void* base, int32_t M, int64_t nnz) {
     s.status = reinterpret_cast<int32_t*>(take(64));
     s.bytes = std::max(off, 16 * n);   // hosts have sized it by 16 bytes an entry
     return s;
-}
-
-// ---- device-wide scan (reduce chunks, scan the spine in one block, apply) --------------------
-// In: functor giving the int32 value at index i.  Out: functor receiving (i, exclusive, value).
-template <typename In>
-__global__ void __launch_bounds__(kScanThreads) scan_reduce_kernel(In in, int64_t n, int64_t* spine) {
-    __shared__ int64_t warp_sum[kScanThreads / 32];
-    const int64_t base = (int64_t)blockIdx.x * kScanChunk;
-    int64_t s = 0;
-    for (int i = threadIdx.x; i < kScanChunk; i += kScanThreads) {
-        const int64_t idx = base + i;
-        if (idx < n) s += in(idx);
-    }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t t = 0;
-        for (int i = 0; i < kScanThreads / 32; i++) t += warp_sum[i];
-        spine[blockIdx.x] = t;
-    }
-}
-
-// One block: exclusive scan of spine[0..nchunks) in place; total -> spine[nchunks] and *total.
-__global__ void __launch_bounds__(1024) scan_spine_kernel(int64_t* spine, int64_t nchunks, int64_t* total) {
-    __shared__ int64_t warp_tot[32];
-    __shared__ int64_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int64_t base = 0; base < nchunks; base += 1024) {
-        const int64_t idx = base + threadIdx.x;
-        const int64_t v = idx < nchunks ? spine[idx] : 0;
-        int64_t x = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) warp_tot[wid] = x;
-        __syncthreads();
-        if (wid == 0) {
-            int64_t w = warp_tot[lane];
-            for (int o = 1; o < 32; o <<= 1) {
-                const int64_t y = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= o) w += y;
-            }
-            warp_tot[lane] = w;  // inclusive over warps
-        }
-        __syncthreads();
-        const int64_t before = carry + (wid > 0 ? warp_tot[wid - 1] : 0);
-        if (idx < nchunks) spine[idx] = before + x - v;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += warp_tot[31];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        spine[nchunks] = carry;
-        if (total) *total = carry;
-    }
-}
-
-template <typename In, typename Out>
-__global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(In in, Out out, int64_t n, const int64_t* spine) {
-    __shared__ int64_t warp_tot[kScanThreads / 32];
-    const int64_t base = (int64_t)blockIdx.x * kScanChunk + (int64_t)threadIdx.x * kScanItems;
-    int32_t v[kScanItems];
-    int64_t s = 0;
-#pragma unroll
-    for (int i = 0; i < kScanItems; i++) {
-        v[i] = (base + i < n) ? in(base + i) : 0;
-        s += v[i];
-    }
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int64_t x = s;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (lane == 31) warp_tot[wid] = x;
-    __syncthreads();
-    int64_t before = spine[blockIdx.x] + x - s;
-    for (int i = 0; i < wid; i++) before += warp_tot[i];
-#pragma unroll
-    for (int i = 0; i < kScanItems; i++) {
-        if (base + i < n) out(base + i, before, v[i]);
-        before += v[i];
-    }
-}
-
-// The whole scan in one block, for counts that three launches would take longer for.
-template <typename In, typename Out>
-__global__ void __launch_bounds__(1024) scan_small_kernel(In in, Out out, int64_t n, int64_t* total) {
-    __shared__ int64_t warp_tot[32];
-    int64_t carry = 0;
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int64_t c = 0; c < n; c += 1024 * kSmallItems) {
-        const int64_t base = c + (int64_t)threadIdx.x * kSmallItems;
-        int32_t v[kSmallItems];
-        int64_t s = 0;
-#pragma unroll
-        for (int i = 0; i < kSmallItems; i++) {
-            v[i] = (base + i < n) ? in(base + i) : 0;
-            s += v[i];
-        }
-        int64_t x = s;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) warp_tot[wid] = x;
-        __syncthreads();
-        int64_t before = carry + x - s;
-        for (int i = 0; i < 32; i++) {
-            const int64_t t = warp_tot[i];
-            if (i < wid) before += t;
-            carry += t;
-        }
-#pragma unroll
-        for (int i = 0; i < kSmallItems; i++) {
-            if (base + i < n) out(base + i, before, v[i]);
-            before += v[i];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0 && total) *total = carry;
-}
-
-template <typename In, typename Out>
-static int device_scan(In in, Out out, int64_t n, int64_t* spine, int64_t* d_total, cudaStream_t st) {
-    if (n <= kSmallScan) {
-        scan_small_kernel<<<1, 1024, 0, st>>>(in, out, n, d_total);
-        MASK_CUDA_TRY(cudaGetLastError());
-        return MASK_OK;
-    }
-    const int64_t chunks = (n + kScanChunk - 1) / kScanChunk;
-    if (chunks > 0) {
-        scan_reduce_kernel<<<(unsigned)chunks, kScanThreads, 0, st>>>(in, n, spine);
-        MASK_CUDA_TRY(cudaGetLastError());
-    }
-    scan_spine_kernel<<<1, 1024, 0, st>>>(spine, chunks, d_total);
-    MASK_CUDA_TRY(cudaGetLastError());
-    if (chunks > 0) {
-        scan_apply_kernel<<<(unsigned)chunks, kScanThreads, 0, st>>>(in, out, n, spine);
-        MASK_CUDA_TRY(cudaGetLastError());
-    }
-    return MASK_OK;
 }
 
 // ---- condensed positions ---------------------------------------------------------------------
@@ -341,7 +191,6 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
     __shared__ int warp_sum[32];
     const int tid = threadIdx.x;
     const int n_big = status[4];
-    if ((int)blockIdx.x >= n_big) return;
     MarkSet marks{reinterpret_cast<uint32_t*>(smem), reinterpret_cast<uint16_t*>(smem + kBigBits / 8), run_before,
                   (min(K, kBigBits) + 4095) / 4096};
     for (int i = tid; i < marks.n_runs * 128; i += kBigThreads) marks.bits[i] = 0;
@@ -389,6 +238,7 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
         if (bad) atomicOr(status, bad);
         if (tid == 0) distinct[w] = total;
     }
+    wait_for_previous_kernel();   // the hub windows' kernel, if any, has ended when this one has
 }
 
 // Windows of more than kHubMin entries, dealt to clusters of kHubBlocks blocks.  Every block takes a range of
@@ -410,6 +260,7 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
     __shared__ int first[kWinRows + 1];        // list index of the row's first entry
     __shared__ int warp_sum[32];
     __shared__ int range_marks[2][kHubBlocks]; // two windows: a block may be one ahead of another
+    let_next_kernel_start();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int me = (int)cluster.block_rank();
     const int n_hub = status[5], n_clusters = gridDim.x / kHubBlocks;
@@ -805,22 +656,31 @@ extern "C" int mask_pack_analyze(const int32_t* d_rowptr, const int32_t* d_colin
     else
         condense_kernel<unsigned long long><<<blocks_for(W, 4), 128, 0, st>>>(d_rowptr, d_colind, M, K, W, s.pos, s.cols, s.rows, s.distinct, s.big_list, s.hub_list, s.status);
     MASK_CUDA_TRY(cudaGetLastError());
-    if (nnz > kSortMax) {
-        constexpr int kSmem = kBigBits / 8 + kBigBits / 16;
-        MASK_CUDA_TRY(cudaFuncSetAttribute(condense_big_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
-        const int64_t most = std::min<int64_t>(W, nnz / kSortMax);
-        condense_big_kernel<<<(unsigned)std::min<int64_t>(most, 2 * sm_count()), kBigThreads, kSmem, st>>>(
-            d_rowptr, d_colind, M, K, s.pos, s.cols, s.distinct, s.big_list, s.status);
-        MASK_CUDA_TRY(cudaGetLastError());
-    }
     if (nnz > kHubMin) {
         const int span = (int)std::min<int64_t>(((int64_t)K + 4095) / 4096 * 4096, kHubBits);   // columns a block marks at a time
         const int smem = span / 8 + span / 16;
-        MASK_CUDA_TRY(cudaFuncSetAttribute(condense_hub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHubBits / 8 + kHubBits / 16));
+        static std::atomic<uint64_t> opted_in;
+        const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(condense_hub_kernel), kHubBits / 8 + kHubBits / 16, opted_in);
+        if (rc != MASK_OK) return rc;
         const int64_t most = std::min<int64_t>(W, nnz / kHubMin);
         condense_hub_kernel<<<(unsigned)(kHubBlocks * std::min<int64_t>(most, std::max(1, sm_count() / kHubBlocks))), kHubThreads, smem, st>>>(
             d_rowptr, d_colind, M, K, span, s.pos, s.cols, s.distinct, s.hub_list, s.status);
         MASK_CUDA_TRY(cudaGetLastError());
+    }
+    if (nnz > kSortMax) {
+        constexpr int kSmem = kBigBits / 8 + kBigBits / 16;
+        static std::atomic<uint64_t> opted_in;
+        int rc = opt_in_shared_memory(reinterpret_cast<const void*>(condense_big_kernel), kSmem, opted_in);
+        if (rc != MASK_OK) return rc;
+        const int64_t most = std::min<int64_t>(W, nnz / kSortMax);
+        const dim3 grid((unsigned)std::min<int64_t>(most, 2 * sm_count()));
+        if (nnz > kHubMin) {   // independent of the hub windows: starts as their blocks leave
+            rc = launch_overlapped(condense_big_kernel, grid, kBigThreads, kSmem, st, d_rowptr, d_colind, M, K, s.pos, s.cols, s.distinct, s.big_list, s.status);
+            if (rc != MASK_OK) return rc;
+        } else {
+            condense_big_kernel<<<grid, kBigThreads, kSmem, st>>>(d_rowptr, d_colind, M, K, s.pos, s.cols, s.distinct, s.big_list, s.status);
+            MASK_CUDA_TRY(cudaGetLastError());
+        }
     }
     int rc = device_scan(WindowTilesIn{s.distinct, W}, SoffOut{d_val_soff, s.first_window}, (int64_t)W + 1, s.spine,
                          reinterpret_cast<int64_t*>(s.status + 2), st);

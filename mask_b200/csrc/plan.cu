@@ -3,10 +3,12 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 
 #include "common.cuh"
 #include "column_stats.h"
+#include "scan.cuh"
 
 namespace mask {
 
@@ -94,7 +96,7 @@ static int32_t default_group_tiles(int64_t T) {
     return (int32_t)std::max<int64_t>(16, std::min<int64_t>(128, g));
 }
 
-// Fills the fragment / group tables of `p` from val_soff on the host.
+// Fills the fragment / group tables of `p` from val_soff on the host: the reference's mappings, and one group per window.
 static void build_tables(mask_plan& p, const int32_t* soff) {
     const int32_t W = p.W;
     const int32_t G = p.group_tiles;
@@ -135,96 +137,312 @@ static void build_tables(mask_plan& p, const int32_t* soff) {
             if (++in_group == kMaxFragsPerGroup) { go.push_back((int32_t)fw.size()); in_group = 0; }
         }
         if (go.back() != (int32_t)fw.size()) go.push_back((int32_t)fw.size());
-    } else {
-        // Groups are closed on fragment boundaries once their cost (tiles plus a fixed share per fragment
-        // for the rows of C it writes) reaches G; a window of more than 5/4 of a piece is cut into near-equal
-        // pieces (each piece costs one partial tile in scratch and the fix-up pass sums them in tile order).
-        constexpr int32_t kWindowCost = 4;
-        const int32_t piece = p.piece_tiles;
-        const int32_t split_above = piece + piece / 4;
-        const size_t most = (size_t)W + (size_t)(p.T / std::max(piece, 1)) + 1;   // fragments
-        fo.resize(most + 1);
-        fw.resize(most);
-        go.resize(most + 1);
-        int32_t *fo_at = fo.data(), *fw_at = fw.data(), *go_at = go.data() + 1;
-        int32_t load = 0, n_frag = 0, closed = 0;
-        auto add = [&](int32_t tile, int32_t w) { *fo_at++ = tile; *fw_at++ = w; n_frag++; };
-        auto close = [&]() {
-            if (closed != n_frag) *go_at++ = closed = n_frag;
-            load = 0;
-        };
+    } else {   // MASK_POLICY_ROW
         for (int32_t w = 0; w < W; w++) {
-            const int32_t s = soff[w], x = soff[w + 1] - s;
-            if (p.policy == MASK_POLICY_ROW) {
-                add(s, w); close();
-                continue;
-            }
-            if (x > split_above) {
-                const int32_t parts = (x + piece - 1) / piece, base = x / parts, rem = x % parts;
-                int32_t at = s;
-                if (piece >= G) close();
-                for (int32_t i = 0; i < parts; i++) {
-                    add(at, w);
-                    at += base + (i < rem ? 1 : 0);
-                    load += base + kWindowCost;
-                    if (load >= G || piece >= G) close();
-                }
-                continue;
-            }
-            if (load > 0 && load + x + kWindowCost > G + G / 8) close();
-            add(s, w);
-            load += x + kWindowCost;
-            if (load >= G) close();
+            fo.push_back(soff[w]); fw.push_back(w); go.push_back(w + 1);
         }
-        close();
-        fo.resize(n_frag);
-        fw.resize(n_frag);
-        go.resize(go_at - go.data());
     }
     fo.push_back(soff[W]);
 
     p.F = (int64_t)fw.size();
     p.G = (int64_t)go.size() - 1;
-
 }
 
-// Groups of the warp-level kernel: the same fragments in shorter runs, closed before their cost passes 5/4 of a
-// target.  Two reasons to keep them short.  Balance: 15 x 148 blocks are resident and take groups in order as they
-// come free, so the target is a resident block's share of what is still left: long groups first, short ones at
-// the end.  Twice the share leaves a second round half empty (100 000 rows, 20 tiles a window, N = 64: 67 us
-// against 44), half of it starts more blocks for nothing (a start costs about three tiles' time; power-law graph
-// with 130 000 nodes, N = 48: 82 us against 80).  Locality: what the resident warps touch together should stay
-// in L2; where windows share rows of B with their neighbours, a window a group keeps the band narrow
-// (27-point stencil with 10^6 rows, N = 128: 517 us, with 128 tiles a group 585 us).
-static void build_warp_groups(mask_plan& p) {
-    p.h_warp_off.clear();
-    if (p.policy != MASK_POLICY_AUTO || !p.auto_groups) return;   // the plan's own groups
-    constexpr int32_t kFragCost = 4, kMaxTarget = 128;
-    const int64_t takers = (int64_t)sm_count() * kWarpBlocksPerSm;
-    const auto& fo = p.h_frag_off;
-    int64_t left = p.T + kFragCost * p.F;   // cost of the fragments not dealt yet
-    auto target_now = [&]() { return p.local ? (int64_t)kMinPiece : std::max<int64_t>(kMinPiece, std::min<int64_t>(kMaxTarget, left / takers)); };
-    int64_t load = 0, limit = target_now() * 5 / 4;
-    p.h_warp_off.reserve((size_t)p.F + 1);
-    p.h_warp_off.push_back(0);
-    for (int64_t f = 0; f < p.F; f++) {
-        const int64_t cost = fo[f + 1] - fo[f] + kFragCost;
-        if (load > 0 && load + cost > limit) {
-            p.h_warp_off.push_back((int32_t)f);
-            left -= load;
-            load = 0;
-            limit = target_now() * 5 / 4;
-        }
-        load += cost;
+// ---- MASK_POLICY_AUTO: tables built on the device ---------------------------------------------------
+// A window of more than 5/4 of a piece is cut into near-equal pieces (each costs one partial tile in scratch, and
+// the fix-up pass sums them in tile order).  Groups are runs of fragments of about equal cost: tiles plus
+// kFragCost per fragment for the rows of C it writes.  Walking the windows one by one on the host, with their
+// tile counts copied there and the tables back, took 0.4 ms for 65 536 windows; this takes 0.1.
+constexpr int32_t kFragCost = 4;
+constexpr int64_t kHigh = (int64_t)1 << 32;   // the scans carry two counts: one in each half
+
+struct PlanCounts {          // on the device in front of the tables, and back on the host
+    int32_t frags, heads, groups, warp_groups, bad, pad[3];
+    int32_t status[4];
+};
+
+struct TableArgs {
+    const int32_t* soff;
+    int32_t W, piece, group;
+    int64_t T, max_frags;
+    int32_t* frag_off; int32_t* frag_win; int32_t* frag_slot; int2* heads;
+    int32_t* group_off; int32_t* group_tile; int32_t* warp_off; int32_t* warp_tile;
+    PlanCounts* counts;
+    const int32_t* local;    // NULL: not known to be
+    int32_t resident;        // resident blocks of the tcgen05 kernel
+    int32_t takers;          // resident blocks of the warp-level kernel
+    int32_t same_groups;     // the warp-level kernel takes the plan's own groups
+};
+
+struct PiecesIn {            // pieces of a window | 1 if it is split
+    TableArgs a;
+    __device__ int64_t operator()(int64_t w) const {
+        const int32_t x = a.soff[w + 1] - a.soff[w];
+        return x > a.piece + a.piece / 4 ? (x + a.piece - 1) / a.piece + kHigh : 1;
     }
-    if (p.F > 0) p.h_warp_off.push_back((int32_t)p.F);
+};
+struct PiecesOut {
+    TableArgs a;
+    __device__ void operator()(int64_t w, int64_t before, int64_t v) const {
+        const int64_t first = before & (kHigh - 1), parts = v & (kHigh - 1);
+        const int32_t split_before = (int32_t)(before >> 32);
+        const bool split = v >= kHigh;
+        const int32_t s = a.soff[w], x = a.soff[w + 1] - s;
+        if (w == 0) {
+            for (int i = 0; i < 4; i++) a.counts->status[i] = 0;
+            if (s != 0) a.counts->bad = 1;
+        }
+        if (first + parts > a.max_frags || x < 0) {   // only if val_soff is not what it should be
+            a.counts->bad = 1;
+            return;
+        }
+        const int32_t base = (int32_t)(x / parts), rem = (int32_t)(x % parts);
+        const int32_t slot = split ? (int32_t)(first - (w - split_before)) : -1;   // unsplit windows are one fragment each
+        int32_t at = s;
+        for (int32_t i = 0; i < parts; i++) {
+            a.frag_off[first + i] = at;
+            a.frag_win[first + i] = (int32_t)w;
+            a.frag_slot[first + i] = split ? slot + i : -1;
+            at += base + (i < rem ? 1 : 0);
+        }
+        if (split) a.heads[split_before] = make_int2((int)first, (int)parts);
+        if (w == a.W - 1) {
+            a.frag_off[first + parts] = at;
+            if (at != a.T) a.counts->bad = 1;
+            a.counts->frags = (int32_t)(first + parts);
+            a.counts->heads = split_before + (split ? 1 : 0);
+        }
+    }
+};
+
+__device__ __forceinline__ int64_t cost_before(const TableArgs& a, int64_t f) { return (int64_t)a.frag_off[f] + kFragCost * f; }
+
+// The tcgen05 kernel's groups.  Its blocks take every resident-th group, so there are a whole number of groups for
+// each of them, of at most 9/8 of the plan's group size (100 000 rows, N = 100: 4.02 rounds 85 us, 4 rounds 72 us).
+// A fragment belongs to the group that the cost before its middle falls into.
+struct GroupsIn {
+    TableArgs a;
+    __device__ int32_t operator()(int64_t f) const {
+        const int32_t F = a.counts->frags;
+        if (a.counts->bad || f >= F) return 0;
+        if (f == 0) return 1;
+        const int64_t total = a.T + (int64_t)kFragCost * F;
+        const int64_t c0 = cost_before(a, f - 1), c1 = cost_before(a, f), c2 = cost_before(a, f + 1);
+        int64_t size2 = 2 * (int64_t)a.group;
+        if (!a.same_groups) {
+            const int64_t most = (int64_t)a.resident * (a.group + a.group / 8), rounds = (total + most - 1) / most;
+            size2 = 2 * total / (a.resident * rounds) + 1;
+            if (size2 < 2 * kMinPiece) size2 = 2 * kMinPiece;
+        }
+        return (c0 + c1) / size2 != (c1 + c2) / size2;
+    }
+};
+struct GroupsOut {
+    TableArgs a;
+    __device__ void operator()(int64_t f, int64_t before, int32_t v) const {
+        const int32_t F = a.counts->frags;
+        if (a.counts->bad || f >= F) return;
+        const int32_t g = (int32_t)before;
+        if (v) { a.group_off[g] = (int32_t)f; a.group_tile[g] = a.frag_off[f]; }
+        if (f == F - 1) {
+            a.group_off[g + v] = F;
+            a.group_tile[g + v] = (int32_t)a.T;
+            a.counts->groups = g + v;
+        }
+    }
+};
+
+// The warp-level kernel's groups: runs of fragments, closed before their cost passes 5/4 of a target.
+//
+// Balance: 15 x 148 blocks are resident and take groups in order as they come free, so the target is a resident
+// block's share of the cost still left, between 16 and 128 tiles: long groups first, short ones at the end.  Twice
+// the share leaves a second round half empty (100 000 rows, 20 tiles a window, N = 64: 67 us against 44), half of it
+// starts more blocks for nothing (a start costs about three tiles' time; power-law graph with 130 000 nodes, N = 48:
+// 82 us against 80), and groups cut by the middles of their fragments as above are too uneven (N = 64: 46 us).
+// Locality: what the resident warps touch together should stay in L2; where windows share rows of B with their
+// neighbours, short groups keep the band narrow (27-point stencil with 10^6 rows, N = 128: one window a group
+// 517 us, 128 tiles a group 585 us).
+//
+// Where a group ends depends on where it begins, so this is a walk; but from every fragment the end is known at
+// once.  Pointer doubling in shared memory finds for every fragment of a chunk where a walk that enters there leaves
+// the chunk and after how many groups; one thread then walks from chunk to chunk; and every chunk writes the groups of
+// the walk that enters it, itself cut into 32 parts in the same way.
+constexpr int kChunk = 2048, kChunkThreads = 1024, kPart = kChunk / 32;   // a group has at most 41 fragments: less than a part
+
+__device__ __forceinline__ int64_t warp_group_end(const TableArgs& a, int64_t f, int64_t F, int64_t total) {
+    const int64_t c = cost_before(a, f);
+    int64_t target = kMinPiece;
+    if (!(a.local && *a.local)) {
+        target = (total - c) / a.takers;
+        target = target < kMinPiece ? kMinPiece : (target > 128 ? 128 : target);
+    }
+    const int64_t limit = c + target * 5 / 4;
+    int64_t lo = f + 1, hi = f + 2 + target * 5 / 4 / kFragCost;   // the end is in [lo, hi)
+    if (hi > F + 1) hi = F + 1;
+    while (hi - lo > 1) {
+        const int64_t mid = (lo + hi) >> 1;
+        if (cost_before(a, mid) <= limit) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// to[i] (i of n): next fragment of a walk -> where the walk leaves i's block of `width`; cnt[i]: groups begun there
+__device__ __forceinline__ void double_pointers(int32_t* to, int32_t* cnt, int n, int width) {
+    constexpr int kPer = kChunk / kChunkThreads;
+    for (int step = 1; step < width; step *= 2) {
+        int32_t t[kPer], c[kPer];
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            const int i = j * kChunkThreads + threadIdx.x, end = min(n, (i / width + 1) * width);
+            const bool inside = i < n && to[i] < end;
+            t[j] = inside ? to[to[i]] : (i < n ? to[i] : 0);
+            c[j] = inside ? cnt[i] + cnt[to[i]] : (i < n ? cnt[i] : 0);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            const int i = j * kChunkThreads + threadIdx.x;
+            if (i < n) { to[i] = t[j]; cnt[i] = c[j]; }
+        }
+    }
+    __syncthreads();
+}
+
+// exit_to[f], groups[f]: where a walk that enters its chunk at f leaves it, and how many groups it begins there
+__global__ void __launch_bounds__(kChunkThreads) warp_group_jumps_kernel(const TableArgs a, int32_t* __restrict__ exit_to, int32_t* __restrict__ groups) {
+    __shared__ int32_t to[kChunk], cnt[kChunk];
+    const int64_t F = a.counts->frags, base = (int64_t)blockIdx.x * kChunk;
+    if (a.counts->bad || base >= F) return;
+    const int n = (int)(F - base < kChunk ? F - base : kChunk);
+    const int64_t total = a.T + (int64_t)kFragCost * F;
+    for (int i = threadIdx.x; i < n; i += kChunkThreads) {
+        to[i] = (int32_t)(warp_group_end(a, base + i, F, total) - base);
+        cnt[i] = 1;
+    }
+    double_pointers(to, cnt, n, kChunk);
+    for (int i = threadIdx.x; i < n; i += kChunkThreads) {
+        exit_to[base + i] = (int32_t)base + to[i];
+        groups[base + i] = cnt[i];
+    }
+}
+// entry[c], first[c]: where the walk from fragment 0 enters chunk c, and how many groups begin before
+__global__ void warp_group_walk_kernel(const TableArgs a, const int32_t* __restrict__ exit_to, const int32_t* __restrict__ groups,
+                                       int32_t* __restrict__ entry, int32_t* __restrict__ first) {
+    const int32_t F = a.counts->frags;
+    if (a.counts->bad) return;
+    int32_t f = 0, g = 0;
+    for (int c = 0; f < F; c++) {   // a group is shorter than a chunk, so no chunk is passed over
+        entry[c] = f;
+        first[c] = g;
+        g += groups[f];
+        f = exit_to[f];
+    }
+}
+__global__ void __launch_bounds__(kChunkThreads) warp_group_write_kernel(const TableArgs a, const int32_t* __restrict__ entry, const int32_t* __restrict__ first) {
+    __shared__ int32_t next[kChunk], to[kChunk], cnt[kChunk], part_entry[32], part_first[32];
+    const int64_t F = a.counts->frags, base = (int64_t)blockIdx.x * kChunk;
+    if (a.counts->bad || base >= F) return;
+    const int n = (int)(F - base < kChunk ? F - base : kChunk);
+    const int64_t total = a.T + (int64_t)kFragCost * F;
+    for (int i = threadIdx.x; i < n; i += kChunkThreads) {
+        next[i] = to[i] = (int32_t)(warp_group_end(a, base + i, F, total) - base);
+        cnt[i] = 1;
+    }
+    double_pointers(to, cnt, n, kPart);
+    if (threadIdx.x == 0) {
+        int32_t i = entry ? entry[blockIdx.x] - (int32_t)base : 0, g = first ? first[blockIdx.x] : 0;
+        for (int p = 0; p < 32; p++) {
+            part_entry[p] = i;
+            part_first[p] = g;
+            if (i < n) { g += cnt[i]; i = to[i]; }
+        }
+        if (base + n == F) {
+            a.warp_off[g] = (int32_t)F;
+            a.warp_tile[g] = (int32_t)a.T;
+            a.counts->warp_groups = g;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const int end = min(n, ((int)threadIdx.x + 1) * kPart);
+        int32_t g = part_first[threadIdx.x];
+        for (int32_t i = part_entry[threadIdx.x]; i < end; i = next[i], g++) {
+            a.warp_off[g] = (int32_t)base + i;
+            a.warp_tile[g] = a.frag_off[base + i];
+        }
+    }
+}
+
+static int enqueue_warp_groups(const TableArgs& a, DevScratch& work, cudaStream_t st) {
+    const int64_t chunks = (a.max_frags + kChunk - 1) / kChunk;
+    int32_t *entry = nullptr, *first = nullptr;
+    if (chunks > 1) {
+        int rc = work.alloc((size_t)(2 * a.max_frags + 2 * chunks) * 4, st);
+        if (rc != MASK_OK) return rc;
+        int32_t* exit_to = work.as<int32_t>();
+        int32_t* groups = exit_to + a.max_frags;
+        entry = groups + a.max_frags;
+        first = entry + chunks;
+        warp_group_jumps_kernel<<<(unsigned)chunks, kChunkThreads, 0, st>>>(a, exit_to, groups);
+        MASK_CUDA_TRY(cudaGetLastError());
+        warp_group_walk_kernel<<<1, 1, 0, st>>>(a, exit_to, groups, entry, first);
+        MASK_CUDA_TRY(cudaGetLastError());
+    }
+    warp_group_write_kernel<<<(unsigned)chunks, kChunkThreads, 0, st>>>(a, entry, first);
+    MASK_CUDA_TRY(cudaGetLastError());
+    return MASK_OK;
+}
+
+// Enqueues the tables of an AUTO plan and the copy of their sizes to `counts` (pinned).
+static int enqueue_auto_tables(mask_plan& p, const int32_t* d_val_soff, bool same_groups, const int32_t* d_local, DevScratch& spine,
+                               DevScratch& work, PlanCounts* counts, cudaStream_t st) {
+    TableArgs a{};
+    a.soff = d_val_soff;
+    a.W = p.W;
+    a.piece = p.piece_tiles;
+    a.group = p.group_tiles;
+    a.T = p.T;
+    a.max_frags = (int64_t)p.W + p.T / p.piece_tiles + 1;
+    a.local = d_local;
+    a.resident = 2 * sm_count();
+    a.takers = sm_count() * kWarpBlocksPerSm;
+    a.same_groups = same_groups;
+    if (a.max_frags >= ((int64_t)1 << 31) - 1) return fail(MASK_ERR_INDEX_OVERFLOW, "the number of tasks does not fit int32");
+    size_t at = sizeof(PlanCounts) / 4;
+    auto section = [&](int64_t n) { const size_t o = at; at += ((size_t)n + 3) & ~(size_t)3; return o; };
+    const int64_t n = a.max_frags;
+    const size_t o_fo = section(n + 1), o_fw = section(n), o_fs = section(n), o_go = section(n + 1), o_gt = section(n + 1),
+                 o_wo = section(n + 1), o_wt = section(n + 1), o_hd = section(2 * std::min<int64_t>(p.W, p.T / p.piece_tiles + 1));
+    int rc = device_alloc(reinterpret_cast<void**>(&p.d_tables), at * sizeof(int32_t), st);
+    if (rc == MASK_OK) rc = spine.alloc(scan_spine_words(n) * 8, st);
+    if (rc != MASK_OK) return rc;
+    a.counts = reinterpret_cast<PlanCounts*>(p.d_tables);
+    a.frag_off = p.d_frag_off = p.d_tables + o_fo;
+    a.frag_win = p.d_frag_win = p.d_tables + o_fw;
+    a.frag_slot = p.d_frag_slot = p.d_tables + o_fs;
+    a.group_off = p.d_group_off = p.d_tables + o_go;
+    a.group_tile = p.d_group_tile = p.d_tables + o_gt;
+    a.warp_off = p.d_tables + o_wo;
+    a.warp_tile = p.d_tables + o_wt;
+    p.d_warp_off = same_groups ? p.d_group_off : a.warp_off;
+    p.d_warp_tile = same_groups ? p.d_group_tile : a.warp_tile;
+    a.heads = reinterpret_cast<int2*>(p.d_tables + o_hd);
+    p.d_heads = a.heads;
+    p.d_status = p.d_tables + offsetof(PlanCounts, status) / 4;
+    MASK_CUDA_TRY(cudaMemsetAsync(a.counts, 0, sizeof(PlanCounts), st));
+    rc = device_scan(PiecesIn{a}, PiecesOut{a}, p.W, spine.as<int64_t>(), nullptr, st);
+    if (rc == MASK_OK) rc = device_scan(GroupsIn{a}, GroupsOut{a}, n, spine.as<int64_t>(), nullptr, st);
+    if (rc == MASK_OK && !same_groups) rc = enqueue_warp_groups(a, work, st);
+    if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(cudaMemcpyAsync(counts, a.counts, sizeof(PlanCounts), cudaMemcpyDeviceToHost, st));
+    return MASK_OK;
 }
 
 // One device array for all tables, filled by one copy: sections start on 16-byte boundaries.
 static int upload_tables(mask_plan& p, const int32_t* soff, cudaStream_t st) {
     const auto& fo = p.h_frag_off; const auto& fw = p.h_frag_win; const auto& go = p.h_group_off;
-    const auto& wo = p.h_warp_off.empty() ? p.h_group_off : p.h_warp_off;
-    p.Gw = (int64_t)wo.size() - 1;
+    p.Gw = p.G;
     // split windows: first fragment and number of pieces; pieces are numbered in fragment order
     std::vector<int32_t> heads;
     p.P = 0;
@@ -239,8 +457,7 @@ static int upload_tables(mask_plan& p, const int32_t* soff, cudaStream_t st) {
     size_t at = 0;
     auto section = [&](size_t n) { const size_t o = at; at += (n + 3) & ~(size_t)3; return o; };
     const size_t o_fo = section(fo.size()), o_fw = section(fw.size()), o_fs = section(fw.size()), o_go = section(go.size()),
-                 o_gt = section(go.size()), o_wo = section(wo.size()), o_wt = section(wo.size()), o_hd = section(heads.size()),
-                 o_st = section(4);
+                 o_gt = section(go.size()), o_hd = section(heads.size()), o_st = section(4);
     HostStage stage;
     int rc = stage.get(at * sizeof(int32_t));
     if (rc != MASK_OK) return rc;
@@ -248,13 +465,11 @@ static int upload_tables(mask_plan& p, const int32_t* soff, cudaStream_t st) {
     std::copy(fo.begin(), fo.end(), h + o_fo);
     std::copy(fw.begin(), fw.end(), h + o_fw);
     std::copy(go.begin(), go.end(), h + o_go);
-    std::copy(wo.begin(), wo.end(), h + o_wo);
     std::copy(heads.begin(), heads.end(), h + o_hd);
     std::fill(h + o_st, h + o_st + 4, 0);
     int32_t slot = 0;
     for (int64_t f = 0; f < p.F; f++) h[o_fs + f] = whole(f) ? -1 : slot++;
     for (size_t g = 0; g < go.size(); g++) h[o_gt + g] = fo[go[g]];
-    for (size_t g = 0; g < wo.size(); g++) h[o_wt + g] = fo[wo[g]];
     rc = device_alloc(reinterpret_cast<void**>(&p.d_tables), at * sizeof(int32_t), st);
     if (rc != MASK_OK) return rc;
     p.d_frag_off = p.d_tables + o_fo;
@@ -262,8 +477,8 @@ static int upload_tables(mask_plan& p, const int32_t* soff, cudaStream_t st) {
     p.d_frag_slot = p.d_tables + o_fs;
     p.d_group_off = p.d_tables + o_go;
     p.d_group_tile = p.d_tables + o_gt;
-    p.d_warp_off = p.d_tables + o_wo;
-    p.d_warp_tile = p.d_tables + o_wt;
+    p.d_warp_off = p.d_group_off;
+    p.d_warp_tile = p.d_group_tile;
     p.d_heads = reinterpret_cast<const int2*>(p.d_tables + o_hd);
     p.d_status = p.d_tables + o_st;
     cudaError_t e = cudaMemcpyAsync(p.d_tables, h, at * sizeof(int32_t), cudaMemcpyHostToDevice, st);
@@ -305,8 +520,7 @@ extern "C" int mask_plan_multi_bind(const int32_t* h_val_soff, int32_t M, int32_
 
 namespace mask {
 
-// With d_val_sidx the column features are measured and the plan table is applied as well: the kernels that
-// measure run while the host builds the tables (both take 0.15 to 0.2 ms on a graph with 2^20 nodes).
+// With d_val_sidx the column features are measured and the plan table is applied as well.
 static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t M, int32_t K, int64_t T, int policy,
                        int32_t group_tiles, cudaStream_t st, mask_plan** out) {
     mask_plan* p = new mask_plan();
@@ -315,28 +529,42 @@ static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int
     p->T = T;
     p->policy = policy;
     p->group_tiles = group_tiles > 0 ? group_tiles : (policy == MASK_POLICY_STRICT_LB ? 64 : default_group_tiles(T));
-    p->auto_groups = group_tiles <= 0;
     // a piece may be longer than a group: it then is a group of its own
     p->piece_tiles = (group_tiles > 0 || policy != MASK_POLICY_AUTO) ? p->group_tiles : default_piece_tiles(T, p->W);
     HostStage stage;
     ColumnStatsJob job;
-    cudaEvent_t have_soff = nullptr;
+    DevScratch spine, work;
     auto body = [&]() -> int {
         MASK_CUDA_TRY(cudaGetDevice(&p->device));
-        const size_t bytes = ((size_t)p->W + 1) * sizeof(int32_t);
-        int rc = stage.get(bytes);
+        int rc = d_val_sidx ? job.enqueue(d_val_soff, d_val_sidx, M, K, T, 512, st) : MASK_OK;
         if (rc != MASK_OK) return rc;
-        const int32_t* soff = stage.as<int32_t>();
-        MASK_CUDA_TRY(cudaMemcpyAsync(stage.as<int32_t>(), d_val_soff, bytes, cudaMemcpyDeviceToHost, st));
-        if (d_val_sidx) {
-            MASK_CUDA_TRY(cudaEventCreateWithFlags(&have_soff, cudaEventDisableTiming));
-            MASK_CUDA_TRY(cudaEventRecord(have_soff, st));
-            rc = job.enqueue(d_val_soff, d_val_sidx, M, K, T, 512, st);
+        const bool on_device = policy == MASK_POLICY_AUTO;
+        const size_t bytes = on_device ? sizeof(PlanCounts) : ((size_t)p->W + 1) * sizeof(int32_t);
+        rc = stage.get(bytes);
+        if (rc != MASK_OK) return rc;
+        if (on_device) {
+            rc = enqueue_auto_tables(*p, d_val_soff, group_tiles > 0, job.device_local(), spine, work, stage.as<PlanCounts>(), st);
             if (rc != MASK_OK) return rc;
-            MASK_CUDA_TRY(cudaEventSynchronize(have_soff));
         } else {
-            MASK_CUDA_TRY(cudaStreamSynchronize(st));
+            MASK_CUDA_TRY(cudaMemcpyAsync(stage.as<int32_t>(), d_val_soff, bytes, cudaMemcpyDeviceToHost, st));
         }
+        MASK_CUDA_TRY(cudaStreamSynchronize(st));   // the plan may be used on any stream from here on
+        if (d_val_sidx) {
+            mask_column_features f;
+            job.finish(&f);
+            choose_plan_parameters(p, f);
+        }
+        if (on_device) {
+            const PlanCounts& c = *stage.as<PlanCounts>();
+            if (c.bad) return fail(MASK_ERR_INVALID_ARGUMENT, "val_soff does not start at 0 / end at T");
+            p->F = c.frags;
+            p->H = c.heads;
+            p->P = p->F - (p->W - p->H);
+            p->G = c.groups;
+            p->Gw = group_tiles > 0 ? p->G : c.warp_groups;
+            return MASK_OK;
+        }
+        const int32_t* soff = stage.as<int32_t>();
         if (soff[0] != 0 || (int64_t)soff[p->W] != T) return fail(MASK_ERR_INVALID_ARGUMENT, "val_soff does not start at 0 / end at T");
         if (policy == MASK_POLICY_REF_AUTO) {  // the bridge's automatic choice between its own two mappings
             mask_features f;
@@ -345,18 +573,10 @@ static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int
             if (group_tiles <= 0) p->group_tiles = 64;
         }
         build_tables(*p, soff);
-        if (d_val_sidx) {
-            MASK_CUDA_TRY(cudaStreamSynchronize(st));
-            mask_column_features f;
-            job.finish(&f);
-            choose_plan_parameters(p, f);
-        }
-        build_warp_groups(*p);
         return upload_tables(*p, soff, st);
     };
     const int rc = body();
     if (rc != MASK_OK) cudaStreamSynchronize(st);   // copies into the staging buffers may be in flight
-    if (have_soff) cudaEventDestroy(have_soff);
     if (rc != MASK_OK) {
         mask_plan_destroy(p);
         return rc;
@@ -450,6 +670,12 @@ extern "C" int mask_plan_status(const mask_plan* p, int32_t* h_status, void* str
 extern "C" int mask_plan_export(const mask_plan* p, int32_t* frag_offset, int32_t* frag_window, int32_t* group_offset) {
     using namespace mask;
     MASK_REQUIRE(p != nullptr, "plan is NULL");
+    if (p->policy == MASK_POLICY_AUTO) {   // these tables were built on the device
+        if (frag_offset) MASK_CUDA_TRY(cudaMemcpy(frag_offset, p->d_frag_off, ((size_t)p->F + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost));
+        if (frag_window && p->F) MASK_CUDA_TRY(cudaMemcpy(frag_window, p->d_frag_win, (size_t)p->F * sizeof(int32_t), cudaMemcpyDeviceToHost));
+        if (group_offset) MASK_CUDA_TRY(cudaMemcpy(group_offset, p->d_group_off, ((size_t)p->G + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost));
+        return MASK_OK;
+    }
     if (frag_offset) std::memcpy(frag_offset, p->h_frag_off.data(), p->h_frag_off.size() * sizeof(int32_t));
     if (frag_window && p->F) std::memcpy(frag_window, p->h_frag_win.data(), p->h_frag_win.size() * sizeof(int32_t));
     if (group_offset) std::memcpy(group_offset, p->h_group_off.data(), p->h_group_off.size() * sizeof(int32_t));

@@ -24,14 +24,12 @@ struct mask_plan {
     int64_t F = 0;  // fragments
     int64_t G = 0;  // groups (thread blocks)
     int64_t Gw = 0; // groups of the warp-level kernel
-    bool auto_groups = false; // nobody asked for a group size
     int32_t piece_tiles = 0;  // windows of more than 5/4 of this are split
     int64_t P = 0;  // fragments that are part of a split window
     int64_t H = 0;  // split windows
     int32_t nslab = 0;  // persistent kernel: 128-column slabs per column block (0 = the widest N fills)
     int device = 0;
-    std::vector<int32_t> h_frag_off, h_frag_win, h_group_off;
-    std::vector<int32_t> h_warp_off;     // empty: the same groups
+    std::vector<int32_t> h_frag_off, h_frag_win, h_group_off;   // tables built on the host (every policy but AUTO)
     int32_t* d_tables = nullptr;         // owned: one array that holds all of the following
     int32_t* d_frag_off = nullptr;
     int32_t* d_frag_win = nullptr;
