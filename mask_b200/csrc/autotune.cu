@@ -34,7 +34,8 @@ struct StatsHead {                 // what goes back to the host in one copy, fo
     uint32_t bins[kCountBins];     // columns by number of gathers
     uint32_t listed;
     int32_t local;                 // local_share >= kLocalShare, for the kernels that group the tiles
-    uint32_t pad[2];
+    uint32_t top_bin;              // largest of them that is not empty
+    uint32_t pad;
 };
 constexpr double kLocalShare = 0.9;
 
@@ -106,8 +107,14 @@ __global__ void __launch_bounds__(512) count_bins_kernel(const uint32_t* __restr
         else list[atomicAdd(&head->listed, 1u)] = c;
     }
     __syncthreads();
+    int top = 0;
     for (int i = threadIdx.x; i < kCountBins; i += 512)
-        if (bins[i]) atomicAdd(&head->bins[i], bins[i]);
+        if (bins[i]) {
+            atomicAdd(&head->bins[i], bins[i]);
+            top = i;
+        }
+    for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if ((threadIdx.x & 31) == 0 && top) atomicMax(&head->top_bin, (uint32_t)top);
 }
 
 }  // namespace
@@ -158,16 +165,20 @@ void ColumnStatsJob::finish(mask_column_features* out) const {
     std::vector<uint32_t> top(list, list + head.listed);
     std::sort(top.begin(), top.end(), std::greater<uint32_t>());
     unsigned long long reach[3] = {0, 0, 0};
+    int64_t left[3];
     for (int i = 0; i < 3; i++) {
         const int width = std::min(N_, 512 >> i);                               // columns of one gathered row at 4, 2, 1 slabs
         const int64_t rows = std::max<int64_t>(1, (int64_t)(l2_ / 2) / ((int64_t)width * 4));
         out->hub_columns[i] = (int32_t)std::min<int64_t>(rows, K_);
-        int64_t left = out->hub_columns[i];
-        for (size_t j = 0; j < top.size() && left > 0; j++, left--) reach[i] += top[j];
-        for (int b = kCountBins - 1; b > 0 && left > 0; b--) {
-            const int64_t take = std::min<int64_t>(left, head.bins[b]);
-            reach[i] += (unsigned long long)take * (unsigned)b;
-            left -= take;
+        left[i] = out->hub_columns[i];
+        for (size_t j = 0; j < top.size() && left[i] > 0; j++, left[i]--) reach[i] += top[j];
+    }
+    for (uint32_t b = head.top_bin; b > 0; b--) {
+        if (head.bins[b] == 0) continue;
+        for (int i = 0; i < 3; i++) {
+            const int64_t take = std::min<int64_t>(left[i], head.bins[b]);
+            reach[i] += (unsigned long long)take * b;
+            left[i] -= take;
         }
     }
     unsigned long long total = 0;
