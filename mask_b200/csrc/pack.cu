@@ -13,17 +13,16 @@
 //                  costs the same whatever the row lengths.  Rows that are not strictly ascending or columns
 //                  outside [0, K) raise an error flag.
 //   2. tiles       ceil(distinct / 8) per window, exclusive scan -> val_soff, total T; the scan also notes
-//                  the window in which every 128th tile lies.
-//   3. fill        one block per 128 consecutive tiles composes them 32 at a time in shared memory (a row of
-//                  the window is walked by 8 lanes from the entry where the tiles begin; positions ascend
-//                  along a row) and writes whole tiles, so a value array of 512 bytes a tile is written once,
-//                  coalesced, and never read.  ME-TCF and MCO count the entries per tile the same way first
-//                  (16 x 4-bit row histogram, 128-bit mask), scan the run lengths and place the entries.
+//                  the window in which every 64th tile lies.
+//   3. fill        one warp per 16 to 64 consecutive tiles composes them 8 at a time in shared memory (a row of
+//                  the window is walked from the entry where the tiles begin; positions ascend along a row)
+//                  and writes whole tiles, so a value array of 512 bytes a tile is written once, coalesced,
+//                  and never read.  ME-TCF and MCO count the entries per tile the same way first (16 x 4-bit row
+//                  histogram, 128-bit mask), scan the run lengths and place the entries.
 //
 // Measured on a power-law graph with 2^20 nodes (17.1 M entries, 1.97 M tiles; one read of the CSR and one
-// write of the packed arrays is 0.2 ms at copy speed): condense 0.45 ms, scan 0.02, SR-BCRS fill
-// 0.40; a binary search of every entry in its 15 sibling rows, two more scans and a scatter into cleared tiles took
-// 2.3 ms.
+// write of the packed arrays is 0.2 ms at copy speed): condense 0.37 ms, scan 0.01, SR-BCRS fill 0.32; a binary
+// search of every entry in its 15 sibling rows, two more scans and a scatter into cleared tiles took 2.3 ms.
 #include <algorithm>
 
 #include <cooperative_groups.h>
@@ -36,8 +35,8 @@
 
 namespace mask {
 
-constexpr int kFillTiles = 128;   // tiles a block of the fill writes ...
-constexpr int kFillSub = 32;      // ... and composes at a time
+constexpr int kFillTiles = 64;   // most tiles a warp of the fill writes, not counting the rest of a small window
+constexpr int kFillThreads = 128;
 
 struct PackScratch {
     int32_t* pos;           // nnz: condensed position of every entry
@@ -48,7 +47,7 @@ struct PackScratch {
     int32_t* hub_list;      // windows of condense_hub_kernel
     int32_t* first_window;  // per kFillTiles tiles (at most nnz tiles)
     int64_t* spine;         // per scan chunk
-    int32_t* status;        // [0] error flags, [2..3] int64 total, [4], [5] lengths of the lists
+    int32_t* status;        // [0] error flags, [4], [5] lengths of the lists
     size_t bytes;
 };
 
@@ -377,18 +376,31 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
     cluster.sync();   // nobody leaves while another block may still write its counts here
 }
 
+// What a host waits for: pinned memory that the last kernel writes itself, a copy's 6 us cheaper than a copy.
+struct HostWords {
+    int64_t total;
+    int32_t status;
+};
+
 // tiles per window, and their exclusive scan
 struct WindowTilesIn {
     const int32_t* distinct;
     int32_t W;
     __device__ int32_t operator()(int64_t w) const { return w < W ? (distinct[w] + kTileCols - 1) / kTileCols : 0; }
 };
-// first_window[c]: the window that holds tile c * kFillTiles (where the fill's block c begins)
+// first_window[c]: the window that holds tile c * kFillTiles
 struct SoffOut {
     int32_t* soff;
     int32_t* first_window;
+    int32_t W;
+    const int32_t* status;
+    HostWords* host;
     __device__ void operator()(int64_t w, int64_t before, int32_t tiles) const {
         soff[w] = (int32_t)before;
+        if (w == W) {
+            host->total = before;
+            host->status = *status;
+        }
         for (int64_t c = (before + kFillTiles - 1) / kFillTiles; c * kFillTiles < before + tiles; c++) first_window[c] = (int32_t)w;
     }
 };
@@ -410,7 +422,9 @@ struct FillArgs {
     const int32_t* pos;
     const int32_t* soff;
     const int32_t* first_window;
+    int32_t W;
     int64_t T;
+    int32_t chunk;             // tiles per warp: 16, 32 or 64
     int32_t skip_zero;         // MCO: entries with value 0 are not stored
     int32_t* sidx;
     float* block_val;          // SR-BCRS
@@ -423,142 +437,229 @@ struct FillArgs {
     float* out_val;
 };
 
-// One block per kFillTiles consecutive tiles, kFillSub at a time.  The entries of a row that fall into the
-// tiles are consecutive (positions ascend along a row): the 8 lanes of group tid / 8 find their number with an
-// 8-way search, then all threads take the entries of the 16 rows as one list -- a hub row with most of the
-// entries is not left to 8 lanes.  What bounds it is writing the tiles (SR-BCRS); several blocks per SM
-// cover the chain first_window -> val_soff -> rows -> positions -> values.
+// 32-bit halves of the words that hold a tile's row counts (16 nibbles) and its mask (128 bits)
+__device__ __forceinline__ void count_entry(uint32_t* words, int tile, int row) {
+    atomicAdd(words + 2 * tile + (row >> 3), 1u << (4 * (row & 7)));
+}
+__device__ __forceinline__ void mark_entry(uint32_t* words, int tile, int phys) {
+    atomicOr(words + 4 * tile + (phys >> 5), 1u << (phys & 31));
+}
+
+// One warp per `chunk` consecutive tiles, kSub at a time, composed in shared memory; nothing waits for another
+// warp.  The entries of a row that fall into the tiles are consecutive (positions ascend along a row): a few lanes
+// take each of the 16 rows, eight entries of it per turn, until one lies behind the tiles; a few rows that go on are
+// then taken by all lanes, one after the other.  A window that fits into a chunk is written by the warp in whose chunk
+// it begins, so that only larger ones cost a search for where a chunk begins in each row.  What bounds it is the chain
+// rows -> positions and values -> tile of every step, which 40 warps an SM cover.  Blocks of 128 threads that composed
+// 32 tiles together took, against this: 396 us, now 323 (SR-BCRS, 2^20 nodes, 1.97 M tiles); 97 us, now 15 (47 000 nodes);
+// ME-TCF of 30 000 nodes 144 us in two passes, now 31.
 template <int MODE>
-__global__ void __launch_bounds__(128) fill_kernel(const FillArgs p) {
+__global__ void __launch_bounds__(kFillThreads, 10) fill_kernel(const FillArgs p) {
     constexpr bool kIds = MODE == kFillSrbcrs || MODE == kFillMetcf || MODE == kFillMco;
     constexpr bool kMco = MODE == kMaskMco || MODE == kFillMco;
-    __shared__ __align__(16) float tile[MODE == kFillSrbcrs ? kFillSub * kTileElems : 4];
-    __shared__ unsigned long long words[MODE == kFillSrbcrs ? 1 : (kMco ? 2 * kFillSub : kFillSub)];
-    __shared__ int32_t begin[kFillSub];
-    __shared__ int row_entry[kWinRows], row_first[kWinRows + 1], row_begin[kWinRows];
-    const int tid = threadIdx.x, r = tid >> 3, l = tid & 7, group = (tid & 31) & ~7;
-    const int64_t block_end = min(p.T, ((int64_t)blockIdx.x + 1) * kFillTiles);
-    int64_t t = (int64_t)blockIdx.x * kFillTiles;
-    int w = p.first_window[blockIdx.x];
-    int64_t s0 = p.soff[w], s1 = p.soff[w + 1];
-    while (t < block_end) {
-        const int row = w * kWinRows + r;
-        const int beg = __ldg(p.rows + row), end = __ldg(p.rows + row + 1);
-        const int base = kIds ? __ldg(p.rows + w * kWinRows) : 0, n_cols = kIds ? __ldg(p.distinct + w) : 0;
-        const int64_t te = s1 < block_end ? s1 : block_end;
-        const int64_t next_s1 = te < block_end ? p.soff[w + 2] : 0;
-        int e = beg;
-        if (t > s0) {   // the block begins inside this window: first entry of the row at or after tile t
-            const int first = (int)(t - s0) * kTileCols;
-            int hi = end;
-            while (e < hi) {
-                const int mid = (e + hi) >> 1;
-                if (__ldg(p.pos + mid) < first) e = mid + 1; else hi = mid;
+    constexpr int kWarps = kFillThreads / 32;
+    // lanes of a row, rows at once; entries of a lane: eight of a row per turn.  A load touches as many lines as rows:
+    // with sixteen L1 is what bounds the SR-BCRS fill, with four the turns cost too many instructions.
+    constexpr int kLanes = MODE == kFillSrbcrs ? 4 : 2, kAtOnce = 32 / kLanes, kSets = kWinRows / kAtOnce, kPer = 8 / kLanes;
+    constexpr unsigned kGroup = (1u << kLanes) - 1;
+    constexpr int kSub = MODE == kFillSrbcrs ? 8 : 32, kWords = kMco ? 2 * kSub : kSub;
+    __shared__ __align__(16) float tiles[MODE == kFillSrbcrs ? kWarps * kSub * kTileElems : 4];
+    __shared__ unsigned long long word_store[MODE == kFillSrbcrs ? 1 : kWarps * kWords];
+    __shared__ int32_t begin_store[MODE == kFillMetcf || MODE == kFillMco ? kWarps * kSub : 1];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane / kLanes, l = lane % kLanes, group = g * kLanes;
+    float* const tile = tiles + (MODE == kFillSrbcrs ? warp * kSub * kTileElems : 0);
+    unsigned long long* const words = word_store + (MODE == kFillSrbcrs ? 0 : warp * kWords);
+    uint32_t* const half_words = reinterpret_cast<uint32_t*>(words);
+    int32_t* const begin = begin_store + (MODE == kFillMetcf || MODE == kFillMco ? warp * kSub : 0);
+
+    const int64_t chunk_begin = ((int64_t)blockIdx.x * kWarps + warp) * p.chunk;
+    if (chunk_begin >= p.T) return;
+    // window of tile t
+    auto locate = [&](int64_t t) {
+        int w = p.first_window[t / kFillTiles];
+        for (;;) {   // windows from w on that end at or before t
+            const int behind = __popc(__ballot_sync(0xffffffffu, __ldg(p.soff + min(w + 1 + lane, p.W)) <= t));
+            w += behind;
+            if (behind < 32) return w;
+        }
+    };
+    int w = locate(chunk_begin);
+    int64_t s0 = p.soff[w], s1 = p.soff[w + 1], t = chunk_begin, chunk_end = min(p.T, chunk_begin + p.chunk);
+    if (t > s0 && s1 - s0 <= p.chunk) t = s1;
+    if (chunk_end < p.T) {
+        const int last = locate(chunk_end);
+        const int64_t b0 = p.soff[last], b1 = p.soff[last + 1];
+        if (b0 < chunk_end && b1 - b0 <= p.chunk) chunk_end = b1;
+    }
+    if (t >= chunk_end) return;
+    while (s1 <= t) {
+        w++;
+        s0 = s1;
+        s1 = p.soff[w + 1];
+    }
+    if (MODE == kFillSrbcrs) {
+        for (int i = lane; i < kSub * kTileElems / 4; i += 32) reinterpret_cast<float4*>(tile)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncwarp();
+    }
+    // entry ee of window row rr (whose first is row_beg), at position q, in tiles from position p0 on
+    auto place = [&](int rr, int row_beg, int ee, int q, float v, int p0) {
+        const int lt = (q - p0) >> 3, cc = q & 7;
+        if (MODE == kFillSrbcrs) {
+            tile[lt * kTileElems + sw223(rr * kTileCols + cc)] = v;
+            if (p.edge_to_col) p.edge_to_col[ee] = q;
+            if (p.edge_to_row) p.edge_to_row[ee] = w * kWinRows + rr;
+        } else if (MODE == kCountMetcf) {
+            count_entry(half_words, lt, rr);
+        } else if (MODE == kFillMetcf) {   // entries of earlier rows, then earlier entries of this row
+            int at = begin[lt] + (rr == 0 ? 0 : nibble_sum(words[lt] & ((1ull << (4 * rr)) - 1ull)));
+            for (int j = ee - 1; j >= row_beg && (__ldg(p.pos + j) >> 3) == (q >> 3); j--) at++;
+            p.coo_idx[at] = sw123(rr * kTileCols + cc);
+            p.out_val[at] = v;
+        } else if (!(p.skip_zero && v == 0.0f)) {
+            const int phys = sw123(rr * kTileCols + cc), upper = phys >> 6;
+            if (MODE == kMaskMco) {
+                mark_entry(half_words, lt, phys);
+            } else {   // values in ascending bit order: the slot is the number of bits below
+                const int below = __popcll(words[2 * lt + upper] & ((1ull << (phys & 63)) - 1ull));
+                p.out_val[begin[lt] + below + (upper ? __popcll(words[2 * lt]) : 0)] = v;
             }
         }
-        for (int64_t c = t; c < te; c += kFillSub) {
-            const int nt = (int)min((int64_t)kFillSub, te - c);
+    };
+    for (;;) {
+                int beg[kSets], e[kSets], end[kSets];
+#pragma unroll
+        for (int k = 0; k < kSets; k++) {
+            e[k] = beg[k] = __ldg(p.rows + w * kWinRows + kAtOnce * k + g);
+            end[k] = __ldg(p.rows + w * kWinRows + kAtOnce * k + g + 1);
+        }
+        const int base = kIds || t > s0 ? __ldg(p.rows + w * kWinRows) : 0, n_cols = kIds ? __ldg(p.distinct + w) : 0;
+        const int64_t te = min(s1, chunk_end);
+        const int64_t next_s1 = te < chunk_end ? p.soff[w + 2] : 0;
+        if (t > s0) {   // the chunk begins inside this window: first entry of every row at or after tile t
+            // `first` columns come before it, all of them in the row but for those that only other rows have
+            const int first = (int)(t - s0) * kTileCols, all = __ldg(p.rows + (w + 1) * kWinRows) - base;
+#pragma unroll
+            for (int k = 0; k < kSets; k++) {
+                int at = min(end[k], beg[k] + max(0, first - (all - (end[k] - beg[k]))));
+                for (int left = min(end[k], beg[k] + first) - at; __any_sync(0xffffffffu, left > 0);) {   // kLanes + 1 parts
+                    const int stride = left / (kLanes + 1) + 1, probe = (l + 1) * stride;
+                    const bool below = left > 0 && probe <= left && __ldg(p.pos + at + probe - 1) < first;
+                    const int hits = __popc((__ballot_sync(0xffffffffu, below) >> group) & kGroup);   // the probes that hit come first
+                    at += hits * stride;
+                    left = min(hits == kLanes ? left : stride - 1, left - hits * stride);
+                }
+                e[k] = at;
+            }
+        }
+        for (int64_t c = t; c < te; c += kSub) {
+            const int nt = (int)min((int64_t)kSub, te - c);
             const int p0 = (int)(c - s0) * kTileCols, limit = p0 + nt * kTileCols;
-            if (MODE == kFillSrbcrs) {
-                for (int i = tid; i < nt * 32; i += 128) reinterpret_cast<float4*>(tile)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            } else if (MODE == kCountMetcf) {
-                if (tid < nt) words[tid] = 0ull;
+            if (MODE == kCountMetcf) {
+                words[lane] = 0ull;
             } else if (MODE == kMaskMco) {
-                if (tid < 2 * nt) words[tid] = 0ull;
+                words[lane] = words[lane + 32] = 0ull;
             } else if (MODE == kFillMetcf) {
-                if (tid < nt) { words[tid] = p.tile_rows[c + tid]; begin[tid] = p.off[2 * (c + tid)]; }
-            } else {
-                if (tid < 2 * nt) words[tid] = p.masks[2 * c + tid];
-                if (tid < nt) begin[tid] = p.off[c + tid];
+                if (lane < nt) { words[lane] = p.tile_rows[c + lane]; begin[lane] = p.off[2 * (c + lane)]; }
+            } else if (MODE == kFillMco) {
+                for (int i = lane; i < 2 * nt; i += 32) words[i] = p.masks[2 * c + i];
+                if (lane < nt) begin[lane] = p.off[c + lane];
             }
             if (kIds) {   // tail slots of a window repeat its last column, or are 0 (ME-TCF)
-                for (int i = tid; i < nt * kTileCols; i += 128) {
+                for (int i = lane; i < nt * kTileCols; i += 32) {
                     const int q = p0 + i;
                     p.sidx[c * kTileCols + i] = (MODE == kFillMetcf && q >= n_cols) ? 0 : __ldg(p.cols + base + min(q, n_cols - 1));
                 }
             }
-            // entries of this row that lie in the tiles: [e, e + cnt)
-            int cnt = 0;
-            for (int left = min(end - e, nt * kTileCols);;) {
-                const int stride = (left + 7) >> 3, probe = min((l + 1) * stride, left);
-                const bool below = left > 0 && __ldg(p.pos + e + cnt + probe - 1) < limit;
-                const int hits = __popc((__ballot_sync(0xffffffffu, below) >> group) & 0xffu);   // the probes that hit come first
-                const int step = hits == 8 ? left : hits * stride;
-                cnt += step;
-                left = hits == 8 ? 0 : min(stride - 1, left - step);
-                if (!__any_sync(0xffffffffu, left > 0)) break;
-            }
-            if (l == 0) { row_entry[r] = e; row_begin[r] = beg; row_first[r + 1] = cnt; }
-            e += cnt;
-            __syncthreads();
-            if (tid < 32) {
-                int x = tid < kWinRows ? row_first[tid + 1] : 0;
-                for (int o = 1; o < kWinRows; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, x, o);
-                    if (tid >= o) x += y;
-                }
-                if (tid < kWinRows) row_first[tid + 1] = x;
-                if (tid == 0) row_first[0] = 0;
-            }
-            __syncthreads();
-            for (int i = tid; i < row_first[kWinRows]; i += 128) {
-                int rr = 0;   // last row whose first list index is <= i
+            if (MODE != kFillSrbcrs) __syncwarp();
+            unsigned open = (1u << kSets) - 1;   // this lane's rows that may have more
+            for (int turn = 1;; turn++) {
+                int q[kSets][kPer];
+                float v[kSets][kPer];
 #pragma unroll
-                for (int half = kWinRows / 2; half > 0; half >>= 1)
-                    if (row_first[rr + half] <= i) rr += half;
-                const int ee = row_entry[rr] + i - row_first[rr];
-                const int q = __ldg(p.pos + ee), lt = (q - p0) >> 3, cc = q & 7;
-                if (MODE == kFillSrbcrs) {
-                    tile[lt * kTileElems + sw223(rr * kTileCols + cc)] = __ldg(p.values + ee);
-                    if (p.edge_to_col) p.edge_to_col[ee] = q;
-                    if (p.edge_to_row) p.edge_to_row[ee] = w * kWinRows + rr;
-                } else if (MODE == kCountMetcf) {
-                    atomicAdd(words + lt, 1ull << (4 * rr));
-                } else if (MODE == kFillMetcf) {   // entries of earlier rows, then earlier entries of this row
-                    int at = begin[lt] + (rr == 0 ? 0 : nibble_sum(words[lt] & ((1ull << (4 * rr)) - 1ull)));
-                    for (int j = ee - 1; j >= row_begin[rr] && (__ldg(p.pos + j) >> 3) == (q >> 3); j--) at++;
-                    p.coo_idx[at] = sw123(rr * kTileCols + cc);
-                    p.out_val[at] = p.values ? __ldg(p.values + ee) : 1.0f;
-                } else {
-                    const float v = p.values ? __ldg(p.values + ee) : 1.0f;
-                    if (!(p.skip_zero && p.values && v == 0.0f)) {
-                        const int phys = sw123(rr * kTileCols + cc), upper = phys >> 6;
-                        if (MODE == kMaskMco) {
-                            atomicOr(words + 2 * lt + upper, 1ull << (phys & 63));
-                        } else {   // values in ascending bit order: the slot is the number of bits below
-                            const int below = __popcll(words[2 * lt + upper] & ((1ull << (phys & 63)) - 1ull));
-                            p.out_val[begin[lt] + below + (upper ? __popcll(words[2 * lt]) : 0)] = v;
-                        }
+                for (int k = 0; k < kSets; k++)
+#pragma unroll
+                    for (int j = 0; j < kPer; j++) {
+                        const int i = e[k] + l + kLanes * j;
+                        const bool have = (open >> k & 1) && i < end[k];
+                        q[k][j] = have ? __ldg(p.pos + i) : 0x7fffffff;
+                        v[k][j] = p.values && have ? __ldg(p.values + i) : 1.0f;
+                    }
+                int rows_open = 0;
+#pragma unroll
+                for (int k = 0; k < kSets; k++) {
+                    int n = 0;
+#pragma unroll
+                    for (int j = 0; j < kPer; j++) {
+                        const bool in = q[k][j] < limit;
+                        if (in) place(kAtOnce * k + g, beg[k], e[k] + l + kLanes * j, q[k][j], v[k][j], p0);
+                        n += __popc((__ballot_sync(0xffffffffu, in) >> group) & kGroup);
+                    }
+                    e[k] += n;
+                    if (n < kLanes * kPer) open &= ~(1u << k);
+                    rows_open += __popc(__ballot_sync(0xffffffffu, n == kLanes * kPer)) / kLanes;
+                }
+                if (rows_open == 0) break;
+                if (rows_open > turn) continue;
+                // few rows that go on and on: all lanes on one after the other
+#pragma unroll
+                for (int k = 0; k < kSets; k++) {
+                    for (unsigned left = __ballot_sync(0xffffffffu, (open >> k & 1) && l == 0); left != 0; left &= left - 1) {
+                        const int from = __ffs(left) - 1, row_beg = __shfl_sync(0xffffffffu, beg[k], from), row_end = __shfl_sync(0xffffffffu, end[k], from);
+                        int at = __shfl_sync(0xffffffffu, e[k], from), taken;
+                        do {
+                            int q2[2];
+                            float v2[2];
+#pragma unroll
+                            for (int j = 0; j < 2; j++) {
+                                const int i = at + lane + 32 * j;
+                                q2[j] = i < row_end ? __ldg(p.pos + i) : 0x7fffffff;
+                                v2[j] = p.values && i < row_end ? __ldg(p.values + i) : 1.0f;
+                            }
+                            taken = 0;
+#pragma unroll
+                            for (int j = 0; j < 2; j++) {
+                                if (q2[j] < limit) place(kAtOnce * k + from / kLanes, row_beg, at + lane + 32 * j, q2[j], v2[j], p0);
+                                taken += __popc(__ballot_sync(0xffffffffu, q2[j] < limit));
+                            }
+                            at += taken;
+                        } while (taken == 64);
+                        if (group == from) e[k] = at;
                     }
                 }
+                break;
             }
-            __syncthreads();
-            if (MODE == kFillSrbcrs) {
+            __syncwarp();
+            if (MODE == kFillSrbcrs) {   // and clear what was read for the next tiles
                 float4* out = reinterpret_cast<float4*>(p.block_val + c * kTileElems);
-                for (int i = tid; i < nt * 32; i += 128) out[i] = reinterpret_cast<const float4*>(tile)[i];
+#pragma unroll
+                for (int i = 0; i < kSub; i++) {
+                    if (i >= nt) break;
+                    float4* from = reinterpret_cast<float4*>(tile) + i * 32 + lane;
+                    out[i * 32 + lane] = *from;
+                    *from = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
             } else if (MODE == kCountMetcf) {
-                if (tid < nt) p.tile_rows[c + tid] = words[tid];
+                if (lane < nt) p.tile_rows[c + lane] = words[lane];
             } else if (MODE == kMaskMco) {
-                if (tid < 2 * nt) p.masks[2 * c + tid] = words[tid];
-            } else if (tid < nt) {   // the padding at the end of the tile's run
-                const int cnt = MODE == kFillMetcf ? nibble_sum(words[tid]) : __popcll(words[2 * tid]) + __popcll(words[2 * tid + 1]);
+                for (int i = lane; i < 2 * nt; i += 32) p.masks[2 * c + i] = words[i];
+            } else if (lane < nt) {   // the padding at the end of the tile's run
+                const int cnt = MODE == kFillMetcf ? nibble_sum(words[lane]) : __popcll(words[2 * lane]) + __popcll(words[2 * lane + 1]);
                 const int pad = MODE == kFillMetcf ? (cnt + 7) & ~7 : (cnt + 3) & ~3;
                 for (int i = cnt; i < pad; i++) {
-                    if (MODE == kFillMetcf) p.coo_idx[begin[tid] + i] = 0;
-                    p.out_val[begin[tid] + i] = 0.f;
+                    if (MODE == kFillMetcf) p.coo_idx[begin[lane] + i] = 0;
+                    p.out_val[begin[lane] + i] = 0.f;
                 }
             }
-            __syncthreads();
+            __syncwarp();
         }
         t = te;
-        if (t == s1 && t < block_end) {   // on to the next window with tiles
+        if (t == chunk_end) return;
+        w++;   // on to the next window with tiles
+        s0 = s1;
+        s1 = next_s1;
+        while (s1 == s0) {
             w++;
-            s0 = s1;
-            s1 = next_s1;
-            while (s1 == s0) {
-                w++;
-                s1 = p.soff[w + 1];
-            }
+            s1 = p.soff[w + 1];
         }
     }
 }
@@ -577,10 +678,14 @@ struct CooOffOut {
     const unsigned long long* tile_rows;
     int32_t* off;
     int64_t T;
+    HostWords* host;
     __device__ void operator()(int64_t t, int64_t before, int32_t v) const {
         off[2 * t] = (int32_t)before;
         off[2 * t + 1] = (int32_t)before + nibble_sum(tile_rows[t]);
-        if (t == T - 1) off[2 * T] = (int32_t)(before + v);
+        if (t == T - 1) {
+            off[2 * T] = (int32_t)(before + v);
+            host->total = before + v;
+        }
     }
 };
 struct McoCountIn {
@@ -590,9 +695,13 @@ struct McoCountIn {
 struct McoOffOut {
     int32_t* off;
     int64_t T;
+    HostWords* host;
     __device__ void operator()(int64_t t, int64_t before, int32_t v) const {
         off[t] = (int32_t)before;
-        if (t == T - 1) off[T] = (int32_t)(before + v);
+        if (t == T - 1) {
+            off[T] = (int32_t)(before + v);
+            host->total = before + v;
+        }
     }
 };
 
@@ -600,13 +709,17 @@ static inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n
 
 template <int MODE>
 static int launch_fill(const FillArgs& a, cudaStream_t st) {
-    fill_kernel<MODE><<<blocks_for(a.T, kFillTiles), 128, 0, st>>>(a);
+    fill_kernel<MODE><<<blocks_for(a.T, a.chunk * (kFillThreads / 32)), kFillThreads, 0, st>>>(a);
     MASK_CUDA_TRY(cudaGetLastError());
     return MASK_OK;
 }
 
-static FillArgs fill_args(const PackScratch& s, const float* d_values, const int32_t* d_val_soff, int64_t T) {
+static FillArgs fill_args(const PackScratch& s, int32_t M, const float* d_values, const int32_t* d_val_soff, int64_t T) {
     FillArgs a{};
+    a.W = (M + kWinRows - 1) / kWinRows;
+    // a chunk costs its searches, so it is as long as leaves the resident warps (48 an SM) one each
+    a.chunk = kFillTiles;
+    while (a.chunk > 16 && T < (int64_t)48 * sm_count() * a.chunk) a.chunk /= 2;
     a.rows = s.rows;
     a.cols = s.cols;
     a.distinct = s.distinct;
@@ -616,17 +729,6 @@ static FillArgs fill_args(const PackScratch& s, const float* d_values, const int
     a.first_window = s.first_window;
     a.T = T;
     return a;
-}
-
-// Copies n int32 words at d_src to the host and waits for them.
-static int read_words(const int32_t* d_src, int32_t* out, int n, cudaStream_t st) {
-    HostStage stage;
-    int rc = stage.get((size_t)n * 4);
-    if (rc != MASK_OK) return rc;
-    MASK_CUDA_TRY(cudaMemcpyAsync(stage.as<int32_t>(), d_src, (size_t)n * 4, cudaMemcpyDeviceToHost, st));
-    MASK_CUDA_TRY(cudaStreamSynchronize(st));
-    memcpy(out, stage.as<int32_t>(), (size_t)n * 4);
-    return MASK_OK;
 }
 
 }  // namespace mask
@@ -682,16 +784,17 @@ extern "C" int mask_pack_analyze(const int32_t* d_rowptr, const int32_t* d_colin
             MASK_CUDA_TRY(cudaGetLastError());
         }
     }
-    int rc = device_scan(WindowTilesIn{s.distinct, W}, SoffOut{d_val_soff, s.first_window}, (int64_t)W + 1, s.spine,
-                         reinterpret_cast<int64_t*>(s.status + 2), st);
+    HostStage stage;
+    int rc = stage.get(sizeof(HostWords));
     if (rc != MASK_OK) return rc;
-    int32_t host_status[4] = {0, 0, 0, 0};
-    rc = read_words(s.status, host_status, 4, st);
+    HostWords* host = stage.as<HostWords>();
+    rc = device_scan(WindowTilesIn{s.distinct, W}, SoffOut{d_val_soff, s.first_window, W, s.status, host}, (int64_t)W + 1, s.spine, st);
+    const cudaError_t e = cudaStreamSynchronize(st);   // also after a failure: a kernel may still write the host's words
     if (rc != MASK_OK) return rc;
-    if (host_status[0] & 2) return fail(MASK_ERR_COLUMN_RANGE, "a column id is outside [0, K)");
-    if (host_status[0] & 1) return fail(MASK_ERR_UNSORTED_ROWS, "CSR rows must hold strictly ascending column ids");
-    int64_t T;
-    memcpy(&T, host_status + 2, 8);
+    MASK_CUDA_TRY(e);
+    if (host->status & 2) return fail(MASK_ERR_COLUMN_RANGE, "a column id is outside [0, K)");
+    if (host->status & 1) return fail(MASK_ERR_UNSORTED_ROWS, "CSR rows must hold strictly ascending column ids");
+    const int64_t T = host->total;
     if (T >= (int64_t)1 << 31 || T * kTileElems < 0) return fail(MASK_ERR_INDEX_OVERFLOW, "tile count does not fit int32");
     *h_T = T;
     return MASK_OK;
@@ -711,7 +814,7 @@ extern "C" int mask_srbcrs_fill(const int32_t* d_rowptr, const int32_t* d_colind
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int W = (M + kWinRows - 1) / kWinRows;
     if (T > 0) {
-        FillArgs a = fill_args(s, d_values, d_val_soff, T);
+        FillArgs a = fill_args(s, M, d_values, d_val_soff, T);
         a.sidx = d_val_sidx;
         a.block_val = d_val_block_val;
         a.edge_to_col = d_edge_to_col;
@@ -742,16 +845,19 @@ extern "C" int mask_metcf_offsets(const int32_t* d_rowptr, int32_t M, int64_t nn
         MASK_CUDA_TRY(cudaMemsetAsync(d_val_coo_off, 0, 4, st));
         return MASK_OK;
     }
-    FillArgs a = fill_args(s, nullptr, d_val_soff, T);
+    FillArgs a = fill_args(s, M, nullptr, d_val_soff, T);
     a.tile_rows = rows;
     int rc = launch_fill<kCountMetcf>(a, st);
     if (rc != MASK_OK) return rc;
     // the spine is sized for max(nnz, W+1) items and T <= nnz
-    rc = device_scan(TilePadIn{rows}, CooOffOut{rows, d_val_coo_off, T}, T, s.spine, reinterpret_cast<int64_t*>(s.status + 2), st);
+    HostStage stage;
+    rc = stage.get(sizeof(HostWords));
     if (rc != MASK_OK) return rc;
-    int64_t total = 0;
-    rc = read_words(s.status + 2, reinterpret_cast<int32_t*>(&total), 2, st);
+    rc = device_scan(TilePadIn{rows}, CooOffOut{rows, d_val_coo_off, T, stage.as<HostWords>()}, T, s.spine, st);
+    const cudaError_t e = cudaStreamSynchronize(st);
     if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(e);
+    const int64_t total = stage.as<HostWords>()->total;
     if (total >= (int64_t)1 << 31) return fail(MASK_ERR_INDEX_OVERFLOW, "nnz_pad does not fit int32");
     *h_nnz_pad = total;
     return MASK_OK;
@@ -770,7 +876,7 @@ extern "C" int mask_metcf_fill(const int32_t* d_rowptr, const int32_t* d_colind,
     PackScratch s = carve(const_cast<void*>(d_scratch), M, nnz);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (T == 0) return MASK_OK;
-    FillArgs a = fill_args(s, d_values, d_val_soff, T);
+    FillArgs a = fill_args(s, M, d_values, d_val_soff, T);
     a.sidx = d_val_sidx;
     a.tile_rows = const_cast<unsigned long long*>(reinterpret_cast<const unsigned long long*>(d_tile_rows));
     a.off = d_val_coo_off;
@@ -794,16 +900,19 @@ extern "C" int mask_mco_offsets(const float* d_values, int32_t M, int64_t nnz, c
         MASK_CUDA_TRY(cudaMemsetAsync(d_val_mco_off, 0, 4, st));
         return MASK_OK;
     }
-    FillArgs a = fill_args(s, d_values, d_val_soff, T);
+    FillArgs a = fill_args(s, M, d_values, d_val_soff, T);
     a.skip_zero = skip_zero_values;
     a.masks = masks;
     int rc = launch_fill<kMaskMco>(a, st);
     if (rc != MASK_OK) return rc;
-    rc = device_scan(McoCountIn{masks}, McoOffOut{d_val_mco_off, T}, T, s.spine, reinterpret_cast<int64_t*>(s.status + 2), st);
+    HostStage stage;
+    rc = stage.get(sizeof(HostWords));
     if (rc != MASK_OK) return rc;
-    int64_t total = 0;
-    rc = read_words(s.status + 2, reinterpret_cast<int32_t*>(&total), 2, st);
+    rc = device_scan(McoCountIn{masks}, McoOffOut{d_val_mco_off, T, stage.as<HostWords>()}, T, s.spine, st);
+    const cudaError_t e = cudaStreamSynchronize(st);
     if (rc != MASK_OK) return rc;
+    MASK_CUDA_TRY(e);
+    const int64_t total = stage.as<HostWords>()->total;
     if (total >= (int64_t)1 << 31) return fail(MASK_ERR_INDEX_OVERFLOW, "value count does not fit int32");
     *h_nval = total;
     return MASK_OK;
@@ -821,7 +930,7 @@ extern "C" int mask_mco_fill(const int32_t* d_rowptr, const float* d_values, int
     PackScratch s = carve(const_cast<void*>(d_scratch), M, nnz);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (T == 0) return MASK_OK;
-    FillArgs a = fill_args(s, d_values, d_val_soff, T);
+    FillArgs a = fill_args(s, M, d_values, d_val_soff, T);
     a.skip_zero = skip_zero_values;
     a.masks = const_cast<unsigned long long*>(reinterpret_cast<const unsigned long long*>(d_val_mco_mask));
     a.off = d_val_mco_off;

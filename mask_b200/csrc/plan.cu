@@ -156,7 +156,7 @@ static void build_tables(mask_plan& p, const int32_t* soff) {
 constexpr int32_t kFragCost = 4;
 constexpr int64_t kHigh = (int64_t)1 << 32;   // the scans carry two counts: one in each half
 
-struct PlanCounts {          // on the device in front of the tables, and back on the host
+struct PlanCounts {          // on the device in front of the tables, and on the host
     int32_t frags, heads, groups, warp_groups, bad, pad[3];
     int32_t status[4];
 };
@@ -168,6 +168,7 @@ struct TableArgs {
     int32_t* frag_off; int32_t* frag_win; int32_t* frag_slot; int2* heads;
     int32_t* group_off; int32_t* group_tile; int32_t* warp_off; int32_t* warp_tile;
     PlanCounts* counts;
+    PlanCounts* host;        // pinned: the counts for the host, `bad` until the kernels that know them write them
     const int32_t* local;    // NULL: not known to be
     int32_t resident;        // resident blocks of the tcgen05 kernel
     int32_t takers;          // resident blocks of the warp-level kernel
@@ -248,6 +249,10 @@ struct GroupsOut {
             a.group_off[g + v] = F;
             a.group_tile[g + v] = (int32_t)a.T;
             a.counts->groups = g + v;
+            a.host->frags = F;
+            a.host->heads = a.counts->heads;
+            a.host->groups = g + v;
+            a.host->bad = 0;
         }
     }
 };
@@ -360,7 +365,7 @@ __global__ void __launch_bounds__(kChunkThreads) warp_group_write_kernel(const T
         if (base + n == F) {
             a.warp_off[g] = (int32_t)F;
             a.warp_tile[g] = (int32_t)a.T;
-            a.counts->warp_groups = g;
+            a.host->warp_groups = g;
         }
     }
     __syncthreads();
@@ -394,7 +399,7 @@ static int enqueue_warp_groups(const TableArgs& a, DevScratch& work, cudaStream_
     return MASK_OK;
 }
 
-// Enqueues the tables of an AUTO plan and the copy of their sizes to `counts` (pinned).
+// Enqueues the tables of an AUTO plan; their sizes are in `counts` (pinned) when they are complete.
 static int enqueue_auto_tables(mask_plan& p, const int32_t* d_val_soff, bool same_groups, const int32_t* d_local, DevScratch& spine,
                                DevScratch& work, PlanCounts* counts, cudaStream_t st) {
     TableArgs a{};
@@ -408,6 +413,9 @@ static int enqueue_auto_tables(mask_plan& p, const int32_t* d_val_soff, bool sam
     a.resident = 2 * sm_count();
     a.takers = sm_count() * kWarpBlocksPerSm;
     a.same_groups = same_groups;
+    a.host = counts;
+    *counts = PlanCounts{};
+    counts->bad = 1;
     if (a.max_frags >= ((int64_t)1 << 31) - 1) return fail(MASK_ERR_INDEX_OVERFLOW, "the number of tasks does not fit int32");
     size_t at = sizeof(PlanCounts) / 4;
     auto section = [&](int64_t n) { const size_t o = at; at += ((size_t)n + 3) & ~(size_t)3; return o; };
@@ -431,11 +439,10 @@ static int enqueue_auto_tables(mask_plan& p, const int32_t* d_val_soff, bool sam
     p.d_heads = a.heads;
     p.d_status = p.d_tables + offsetof(PlanCounts, status) / 4;
     MASK_CUDA_TRY(cudaMemsetAsync(a.counts, 0, sizeof(PlanCounts), st));
-    rc = device_scan(PiecesIn{a}, PiecesOut{a}, p.W, spine.as<int64_t>(), nullptr, st);
-    if (rc == MASK_OK) rc = device_scan(GroupsIn{a}, GroupsOut{a}, n, spine.as<int64_t>(), nullptr, st);
+    rc = device_scan(PiecesIn{a}, PiecesOut{a}, p.W, spine.as<int64_t>(), st);
+    if (rc == MASK_OK) rc = device_scan(GroupsIn{a}, GroupsOut{a}, n, spine.as<int64_t>(), st);
     if (rc == MASK_OK && !same_groups) rc = enqueue_warp_groups(a, work, st);
     if (rc != MASK_OK) return rc;
-    MASK_CUDA_TRY(cudaMemcpyAsync(counts, a.counts, sizeof(PlanCounts), cudaMemcpyDeviceToHost, st));
     return MASK_OK;
 }
 

@@ -203,3 +203,25 @@ def test_session_column_chunks(oracle_mod, rows, N):
             _assert_close(oracle_mod, m, B, out)
     finally:
         L.mask_session_destroy(h)
+
+
+# tiles a warp of the fill takes (16, 32, 64: more of them than 48 warps an SM take in shorter runs), and scans by
+# one block, by chunks, and by chunks whose sums are scanned in turn (more than 2^22 tiles)
+@pytest.mark.parametrize("rows", [3_000, 9_001, 250_000, 520_000, 4_300_000])
+def test_pack_tile_counts(oracle_mod, rows):
+    from mask_b200 import engine
+    K = 4000
+    rng = np.random.Generator(np.random.PCG64(rows))
+    length = np.where(np.arange(rows) % 4096 == 5, 1500, 8)
+    step = np.where(length == 8, rng.integers(1, 400, rows), 2)
+    start = (rng.random(rows) * (K - length * step)).astype(np.int64)
+    rowptr = np.concatenate([[0], np.cumsum(length)])
+    at = np.arange(rowptr[-1]) - np.repeat(rowptr[:-1], length)
+    colind = (np.repeat(start, length) + at * np.repeat(step, length)).astype(np.int32)
+    m = G.CSR(rows, K, rowptr.astype(np.int32), colind, rng.random(colind.size, dtype=np.float32))
+    rp, ci, va = _dev(m)
+    _check_metcf(engine.pack_metcf(rp, ci, va, m.M, m.K), oracle_mod.pack_metcf(m.M, m.rowptr, m.colind, m.values))
+    if rows > 1_000_000:
+        return
+    _check_srbcrs(engine.pack_srbcrs(rp, ci, va, m.M, m.K), oracle_mod.pack_srbcrs(m.M, m.rowptr, m.colind, m.values))
+    _check_mco(engine.pack_mco(rp, ci, va, m.M, m.K), oracle_mod.pack_mco(m.M, m.rowptr, m.colind, m.values))
