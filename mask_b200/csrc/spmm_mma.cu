@@ -332,32 +332,37 @@ static int sweep_slabs(const mask_plan* plan, int N) {
 // Which kernel: one warp per block (spmm_warp.cu) or the persistent tcgen05 kernel (spmm_sweep.cu).  The tcgen05
 // kernel takes up to 512 columns of a tile at once: tile values and ids are read once and every gathered byte goes
 // through shared memory once to and once from, so it wins where full-width rows are gathered at the L2's or
-// shared memory's rate.  The warp kernel takes 128 columns at a time, has no minimum width, spreads small
-// matrices over 2220 blocks instead of 296, and re-reads the tiles once per 128 columns.  Measured (us, tcgen05 /
-// warp; power-law graphs of 20 000 / 300 000 / 2^20 / 2^22 nodes, stencils of 40^3 / 100^3, uniform 10^5 / 2 10^5 rows):
-//   N = 16     39 / 18,   172 / 98,   -,           -,               41 / 18,   -,           45 / 25,   -
-//   N = 128    41 / 23,   283 / 216,  1020 / 870,  -,               48 / 37,   586 / 517,   64 / 60,   132 / 136
-//   N = 192    47 / 31,   -,          1498 / 1362, -,               68 / 57,   880 / 929,   94 / 95,   206 / 209
-//   N = 256    47 / 36,   416 / 424,  1688 / 1681, -,               67 / 70,   945 / 1145,  108 / 116, 266 / 265
-//   N = 512    70 / 59,   798 / 813,  3363 / 3338, 28 500 / 26 900, 115 / 131, 1800 / 2050, 253 / 221, 599 / 512
+// shared memory's rate.  The warp kernel takes at most 128 columns at a time, has no minimum width, spreads small
+// matrices over up to 3256 blocks instead of 296, and re-reads (and rebuilds) the tiles for every block of columns.
+// Measured (us, tcgen05 / warp), SR-BCRS; power-law graphs of 20 000 / 300 000 / 2^20 / 2^22 nodes, stencils of
+// 27^3 / 100^3, uniform 700 / 4096 / 10^5 / 2 10^5 rows:
+//   N = 32     26 / 12,   -,         -,           -,               16 / 7,    -,           7.5 / 7.4,  9.1 / 9.3,  -,         -
+//   N = 128    28 / 23,   283 / 216, 1020 / 870,  -,               17 / 15,   586 / 517,   7.7 / 7.5,  9.6 / 11.6, 64 / 60,   132 / 136
+//   N = 192    32 / 28,   -,         1498 / 1362, -,               23 / 20,   880 / 929,   9.4 / 7.9,  12.0 / 12.9, 94 / 95,  206 / 209
+//   N = 256    32 / 33,   416 / 424, 1688 / 1681, -,               22 / 25,   945 / 1145,  9.4 / 8.2,  12.0 / 12.7, 108 / 116, 266 / 265
+//   N = 512    51 / 56,   798 / 813, 3363 / 3338, 28 500 / 26 900, 37 / 43,   1760 / 2050, 13.2 / 8.5, 17.2 / 19.1, 253 / 221, 599 / 512
+// ME-TCF and MCO, 20 000 nodes: N = 128 30 / 27, N = 256 33 / 39, N = 512 54 / 64; 4096 rows: 10 / 20, 13 / 21, 17 / 27.
 static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, bool sidx_aligned) {
     if (tf32x3) return true;                    // compensated products: the warp kernel only
     if (!sidx_aligned || g_tune_sweep == 2) return false;
     if (g_tune_async == 0) return false;
     if (g_tune_sweep == 0) return true;
     if (g_tune_tma != 0 && fmt == kFmtSrbcrs && plan->d_vals_tf32 != nullptr) return false;
-    // a handful of long groups: one warp takes half a microsecond per tile, a tcgen05 block a quarter of that
-    if (plan->Gw < 4 * sm_count() && plan->T > 24 * plan->Gw) return false;
-    const int64_t slabs = (N + 127) / 128;
+    const bool dense = fmt == kFmtSrbcrs;
+    const int64_t slabs = (N + 127) / 128, work = plan->T * slabs;
+    const int64_t block = 128 * sweep_slabs(plan, N), padded = (N + block - 1) / block * block;
+    const bool pads = 4 * padded >= 5 * (int64_t)N;   // columns that the tcgen05 kernel's blocks would only pad: a quarter of N and more
+    // A handful of long groups: one warp takes a quarter of a microsecond per tile and twice that for one that it
+    // rebuilds, a tcgen05 block an eighth.  With enough columns the warp kernel has more blocks to deal them to.
+    if (plan->Gw < 4 * sm_count() && plan->T > (dense ? 24 : 16) * plan->Gw)
+        return dense && (N > 128 ? plan->Gw * slabs <= (N > 256 ? 4 : 2) * sm_count() : N <= 64 && plan->Gw > 2 * sm_count());
     if (N <= 128)   // a bitmap tile costs the warp kernel more to expand, and unaligned rows two passes a quarter-warp
         return !(fmt == kFmtMco && N > 96 && N < 128 && !plan->hub_heavy && !plan->local);
-    if (plan->T * slabs <= (fmt == kFmtMco ? 100000 : 150000)) return true;   // too little work for long-lived blocks
+    if (dense && work <= 150000 && (work <= 15000 || pads || (N <= 256 && !plan->local))) return true;   // too little work for long-lived blocks
     if (fmt == kFmtMco) return false;
-    if (plan->far_beyond_l2 && fmt == kFmtSrbcrs) return true;   // narrower rows of B: more of the hubs stay in L2
+    if (plan->far_beyond_l2 && dense) return true;   // narrower rows of B: more of the hubs stay in L2
     if (plan->slab_fits && N > 256) return true;
-    // columns that the tcgen05 kernel's blocks would only pad: a quarter of N and more
-    const int64_t block = 128 * sweep_slabs(plan, N), padded = (N + block - 1) / block * block;
-    return !plan->local && 4 * padded >= 5 * (int64_t)N;
+    return !plan->local && pads;
 }
 
 template <int FMT>

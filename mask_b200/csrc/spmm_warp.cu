@@ -230,13 +230,16 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
                 const float4 v0 = *reinterpret_cast<const float4*>(bt + q * 1024);
                 const float4 v1 = *reinterpret_cast<const float4*>(bt + q * 1024 + 128);
                 const float b0[4] = {v0.x, v0.y, v0.z, v0.w}, b1[4] = {v1.x, v1.y, v1.z, v1.w};
+                uint32_t h0[4], h1[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const uint32_t h0 = tf32_hi(b0[j]), h1 = tf32_hi(b1[j]);
-                    mma_tf32(acc[q][j], al, h0, h1);                                       // small terms first
-                    mma_tf32(acc[q][j], a, tf32_lo(b0[j], h0), tf32_lo(b1[j], h1));
-                    mma_tf32(acc[q][j], a, h0, h1);
-                }
+                for (int j = 0; j < 4; j++) { h0[j] = tf32_hi(b0[j]); h1[j] = tf32_hi(b1[j]); }
+                // small terms first; four accumulators in turn, so that no product waits for the one before it
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], al, h0[j], h1[j]);
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], a, tf32_lo(b0[j], h0[j]), tf32_lo(b1[j], h1[j]));
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], a, h0[j], h1[j]);
             }
         } else {
             const uint32_t a[4] = {rna_bits(af[0]), rna_bits(af[1]), rna_bits(af[2]), rna_bits(af[3])};
@@ -254,10 +257,47 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
     cpa_wait<0>();
 }
 
-template <int NQ, int KT, int S, int MINB, int FMT, bool GUARD, bool COMP>
+// Tiles per step: one (two at 32 columns) where many blocks are resident, up to four times as many where few are.
+static constexpr int warp_step_tiles(int nq, int depth) { return (nq == 1 ? 2 : 1) << depth; }
+// Blocks per SM: as many as shared memory holds, except where the registers of the compensated products need
+// more room (N = 256, 200 000-node power-law graph: 12 blocks of 165 registers 475 us, 15 of 128 490 us).
+static constexpr int warp_blocks_per_sm(int nq, int depth, bool comp) {
+    constexpr int blocks[4][3] = {{22, 12, 6}, {24, 13, 7}, {18, 10, 5}, {15, 8, 4}};
+    constexpr int comp_blocks[4] = {22, 16, 14, 12};
+    return comp && depth == 0 ? comp_blocks[nq - 1] : blocks[nq - 1][depth];
+}
+
+// Columns per warp (32 nq) and tiles per step for `groups` groups of tiles.  With fewer blocks than an SM holds the
+// gathers are bound by their latency: a block has two steps in flight, so the steps get longer, and the columns are
+// dealt to more blocks, as long as all of them are resident at once (short groups: within a sixteenth; a second
+// round of long ones doubles the time).  The longest step that fits comes first, then the fewest columns that pad no
+// more than the widest block would.  us, one tile and all columns a step / as chosen here: uniform 16 384
+// rows, N = 64 18.6 / 9.1, N = 128 20.6 / 13.6; 15^3 stencil, N = 64 7.2 / 5.2, N = 256 10.7 / 6.8; power-law graph
+// of 20 000 nodes, N = 64 21.3 / 15.2.  With four times the resident blocks, long steps lose a quarter to a half.
+static void choose_warp_shape(int64_t groups, int64_t T, int N, bool comp, int tuned_nq, int* nq_out, int* depth_out) {
+    const int slabs = (N + 127) / 128, widest = (N + 32 * slabs - 1) / (32 * slabs);
+    const bool tuned = tuned_nq >= 1 && tuned_nq <= 4;
+    for (int depth = 2; depth >= 0; depth--) {
+        for (int nq = tuned ? tuned_nq : 1; nq <= (tuned ? tuned_nq : widest); nq++) {
+            const int blocks = (N + 32 * nq - 1) / (32 * nq);
+            if (blocks * nq > slabs * widest && !tuned) continue;
+            const int64_t resident = (int64_t)sm_count() * warp_blocks_per_sm(nq, depth, comp);
+            if (groups * blocks <= resident + (T <= 24 * groups ? resident / 16 : 0)) {
+                *nq_out = nq;
+                *depth_out = depth;
+                return;
+            }
+        }
+    }
+    *nq_out = tuned ? tuned_nq : widest;
+    *depth_out = 0;
+}
+
+template <int NQ, int DEPTH, int FMT, bool GUARD, bool COMP>
 static int launch_warp_variant(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st) {
+    constexpr int KT = warp_step_tiles(NQ, DEPTH), S = 3;
     using L = WarpLayout<NQ, KT, S, FMT>;
-    auto kern = spmm_warp_kernel<NQ, KT, S, MINB, FMT, GUARD, COMP>;
+    auto kern = spmm_warp_kernel<NQ, KT, S, warp_blocks_per_sm(NQ, DEPTH, COMP), FMT, GUARD, COMP>;
     static std::atomic<uint64_t> opted_in;
     const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(kern), L::kBytes, opted_in);
     if (rc != MASK_OK) return rc;
@@ -266,36 +306,31 @@ static int launch_warp_variant(const mask_plan* plan, const SpmmArgs& a, cudaStr
     return launch_overlapped(kern, grid, 32, L::kBytes, st, a);
 }
 
+template <int FMT, bool COMP>
+static int launch_warp_shape(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st, int nq, int depth) {
+    const bool guard = a.N % (32 * nq) != 0;
+#define MASK_CASE(NQ, DEPTH)                                                               \
+    case NQ * 3 + DEPTH:                                                                   \
+        return guard ? launch_warp_variant<NQ, DEPTH, FMT, true, COMP>(plan, a, st)        \
+                     : launch_warp_variant<NQ, DEPTH, FMT, false, COMP>(plan, a, st);
+#define MASK_CASES(NQ) MASK_CASE(NQ, 0) MASK_CASE(NQ, 1) MASK_CASE(NQ, 2)
+    switch (nq * 3 + depth) { MASK_CASES(1) MASK_CASES(2) MASK_CASES(3) MASK_CASES(4) }
+#undef MASK_CASES
+#undef MASK_CASE
+    return fail(MASK_ERR_INVALID_ARGUMENT, "no such kernel");
+}
+
 template <int FMT>
-int launch_spmm_warp(const mask_plan* plan, const SpmmArgs& a_in, cudaStream_t st, int nq) {
+int launch_spmm_warp(const mask_plan* plan, const SpmmArgs& a_in, cudaStream_t st, int tuned_nq) {
     SpmmArgs a = a_in;
     a.group_off = plan->d_warp_off;
     a.group_tile = plan->d_warp_tile;
     a.n_frag = plan->F;
-    const int slabs = (a.N + 127) / 128;
-    if (nq < 1 || nq > 4) nq = (a.N + 32 * slabs - 1) / (32 * slabs);
-    const bool guard = a.N % (32 * nq) != 0;
-#define MASK_GO(NQ, KT, MINB, COMP) (guard ? launch_warp_variant<NQ, KT, 3, MINB, FMT, true, COMP>(plan, a, st) \
-                                           : launch_warp_variant<NQ, KT, 3, MINB, FMT, false, COMP>(plan, a, st))
-    // Blocks per SM: as many as shared memory holds, except where the registers of the compensated products need
-    // more room (N = 256, 200 000-node power-law graph: 12 blocks of 138 registers 475 us, 15 of 128 490 us).
-    if constexpr (FMT == kFmtSrbcrs) {
-        if (a.tf32x3) {
-            switch (nq) {
-                case 4: return MASK_GO(4, 1, 12, true);
-                case 3: return MASK_GO(3, 1, 14, true);
-                case 2: return MASK_GO(2, 1, 16, true);
-                default: return MASK_GO(1, 2, 22, true);
-            }
-        }
-    }
-    switch (nq) {
-        case 4: return MASK_GO(4, 1, 15, false);
-        case 3: return MASK_GO(3, 1, 18, false);
-        case 2: return MASK_GO(2, 1, 24, false);
-        default: return MASK_GO(1, 2, 22, false);
-    }
-#undef MASK_GO
+    int nq, depth;
+    choose_warp_shape(plan->Gw, plan->T, a.N, a.tf32x3, tuned_nq, &nq, &depth);
+    if constexpr (FMT == kFmtSrbcrs)
+        if (a.tf32x3) return launch_warp_shape<FMT, true>(plan, a, st, nq, depth);
+    return launch_warp_shape<FMT, false>(plan, a, st, nq, depth);
 }
 template int launch_spmm_warp<kFmtSrbcrs>(const mask_plan*, const SpmmArgs&, cudaStream_t, int);
 template int launch_spmm_warp<kFmtMetcf>(const mask_plan*, const SpmmArgs&, cudaStream_t, int);

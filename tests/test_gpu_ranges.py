@@ -97,6 +97,32 @@ def test_warp_kernel_column_counts(oracle_mod, fmt, N):
         engine.tune("sweep", 1)
 
 
+# numbers of windows at which the warp kernel takes more or fewer tiles a step and columns a block
+@pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
+@pytest.mark.parametrize("N", [32, 64, 96, 124, 256])
+@pytest.mark.parametrize("windows", [37, 440, 1000, 1700, 4100])
+def test_warp_kernel_step_lengths(oracle_mod, fmt, N, windows):
+    import torch
+    from mask_b200 import engine
+    rng = np.random.Generator(np.random.PCG64(windows))
+    K, length = 1900, rng.integers(0, 25, 16 * windows - 3)
+    rows = [np.sort(rng.choice(K, n, replace=False)) for n in length]
+    m = _rows_to_csr(rows, K, 3)
+    p = {"srbcrs": engine.pack_srbcrs, "metcf": engine.pack_metcf, "mco": engine.pack_mco}[fmt](*_dev(m), m.M, m.K)
+    B = rng.standard_normal((K, N), dtype=np.float32)
+    Bd = torch.from_numpy(B).cuda()
+    engine.tune("sweep", 0)
+    try:
+        _assert_close(oracle_mod, m, B, engine.spmm(p, Bd).cpu().numpy())
+        if fmt == "srbcrs":
+            out = engine.spmm(p, Bd, tf32x3=True).cpu().numpy()
+            bad, worst = oracle_mod.check_tolerance(out, oracle_mod.spmm_f32(m.M, m.rowptr, m.colind, m.values, B),
+                                                    oracle_mod.spmm_abs_f64(m.M, m.rowptr, m.colind, m.values, B), 2e-5, 1e-6)
+            assert bad == 0, worst
+    finally:
+        engine.tune("sweep", 1)
+
+
 @pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
 @pytest.mark.parametrize("N,offset,sweep", [(1, 0, 1), (3, 0, 1), (47, 0, 1), (47, 1, 2), (64, 3, 1), (129, 2, 1), (515, 0, 2)])
 def test_rows_that_are_not_whole_vectors(oracle_mod, fmt, N, offset, sweep):
