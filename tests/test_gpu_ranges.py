@@ -170,6 +170,14 @@ GRAPHS = {
     "one_way": lambda: _graph({(i, (i + 1) % 500) for i in range(500)} | {(i, (7 * i) % 500) for i in range(500)} | {(i, i) for i in range(0, 500, 3)}, 500),
     # hundreds of components of different sizes, isolated nodes between them
     "components": lambda: _graph(_both((10 * c + i, 10 * c + i + 1) for c in range(300) for i in range(c % 8)), 3000),
+    # more edges than are united at once: two grids, long lists that join some of their nodes, lone paths
+    "many_edges": lambda: _graph(_both([(i, i + d) for i in range(18_000) for d in (1, 150) if (i + d) // 9_000 == i // 9_000]
+                                       + [(18_200, i) for i in range(0, 9_000, 4)] + [(18_201, i) for i in range(9_000, 18_000, 5)]
+                                       + [(18_300 + 3 * i, 18_301 + 3 * i) for i in range(50)]
+                                       + [(i, (i * 7919) % 8_000) for i in range(8_000) if i != (i * 7919) % 8_000]
+                                       + [(9_000 + i, 9_000 + (i * 5171) % 8_000) for i in range(8_000) if i != (i * 5171) % 8_000]
+                                       + [(i, (i * 6007 + 5) % 8_000) for i in range(8_000) if i != (i * 6007 + 5) % 8_000]
+                                       + [(i, (i * 3001 + 9) % 8_000) for i in range(8_000) if i != (i * 3001 + 9) % 8_000]), 18_500),
     "no_edges": lambda: _graph({(3, 3)}, 50),
     "single": lambda: _graph({(0, 0)}, 1),
 }
