@@ -384,7 +384,7 @@ int mask_spmm_srbcrs_static_scratch(const mask_plan* plan, const int32_t* d_val_
  * where the warp-level one measures faster (by N and the plan), 2 = always, 0 = warp-level kernels only),
  * "nslab" (tcgen05 kernel: 128-column slabs per sweep, 1 / 2 / 4; 0 = the plan table's choice),
  * "tma" (1 = the TMA-fed kernel for plans prepared with mask_plan_prepare_values), and for the
- * warp-level kernels "nq" (32-column groups per warp: 1..4; 0 = chosen from N), "min_blocks"
+ * warp-level kernels "nq" (32-column groups per warp: 1..4; 0 = chosen from N and the plan), "min_blocks"
  * (occupancy target; 0 = default), "async" (0 = register-pipelined kernel instead of the cp.async
  * ring), "stages" (no effect); "session_chunk" (columns per chunk of mask_session_spmm_host).
  * Replaces the reference's tile_b environment switches SRBCRS_TILE_B / DTC_TILE_B
