@@ -2,6 +2,7 @@
 // block.  Used by the format builder (columns of a window) and the row reorders (neighbours of a node).
 #pragma once
 
+#include <climits>
 #include <cstdint>
 
 #include <cuda_runtime.h>
@@ -54,6 +55,17 @@ __device__ __forceinline__ void warp_sort(Key (&key)[E], int lane) {
             for (int i = 0; i < E; i++)
                 if ((i ^ s) > i) order2(key[i], key[i ^ s]);
     }
+}
+
+// The least of the values that the THREADS threads of a block hand in, to all of them (INT_MAX: none).  `word`: one per
+// warp; nobody may still read or write them.
+template <int THREADS>
+__device__ __forceinline__ int block_least(int x, int* word) {
+    const int lane = threadIdx.x & 31;
+    x = __reduce_min_sync(0xffffffffu, x);
+    if (lane == 0) word[threadIdx.x >> 5] = x;
+    __syncthreads();
+    return __reduce_min_sync(0xffffffffu, lane < THREADS / 32 ? word[lane] : INT_MAX);
 }
 
 constexpr int kMarkMax = 1 << 20;   // most keys a MarkSet holds (its shared memory: 3/16 of a byte per key)

@@ -179,7 +179,8 @@ __global__ void __launch_bounds__(128) condense_kernel(const int32_t* __restrict
 }
 
 // Windows of kSortMax + 1 to kHubMin entries, dealt to the blocks round-robin: the entries stay in registers,
-// kBigBits columns are marked, counted, ranked and unmarked at a time.
+// kBigBits columns are marked, counted, ranked and unmarked at a time, each time from the smallest column that is
+// left: columns up to 2^31 - 2 are 4096 such ranges, most of them without an entry of the window.
 __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
                                                                    int32_t M, int32_t K, int32_t* __restrict__ pos,
                                                                    int32_t* __restrict__ cols, int32_t* __restrict__ distinct,
@@ -213,8 +214,18 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
 #pragma unroll
             for (int r = 0; r < kWinRows; r++) start |= e == bound[r];
             if (e - e0 < n) bad |= entry_faults(colind, e, c[i], K, start);
+            if (c[i] >= K) c[i] = -1;
         }
-        for (int c0 = 0; c0 < K; c0 += kBigBits) {
+        // the smallest column from `from` on, INT_MAX if there is none
+        auto least_from = [&](int from) {
+            int x = INT_MAX;
+#pragma unroll
+            for (int i = 0; i < kBigKeep; i++)
+                if (c[i] >= from) x = min(x, c[i]);
+            return block_least<kBigThreads>(x, warp_sum);
+        };
+        const bool one_range = K <= kBigBits;
+        for (int c0 = one_range ? 0 : least_from(0); c0 < K;) {
             const int span = min(kBigBits, K - c0);
 #pragma unroll
             for (int i = 0; i < kBigKeep; i++)
@@ -233,6 +244,8 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
                 if (c[i] >= c0 && c[i] - c0 < span) marks.unmark(c[i] - c0);
             total += all;
             __syncthreads();
+            if (one_range || span == K - c0) break;
+            c0 = least_from(c0 + span);
         }
         if (bad) atomicOr(status, bad);
         if (tid == 0) distinct[w] = total;
@@ -244,7 +257,7 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
 // columns -- cut at the eighths of the window's longest row, so that the ranges hold about as many entries each --
 // which is a run of entries in each of the 16 rows, found by a 32-way search; the blocks exchange their counts
 // through distributed shared memory and rank what they marked themselves.  A range wider than kHubBits is taken in
-// parts (marked once to count, once more to rank).  With one block per window the 150 000 entries of the largest
+// parts (marked once to count, once more to rank), each from the smallest column that is left.  With one block per window the 150 000 entries of the largest
 // window of a power-law graph with 2^20 nodes took 0.3 ms while the rest of the GPU had finished.
 __global__ void __cluster_dims__(kHubBlocks, 1, 1) __launch_bounds__(kHubThreads, 1)
 condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M, int32_t K, int32_t span,
@@ -325,24 +338,30 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
         auto mark_part = [&](int c0, int part) {
             marks.n_runs = (part + 4095) / 4096;
             for (int i0 = 0; i0 < m; i0 += kHubThreads) {
-                const int i = i0 + tid, d = i < m ? __ldg(colind + entry(i)) - c0 : -1;
-                marks.mark_ascending(d < part ? d : -1);
+                const int i = i0 + tid, c = i < m ? __ldg(colind + entry(i)) : -1;
+                marks.mark_ascending(c >= c0 && c - c0 < part ? c - c0 : -1);
             }
-        };
-        auto unmark_part = [&](int c0, int part) {
-            __syncthreads();
-            for (int i = tid; i < m; i += kHubThreads) {
-                const int d = __ldg(colind + entry(i)) - c0;
-                if (d >= 0 && d < part) marks.unmark(d);
-            }
-            __syncthreads();
         };
         const bool whole = c_hi - c_lo <= span;
+        // returns where the next part begins: the smallest column behind this one, c_hi or more if there is none
+        auto unmark_part = [&](int c0, int part) {
+            int behind = INT_MAX;
+            __syncthreads();
+            for (int i = tid; i < m; i += kHubThreads) {
+                const int c = __ldg(colind + entry(i));
+                if (c < c0) continue;
+                if (c - c0 < part) marks.unmark(c - c0);
+                else behind = min(behind, c);
+            }
+            __syncthreads();
+            return whole ? c_hi : block_least<kHubThreads>(behind, warp_sum);
+        };
         int mine = 0;
-        for (int c0 = c_lo; c0 < c_hi; c0 += span) {
-            mark_part(c0, min(span, c_hi - c0));
+        for (int c0 = c_lo; c0 < c_hi;) {
+            const int part = min(span, c_hi - c0);
+            mark_part(c0, part);
             mine += marks.count<kHubThreads>(warp_sum);
-            if (!whole) unmark_part(c0, min(span, c_hi - c0));
+            c0 = whole ? c_hi : unmark_part(c0, part);
         }
         if (tid < kHubBlocks) cluster.map_shared_rank(range_marks[turn], tid)[me] = mine;
         cluster.sync();
@@ -352,7 +371,7 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
             total += v;
             if (i < me) ahead += v;
         }
-        for (int c0 = c_lo; c0 < c_hi; c0 += span) {
+        for (int c0 = c_lo; c0 < c_hi;) {
             const int part = min(span, c_hi - c0);
             int here = mine;
             if (!whole) {
@@ -361,14 +380,14 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
             }
 #pragma unroll 2
             for (int i = tid; i < m; i += kHubThreads) {
-                const int e = entry(i), c = __ldg(colind + e), d = c - c0;
-                if (d >= 0 && d < part) {
-                    const int q = ahead + marks.rank(d);
+                const int e = entry(i), c = __ldg(colind + e);
+                if (c >= c0 && c - c0 < part) {
+                    const int q = ahead + marks.rank(c - c0);
                     pos[e] = q;
                     cols[e0 + q] = c;
                 }
             }
-            unmark_part(c0, part);
+            c0 = unmark_part(c0, part);
             ahead += here;
         }
         if (me == 0 && tid == 0) distinct[w] = total;

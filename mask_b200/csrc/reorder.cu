@@ -288,7 +288,8 @@ __global__ void __launch_bounds__(128) sort_adjacency_kernel(const int32_t* __re
 }
 
 constexpr int kLongBits = 1 << 19;
-// the same for long lists: one block marks the ranks and places every one by the number of marks below it
+// the same for long lists: one block marks the ranks, kLongBits at a time from the smallest one left, and places
+// every one by the number of marks below it
 __global__ void __launch_bounds__(512) sort_long_adjacency_kernel(const int32_t* __restrict__ ptr, const int32_t* __restrict__ col, int32_t M,
                                                                   const int32_t* __restrict__ starts, const int32_t* __restrict__ rank,
                                                                   const int32_t* __restrict__ out_ptr, int32_t* __restrict__ out,
@@ -302,8 +303,9 @@ __global__ void __launch_bounds__(512) sort_long_adjacency_kernel(const int32_t*
     for (int j = blockIdx.x; j < total; j += gridDim.x) {
         const int i = long_list[j], v = starts[i], b = ptr[v], n = ptr[v + 1] - b, o = out_ptr[i];
         int placed = 0;
-        for (int r0 = 0; r0 < M; r0 += kLongBits) {
+        for (int r0 = 0; r0 < M;) {
             const int span = min(kLongBits, M - r0);
+            int behind = INT_MAX;   // smallest rank behind this range
             __syncthreads();
             for (int k = threadIdx.x; k < marks.n_runs * 128; k += 512) marks.bits[k] = 0;
             __syncthreads();
@@ -313,13 +315,15 @@ __global__ void __launch_bounds__(512) sort_long_adjacency_kernel(const int32_t*
                     const int c = __ldg(col + b + e);
                     if (c < 0 || c >= M || c == v) continue;
                     const int d = rank[c] - r0;
-                    if (d >= 0 && d < span) f(d);
+                    if (d >= span) behind = min(behind, r0 + d);
+                    else if (d >= 0) f(d);
                 }
             };
             each([&](int d) { marks.mark(d); });
             const int here = marks.count<512>(warp_sum);
             each([&](int d) { out[o + placed + marks.rank(d)] = r0 + d; });
             placed += here;
+            r0 = M <= kLongBits ? M : block_least<512>(behind, warp_sum);
         }
     }
 }

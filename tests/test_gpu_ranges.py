@@ -259,3 +259,43 @@ def test_pack_tile_counts(oracle_mod, rows):
         return
     _check_srbcrs(engine.pack_srbcrs(rp, ci, va, m.M, m.K), oracle_mod.pack_srbcrs(m.M, m.rowptr, m.colind, m.values))
     _check_mco(engine.pack_mco(rp, ci, va, m.M, m.K), oracle_mod.pack_mco(m.M, m.rowptr, m.colind, m.values))
+
+
+@pytest.mark.parametrize("n", [1100, 5000, 9000, 20_000])
+def test_pack_columns_up_to_the_end_of_int32(oracle_mod, n):
+    """Windows that one block and that a cluster ranks, columns spread over 2^31 - 1 (hundreds to thousands of the
+    ranges that a block marks at a time) or all in the last range, which is narrower than a step."""
+    from mask_b200 import engine
+    K = 2**31 - 1
+    rng = np.random.Generator(np.random.PCG64(n))
+    rows = []
+    for span in (K, 300_000, K):
+        for i in range(16):
+            c = np.unique(np.concatenate([K - 1 - rng.integers(0, span, n // 40 if i else n - 15 * (n // 40)), [K - 1 - i, K - span + i]]))
+            rows.append(c.astype(np.int32))
+    m = _rows_to_csr(rows[:-3], K, 7)
+    rp, ci, va = _dev(m)
+    _check_srbcrs(engine.pack_srbcrs(rp, ci, va, m.M, m.K), oracle_mod.pack_srbcrs(m.M, m.rowptr, m.colind, m.values))
+    _check_metcf(engine.pack_metcf(rp, ci, va, m.M, m.K), oracle_mod.pack_metcf(m.M, m.rowptr, m.colind, m.values))
+
+
+def test_rcm_long_lists_over_many_ranks(oracle_mod):
+    """Neighbour lists longer than a warp sorts whose ranks lie in several of the ranges that a block marks at a time,
+    some of which hold none of them."""
+    from mask_b200 import engine
+    n = 2_300_000
+    rng = np.random.Generator(np.random.PCG64(4))
+    a = np.arange(2, n - n % 2, 2)                 # pairs of neighbours, but for the nodes next to one of the hubs 0 and 1
+    near = [np.sort(rng.choice(np.arange(1000, 400_000), 1500, replace=False)), np.sort(rng.choice(np.arange(1_700_000, n - 2), 2500, replace=False))]
+    taken = np.zeros(n, bool)
+    for x in near:
+        taken[x] = True
+    a = a[~(taken[a] | taken[a + 1])]
+    src = np.concatenate([a, a + 1] + [np.full(len(x), h) for h, x in enumerate(near)] + near)
+    dst = np.concatenate([a + 1, a] + near + [np.full(len(x), h) for h, x in enumerate(near)])
+    order = np.lexsort((dst, src))
+    rowptr = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+    m = G.CSR(n, n, rowptr, dst[order].astype(np.int32), np.ones(len(src), np.float32))
+    rp, ci, _ = _dev(m)
+    got = engine.reorder_rows(rp, ci, n, n, "row_rcm").cpu().numpy()
+    assert np.array_equal(got, oracle_mod.reorder_rows("row_rcm", n, n, m.rowptr, m.colind))
