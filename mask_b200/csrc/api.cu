@@ -163,7 +163,7 @@ extern "C" int mask_session_create_srbcrs(int32_t M, int32_t K, int64_t T, const
     MASK_REQUIRE(T == 0 || (h_val_sidx && h_val_block_val), "packed arrays are NULL");
     mask_session* s = new mask_session();
     s->M = M; s->K = K; s->T = T;
-    const size_t W = (size_t)(M + kWinRows - 1) / kWinRows;
+    const size_t W = (size_t)window_count(M);
     auto body = [&]() -> int {
         int rc = session_common_init(s);
         if (rc != MASK_OK) return rc;
@@ -193,7 +193,7 @@ extern "C" int mask_session_create_csr(int32_t M, int32_t K, int64_t nnz, const 
     MASK_REQUIRE(nnz == 0 || (h_colind && h_values), "colind or values is NULL");
     mask_session* s = new mask_session();
     s->M = M; s->K = K;
-    const size_t W = (size_t)(M + kWinRows - 1) / kWinRows;
+    const size_t W = (size_t)window_count(M);
     DevScratch rowptr_b, colind_b, values_b, work_b;
     auto body = [&]() -> int {
         int rc = session_common_init(s);

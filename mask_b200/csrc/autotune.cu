@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(512) count_bins_kernel(const uint32_t* __restr
     }
     for (int i = threadIdx.x; i < kCountBins; i += 512) bins[i] = 0;
     __syncthreads();
-    for (int i = blockIdx.x * 512 + threadIdx.x; i < K; i += gridDim.x * 512) {
+    for (uint32_t i = blockIdx.x * 512 + threadIdx.x; i < (uint32_t)K; i += gridDim.x * 512) {
         const uint32_t c = counts[i];
         if (c < (uint32_t)kCountBins) atomicAdd(&bins[c], 1u);
         else list[atomicAdd(&head->listed, 1u)] = c;
@@ -127,7 +127,7 @@ int ColumnStatsJob::enqueue(const int32_t* d_val_soff, const int32_t* d_val_sidx
     N_ = N;
     T_ = T;
     if (T == 0) return MASK_OK;
-    const int32_t W = (M + kWinRows - 1) / kWinRows;
+    const int32_t W = window_count(M);
     // one allocation: what goes back to the host (with room for every column that can be listed), then counts
     const int64_t most_listed = std::min<int64_t>(K, T * kTileCols / kCountBins) + 1;
     const size_t counts_at = (sizeof(StatsHead) + (size_t)most_listed * 4 + 15) & ~(size_t)15;

@@ -67,7 +67,7 @@ extern "C" int mask_metcf_checkpoint_write(const char* path, int32_t M, int64_t 
     FILE* f = std::fopen(path, "wb");
     if (!f) return fail(MASK_ERR_INVALID_ARGUMENT, "cannot open checkpoint file for writing");
     const int32_t t32 = (int32_t)T, p32 = (int32_t)nnz_pad;
-    const size_t W = (size_t)(M + kWinRows - 1) / kWinRows;
+    const size_t W = (size_t)window_count(M);
     bool ok = std::fwrite(&t32, 4, 1, f) == 1 && std::fwrite(&p32, 4, 1, f) == 1;
     ok = ok && std::fwrite(val_soff, 4, W + 1, f) == W + 1;
     ok = ok && (T == 0 || std::fwrite(val_sidx, 4, (size_t)T * 8, f) == (size_t)T * 8);
@@ -102,7 +102,7 @@ extern "C" int mask_metcf_checkpoint_read(const char* path, int32_t M, int32_t K
     FILE* f = std::fopen(path, "rb");
     if (!f) return fail(MASK_ERR_INVALID_ARGUMENT, "cannot open checkpoint file");
     int32_t h[2] = {-1, -1};
-    const size_t W = (size_t)(M + kWinRows - 1) / kWinRows;
+    const size_t W = (size_t)window_count(M);
     bool ok = std::fread(h, 4, 2, f) == 2 && h[0] == T && h[1] == nnz_pad;
     ok = ok && std::fread(val_soff, 4, W + 1, f) == W + 1;
     ok = ok && (T == 0 || std::fread(val_sidx, 4, (size_t)T * 8, f) == (size_t)T * 8);
@@ -124,7 +124,7 @@ extern "C" int mask_metcf_checkpoint_read(const char* path, int32_t M, int32_t K
 extern "C" int mask_features_from_soff(const int32_t* h_val_soff, int32_t M, int64_t nnz, mask_features* out) {
     using namespace mask;
     MASK_REQUIRE(h_val_soff && out && M >= 1 && nnz >= 0, "bad arguments");
-    const int W = (M + kWinRows - 1) / kWinRows;
+    const int W = window_count(M);
     std::vector<int32_t> len((size_t)W);
     for (int w = 0; w < W; w++) len[w] = h_val_soff[w + 1] - h_val_soff[w];
     std::sort(len.begin(), len.end());

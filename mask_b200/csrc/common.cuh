@@ -39,6 +39,15 @@ constexpr int kWinRows = 16;   // rows per window
 constexpr int kTileCols = 8;   // condensed columns per tile
 constexpr int kTileElems = 128;
 
+// Windows of M >= 1 rows; M + 15 need not fit int32.
+__host__ __device__ inline int32_t window_count(int32_t M) { return (M - 1) / kWinRows + 1; }
+
+inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
+
+// Number of the thread, and of the warp, in the grid.  A warp per row passes 2^32 threads at 2^27 rows.
+__device__ __forceinline__ int64_t grid_thread() { return (int64_t)blockIdx.x * blockDim.x + threadIdx.x; }
+__device__ __forceinline__ int64_t grid_warp() { return grid_thread() >> 5; }
+
 // Swizzle<2,2,3> over a row-major 16x8 tile (SR-BCRS value layout).
 __host__ __device__ inline int sw223(int i) { return i ^ (((i >> 5) & 3) << 2); }
 // Swizzle<1,2,3> over the same tile (ME-TCF COO index).

@@ -57,7 +57,7 @@ static PackScratch carve(void* base, int32_t M, int64_t nnz) {
     PackScratch s{};
     char* p = static_cast<char*>(base);
     size_t off = 0;
-    const size_t n = (size_t)std::max<int64_t>(nnz, 1), W = (size_t)(M + kWinRows - 1) / kWinRows;
+    const size_t n = (size_t)std::max<int64_t>(nnz, 1), W = (size_t)window_count(M);
     auto take = [&](size_t bytes) { char* r = p ? p + off : nullptr; off += align_up(bytes); return r; };
     s.pos = reinterpret_cast<int32_t*>(take(n * 4));
     s.cols = reinterpret_cast<int32_t*>(take(n * 4));
@@ -149,9 +149,9 @@ __global__ void __launch_bounds__(128) condense_kernel(const int32_t* __restrict
     const int w = blockIdx.x * 4 + warp;
     if (w >= W) return;
     const int r0 = w * kWinRows;
-    const int bound = __ldg(rowptr + min(r0 + min(lane, kWinRows), M));   // lane i: where row i of the window begins
+    const int bound = __ldg(rowptr + r0 + min(min(lane, kWinRows), M - r0));   // lane i: where row i of the window begins
     const int base = __shfl_sync(0xffffffffu, bound, 0), n = __shfl_sync(0xffffffffu, bound, kWinRows) - base;
-    if (lane <= kWinRows) rows[r0 + lane] = bound;   // entry 16 is the next window's entry 0
+    if (lane <= kWinRows) (rows + r0)[lane] = bound;   // entry 16 is the next window's entry 0
     if (n > kSortMax) {
         if (lane == 0) {
             if (n > kHubMin) hub_list[atomicAdd(status + 5, 1)] = w;
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
     for (int b = blockIdx.x; b < n_big; b += gridDim.x) {
         const int w = big_list[b];
         __syncthreads();
-        if (tid <= kWinRows) bound[tid] = rowptr[min(w * kWinRows + tid, M)];
+        if (tid <= kWinRows) bound[tid] = (rowptr + w * kWinRows)[min(tid, M - w * kWinRows)];
         __syncthreads();
         const int e0 = bound[0], n = bound[kWinRows] - e0;
         int total = 0, bad = 0;
@@ -282,12 +282,12 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
     for (int b = blockIdx.x / kHubBlocks; b < n_hub; b += n_clusters, turn ^= 1) {
         const int w = hub_list[b];
         __syncthreads();
-        if (tid <= kWinRows) bound[tid] = rowptr[min(w * kWinRows + tid, M)];
+        if (tid <= kWinRows) bound[tid] = (rowptr + w * kWinRows)[min(tid, M - w * kWinRows)];
         __syncthreads();
         const int e0 = bound[0], n = bound[kWinRows] - e0;
         int bad = 0;
-        for (int j = me * kHubThreads + tid; j < n; j += kHubBlocks * kHubThreads) {
-            const int e = e0 + j;
+        for (uint32_t j = me * kHubThreads + tid; j < (uint32_t)n; j += kHubBlocks * kHubThreads) {
+            const int e = e0 + (int)j;
             bool start = false;
 #pragma unroll
             for (int r = 0; r < kWinRows; r++) start |= e == bound[r];
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(kFillThreads, 10) fill_kernel(const FillArgs p
         const int64_t next_s1 = te < chunk_end ? p.soff[w + 2] : 0;
         if (t > s0) {   // the chunk begins inside this window: first entry of every row at or after tile t
             // `first` columns come before it, all of them in the row but for those that only other rows have
-            const int first = (int)(t - s0) * kTileCols, all = __ldg(p.rows + (w + 1) * kWinRows) - base;
+            const int first = (int)(t - s0) * kTileCols, all = __ldg(p.rows + w * kWinRows + kWinRows) - base;
 #pragma unroll
             for (int k = 0; k < kSets; k++) {
                 int at = min(end[k], beg[k] + max(0, first - (all - (end[k] - beg[k]))));
@@ -724,8 +724,6 @@ struct McoOffOut {
     }
 };
 
-static inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
-
 template <int MODE>
 static int launch_fill(const FillArgs& a, cudaStream_t st) {
     fill_kernel<MODE><<<blocks_for(a.T, a.chunk * (kFillThreads / 32)), kFillThreads, 0, st>>>(a);
@@ -735,7 +733,7 @@ static int launch_fill(const FillArgs& a, cudaStream_t st) {
 
 static FillArgs fill_args(const PackScratch& s, int32_t M, const float* d_values, const int32_t* d_val_soff, int64_t T) {
     FillArgs a{};
-    a.W = (M + kWinRows - 1) / kWinRows;
+    a.W = window_count(M);
     // a chunk costs its searches, so it is as long as leaves the resident warps (48 an SM) one each
     a.chunk = kFillTiles;
     while (a.chunk > 16 && T < (int64_t)48 * sm_count() * a.chunk) a.chunk /= 2;
@@ -769,7 +767,7 @@ extern "C" int mask_pack_analyze(const int32_t* d_rowptr, const int32_t* d_colin
     PackScratch s = carve(d_scratch, M, nnz);
     if (scratch_bytes < s.bytes) return fail(MASK_ERR_SCRATCH_TOO_SMALL, "scratch smaller than mask_pack_scratch_bytes");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int W = (M + kWinRows - 1) / kWinRows;
+    const int W = window_count(M);
     MASK_CUDA_TRY(cudaMemsetAsync(s.status, 0, 64, st));
     // a key is the column and the entry's index within the window
     if (K <= (1 << (32 - kSortIdxBits)))
@@ -831,7 +829,7 @@ extern "C" int mask_srbcrs_fill(const int32_t* d_rowptr, const int32_t* d_colind
     MASK_REQUIRE(T == 0 || (d_val_sidx && d_val_block_val), "output arrays are NULL");
     PackScratch s = carve(const_cast<void*>(d_scratch), M, nnz);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int W = (M + kWinRows - 1) / kWinRows;
+    const int W = window_count(M);
     if (T > 0) {
         FillArgs a = fill_args(s, M, d_values, d_val_soff, T);
         a.sidx = d_val_sidx;

@@ -178,8 +178,8 @@ struct TableArgs {
 struct PiecesIn {            // pieces of a window | 1 if it is split
     TableArgs a;
     __device__ int64_t operator()(int64_t w) const {
-        const int32_t x = a.soff[w + 1] - a.soff[w];
-        return x > a.piece + a.piece / 4 ? (x + a.piece - 1) / a.piece + kHigh : 1;
+        const int64_t x = a.soff[w + 1] - a.soff[w], piece = a.piece;
+        return x > piece + piece / 4 ? (x + piece - 1) / piece + kHigh : 1;
     }
 };
 struct PiecesOut {
@@ -503,7 +503,7 @@ extern "C" int mask_plan_strict_lb(const int32_t* h_val_soff, int32_t M, int32_t
     using namespace mask;
     MASK_REQUIRE(h_val_soff != nullptr && M >= 1 && workload >= 1 && n_frag && n_groups, "bad arguments");
     std::vector<int32_t> rbo, rb2w, go;
-    strict_lb(h_val_soff, (M + kWinRows - 1) / kWinRows, workload, rbo, rb2w, go);
+    strict_lb(h_val_soff, window_count(M), workload, rbo, rb2w, go);
     *n_frag = (int64_t)rb2w.size();
     *n_groups = (int64_t)go.size() - 1;
     if (row_block_offset) std::memcpy(row_block_offset, rbo.data(), rbo.size() * sizeof(int32_t));
@@ -517,7 +517,7 @@ extern "C" int mask_plan_multi_bind(const int32_t* h_val_soff, int32_t M, int32_
     using namespace mask;
     MASK_REQUIRE(h_val_soff != nullptr && M >= 1 && n_tasks, "bad arguments");
     std::vector<int32_t> tw, ws, ts;
-    multi_bind(h_val_soff, (M + kWinRows - 1) / kWinRows, tw, ws, ts);
+    multi_bind(h_val_soff, window_count(M), tw, ws, ts);
     *n_tasks = (int64_t)tw.size();
     if (task_window && !tw.empty()) std::memcpy(task_window, tw.data(), tw.size() * sizeof(int32_t));
     if (window_split && !ws.empty()) std::memcpy(window_split, ws.data(), ws.size() * sizeof(int32_t));
@@ -532,7 +532,7 @@ static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int
                        int32_t group_tiles, cudaStream_t st, mask_plan** out) {
     mask_plan* p = new mask_plan();
     p->M = M;
-    p->W = (M + kWinRows - 1) / kWinRows;
+    p->W = window_count(M);
     p->T = T;
     p->policy = policy;
     p->group_tiles = group_tiles > 0 ? group_tiles : (policy == MASK_POLICY_STRICT_LB ? 64 : default_group_tiles(T));

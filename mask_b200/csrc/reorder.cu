@@ -54,8 +54,9 @@ __device__ __forceinline__ uint64_t mix_column(uint64_t v) {   // the bridge's c
 // one warp per row: first in-range column (K if none) and the min-hash signature over all its columns
 __global__ void row_keys_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M, int32_t K,
                                 uint32_t* __restrict__ first, uint64_t* __restrict__ sig) {
-    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (r >= M) return;
+    const int64_t row = grid_warp();
+    if (row >= M) return;
+    const int r = (int)row, lane = threadIdx.x & 31;
     uint32_t f = (uint32_t)K;
     uint64_t s = ~0ULL;
     for (int q = rowptr[r] + lane; q < rowptr[r + 1]; q += 32) {
@@ -88,7 +89,7 @@ int sort_rows_by(const KeyT* key_of_row, int32_t* rows_in, int32_t* rows_out, in
     int rc = keys.alloc(2 * half, st);
     if (rc != MASK_OK) return rc;
     KeyT *kin = keys.as<KeyT>(), *kout = keys.as<KeyT>(half);
-    gather_keys_kernel<KeyT><<<(n + 255) / 256, 256, 0, st>>>(key_of_row, rows_in, n, kin);
+    gather_keys_kernel<KeyT><<<blocks_for(n, 256), 256, 0, st>>>(key_of_row, rows_in, n, kin);
     MASK_CUDA_TRY(cudaGetLastError());
     size_t bytes = 0;
     MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kin, kout, rows_in, rows_out, n, 0, end_bit, st));
@@ -174,8 +175,9 @@ __global__ void __launch_bounds__(256) jaccard_chain_kernel(const int32_t* __res
 __global__ void sym_edge_keys_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M,
                                      uint64_t* __restrict__ keys) {
     // one warp per row; every stored (r, c) with c != r in range gives (r, c) and (c, r); others give a sentinel
-    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (r >= M) return;
+    const int64_t row = grid_warp();
+    if (row >= M) return;
+    const int r = (int)row, lane = threadIdx.x & 31;
     for (int q = rowptr[r] + lane; q < rowptr[r + 1]; q += 32) {
         const int c = colind[q];
         const bool ok = c >= 0 && c < M && c != r;
@@ -271,8 +273,9 @@ __global__ void __launch_bounds__(128) sort_adjacency_kernel(const int32_t* __re
                                                              const int32_t* __restrict__ starts, const int32_t* __restrict__ rank,
                                                              const int32_t* __restrict__ out_ptr, int32_t* __restrict__ out,
                                                              int32_t* __restrict__ long_list, int32_t* __restrict__ n_long) {
-    const int i = (blockIdx.x * 128 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= M) return;
+    const int64_t node = grid_warp();
+    if (node >= M) return;
+    const int i = (int)node, lane = threadIdx.x & 31;
     const int v = starts[i], b = ptr[v], n = ptr[v + 1] - b, o = out_ptr[i], n_out = out_ptr[i + 1] - o;
     if (n > kAdjSortMax) {
         if (lane == 0) long_list[atomicAdd(n_long, 1)] = i;
@@ -397,8 +400,10 @@ __global__ void __launch_bounds__(256) common_label_kernel(const int32_t* __rest
 // The remaining edges: a warp per node, lists longer than kAdjSortMax in the next kernel.
 __global__ void __launch_bounds__(256) hook_rest_kernel(const int32_t* __restrict__ ptr, const int32_t* __restrict__ adj, int32_t M,
                                                         int32_t* label, const int32_t* __restrict__ most) {
-    const int i = (blockIdx.x * 256 + threadIdx.x) >> 5;
-    if (i >= M || __ldcg(label + i) == *most) return;
+    const int64_t node = grid_warp();
+    if (node >= M) return;
+    const int i = (int)node;
+    if (__ldcg(label + i) == *most) return;
     const int b = ptr[i], e = ptr[i + 1];
     if (e - b > kAdjSortMax) return;
     for (int q = b + (threadIdx.x & 31); q < e; q += 32) unite(label, i, adj[q]);
@@ -428,13 +433,14 @@ struct IsRoot {
 // Per level: (1) every unvisited neighbour records the earliest queue position that reaches it, (2) every queue
 // node counts the neighbours that recorded it, (3) the counts are scanned and the children written behind the
 // queue.  A block takes a run of consecutive queue nodes, a warp a node (nodes with long lists: the block).
-// Levels of at most kSmallLevel nodes are walked by one block alone, without grid-wide barriers.
+// Levels of at most kSmallLevel nodes are walked by one block alone, without grid-wide barriers.  Positions are
+// unsigned: a stride past the last of 2^31 - 1 nodes stays a number.
 struct BfsArgs {
     const int32_t* ptr;
     const int32_t* adj;
     int32_t* queue;
     int32_t* pos;        // queue position, -1 before
-    int32_t* parent;     // earliest queue position that reaches the node
+    uint32_t* parent;    // earliest queue position that reaches the node, ~0u before
     int32_t* children;   // per node of the level
     int32_t* block_sum;  // per block
     int32_t* state;      // [0] base of the level, [1] its size
@@ -462,12 +468,12 @@ struct BfsKept {
 struct BfsShared {
     int warp_sum[kBfsWarps];
     int n_long;            // nodes of the block's share with long lists; too many of them: every node to a warp
-    int long_at[kMaxLong];
+    uint32_t long_at[kMaxLong];
     __device__ __forceinline__ bool by_block(int len) const { return len > kBlockList && n_long <= kMaxLong; }
 };
 
 // `width` lanes (a warp or the block) record queue position qpos with the unvisited neighbours of its node.
-__device__ __forceinline__ void bfs_mark(const BfsArgs& p, int qpos, int lane, int width) {
+__device__ __forceinline__ void bfs_mark(const BfsArgs& p, uint32_t qpos, int lane, int width) {
     const int v = __ldcg(p.queue + qpos), b = p.ptr[v], e = p.ptr[v + 1];
     for (int q = b + lane; q < e; q += width) {
         const int nb = p.adj[q];
@@ -499,12 +505,12 @@ __device__ __forceinline__ int block_exclusive(int x, BfsShared& s, int* total) 
 }
 
 // The queue nodes [lo, hi) of the level that begins at `base`: marks.
-__device__ __forceinline__ void bfs_mark_range(const BfsArgs& p, int base, int lo, int hi, BfsShared& s, BfsKept& keep) {
+__device__ __forceinline__ void bfs_mark_range(const BfsArgs& p, uint32_t base, uint32_t lo, uint32_t hi, BfsShared& s, BfsKept& keep) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) s.n_long = 0;
     if (*p.n_sorted_long > 0) {
         __syncthreads();
-        for (int i = lo + threadIdx.x; i < hi; i += kBfsThreads) {
+        for (uint32_t i = lo + threadIdx.x; i < hi; i += kBfsThreads) {
             const int v = __ldcg(p.queue + base + i);
             if (p.ptr[v + 1] - p.ptr[v] > kBlockList) {
                 const int k = atomicAdd(&s.n_long, 1);
@@ -515,7 +521,7 @@ __device__ __forceinline__ void bfs_mark_range(const BfsArgs& p, int base, int l
     __syncthreads();
 #pragma unroll
     for (int t = 0; t < kKept; t++) {
-        const int i = lo + warp + t * kBfsWarps;
+        const uint32_t i = lo + warp + t * kBfsWarps;
         keep.kept[t] = false;
         if (i >= hi) continue;
         const int v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
@@ -528,7 +534,7 @@ __device__ __forceinline__ void bfs_mark_range(const BfsArgs& p, int base, int l
         keep.nb[t] = nb;
         if (nb >= 0 && __ldcg(p.pos + nb) < 0 && __ldcg(p.parent + nb) > base + i) atomicMin(p.parent + nb, base + i);
     }
-    for (int i = lo + warp + kKept * kBfsWarps; i < hi; i += kBfsWarps) {
+    for (uint32_t i = lo + warp + kKept * kBfsWarps; i < hi; i += kBfsWarps) {
         const int v = __ldcg(p.queue + base + i);
         if (!s.by_block(p.ptr[v + 1] - p.ptr[v])) bfs_mark(p, base + i, lane, 32);
     }
@@ -542,18 +548,19 @@ __device__ __forceinline__ bool is_kept(const BfsKept& keep, int t) {
     return x;
 }
 // Counts children per node; returns the sum over the range (to every thread).
-__device__ __forceinline__ int bfs_count_range(const BfsArgs& p, int base, int lo, int hi, BfsShared& s, BfsKept& keep) {
+__device__ __forceinline__ int bfs_count_range(const BfsArgs& p, uint32_t base, uint32_t lo, uint32_t hi, BfsShared& s, BfsKept& keep) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int sum = 0;
 #pragma unroll
     for (int t = 0; t < kKept; t++) {
         if (!keep.kept[t]) continue;
-        const int i = lo + warp + t * kBfsWarps;
+        const uint32_t i = lo + warp + t * kBfsWarps;
         keep.child[t] = __ballot_sync(0xffffffffu, keep.nb[t] >= 0 && __ldcg(p.parent + max(keep.nb[t], 0)) == base + i);
         const int c = __popc(keep.child[t]);
         if (lane == 0) { p.children[i] = c; sum += c; }
     }
-    for (int t = 0, i = lo + warp; i < hi; i += kBfsWarps, t++) {
+    uint32_t i = lo + warp;
+    for (int t = 0; i < hi; i += kBfsWarps, t++) {
         if (is_kept(keep, t)) continue;
         const int v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
         if (s.by_block(e - b)) continue;
@@ -563,7 +570,8 @@ __device__ __forceinline__ int bfs_count_range(const BfsArgs& p, int base, int l
         if (lane == 0) { p.children[i] = c; sum += c; }
     }
     for (int k = 0; k < s.n_long && s.n_long <= kMaxLong; k++) {
-        const int i = s.long_at[k], v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
+        const uint32_t i = s.long_at[k];
+        const int v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
         int c = 0, all = 0;
         for (int q = b + threadIdx.x; q < e; q += kBfsThreads) c += __ldcg(p.parent + p.adj[q]) == base + i;
         block_exclusive(c, s, &all);
@@ -574,14 +582,14 @@ __device__ __forceinline__ int bfs_count_range(const BfsArgs& p, int base, int l
     return total;
 }
 // Writes the children of the range behind queue position `at` and numbers them.
-__device__ __forceinline__ void bfs_place_range(const BfsArgs& p, int base, int lo, int hi, int at, BfsShared& s, const BfsKept& keep) {
+__device__ __forceinline__ void bfs_place_range(const BfsArgs& p, uint32_t base, uint32_t lo, uint32_t hi, int at, BfsShared& s, const BfsKept& keep) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     __syncthreads();   // children[] of the range has been written by this block
-    for (int c0 = lo; c0 < hi; c0 += kBfsThreads) {
-        const int mine = c0 + (int)threadIdx.x < hi ? __ldcg(p.children + c0 + threadIdx.x) : 0;
+    for (uint32_t c0 = lo; c0 < hi; c0 += kBfsThreads) {
+        const int mine = c0 + threadIdx.x < hi ? __ldcg(p.children + c0 + threadIdx.x) : 0;
         int all = 0;
         const int before = block_exclusive(mine, s, &all);
-        if (c0 + (int)threadIdx.x < hi) p.children[c0 + threadIdx.x] = at + before;   // now: where they go
+        if (c0 + threadIdx.x < hi) p.children[c0 + threadIdx.x] = at + before;   // now: where they go
         at += all;
     }
     __syncthreads();
@@ -594,7 +602,8 @@ __device__ __forceinline__ void bfs_place_range(const BfsArgs& p, int base, int 
             p.pos[keep.nb[t]] = o;
         }
     }
-    for (int t = 0, i = lo + warp; i < hi; i += kBfsWarps, t++) {
+    uint32_t i = lo + warp;
+    for (int t = 0; i < hi; i += kBfsWarps, t++) {
         if (is_kept(keep, t)) continue;
         const int v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
         if (s.by_block(e - b)) continue;
@@ -612,7 +621,8 @@ __device__ __forceinline__ void bfs_place_range(const BfsArgs& p, int base, int 
         }
     }
     for (int k = 0; k < s.n_long && s.n_long <= kMaxLong; k++) {
-        const int i = s.long_at[k], v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
+        const uint32_t i = s.long_at[k];
+        const int v = __ldcg(p.queue + base + i), b = p.ptr[v], e = p.ptr[v + 1];
         int to = __ldcg(p.children + i);
         for (int q0 = b; q0 < e; q0 += kBfsThreads) {
             const int nb = q0 + (int)threadIdx.x < e ? p.adj[q0 + threadIdx.x] : -1;
@@ -635,7 +645,7 @@ __global__ void __launch_bounds__(kBfsThreads) bfs_kernel(const BfsArgs p) {
     __shared__ BfsShared s;
     BfsKept keep;
     int base = 0, n = *p.n_start;
-    for (int i = blockIdx.x * kBfsThreads + threadIdx.x; i < n; i += gridDim.x * kBfsThreads) p.pos[__ldcg(p.queue + i)] = i;
+    for (uint32_t i = blockIdx.x * kBfsThreads + threadIdx.x; i < (uint32_t)n; i += gridDim.x * kBfsThreads) p.pos[__ldcg(p.queue + i)] = i;
     grid.sync();
     while (n > 0) {
         if (n <= kSmallLevel) {
@@ -657,7 +667,7 @@ __global__ void __launch_bounds__(kBfsThreads) bfs_kernel(const BfsArgs p) {
             continue;
         }
         const int share = (n + gridDim.x - 1) / gridDim.x;
-        const int lo = min(n, (int)blockIdx.x * share), hi = min(n, lo + share);
+        const int lo = min(n, (int)blockIdx.x * share), hi = lo + min(share, n - lo);
         bfs_mark_range(p, base, lo, hi, s, keep);
         grid.sync();
         const int sum = bfs_count_range(p, base, lo, hi, s, keep);
@@ -708,14 +718,14 @@ int symmetrised_pattern(const int32_t* rowptr, const int32_t* colind, int32_t M,
     if (rc == MASK_OK) rc = deg_b.alloc(((size_t)M + 1) * 4, st);
     if (rc == MASK_OK) rc = ptr_b.alloc(((size_t)M + 1) * 4, st);
     if (rc != MASK_OK) return rc;
-    const unsigned row_blocks = (unsigned)(((int64_t)M * 32 + 255) / 256);
+    const unsigned row_blocks = blocks_for((int64_t)M * 32, 256);
     sym_edge_keys_kernel<<<row_blocks, 256, 0, st>>>(rowptr, colind, M, keys.as<uint64_t>());
     MASK_CUDA_TRY(cudaGetLastError());
     uint64_t *k0 = keys.as<uint64_t>(), *k1 = keys_sorted.as<uint64_t>();
     size_t b1 = 0, b2 = 0, b3 = 0;
     MASK_CUDA_TRY(cub::DeviceRadixSort::SortKeys(nullptr, b1, k0, k1, (int)n_keys, 0, 64, st));
     MASK_CUDA_TRY(cub::DeviceSelect::Unique(nullptr, b2, k1, k0, n_unique_d.as<int64_t>(), (int)n_keys, st));
-    MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, b3, deg_b.as<int32_t>(), ptr_b.as<int32_t>(), M + 1, st));
+    MASK_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, b3, deg_b.as<int32_t>(), ptr_b.as<int32_t>() + 1, M, st));
     rc = tmp.alloc(std::max(b1, std::max(b2, b3)), st);
     if (rc != MASK_OK) return rc;
     MASK_CUDA_TRY(cub::DeviceRadixSort::SortKeys(tmp.p, b1, k0, k1, (int)n_keys, 0, 64, st));
@@ -735,18 +745,19 @@ int symmetrised_pattern(const int32_t* rowptr, const int32_t* colind, int32_t M,
     if (rc != MASK_OK) return rc;
     MASK_CUDA_TRY(cudaMemsetAsync(deg_b.p, 0, ((size_t)M + 1) * 4, st));
     if (n_edges > 0) {
-        const unsigned eb = (unsigned)((n_edges + 255) / 256);
+        const unsigned eb = blocks_for(n_edges, 256);
         count_sources_kernel<<<eb, 256, 0, st>>>(k0, n_edges, deg_b.as<int32_t>());
         split_targets_kernel<<<eb, 256, 0, st>>>(k0, n_edges, adj_b.as<int32_t>());
         MASK_CUDA_TRY(cudaGetLastError());
     }
-    MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, b3, deg_b.as<int32_t>(), ptr_b.as<int32_t>(), M + 1, st));
+    MASK_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp.p, b3, deg_b.as<int32_t>(), ptr_b.as<int32_t>() + 1, M, st));
+    MASK_CUDA_TRY(cudaMemsetAsync(ptr_b.p, 0, 4, st));
     *n_edges_out = n_edges;
     return MASK_OK;
 }
 
 int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, int64_t nnz, int32_t* order, cudaStream_t st) {
-    const unsigned node_blocks = (unsigned)((M + 255) / 256);
+    const unsigned node_blocks = blocks_for(M, 256);
     const int32_t *ptr = rowptr, *col = colind;
     int64_t n_edges = nnz;
     DevScratch deg_b, flag_b, sym_ptr, sym_adj;
@@ -759,7 +770,7 @@ int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, in
     int32_t* flags = flag_b.as<int32_t>();   // [0] asymmetric, [1] long lists, [2] start nodes, [4..5] state of the traversal, [6] most common label
     MASK_CUDA_TRY(cudaMemsetAsync(flags, 0, 64, st));
     row_lengths_kernel<<<node_blocks, 256, 0, st>>>(ptr, M, deg);
-    if (nnz > 0) check_symmetry_kernel<<<(unsigned)((nnz + 255) / 256), 256, 0, st>>>(ptr, col, M, nnz, deg, flags);
+    if (nnz > 0) check_symmetry_kernel<<<blocks_for(nnz, 256), 256, 0, st>>>(ptr, col, M, nnz, deg, flags);
     MASK_CUDA_TRY(cudaGetLastError());
     MASK_CUDA_TRY(cudaMemcpyAsync(host.as<int32_t>(), flags, 4, cudaMemcpyDeviceToHost, st));
     MASK_CUDA_TRY(cudaStreamSynchronize(st));
@@ -785,7 +796,7 @@ int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, in
     cub::CountingInputIterator<int> counting(0);
     size_t b1 = 0, b2 = 0, b3 = 0;
     MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, b1, udeg, usorted, arr(kIds), arr(kStarts), M, 0, bits, st));
-    MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, b2, arr(kSortedDeg), arr(kOutPtr), M + 1, st));
+    MASK_CUDA_TRY(cub::DeviceScan::InclusiveSum(nullptr, b2, arr(kSortedDeg), arr(kOutPtr) + 1, M, st));
     MASK_CUDA_TRY(cub::DeviceSelect::If(nullptr, b3, counting, arr(kQueue), flags + 2, M, IsRoot{arr(kLabel)}, st));
     rc = tmp.alloc(std::max(b1, std::max(b2, b3)), st);
     if (rc != MASK_OK) return rc;
@@ -793,11 +804,11 @@ int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, in
     iota_kernel<<<node_blocks, 256, 0, st>>>(arr(kIds), M);
     MASK_CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp.p, b1, udeg, usorted, arr(kIds), arr(kStarts), M, 0, bits, st));
     scatter_rank_kernel<<<node_blocks, 256, 0, st>>>(arr(kStarts), M, arr(kRank), arr(kLabel));
-    MASK_CUDA_TRY(cudaMemsetAsync(arr(kSortedDeg) + M, 0, 4, st));
-    MASK_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, b2, arr(kSortedDeg), arr(kOutPtr), M + 1, st));
+    MASK_CUDA_TRY(cudaMemsetAsync(arr(kOutPtr), 0, 4, st));
+    MASK_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp.p, b2, arr(kSortedDeg), arr(kOutPtr) + 1, M, st));
     int32_t* adj = adj_b.as<int32_t>();
-    sort_adjacency_kernel<<<(unsigned)(((int64_t)M * 32 + 127) / 128), 128, 0, st>>>(ptr, col, M, arr(kStarts), arr(kRank), arr(kOutPtr), adj,
-                                                                                  arr(kLong), flags + 1);
+    sort_adjacency_kernel<<<blocks_for((int64_t)M * 32, 128), 128, 0, st>>>(ptr, col, M, arr(kStarts), arr(kRank), arr(kOutPtr), adj, arr(kLong),
+                                                                            flags + 1);
     MASK_CUDA_TRY(cudaGetLastError());
     if (n_edges > kAdjSortMax) {
         constexpr int kSmem = kLongBits / 8 + kLongBits / 16;
@@ -809,7 +820,7 @@ int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, in
     // components; their least ranks, ascending, begin the queue
     if (n_edges > 0) {
         if (n_edges <= kFewEdges) {
-            hook_kernel<<<(unsigned)((n_edges + 255) / 256), 256, 0, st>>>(arr(kOutPtr), adj, M, arr(kLabel));
+            hook_kernel<<<blocks_for(n_edges, 256), 256, 0, st>>>(arr(kOutPtr), adj, M, arr(kLabel));
         } else {
             least_neighbour_kernel<<<node_blocks, 256, 0, st>>>(arr(kOutPtr), adj, M, arr(kLabel));
             flatten_labels_kernel<<<node_blocks, 256, 0, st>>>(arr(kLabel), M);
@@ -818,7 +829,7 @@ int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, in
                 flatten_labels_kernel<<<node_blocks, 256, 0, st>>>(arr(kLabel), M);
             }
             common_label_kernel<<<1, 256, 0, st>>>(arr(kLabel), M, flags + 6);
-            hook_rest_kernel<<<(unsigned)(((int64_t)M * 32 + 255) / 256), 256, 0, st>>>(arr(kOutPtr), adj, M, arr(kLabel), flags + 6);
+            hook_rest_kernel<<<blocks_for((int64_t)M * 32, 256), 256, 0, st>>>(arr(kOutPtr), adj, M, arr(kLabel), flags + 6);
             hook_long_kernel<<<(unsigned)std::min<int64_t>(n_edges / kAdjSortMax, 2 * sm_count()), 512, 0, st>>>(
                 arr(kOutPtr), adj, arr(kLabel), flags + 6, arr(kLong), flags + 1);
         }
@@ -827,8 +838,9 @@ int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, in
     MASK_CUDA_TRY(cudaGetLastError());
     MASK_CUDA_TRY(cub::DeviceSelect::If(tmp.p, b3, counting, arr(kQueue), flags + 2, M, IsRoot{arr(kLabel)}, st));
     MASK_CUDA_TRY(cudaMemsetAsync(arr(kPos), 0xff, (size_t)M * 4, st));
-    MASK_CUDA_TRY(cudaMemsetAsync(arr(kParent), 0x7f, (size_t)M * 4, st));
-    BfsArgs a{arr(kOutPtr), adj, arr(kQueue), arr(kPos), arr(kParent), arr(kChildren), arr(kRow), flags + 4, flags + 2, flags + 1, M};
+    MASK_CUDA_TRY(cudaMemsetAsync(arr(kParent), 0xff, (size_t)M * 4, st));
+    BfsArgs a{arr(kOutPtr), adj, arr(kQueue), arr(kPos), reinterpret_cast<uint32_t*>(arr(kParent)), arr(kChildren), arr(kRow), flags + 4,
+              flags + 2, flags + 1, M};
     // block sums: one word per block, in an array that is not used yet
     const unsigned blocks = (unsigned)std::min<int64_t>(sm_count(), ((int64_t)M + kBfsWarps - 1) / kBfsWarps);
     void* args[] = {&a};
@@ -856,8 +868,9 @@ __global__ void gather_rows_kernel(const int32_t* __restrict__ rowptr, const int
                                    const float* __restrict__ values, const int32_t* __restrict__ order,
                                    const int32_t* __restrict__ rowptr_out, int32_t M, int32_t* __restrict__ colind_out,
                                    float* __restrict__ values_out) {
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (i >= M) return;
+    const int64_t row = grid_warp();
+    if (row >= M) return;
+    const int i = (int)row, lane = threadIdx.x & 31;
     const int r = order[i];
     const int src = rowptr[r], n = rowptr[r + 1] - src, dst = rowptr_out[i];
     for (int j = lane; j < n; j += 32) {
@@ -873,7 +886,7 @@ extern "C" int mask_reorder_rows(int kind, const int32_t* d_rowptr, const int32_
     using namespace mask;
     MASK_REQUIRE(d_rowptr && d_row_order && M >= 1 && K >= 1, "bad arguments");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const unsigned node_blocks = (unsigned)((M + 255) / 256), row_blocks = (unsigned)(((int64_t)M * 32 + 255) / 256);
+    const unsigned node_blocks = blocks_for(M, 256), row_blocks = blocks_for((int64_t)M * 32, 256);
     if (kind == MASK_REORDER_NONE) {
         iota_kernel<<<node_blocks, 256, 0, st>>>(d_row_order, M);
         MASK_CUDA_TRY(cudaGetLastError());
@@ -907,7 +920,7 @@ extern "C" int mask_reorder_rows(int kind, const int32_t* d_rowptr, const int32_
     rc = sort_rows_by<uint32_t>(first.as<uint32_t>(), ids.as<int32_t>(), by_first.as<int32_t>(), M, col_bits, st);
     if (rc == MASK_OK) rc = sort_rows_by<uint64_t>(sig.as<uint64_t>(), by_first.as<int32_t>(), ids.as<int32_t>(), M, 64, st);
     if (rc != MASK_OK) return rc;
-    jaccard_chain_kernel<<<(unsigned)((M + 63) / 64), 256, 0, st>>>(d_rowptr, d_colind, ids.as<int32_t>(), M, d_row_order);
+    jaccard_chain_kernel<<<blocks_for(M, 64), 256, 0, st>>>(d_rowptr, d_colind, ids.as<int32_t>(), M, d_row_order);
     MASK_CUDA_TRY(cudaGetLastError());
     return MASK_OK;
 }
@@ -928,8 +941,8 @@ extern "C" int mask_csr_permute_rows(const int32_t* d_rowptr, const int32_t* d_c
     MASK_CUDA_TRY(cub::DeviceScan::InclusiveSum(tmp.p, bytes, lengths, d_rowptr_out + 1, M, st));
     MASK_CUDA_TRY(cudaMemsetAsync(d_rowptr_out, 0, 4, st));
     if (d_colind && d_values && d_colind_out && d_values_out) {
-        gather_rows_kernel<<<(unsigned)(((int64_t)M * 32 + 255) / 256), 256, 0, st>>>(d_rowptr, d_colind, d_values, d_row_order,
-                                                                                   d_rowptr_out, M, d_colind_out, d_values_out);
+        gather_rows_kernel<<<blocks_for((int64_t)M * 32, 256), 256, 0, st>>>(d_rowptr, d_colind, d_values, d_row_order, d_rowptr_out, M, d_colind_out,
+                                                                             d_values_out);
         MASK_CUDA_TRY(cudaGetLastError());
     }
     return MASK_OK;

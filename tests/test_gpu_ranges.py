@@ -299,3 +299,79 @@ def test_rcm_long_lists_over_many_ranks(oracle_mod):
     rp, ci, _ = _dev(m)
     got = engine.reorder_rows(rp, ci, n, n, "row_rcm").cpu().numpy()
     assert np.array_equal(got, oracle_mod.reorder_rows("row_rcm", n, n, m.rowptr, m.colind))
+
+
+def _scattered(small_rows, at, M):
+    """rowptr of M rows on the GPU: row at[i] is as long as small_rows[i], the others are empty."""
+    import torch
+    rowptr = torch.zeros(M + 1, dtype=torch.int32, device="cuda")
+    for r, row in zip(at, small_rows):
+        rowptr[int(r) + 1:] += len(row)
+    return rowptr
+
+
+@pytest.mark.parametrize("kind", ["row_rcm", "first_col_sort", "jaccard_greedy"])
+def test_reorders_past_2_27_rows(oracle_mod, kind):
+    """A warp per row is more than 2^32 threads.  All but a few hundred rows are empty, so the order follows from those."""
+    import torch
+    from mask_b200 import engine
+    M = 2**27 + 1000
+    rng = np.random.Generator(np.random.PCG64(6))
+    at = np.unique(np.concatenate([rng.integers(0, M, 150), np.arange(2**27 - 40, 2**27 + 40), np.arange(M - 30, M)]))
+    n = len(at)
+    pairs = _both((int(a), int(b)) for a, b in rng.integers(0, n, (2 * n, 2)) if a != b) | _both((i, (i + 1) % n) for i in range(n))
+    small = _graph(pairs, n)
+    rows = [at[small.colind[small.rowptr[i]:small.rowptr[i + 1]]].astype(np.int32) for i in range(n)]
+    rp, ci = _scattered(rows, at, M), torch.from_numpy(np.concatenate(rows)).cuda()
+    order = engine.reorder_rows(rp, ci, M, M, kind)
+    full = torch.zeros(M, dtype=torch.bool, device="cuda")
+    full[torch.from_numpy(at).cuda()] = True
+    empty = torch.nonzero(~full).squeeze(1).to(torch.int32)
+    if kind == "row_rcm":               # isolated nodes are components of their own and come first
+        want = np.concatenate([at[oracle_mod.reorder_rows(kind, n, n, small.rowptr, small.colind)]])
+        assert torch.equal(order[:M - n], empty)
+        assert np.array_equal(order[M - n:].cpu().numpy(), want)
+    else:                               # empty rows come last; the first of them share a bucket of 64 with the others
+        more = -n % 64
+        ids = np.sort(np.concatenate([at, empty[:more].cpu().numpy()]))
+        some = _rows_to_csr([rows[np.searchsorted(at, r)] if r in at else np.zeros(0, np.int32) for r in ids], M, 1)
+        want = ids[oracle_mod.reorder_rows(kind, len(ids), M, some.rowptr, some.colind)]
+        assert np.array_equal(order[:len(ids)].cpu().numpy(), want)
+        assert torch.equal(order[len(ids):], empty[more:])
+    va = torch.arange(ci.numel(), dtype=torch.float32, device="cuda")
+    rp2, ci2, va2 = engine.permute_rows(rp, ci, va, M, order)
+    place = torch.nonzero(full[order.long()]).squeeze(1)
+    taken = [int(np.searchsorted(at, r)) for r in order[place].cpu().numpy()]
+    assert np.array_equal(ci2.cpu().numpy(), np.concatenate([rows[i] for i in taken]))
+    assert np.array_equal(va2.cpu().numpy(), np.concatenate([np.arange(small.rowptr[i], small.rowptr[i + 1], dtype=np.float32) for i in taken]))
+    assert torch.equal(rp2[1:] - rp2[:-1], (rp[1:] - rp[:-1])[order.long()])
+
+
+def test_pack_and_product_rows_up_to_the_end_of_int32(oracle_mod):
+    """M = 2^31 - 1: 16 times the number of windows, and the index of the row behind the last window, do not fit int32."""
+    import torch
+    from mask_b200 import engine
+    M, K, N = 2**31 - 1, 3000, 4
+    rng = np.random.Generator(np.random.PCG64(8))
+    at = np.concatenate([np.arange(3, 20), np.arange(2**30 - 5, 2**30 + 9), [2**31 - 100], np.arange(M - 20, M)])
+    rows = [np.sort(rng.choice(K, int(c), replace=False)).astype(np.int32) for c in rng.integers(1, 60, len(at))]
+    rows[20] = np.sort(rng.choice(K, 1500, replace=False)).astype(np.int32)   # a window that a block ranks
+    windows = np.unique(at // 16)
+    by_row = dict(zip(at.tolist(), rows))
+    small = _rows_to_csr([by_row.get(int(r), np.zeros(0, np.int32)) for w in windows for r in range(16 * w, min(16 * w + 16, M))], K, 5)
+    rp, ci, va = _scattered(rows, at, M), torch.from_numpy(small.colind).cuda(), torch.from_numpy(small.values).cuda()
+    p = engine.pack_srbcrs(rp, ci, va, M, K)
+    del rp
+    want = oracle_mod.pack_srbcrs(small.M, small.rowptr, small.colind, small.values)
+    for k in ("val_sidx", "val_block_val"):
+        assert np.array_equal(getattr(p, k).cpu().numpy().view(np.int32), want[k].view(np.int32)), k
+    tiles = torch.diff(p.val_soff)
+    assert np.array_equal(tiles[torch.from_numpy(windows).cuda()].cpu().numpy(), np.diff(want["val_soff"]))
+    assert int(p.val_soff[0]) == 0 and int(p.val_soff[-1]) == p.T == int(tiles.sum())
+    B = rng.standard_normal((K, N), dtype=np.float32)
+    out = engine.spmm(p, torch.from_numpy(B).cuda())
+    assert p.plan().status() == 0
+    ids = torch.from_numpy(np.concatenate([np.arange(16 * w, min(16 * w + 16, M)) for w in windows])).cuda()
+    _assert_close(oracle_mod, small, B, out[ids].cpu().numpy())
+    out[ids] = 0
+    assert not bool(out.any())
