@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
                 if (c[i] >= from) x = min(x, c[i]);
             return block_least<kBigThreads>(x, warp_sum);
         };
-        const bool one_range = K <= kBigBits;
-        for (int c0 = one_range ? 0 : least_from(0); c0 < K;) {
+        const bool few = K <= 4 * kBigBits;   // looking for the next column costs about what an empty range does
+        for (int c0 = few ? 0 : least_from(0); c0 < K;) {
             const int span = min(kBigBits, K - c0);
 #pragma unroll
             for (int i = 0; i < kBigKeep; i++)
@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
                 if (c[i] >= c0 && c[i] - c0 < span) marks.unmark(c[i] - c0);
             total += all;
             __syncthreads();
-            if (one_range || span == K - c0) break;
-            c0 = least_from(c0 + span);
+            if (span == K - c0) break;
+            c0 = few ? c0 + span : least_from(c0 + span);
         }
         if (bad) atomicOr(status, bad);
         if (tid == 0) distinct[w] = total;
@@ -257,8 +257,9 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
 // columns -- cut at the eighths of the window's longest row, so that the ranges hold about as many entries each --
 // which is a run of entries in each of the 16 rows, found by a 32-way search; the blocks exchange their counts
 // through distributed shared memory and rank what they marked themselves.  A range wider than kHubBits is taken in
-// parts (marked once to count, once more to rank), each from the smallest column that is left.  With one block per window the 150 000 entries of the largest
-// window of a power-law graph with 2^20 nodes took 0.3 ms while the rest of the GPU had finished.
+// parts (marked once to count, once more to rank), each from the smallest column that is left.  With one block per
+// window the 150 000 entries of the largest window of a power-law graph with 2^20 nodes took 0.3 ms while the rest of
+// the GPU had finished.
 __global__ void __cluster_dims__(kHubBlocks, 1, 1) __launch_bounds__(kHubThreads, 1)
 condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M, int32_t K, int32_t span,
                     int32_t* __restrict__ pos, int32_t* __restrict__ cols, int32_t* __restrict__ distinct,
