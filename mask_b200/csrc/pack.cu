@@ -457,6 +457,21 @@ struct FillArgs {
     float* out_val;
 };
 
+// The window that holds tile t, for a whole warp: the last one from w on that begins at or before t (window w does, the
+// end of the last one does not).  32 windows are looked at in a step, then every 32nd, and so on, so that a run of
+// windows without tiles costs a step for each factor of 32 in its length.
+__device__ __forceinline__ int window_of_tile(const int32_t* __restrict__ soff, int32_t W, int w, int64_t t) {
+    const int lane = threadIdx.x & 31;
+    for (int stride = 1;;) {
+        const int at = (int)min((int64_t)w + (int64_t)(lane + 1) * stride, (int64_t)W);
+        const int hits = __popc(__ballot_sync(0xffffffffu, __ldg(soff + at) <= t));   // the probes that hit come first
+        w += hits * stride;
+        if (hits == 32) stride *= 32;
+        else if (stride == 1) return w;
+        else stride /= 32;
+    }
+}
+
 // 32-bit halves of the words that hold a tile's row counts (16 nibbles) and its mask (128 bits)
 __device__ __forceinline__ void count_entry(uint32_t* words, int tile, int row) {
     atomicAdd(words + 2 * tile + (row >> 3), 1u << (4 * (row & 7)));
@@ -494,15 +509,7 @@ __global__ void __launch_bounds__(kFillThreads, 10) fill_kernel(const FillArgs p
 
     const int64_t chunk_begin = ((int64_t)blockIdx.x * kWarps + warp) * p.chunk;
     if (chunk_begin >= p.T) return;
-    // window of tile t
-    auto locate = [&](int64_t t) {
-        int w = p.first_window[t / kFillTiles];
-        for (;;) {   // windows from w on that end at or before t
-            const int behind = __popc(__ballot_sync(0xffffffffu, __ldg(p.soff + min(w + 1 + lane, p.W)) <= t));
-            w += behind;
-            if (behind < 32) return w;
-        }
-    };
+    auto locate = [&](int64_t t) { return window_of_tile(p.soff, p.W, p.first_window[t / kFillTiles], t); };
     int w = locate(chunk_begin);
     int64_t s0 = p.soff[w], s1 = p.soff[w + 1], t = chunk_begin, chunk_end = min(p.T, chunk_begin + p.chunk);
     if (t > s0 && s1 - s0 <= p.chunk) t = s1;
@@ -512,9 +519,9 @@ __global__ void __launch_bounds__(kFillThreads, 10) fill_kernel(const FillArgs p
         if (b0 < chunk_end && b1 - b0 <= p.chunk) chunk_end = b1;
     }
     if (t >= chunk_end) return;
-    while (s1 <= t) {
-        w++;
-        s0 = s1;
+    if (s1 <= t) {
+        w = window_of_tile(p.soff, p.W, w, t);
+        s0 = t;
         s1 = p.soff[w + 1];
     }
     if (MODE == kFillSrbcrs) {
@@ -546,7 +553,7 @@ __global__ void __launch_bounds__(kFillThreads, 10) fill_kernel(const FillArgs p
         }
     };
     for (;;) {
-                int beg[kSets], e[kSets], end[kSets];
+        int beg[kSets], e[kSets], end[kSets];
 #pragma unroll
         for (int k = 0; k < kSets; k++) {
             e[k] = beg[k] = __ldg(p.rows + w * kWinRows + kAtOnce * k + g);
@@ -677,8 +684,8 @@ __global__ void __launch_bounds__(kFillThreads, 10) fill_kernel(const FillArgs p
         w++;   // on to the next window with tiles
         s0 = s1;
         s1 = next_s1;
-        while (s1 == s0) {
-            w++;
+        if (s1 == s0) {
+            w = window_of_tile(p.soff, p.W, w, t);
             s1 = p.soff[w + 1];
         }
     }

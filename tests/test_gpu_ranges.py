@@ -375,3 +375,44 @@ def test_pack_and_product_rows_up_to_the_end_of_int32(oracle_mod):
     _assert_close(oracle_mod, small, B, out[ids].cpu().numpy())
     out[ids] = 0
     assert not bool(out.any())
+
+
+# windows without tiles between others: as many as are looked at in a step, in a step of steps, and one more or less
+@pytest.mark.parametrize("gap", [1, 31, 32, 33, 1023, 1024, 1055, 1056, 32_768, 40_000])
+def test_pack_runs_of_empty_windows(oracle_mod, gap):
+    from mask_b200 import engine
+    rng = np.random.Generator(np.random.PCG64(gap))
+    K, none = 5000, [np.zeros(0, np.int32)]
+    some = lambda n: [np.sort(rng.choice(K, int(c), replace=False)) for c in rng.integers(1, 40, n)]
+    rows = none * (16 * gap) + some(37) + none * (16 * gap + 11) + some(900) + none * (16 * gap) + some(16) + none * (16 * gap)
+    m = _rows_to_csr(rows, K, 7)
+    rp, ci, va = _dev(m)
+    _check_srbcrs(engine.pack_srbcrs(rp, ci, va, m.M, m.K), oracle_mod.pack_srbcrs(m.M, m.rowptr, m.colind, m.values))
+    _check_metcf(engine.pack_metcf(rp, ci, va, m.M, m.K), oracle_mod.pack_metcf(m.M, m.rowptr, m.colind, m.values))
+    _check_mco(engine.pack_mco(rp, ci, va, m.M, m.K), oracle_mod.pack_mco(m.M, m.rowptr, m.colind, m.values))
+
+
+def test_pack_time_does_not_depend_on_where_the_empty_rows_are():
+    """2^21 empty rows in the middle of a matrix cost what they cost at its end.  Walking them window by window took
+    one warp 7.8 ms, against 0.1 in all; three times the other placing leaves room for noise."""
+    import torch
+    from mask_b200 import engine
+    rows, empty, K = 32_000, 1 << 21, 8
+    colind = torch.arange(8, dtype=torch.int32, device="cuda").repeat(rows)   # one tile a window
+    values = torch.rand(8 * rows, device="cuda")
+    length = torch.full((rows,), 8, dtype=torch.int64, device="cuda")
+    gap = torch.zeros(empty, dtype=torch.int64, device="cuda")
+    ms = {}
+    for where, parts in (("middle", (length[:16 * 1003], gap, length[16 * 1003:])), ("end", (length, gap))):
+        rowptr = torch.zeros(rows + empty + 1, dtype=torch.int32, device="cuda")
+        rowptr[1:] = torch.cumsum(torch.cat(parts), 0)
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            engine.pack_srbcrs(rowptr, colind, values, rows + empty, K)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        ms[where] = sorted(times)[3]
+    assert ms["middle"] < 3 * ms["end"], ms
