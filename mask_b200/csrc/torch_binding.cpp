@@ -39,7 +39,7 @@ const at::Tensor* float_tensor(PyObject* o, const char* name) {
 // spmm(format, M, K, val_sidx, offsets, index, values, plan, dense, out or None, epilogue, whole_vectors) -> out, or an
 // int: the status of a C-ABI call that failed.  whole_vectors: only N % 4 == 0 (else -1) and 16-byte aligned dense and
 // out (else -2) are taken.
-PyObject* spmm(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
+PyObject* product(PyObject* const* args, Py_ssize_t n_args) {
     if (n_args != 12) return raise("spmm takes 12 arguments");
     mask_matrix m{};
     m.format = (int32_t)PyLong_AsLong(args[0]);
@@ -62,42 +62,48 @@ PyObject* spmm(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
         return nullptr;
     }
     if (N > 0x7ffffffc) return raise("dense has too many columns");
+    at::Tensor out;
+    if (args[9] == Py_None) {
+        out = at::empty({m.M, N}, dense->options());
+    } else {
+        const at::Tensor* given = float_tensor(args[9], "out");
+        if (!given) return nullptr;
+        if (given->dim() != 2 || given->size(0) != m.M || given->size(1) != N) return raise("out has the wrong shape");
+        out = *given;
+    }
+    if (N > 0) {
+        if (args[11] == Py_True) {
+            if (N % 4) return PyLong_FromLong(-1);
+            if ((reinterpret_cast<uintptr_t>(dense->data_ptr()) | reinterpret_cast<uintptr_t>(out.data_ptr())) & 15) return PyLong_FromLong(-2);
+        }
+        const int32_t n4 = (int32_t)((N + 3) & ~(int64_t)3);
+        const float* B = static_cast<const float*>(dense->data_ptr());
+        // freed to torch's allocator on return: it is reused in stream order
+        at::Tensor pad, scratch;
+        if (n4 != N || (reinterpret_cast<uintptr_t>(B) & 15)) pad = at::empty({K * n4}, dense->options());
+        const size_t need = mask_plan_scratch_bytes(plan, n4);
+        if (need) scratch = at::empty({(int64_t)need}, dense->options().dtype(at::kByte));
+        float* C = static_cast<float*>(out.data_ptr());
+        cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+        int rc;
+        Py_BEGIN_ALLOW_THREADS
+        rc = mask_spmm(plan, &m, (int32_t)N, B, N, C, N, pad.defined() ? static_cast<float*>(pad.data_ptr()) : nullptr,
+                       need ? scratch.data_ptr() : nullptr, need, epilogue, stream);
+        Py_END_ALLOW_THREADS
+        if (rc != MASK_OK) return PyLong_FromLong(rc);
+    }
+    if (args[9] != Py_None) {
+        Py_INCREF(args[9]);
+        return args[9];
+    }
+    return THPVariable_Wrap(std::move(out));
+}
+
+// Tensors without storage or strides (sparse ones, those of torch.func's transforms) throw already when they are asked
+// for an address or whether they are contiguous.
+PyObject* spmm(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
     try {
-        at::Tensor out;
-        if (args[9] == Py_None) {
-            out = at::empty({m.M, N}, dense->options());
-        } else {
-            const at::Tensor* given = float_tensor(args[9], "out");
-            if (!given) return nullptr;
-            if (given->dim() != 2 || given->size(0) != m.M || given->size(1) != N) return raise("out has the wrong shape");
-            out = *given;
-        }
-        if (N > 0) {
-            if (args[11] == Py_True) {
-                if (N % 4) return PyLong_FromLong(-1);
-                if ((reinterpret_cast<uintptr_t>(dense->data_ptr()) | reinterpret_cast<uintptr_t>(out.data_ptr())) & 15) return PyLong_FromLong(-2);
-            }
-            const int32_t n4 = (int32_t)((N + 3) & ~(int64_t)3);
-            const float* B = static_cast<const float*>(dense->data_ptr());
-            // freed to torch's allocator on return: it is reused in stream order
-            at::Tensor pad, scratch;
-            if (n4 != N || (reinterpret_cast<uintptr_t>(B) & 15)) pad = at::empty({K * n4}, dense->options());
-            const size_t need = mask_plan_scratch_bytes(plan, n4);
-            if (need) scratch = at::empty({(int64_t)need}, dense->options().dtype(at::kByte));
-            float* C = static_cast<float*>(out.data_ptr());
-            cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
-            int rc;
-            Py_BEGIN_ALLOW_THREADS
-            rc = mask_spmm(plan, &m, (int32_t)N, B, N, C, N, pad.defined() ? static_cast<float*>(pad.data_ptr()) : nullptr,
-                           need ? scratch.data_ptr() : nullptr, need, epilogue, stream);
-            Py_END_ALLOW_THREADS
-            if (rc != MASK_OK) return PyLong_FromLong(rc);
-        }
-        if (args[9] != Py_None) {
-            Py_INCREF(args[9]);
-            return args[9];
-        }
-        return THPVariable_Wrap(std::move(out));
+        return product(args, n_args);
     } catch (...) {
         torch::translate_exception_to_python(std::current_exception());
         return nullptr;

@@ -492,3 +492,20 @@ def test_product_with_more_than_2_31_elements(oracle_mod):
     bad, worst = oracle_mod.check_tolerance(got, ref, absp, RTOL, ATOL)
     assert bad == 0, worst
     assert not bool(torch.isnan(out[-1]).any()) and not bool(torch.isnan(out[:: 1 << 12]).any())
+
+
+@pytest.mark.parametrize("what", ["sparse", "vmap", "strided"])
+def test_dense_operands_that_are_not_plain_tensors_raise(what):
+    import torch
+    from mask_b200 import engine
+    m = cases.SMALL["m17"]()
+    p = engine.pack_srbcrs(*_dev(m), m.M, m.K)
+    B = torch.ones(m.K, 32, device="cuda")
+    with pytest.raises(RuntimeError):
+        if what == "sparse":
+            engine.spmm(p, B.to_sparse())
+        elif what == "vmap":
+            torch.func.vmap(lambda b: engine.spmm(p, b))(torch.stack([B, B]))
+        else:
+            engine.spmm(p, B.t().contiguous().t())
+    assert engine.spmm(p, B).shape == (m.M, 32)
