@@ -365,9 +365,25 @@ static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, 
     return !plan->local && pads;
 }
 
+static bool aligned(const void* p, unsigned bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+
+// The packed arrays as the asynchronous copies read them: 16 bytes at a time, pairs of offsets 8.  Ids as well in the warp
+// kernel, which other products leave to the tcgen05 kernel when they are not aligned.
+static int check_packed_alignment(const SpmmArgs& a) {
+    MASK_REQUIRE(aligned(a.val_blk, 16) && aligned(a.coo_idx, 16) && aligned(a.coo_val, 16) && aligned(a.mco_mask, 16),
+                 "val_block_val, val_coo_idx, val_coo_val, val_mco_mask and val_mco_val must be 16-byte aligned");
+    MASK_REQUIRE(a.mco_mask || aligned(a.coo_off, 8), "val_coo_off must be 8-byte aligned");
+    MASK_REQUIRE(!a.tf32x3 || aligned(a.val_sidx, 16), "compensated products need 16-byte aligned val_sidx");
+    return MASK_OK;
+}
+
 template <int FMT>
 static int launch_spmm(const mask_plan* plan, SpmmArgs a, cudaStream_t st) {
     if (plan->G == 0) return MASK_OK;
+    if (a.tf32x3 || g_tune_sweep != 0 || g_tune_async != 0) {   // every kernel but the register-pipelined one
+        const int bad = check_packed_alignment(a);
+        if (bad != MASK_OK) return bad;
+    }
     a.frag_off = plan->d_frag_off;
     a.frag_win = plan->d_frag_win;
     a.frag_slot = plan->d_frag_slot;
@@ -377,7 +393,7 @@ static int launch_spmm(const mask_plan* plan, SpmmArgs a, cudaStream_t st) {
     a.n_peer_out = plan->n_peer_out;
     const int N = a.N;
     int rc;
-    if (use_warp_kernel(plan, FMT, N, a.tf32x3, (reinterpret_cast<uintptr_t>(a.val_sidx) & 15) == 0)) {
+    if (use_warp_kernel(plan, FMT, N, a.tf32x3, aligned(a.val_sidx, 16))) {
         rc = launch_spmm_warp<FMT>(plan, a, st, g_tune_nq);
         return rc != MASK_OK ? rc : launch_fixup(plan, a, st);
     }

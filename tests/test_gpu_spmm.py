@@ -509,3 +509,54 @@ def test_dense_operands_that_are_not_plain_tensors_raise(what):
         else:
             engine.spmm(p, B.t().contiguous().t())
     assert engine.spmm(p, B).shape == (m.M, 32)
+
+
+@pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
+def test_packed_arrays_off_their_alignment(oracle_mod, fmt):
+    """Arrays that a kernel copies 16 bytes at a time are refused off that grid, ids are taken by another kernel."""
+    import ctypes as C
+    import torch
+    from mask_b200 import _lib, engine
+    m = cases.SMALL["rmat10"]()
+    p = {"srbcrs": engine.pack_srbcrs, "metcf": engine.pack_metcf, "mco": engine.pack_mco}[fmt](*_dev(m), m.M, m.K)
+    code, offsets, index, values = p._arrays()
+    N = 64
+    B = _dense(m.K, N, 3)
+    Bd = torch.from_numpy(B).cuda()
+    plan = p.new_plan()
+    scratch = torch.empty(plan.scratch_bytes(N) + 16, dtype=torch.uint8, device="cuda")
+
+    def off(t, by):
+        moved = torch.zeros(t.numel() * t.element_size() + 64, dtype=torch.uint8, device="cuda")
+        moved[by:by + t.numel() * t.element_size()] = t.view(torch.uint8)
+        return moved[by:]
+
+    def call(epilogue=0, **moved):
+        arrays = dict(sidx=p.val_sidx, offsets=offsets, index=index, values=values)
+        kept = {k: off(arrays[k], by) for k, by in moved.items()}
+        ptr = {k: None if t is None else t.data_ptr() for k, t in {**arrays, **kept}.items()}
+        out = torch.full((m.M, N), float("nan"), device="cuda")
+        mat = _lib.Matrix(code, m.M, m.K, 0, ptr["sidx"], ptr["offsets"], ptr["index"], ptr["values"])
+        rc = _lib.lib().mask_spmm(plan._h, C.byref(mat), N, Bd.data_ptr(), N, out.data_ptr(), N, None, scratch.data_ptr(), scratch.numel(), epilogue,
+                                  C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        return rc, out
+
+    rc, out = call()
+    assert rc == 0
+    _assert_close(oracle_mod, m, B, out.cpu().numpy())
+    for by in (4, 8, 12):
+        rc, out = call(sidx=by)
+        assert rc == 0
+        _assert_close(oracle_mod, m, B, out.cpu().numpy())
+        assert call(values=by)[0] == 1
+        if fmt != "srbcrs":
+            assert call(index=by)[0] == 1
+        if fmt == "metcf" and by != 8:
+            assert call(offsets=by)[0] == 1
+        if fmt == "srbcrs":
+            assert call(_lib.NUMERICS_TF32X3, sidx=by)[0] == 1
+    if fmt == "srbcrs":
+        assert call(_lib.NUMERICS_TF32X3)[0] == 0
+    else:
+        assert call(offsets=8)[0] == 0
