@@ -539,6 +539,31 @@ static int fill_matrix_args(const mask_plan* plan, const mask_matrix* m, SpmmArg
 
 }  // namespace mask
 
+namespace mask {
+
+// Column blocks, and rows of partial tiles in the fix-up pass, are numbered in the y dimension of a grid (at most
+// 65 535), so wider products are taken in pieces of this many columns, one after the other.  Peers' copies of C are
+// written at the same offsets as C itself: such products stay whole.
+constexpr int32_t kPieceColumns = 1 << 21;
+
+static int launch_pieces(const mask_plan* plan, int format, const SpmmArgs& a, cudaStream_t st) {
+    const int32_t most = plan->n_peer_out ? a.N : kPieceColumns;
+    for (int32_t c0 = 0, width; c0 < a.N; c0 += width) {
+        SpmmArgs piece = a;
+        width = std::min(most, a.N - c0);
+        piece.B += c0;
+        piece.C += c0;
+        piece.N = width;
+        piece.n_out = std::min(width, a.n_out - c0);
+        const int rc = format == kFmtSrbcrs ? launch_spmm<kFmtSrbcrs>(plan, piece, st)
+                                            : (format == kFmtMetcf ? launch_spmm<kFmtMetcf>(plan, piece, st) : launch_spmm<kFmtMco>(plan, piece, st));
+        if (rc != MASK_OK) return rc;
+    }
+    return MASK_OK;
+}
+
+}  // namespace mask
+
 extern "C" int mask_spmm(const mask_plan* plan, const mask_matrix* m, int32_t n, const float* d_B, int64_t ldb, float* d_C, int64_t ldc,
                          float* d_pad, void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
     using namespace mask;
@@ -570,11 +595,7 @@ extern "C" int mask_spmm(const mask_plan* plan, const mask_matrix* m, int32_t n,
                                reinterpret_cast<float4*>(d_pad));
         if (rc != MASK_OK) return rc;
     }
-    switch (m->format) {
-        case kFmtSrbcrs: return launch_spmm<kFmtSrbcrs>(plan, a, st);
-        case kFmtMetcf: return launch_spmm<kFmtMetcf>(plan, a, st);
-        default: return launch_spmm<kFmtMco>(plan, a, st);
-    }
+    return launch_pieces(plan, m->format, a, st);
 }
 
 // The entry points that take a matrix array by array.

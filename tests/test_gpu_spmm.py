@@ -560,3 +560,22 @@ def test_packed_arrays_off_their_alignment(oracle_mod, fmt):
         assert call(_lib.NUMERICS_TF32X3)[0] == 0
     else:
         assert call(offsets=8)[0] == 0
+
+
+@pytest.mark.parametrize("N,tf32x3,gt", [(65_535 * 128 + 132, True, 0), (4_194_304 + 36, False, 1), (2 * (1 << 21) + 3, False, 1)])
+def test_products_of_millions_of_columns(N, tf32x3, gt):
+    """More column blocks, or rows of partial tiles, than the y dimension of a grid holds."""
+    import torch
+    from mask_b200 import engine
+    m = cases.random_csr(5, 40, 24, 0.4)
+    p = engine.pack_srbcrs(*_dev(m), m.M, m.K)
+    plan = p.new_plan("auto", gt)
+    assert (plan.info()["partial"] > 0) == (gt > 0)
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    B = torch.randn(m.K, N, generator=gen, device="cuda")
+    A = torch.zeros(m.M, m.K)
+    A[np.repeat(np.arange(m.M), np.diff(m.rowptr)), m.colind] = torch.from_numpy(m.values)
+    A = A.cuda()
+    C = engine.spmm_any_width(p, B, plan=plan, tf32x3=tf32x3)
+    bound = (2e-5 if tf32x3 else 2e-3) * (A.abs() @ B.abs()) + 1e-6
+    assert bool(((C - A @ B).abs() <= bound).all())
