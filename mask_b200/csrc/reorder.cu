@@ -331,27 +331,31 @@ __global__ void __launch_bounds__(512) sort_long_adjacency_kernel(const int32_t*
     }
 }
 
-// Connected components by hooking: the root of a tree is its least node, so labels end as the component's least rank.
+// Connected components as a forest: label[i] is a node of i's tree that is smaller than i, or i if i is the root, so that
+// labels end as the component's least rank.  Many threads join trees at once (Anderson and Woll, "Wait-free parallel
+// algorithms for the union-find problem", 1991): a root is given a parent by compare-and-swap, everything else only ever
+// moves up.
+
+// The root of i's tree.  Every node on the way is moved up to its grandparent (path splitting: Tarjan and van Leeuwen,
+// "Worst-case analysis of set union algorithms", 1984).
 __device__ __forceinline__ int find_root(int32_t* label, int i) {
-    int cur = __ldcg(label + i);
-    if (cur != i) {
-        int prev = i, next;
-        while (cur > (next = __ldcg(label + cur))) {   // halve the path on the way
-            label[prev] = next;
-            prev = cur;
-            cur = next;
-        }
+    for (int parent = __ldcg(label + i); parent != i;) {
+        const int grandparent = __ldcg(label + parent);
+        if (grandparent != parent) __stcg(label + i, grandparent);
+        i = parent;
+        parent = grandparent;
     }
-    return cur;
+    return i;
 }
+// Joins the trees of i and j: the larger root goes below the smaller one.
 __device__ __forceinline__ void unite(int32_t* label, int i, int j) {
-    int a = find_root(label, i), b = find_root(label, j);
-    while (a != b) {      // the larger root joins the smaller; a failed exchange returns a smaller label
-        if (a < b) { const int t = a; a = b; b = t; }
-        const int was = atomicCAS(label + a, a, b);
-        if (was == a) break;
-        a = was;
-    }
+    for (;;) {
+        i = find_root(label, i);
+        j = find_root(label, j);
+        if (i == j) return;
+        const int below = max(i, j);
+        if (atomicCAS(label + below, below, min(i, j)) == below) return;
+    }   // `below` has got a parent meanwhile: on from there
 }
 constexpr int64_t kFewEdges = 1 << 17;   // up to here along every edge at once: a dozen launches cost more than the contention
 __global__ void __launch_bounds__(256) hook_kernel(const int32_t* __restrict__ ptr, const int32_t* __restrict__ adj, int32_t M, int32_t* label) {
@@ -365,12 +369,14 @@ __global__ void __launch_bounds__(256) hook_kernel(const int32_t* __restrict__ p
     const int j = adj[e];
     if (j < i) unite(label, i, j);   // every edge is listed from both ends
 }
-// Every node points to its least neighbour if that is smaller: no two nodes write the same label.  Then four rounds,
-// each along one more edge of every node and with flat trees, so that nobody follows a chain while it grows: a root
-// joins the least root that its nodes see.  That leaves one component with nearly all nodes where the graph
-// has one; its nodes need not look at their other edges, because an edge out of it is found from its other
-// end.  Uniting along every edge had all of them contend for a few roots: 64 000-node stencil 100 to 230 us, power-law
-// graph of 200 000 nodes 430, now 59 and 73 in all.
+// With more edges: first every node points to its least neighbour if that is smaller (the start of ECL-CC: Jaiganesh and
+// Burtscher, "A high-performance connected components implementation for GPUs", 2018); no two nodes write the same
+// label.  Then four rounds, each along one more edge of every node and with flat trees, so that nobody follows a chain
+// while it grows: a root joins the least root that its nodes see.  That leaves one component with nearly all nodes where
+// the graph has one; a sample of the nodes tells which, and its nodes need not look at their other edges, because an edge
+// out of it is found from its other end (Afforest: Sutton, Ben-Nun and Barak, "Optimizing parallel graph connectivity
+// computation via subgraph sampling", 2018).  Uniting along every edge had all of them contend for a few roots: 64 000-node
+// stencil 100 to 230 us, power-law graph of 200 000 nodes 430, now 59 and 73 in all.
 __global__ void least_neighbour_kernel(const int32_t* __restrict__ ptr, const int32_t* __restrict__ adj, int32_t M, int32_t* __restrict__ label) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < M) label[i] = ptr[i] < ptr[i + 1] ? min(i, adj[ptr[i]]) : i;
@@ -420,9 +426,9 @@ __global__ void __launch_bounds__(512) hook_long_kernel(const int32_t* __restric
 __global__ void flatten_labels_kernel(int32_t* __restrict__ label, int32_t M) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= M) return;
-    int cur = __ldcg(label + i), next;
-    while (cur > (next = __ldcg(label + cur))) cur = next;
-    label[i] = cur;
+    int root = i;
+    for (int parent = __ldcg(label + root); parent != root; parent = __ldcg(label + root)) root = parent;
+    __stcg(label + i, root);
 }
 struct IsRoot {
     const int32_t* label;
