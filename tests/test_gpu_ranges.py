@@ -416,3 +416,64 @@ def test_pack_time_does_not_depend_on_where_the_empty_rows_are():
             times.append(a.elapsed_time(b))
         ms[where] = sorted(times)[3]
     assert ms["middle"] < 3 * ms["end"], ms
+
+
+def _chain(engine, p, plan, x, y, steps, widths):
+    """x -> A x -> A A x ..., alternating between two buffers, nothing waited for."""
+    for _ in range(steps):
+        (engine.spmm if widths else engine.spmm_any_width)(p, x, out=y, plan=plan)
+        x, y = y, x
+    return x
+
+
+# kernels start while the one before them drains: both main kernels, with whole and split windows (fix-up pass), rows that
+# are padded first, products that fill the GPU and that do not
+@pytest.mark.parametrize("sweep", [0, 2])
+@pytest.mark.parametrize("N,gt", [(64, 0), (64, 5), (512, 5), (47, 5)])
+@pytest.mark.parametrize("scale", [9, 14])
+def test_overlapped_launches_keep_their_order(sweep, N, gt, scale):
+    import torch
+    from mask_b200 import engine
+    m = G.rmat_gcn_normalised(scale=scale, samples_per_node=8, seed=5)
+    p = engine.pack_srbcrs(*_dev(m), m.M, m.K)
+    whole = N % 4 == 0
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    first = [torch.randn(m.K, N, generator=gen, device="cuda") for _ in range(3)]
+    engine.tune("sweep", sweep)
+    try:
+        plan = p.new_plan("auto", gt)
+        nan = lambda: torch.full((m.M, N), float("nan"), device="cuda")
+        want = []
+        for f in first:                              # one product at a time
+            x, y = f.clone(), nan()
+            for _ in range(6):
+                torch.cuda.synchronize()
+                (engine.spmm if whole else engine.spmm_any_width)(p, x, out=y, plan=plan)
+                torch.cuda.synchronize()
+                x, y = y, x
+            want.append(x.clone())
+        # back to back: each product reads what the last one wrote and overwrites what it read
+        assert torch.equal(_chain(engine, p, plan, first[0].clone(), nan(), 6, whole), want[0])
+        # on three streams at once, with a copy into the operand between the chains
+        streams, got = [torch.cuda.Stream() for _ in first], []
+        x, y = [nan() for _ in first], [nan() for _ in first]
+        torch.cuda.synchronize()
+        for turn in range(3):
+            for s, f, a, b in zip(streams, first, x, y):
+                with torch.cuda.stream(s):
+                    a.copy_(f)
+                    got.append(_chain(engine, p, plan, a, b, 6, whole))
+        torch.cuda.synchronize()
+        for g, w in zip(got, want * 3):
+            assert torch.equal(g, w)
+        # captured, and replayed with other operands
+        x, y = nan(), nan()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            last = _chain(engine, p, plan, x, y, 6, whole)
+        for f, w in list(zip(first, want)) * 2:
+            x.copy_(f)
+            graph.replay()
+            assert torch.equal(last, w)
+    finally:
+        engine.tune("sweep", 1)
