@@ -35,7 +35,8 @@ typedef enum mask_status {
     MASK_ERR_INDEX_OVERFLOW = 5,   /* a count does not fit the int32 index arrays of the format */
     MASK_ERR_COLUMN_RANGE = 6,     /* a column id is outside [0, K) */
     MASK_ERR_NO_DEVICE = 7,
-    MASK_ERR_KERNEL_TIMEOUT = 8    /* a kernel gave up on one of its bounded waits: the output is invalid */
+    MASK_ERR_KERNEL_TIMEOUT = 8,   /* a kernel gave up on one of its bounded waits: the output is invalid */
+    MASK_ERR_OUT_OF_MEMORY = 9     /* host memory; device memory is reported as MASK_ERR_CUDA */
 } mask_status;
 
 int mask_version(void);

@@ -47,6 +47,7 @@ extern "C" const char* mask_status_string(int status) {
         case MASK_ERR_COLUMN_RANGE: return "column id out of range";
         case MASK_ERR_NO_DEVICE: return "no CUDA device";
         case MASK_ERR_KERNEL_TIMEOUT: return "a kernel gave up on a bounded wait";
+        case MASK_ERR_OUT_OF_MEMORY: return "out of host memory";
         default: return "unknown status";
     }
 }
@@ -161,7 +162,8 @@ extern "C" int mask_session_create_srbcrs(int32_t M, int32_t K, int64_t T, const
     *out = nullptr;
     MASK_REQUIRE(M >= 1 && K >= 1 && T >= 0 && h_val_soff, "bad arguments");
     MASK_REQUIRE(T == 0 || (h_val_sidx && h_val_block_val), "packed arrays are NULL");
-    mask_session* s = new mask_session();
+    mask_session* s = new (std::nothrow) mask_session();
+    if (!s) return fail(MASK_ERR_OUT_OF_MEMORY, "out of host memory");
     s->M = M; s->K = K; s->T = T;
     const size_t W = (size_t)window_count(M);
     auto body = [&]() -> int {
@@ -191,7 +193,8 @@ extern "C" int mask_session_create_csr(int32_t M, int32_t K, int64_t nnz, const 
     *out = nullptr;
     MASK_REQUIRE(M >= 1 && K >= 1 && nnz >= 0 && h_rowptr, "bad arguments");
     MASK_REQUIRE(nnz == 0 || (h_colind && h_values), "colind or values is NULL");
-    mask_session* s = new mask_session();
+    mask_session* s = new (std::nothrow) mask_session();
+    if (!s) return fail(MASK_ERR_OUT_OF_MEMORY, "out of host memory");
     s->M = M; s->K = K;
     const size_t W = (size_t)window_count(M);
     DevScratch rowptr_b, colind_b, values_b, work_b;

@@ -210,8 +210,7 @@ extern "C" int mask_features_columns(const int32_t* d_val_soff, const int32_t* d
     const cudaError_t e = cudaStreamSynchronize(st);   // also after a failure: the copy may be in flight
     if (rc != MASK_OK) return rc;
     MASK_CUDA_TRY(e);
-    job.finish(out);
-    return MASK_OK;
+    return without_exceptions([&] { job.finish(out); return MASK_OK; });
 }
 
 namespace mask {

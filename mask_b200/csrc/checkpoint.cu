@@ -18,11 +18,13 @@
 extern "C" int mask_metcf_checkpoint_name(const char* matrix_name, int32_t M, int32_t K, char* out, size_t out_len) {
     using namespace mask;
     MASK_REQUIRE(out != nullptr && out_len > 0, "bad arguments");
-    std::string base = (matrix_name && matrix_name[0]) ? matrix_name : "synthetic";
-    const std::string name = base + "_M" + std::to_string(M) + "_K" + std::to_string(K) + "_TBK8_RWM16_METCF.checkpoint";
-    if (name.size() + 1 > out_len) return fail(MASK_ERR_INVALID_ARGUMENT, "name buffer too small");
-    std::memcpy(out, name.c_str(), name.size() + 1);
-    return MASK_OK;
+    return without_exceptions([&]() -> int {
+        std::string base = (matrix_name && matrix_name[0]) ? matrix_name : "synthetic";
+        const std::string name = base + "_M" + std::to_string(M) + "_K" + std::to_string(K) + "_TBK8_RWM16_METCF.checkpoint";
+        if (name.size() + 1 > out_len) return fail(MASK_ERR_INVALID_ARGUMENT, "name buffer too small");
+        std::memcpy(out, name.c_str(), name.size() + 1);
+        return MASK_OK;
+    });
 }
 
 // The name the reference's testbed gives the file for a matrix read from `file_path` -- the file
@@ -34,28 +36,30 @@ extern "C" int mask_metcf_checkpoint_name_for(const char* file_path, int32_t M, 
                                               size_t out_len) {
     using namespace mask;
     MASK_REQUIRE(out != nullptr && out_len > 0, "bad arguments");
-    std::string path = file_path ? file_path : "";
-    std::string base = path;
-    const size_t slash = base.find_last_of('/');
-    if (slash != std::string::npos) base = base.substr(slash + 1);
-    const size_t dot = base.find_last_of('.');
-    if (dot != std::string::npos && dot > 0 && base != "..") base = base.substr(0, dot);
-    if (base.empty()) base = "synthetic";
-    std::string name = base + "_M" + std::to_string(M) + "_K" + std::to_string(K) + "_TBK8_RWM16";
-    if (path.empty()) {
-        char buf[64];
-        std::snprintf(buf, sizeof(buf), "%.4f", (double)sparsity);
-        std::string tok = buf;
-        while (!tok.empty() && tok.back() == '0') tok.pop_back();
-        if (!tok.empty() && tok.back() == '.') tok.pop_back();
-        for (char& c : tok)
-            if (c == '.') c = 'p';
-        name += "_sp" + (tok.empty() ? std::string("unknown") : tok);
-    }
-    name += "_METCF.checkpoint";
-    if (name.size() + 1 > out_len) return fail(MASK_ERR_INVALID_ARGUMENT, "name buffer too small");
-    std::memcpy(out, name.c_str(), name.size() + 1);
-    return MASK_OK;
+    return without_exceptions([&]() -> int {
+        std::string path = file_path ? file_path : "";
+        std::string base = path;
+        const size_t slash = base.find_last_of('/');
+        if (slash != std::string::npos) base = base.substr(slash + 1);
+        const size_t dot = base.find_last_of('.');
+        if (dot != std::string::npos && dot > 0 && base != "..") base = base.substr(0, dot);
+        if (base.empty()) base = "synthetic";
+        std::string name = base + "_M" + std::to_string(M) + "_K" + std::to_string(K) + "_TBK8_RWM16";
+        if (path.empty()) {
+            char buf[64];
+            std::snprintf(buf, sizeof(buf), "%.4f", (double)sparsity);
+            std::string tok = buf;
+            while (!tok.empty() && tok.back() == '0') tok.pop_back();
+            if (!tok.empty() && tok.back() == '.') tok.pop_back();
+            for (char& c : tok)
+                if (c == '.') c = 'p';
+            name += "_sp" + (tok.empty() ? std::string("unknown") : tok);
+        }
+        name += "_METCF.checkpoint";
+        if (name.size() + 1 > out_len) return fail(MASK_ERR_INVALID_ARGUMENT, "name buffer too small");
+        std::memcpy(out, name.c_str(), name.size() + 1);
+        return MASK_OK;
+    });
 }
 
 extern "C" int mask_metcf_checkpoint_write(const char* path, int32_t M, int64_t T, int64_t nnz_pad, const int32_t* val_soff,
@@ -124,30 +128,32 @@ extern "C" int mask_metcf_checkpoint_read(const char* path, int32_t M, int32_t K
 extern "C" int mask_features_from_soff(const int32_t* h_val_soff, int32_t M, int64_t nnz, mask_features* out) {
     using namespace mask;
     MASK_REQUIRE(h_val_soff && out && M >= 1 && nnz >= 0, "bad arguments");
-    const int W = window_count(M);
-    std::vector<int32_t> len((size_t)W);
-    for (int w = 0; w < W; w++) len[w] = h_val_soff[w + 1] - h_val_soff[w];
-    std::sort(len.begin(), len.end());
-    auto pct = [&](double q) {  // same rank rule as the bridge's p95 (custom_format_e2e.cu:652-657)
-        const size_t i = std::min(len.size() - 1, (size_t)std::ceil(len.size() * q) - 1);
-        return len[i];
-    };
-    mask_features f{};
-    f.row_windows = W;
-    f.tiles = h_val_soff[W];
-    f.nnz = nnz;
-    f.tiles_mean = W ? (double)f.tiles / W : 0.0;
-    f.tiles_p50 = pct(0.50);
-    f.tiles_p95 = pct(0.95);
-    f.tiles_p99 = pct(0.99);
-    f.tiles_max = len.back();
-    int64_t top5 = 0;
-    for (int i = 0; i < std::min(5, W); i++) top5 += len[(size_t)W - 1 - i];
-    f.top5_window_share = f.tiles ? (double)top5 / (double)f.tiles : 0.0;
-    f.tile_fill = f.tiles ? (double)nnz / (128.0 * (double)f.tiles) : 0.0;
-    // the bridge's heavy-tail test (custom_format_e2e.cu:659-663)
-    f.heavy_tail = f.tiles_max > std::max(64, 4 * std::max(f.tiles_p95, 1)) ? 1 : 0;
-    f.empty_windows = (int32_t)(std::lower_bound(len.begin(), len.end(), 1) - len.begin());
-    *out = f;
-    return MASK_OK;
+    return without_exceptions([&]() -> int {
+        const int W = window_count(M);
+        std::vector<int32_t> len((size_t)W);
+        for (int w = 0; w < W; w++) len[w] = h_val_soff[w + 1] - h_val_soff[w];
+        std::sort(len.begin(), len.end());
+        auto pct = [&](double q) {  // same rank rule as the bridge's p95 (custom_format_e2e.cu:652-657)
+            const size_t i = std::min(len.size() - 1, (size_t)std::ceil(len.size() * q) - 1);
+            return len[i];
+        };
+        mask_features f{};
+        f.row_windows = W;
+        f.tiles = h_val_soff[W];
+        f.nnz = nnz;
+        f.tiles_mean = W ? (double)f.tiles / W : 0.0;
+        f.tiles_p50 = pct(0.50);
+        f.tiles_p95 = pct(0.95);
+        f.tiles_p99 = pct(0.99);
+        f.tiles_max = len.back();
+        int64_t top5 = 0;
+        for (int i = 0; i < std::min(5, W); i++) top5 += len[(size_t)W - 1 - i];
+        f.top5_window_share = f.tiles ? (double)top5 / (double)f.tiles : 0.0;
+        f.tile_fill = f.tiles ? (double)nnz / (128.0 * (double)f.tiles) : 0.0;
+        // the bridge's heavy-tail test (custom_format_e2e.cu:659-663)
+        f.heavy_tail = f.tiles_max > std::max(64, 4 * std::max(f.tiles_p95, 1)) ? 1 : 0;
+        f.empty_windows = (int32_t)(std::lower_bound(len.begin(), len.end(), 1) - len.begin());
+        *out = f;
+        return MASK_OK;
+    });
 }

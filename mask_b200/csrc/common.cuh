@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <cstdio>
+#include <new>
 
 #include "mask_b200.h"
 
@@ -18,6 +19,18 @@ void set_error(const char* fmt, ...);
 inline int fail(int status, const char* what) {
     set_error("%s", what);
     return status;
+}
+
+// Runs the part of an entry point that allocates host memory: nothing may be thrown through the C ABI.
+template <typename Body>
+int without_exceptions(Body body) noexcept {
+    try {
+        return body();
+    } catch (const std::bad_alloc&) {
+        return fail(MASK_ERR_OUT_OF_MEMORY, "out of host memory");
+    } catch (...) {
+        return fail(MASK_ERR_INVALID_ARGUMENT, "unexpected exception");
+    }
 }
 
 #define MASK_CUDA_TRY(expr)                                                              \

@@ -84,9 +84,11 @@ HostStage::~HostStage() {
     {
         std::lock_guard<std::mutex> lock(host_mu());
         if (g_host_kept + size_ <= kHostCacheKeep) {
-            host_free().push_back({p_, size_});
-            g_host_kept += size_;
-            return;
+            const int rc = without_exceptions([&] { host_free().push_back({p_, size_}); return MASK_OK; });
+            if (rc == MASK_OK) {
+                g_host_kept += size_;
+                return;
+            }
         }
     }
     cudaFreeHost(p_);

@@ -502,27 +502,31 @@ extern "C" int mask_plan_strict_lb(const int32_t* h_val_soff, int32_t M, int32_t
                                    int64_t* n_groups) {
     using namespace mask;
     MASK_REQUIRE(h_val_soff != nullptr && M >= 1 && workload >= 1 && n_frag && n_groups, "bad arguments");
-    std::vector<int32_t> rbo, rb2w, go;
-    strict_lb(h_val_soff, window_count(M), workload, rbo, rb2w, go);
-    *n_frag = (int64_t)rb2w.size();
-    *n_groups = (int64_t)go.size() - 1;
-    if (row_block_offset) std::memcpy(row_block_offset, rbo.data(), rbo.size() * sizeof(int32_t));
-    if (row_block_to_window && !rb2w.empty()) std::memcpy(row_block_to_window, rb2w.data(), rb2w.size() * sizeof(int32_t));
-    if (group_offset) std::memcpy(group_offset, go.data(), go.size() * sizeof(int32_t));
-    return MASK_OK;
+    return without_exceptions([&] {
+        std::vector<int32_t> rbo, rb2w, go;
+        strict_lb(h_val_soff, window_count(M), workload, rbo, rb2w, go);
+        *n_frag = (int64_t)rb2w.size();
+        *n_groups = (int64_t)go.size() - 1;
+        if (row_block_offset) std::memcpy(row_block_offset, rbo.data(), rbo.size() * sizeof(int32_t));
+        if (row_block_to_window && !rb2w.empty()) std::memcpy(row_block_to_window, rb2w.data(), rb2w.size() * sizeof(int32_t));
+        if (group_offset) std::memcpy(group_offset, go.data(), go.size() * sizeof(int32_t));
+        return MASK_OK;
+    });
 }
 
 extern "C" int mask_plan_multi_bind(const int32_t* h_val_soff, int32_t M, int32_t* task_window, int32_t* window_split,
                                     int32_t* task_soff, int64_t* n_tasks) {
     using namespace mask;
     MASK_REQUIRE(h_val_soff != nullptr && M >= 1 && n_tasks, "bad arguments");
-    std::vector<int32_t> tw, ws, ts;
-    multi_bind(h_val_soff, window_count(M), tw, ws, ts);
-    *n_tasks = (int64_t)tw.size();
-    if (task_window && !tw.empty()) std::memcpy(task_window, tw.data(), tw.size() * sizeof(int32_t));
-    if (window_split && !ws.empty()) std::memcpy(window_split, ws.data(), ws.size() * sizeof(int32_t));
-    if (task_soff) std::memcpy(task_soff, ts.data(), ts.size() * sizeof(int32_t));
-    return MASK_OK;
+    return without_exceptions([&] {
+        std::vector<int32_t> tw, ws, ts;
+        multi_bind(h_val_soff, window_count(M), tw, ws, ts);
+        *n_tasks = (int64_t)tw.size();
+        if (task_window && !tw.empty()) std::memcpy(task_window, tw.data(), tw.size() * sizeof(int32_t));
+        if (window_split && !ws.empty()) std::memcpy(window_split, ws.data(), ws.size() * sizeof(int32_t));
+        if (task_soff) std::memcpy(task_soff, ts.data(), ts.size() * sizeof(int32_t));
+        return MASK_OK;
+    });
 }
 
 namespace mask {
@@ -530,7 +534,8 @@ namespace mask {
 // With d_val_sidx the column features are measured and the plan table is applied as well.
 static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t M, int32_t K, int64_t T, int policy,
                        int32_t group_tiles, cudaStream_t st, mask_plan** out) {
-    mask_plan* p = new mask_plan();
+    mask_plan* p = new (std::nothrow) mask_plan();
+    if (!p) return fail(MASK_ERR_OUT_OF_MEMORY, "out of host memory");
     p->M = M;
     p->W = window_count(M);
     p->T = T;
@@ -582,7 +587,7 @@ static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int
         build_tables(*p, soff);
         return upload_tables(*p, soff, st);
     };
-    const int rc = body();
+    const int rc = without_exceptions(body);
     if (rc != MASK_OK) cudaStreamSynchronize(st);   // copies into the staging buffers may be in flight
     if (rc != MASK_OK) {
         mask_plan_destroy(p);

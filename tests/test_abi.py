@@ -199,3 +199,31 @@ def test_features_and_ref_auto_rule(oracle_mod):
         if soff[-1]:
             assert abs(f.tile_fill - m.nnz / (128.0 * soff[-1])) < 1e-12
             assert abs(f.top5_window_share - lens[-5:].sum() / soff[-1]) < 1e-12
+
+
+# in a process of its own with its address space limited: an exception that leaves the library ends the process
+OUT_OF_MEMORY = """
+import ctypes as C, resource
+import numpy as np
+from mask_b200 import _lib
+L = _lib.lib()
+n = [C.c_int64(), C.c_int64()]
+f = _lib.Features()
+long = np.array([0, 1 << 28], dtype=np.int32)          # one window: 2^28 pieces of one tile
+many = np.zeros((1 << 27) + 1, dtype=np.int32)         # 2^27 windows
+size = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+resource.setrlimit(resource.RLIMIT_AS, (size + (256 << 20), resource.getrlimit(resource.RLIMIT_AS)[1]))
+got = [L.mask_plan_strict_lb(long.ctypes.data, 16, 1, None, None, None, C.byref(n[0]), C.byref(n[1])),
+       L.mask_plan_multi_bind(many.ctypes.data, 2**31 - 1, None, None, None, C.byref(n[0])),
+       L.mask_features_from_soff(many.ctypes.data, 2**31 - 1, 0, C.byref(f))]
+print(got, L.mask_status_string(9).decode())
+"""
+
+
+def test_out_of_host_memory_is_a_status():
+    import subprocess
+    import sys
+    r = subprocess.run([sys.executable, "-c", OUT_OF_MEMORY], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-500:]
+    assert r.stdout.strip() == "[9, 9, 9] out of host memory"
