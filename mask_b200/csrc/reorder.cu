@@ -762,15 +762,14 @@ int symmetrised_pattern(const int32_t* rowptr, const int32_t* colind, int32_t M,
     return MASK_OK;
 }
 
-int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, int64_t nnz, int32_t* order, cudaStream_t st) {
+// `host`: 4 bytes; after a failure a copy into them may be in flight
+int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, int64_t nnz, int32_t* order, const HostStage& host, cudaStream_t st) {
     const unsigned node_blocks = blocks_for(M, 256);
     const int32_t *ptr = rowptr, *col = colind;
     int64_t n_edges = nnz;
     DevScratch deg_b, flag_b, sym_ptr, sym_adj;
-    HostStage host;
     int rc = deg_b.alloc(((size_t)M + 1) * 4, st);
     if (rc == MASK_OK) rc = flag_b.alloc(64, st);
-    if (rc == MASK_OK) rc = host.get(64);
     if (rc != MASK_OK) return rc;
     int32_t* deg = deg_b.as<int32_t>();
     int32_t* flags = flag_b.as<int32_t>();   // [0] asymmetric, [1] long lists, [2] start nodes, [4..5] state of the traversal, [6] most common label
@@ -909,7 +908,9 @@ extern "C" int mask_reorder_rows(int kind, const int32_t* d_rowptr, const int32_
     MASK_REQUIRE(nnz32 == 0 || d_colind, "colind is NULL");
     if (kind == MASK_REORDER_ROW_RCM) {
         if (M != K) return fail(MASK_ERR_INVALID_ARGUMENT, "row_rcm needs a square matrix");
-        return order_rcm_device(d_rowptr, d_colind, M, nnz32, d_row_order, st);
+        rc = order_rcm_device(d_rowptr, d_colind, M, nnz32, d_row_order, host, st);
+        if (rc != MASK_OK) cudaStreamSynchronize(st);   // before the host words go to someone else
+        return rc;
     }
     DevScratch first, sig, ids, by_first;
     rc = first.alloc((size_t)M * 4, st);
