@@ -380,7 +380,9 @@ static int check_packed_alignment(const SpmmArgs& a) {
 template <int FMT>
 static int launch_spmm(const mask_plan* plan, SpmmArgs a, cudaStream_t st) {
     if (plan->G == 0) return MASK_OK;
-    if (a.tf32x3 || g_tune_sweep != 0 || g_tune_async != 0) {   // every kernel but the register-pipelined one
+    // the register-pipelined kernel writes C 16 bytes at a time: rows that are not whole vectors go to the tcgen05 kernel
+    const bool registers = g_tune_sweep == 0 && g_tune_async == 0 && !a.tf32x3 && a.vec_out;
+    if (!registers) {
         const int bad = check_packed_alignment(a);
         if (bad != MASK_OK) return bad;
     }
@@ -401,7 +403,7 @@ static int launch_spmm(const mask_plan* plan, SpmmArgs a, cudaStream_t st) {
         rc = launch_spmm_tma(plan, a, a.K, st, g_tune_nslab != 0 ? g_tune_nslab : plan->nslab);
         return rc != MASK_OK ? rc : launch_fixup(plan, a, st);
     }
-    if (g_tune_sweep != 0) {
+    if (g_tune_sweep != 0 || !a.vec_out) {
         rc = launch_spmm_sweep(plan, a, st, g_tune_nslab != 0 ? g_tune_nslab : plan->nslab);
         return rc != MASK_OK ? rc : launch_fixup(plan, a, st);
     }

@@ -150,6 +150,26 @@ def test_rows_that_are_not_whole_vectors(oracle_mod, fmt, N, offset, sweep):
         engine.tune("sweep", 1)
 
 
+@pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
+@pytest.mark.parametrize("N", [47, 130])
+def test_rows_that_are_not_whole_vectors_under_the_comparison_knobs(oracle_mod, fmt, N):
+    """The register-pipelined kernel, which only the knobs select, writes C 16 bytes at a time."""
+    import torch
+    from mask_b200 import engine
+    m = _mixed_matrix()
+    p = {"srbcrs": engine.pack_srbcrs, "metcf": engine.pack_metcf, "mco": engine.pack_mco}[fmt](*_dev(m), m.M, m.K)
+    B = np.random.Generator(np.random.PCG64(N)).standard_normal((m.K, N), dtype=np.float32)
+    engine.tune("sweep", 0)
+    engine.tune("async", 0)
+    try:
+        for gt in (0, 5):
+            out = engine.spmm_any_width(p, torch.from_numpy(B).cuda(), plan=p.new_plan("auto", gt))
+            _assert_close(oracle_mod, m, B, out.cpu().numpy())
+    finally:
+        engine.tune("sweep", 1)
+        engine.tune("async", 1)
+
+
 def _graph(edges, n, extra=()):
     e = np.array(sorted(set(edges) | set(extra)), dtype=np.int64)
     order = np.lexsort((e[:, 1], e[:, 0])) if len(e) else np.zeros(0, np.int64)
