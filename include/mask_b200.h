@@ -366,7 +366,10 @@ int mask_spmm(const mask_plan* plan, const mask_matrix* matrix, int32_t n, const
  * cudaMalloc / cudaFree and uses no allocating library routine.
  *   - A plan whose partial tiles for this N exceed the capacity (mask_plan_scratch_bytes(plan, N)
  *     > capacity; 1024 partial tiles at N = 512) is refused with MASK_ERR_SCRATCH_TOO_SMALL and
- *     nothing is launched.
+ *     nothing is launched -- unless it is an AUTO plan of default group size and the partial tiles
+ *     would fit if windows were cut into pieces of that size (mask_plan_info's group_tiles): such a
+ *     plan's own pieces may be shorter, and the product is then taken in several launches of fewer
+ *     columns.
  *   - The first call on each device looks up the array's device address
  *     (cudaGetSymbolAddress, with that device current).  Make that first call during start-up,
  *     before any stream capture begins.  The address is remembered per device ordinal for the

@@ -157,7 +157,7 @@ constexpr int32_t kFragCost = 4;
 constexpr int64_t kHigh = (int64_t)1 << 32;   // the scans carry two counts: one in each half
 
 struct PlanCounts {          // on the device in front of the tables, and on the host
-    int32_t frags, heads, groups, warp_groups, bad, pad[3];
+    int32_t frags, heads, groups, warp_groups, bad, group_pieces, pad[2];
     int32_t status[4];
 };
 
@@ -207,6 +207,8 @@ struct PiecesOut {
             at += base + (i < rem ? 1 : 0);
         }
         if (split) a.heads[split_before] = make_int2((int)first, (int)parts);
+        const int64_t group = a.group;
+        if (x > group + group / 4) atomicAdd(&a.counts->group_pieces, (int32_t)((x + group - 1) / group));
         if (w == a.W - 1) {
             a.frag_off[first + parts] = at;
             if (at != a.T) a.counts->bad = 1;
@@ -252,6 +254,7 @@ struct GroupsOut {
             a.host->frags = F;
             a.host->heads = a.counts->heads;
             a.host->groups = g + v;
+            a.host->group_pieces = a.counts->group_pieces;
             a.host->bad = 0;
         }
     }
@@ -461,6 +464,7 @@ static int upload_tables(mask_plan& p, const int32_t* soff, cudaStream_t st) {
         p.P++;
     }
     p.H = (int64_t)heads.size() / 2;
+    p.P_group = p.P;
     size_t at = 0;
     auto section = [&](size_t n) { const size_t o = at; at += (n + 3) & ~(size_t)3; return o; };
     const size_t o_fo = section(fo.size()), o_fw = section(fw.size()), o_fs = section(fw.size()), o_go = section(go.size()),
@@ -572,6 +576,7 @@ static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int
             p->F = c.frags;
             p->H = c.heads;
             p->P = p->F - (p->W - p->H);
+            p->P_group = c.group_pieces;
             p->G = c.groups;
             p->Gw = group_tiles > 0 ? p->G : c.warp_groups;
             return MASK_OK;

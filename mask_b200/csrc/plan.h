@@ -27,6 +27,7 @@ struct mask_plan {
     int32_t piece_tiles = 0;  // windows of more than 5/4 of this are split
     int64_t P = 0;  // fragments that are part of a split window
     int64_t H = 0;  // split windows
+    int64_t P_group = 0;  // P if windows were split into pieces of group_tiles
     int32_t nslab = 0;  // persistent kernel: 128-column slabs per column block (0 = the widest N fills)
     int device = 0;
     std::vector<int32_t> h_frag_off, h_frag_win, h_group_off;   // tables built on the host (every policy but AUTO)

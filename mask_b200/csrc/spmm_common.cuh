@@ -24,6 +24,7 @@ struct SpmmArgs {
     const unsigned long long* mco_mask;   // MCO: two 64-bit words per tile, bit Swizzle<1,2,3>(8r+c)
     float* const* peer_out;    // optional: n_peer_out more output bases (peer GPUs' copies of C, same layout)
     int32_t n_peer_out;
+    int32_t peer_col;          // column of the peers' copies that column 0 of this launch's C is
     const int32_t* row_map;    // optional: packed row i is output row row_map[i] (row reorder undone on the fly)
     const float* B;
     int64_t ldb;
@@ -137,7 +138,7 @@ __device__ __forceinline__ void flush_fragment(const SpmmArgs& p, int ff, int co
                 if (slot < 0) {  // the same row into every peer's copy of C (plain stores over NVLink)
                     const int64_t off = row - p.C;
                     for (int j = 0; j < p.n_peer_out; j++) {
-                        float* prow = p.peer_out[j] + off;
+                        float* prow = p.peer_out[j] + p.peer_col + off;
                         if (c0 < p.N) *reinterpret_cast<float4*>(prow + c0) = v0;
                         if (c0 + 4 < p.N) *reinterpret_cast<float4*>(prow + c0 + 4) = v1;
                     }
@@ -150,6 +151,11 @@ __device__ __forceinline__ void flush_fragment(const SpmmArgs& p, int ff, int co
             for (int i = 0; i < 4; i++) acc[q][j][i] = 0.f;
     }
 }
+
+// spmm_mma.cu: the array entry points, in pieces of at most `most` columns.  Scratch for one piece.
+int spmm_arrays(const mask_plan* plan, const mask_matrix& m, int32_t N, const float* d_B, int64_t ldb, float* d_C, int64_t ldc, void* d_scratch,
+                size_t scratch_bytes, int epilogue, void* stream, int32_t most);
+constexpr int32_t kPieceColumns = 1 << 21;
 
 // spmm_sweep.cu: persistent tcgen05 kernel, any N % 4 == 0, groups of any length.  nslab = 128-column
 // slabs per column block (1, 2, 4; 0 = by N).

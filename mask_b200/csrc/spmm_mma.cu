@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, MIN_BLOCKS) spmm_mma_kern
                     if (slot < 0) {  // the same row into every peer's copy of C
                         const int64_t off = row - p.C;
                         for (int j = 0; j < p.n_peer_out; j++) {
-                            float* prow = p.peer_out[j] + off;
+                            float* prow = p.peer_out[j] + p.peer_col + off;
                             if (c0 < p.N) *reinterpret_cast<float4*>(prow + c0) = v0;
                             if (c0 + 4 < p.N) *reinterpret_cast<float4*>(prow + c0 + 4) = v1;
                         }
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, MIN_BLOCKS) spmm_mma_kern
 __global__ void __launch_bounds__(256) spmm_fixup_kernel(const int2* heads, const int32_t* frag_win, const int32_t* frag_slot,
                                                         const float* scratch, float* C, int64_t ldc, int32_t M,
                                                         int32_t N, int32_t n_out, int32_t vec_out, int32_t relu, const int32_t* row_map,
-                                                        float* const* peer_out, int32_t n_peer_out) {
+                                                        float* const* peer_out, int32_t n_peer_out, int32_t peer_col) {
     let_next_kernel_start();
     const int2 head = heads[blockIdx.x];
     const int w = frag_win[head.x];
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(256) spmm_fixup_kernel(const int2* heads, cons
             continue;
         }
         *reinterpret_cast<float4*>(C + (int64_t)out_row * ldc + c) = s;
-        for (int j = 0; j < n_peer_out; j++) *reinterpret_cast<float4*>(peer_out[j] + (int64_t)out_row * ldc + c) = s;
+        for (int j = 0; j < n_peer_out; j++) *reinterpret_cast<float4*>(peer_out[j] + peer_col + (int64_t)out_row * ldc + c) = s;
     }
 }
 
@@ -316,7 +316,7 @@ static int launch_fixup(const mask_plan* plan, const SpmmArgs& a, cudaStream_t s
     if (plan->H > 0) {
         dim3 fgrid((unsigned)plan->H, (unsigned)((kWinRows * (a.N >> 2) + 255) / 256));
         return launch_overlapped(spmm_fixup_kernel, fgrid, 256, 0, st, plan->d_heads, plan->d_frag_win, plan->d_frag_slot, a.scratch, a.C,
-                                 a.ldc, a.M, a.N, a.n_out, a.vec_out, a.relu, a.row_map, a.peer_out, a.n_peer_out);
+                                 a.ldc, a.M, a.N, a.n_out, a.vec_out, a.relu, a.row_map, a.peer_out, a.n_peer_out, a.peer_col);
     }
     return MASK_OK;
 }
@@ -431,7 +431,7 @@ static int launch_spmm(const mask_plan* plan, SpmmArgs a, cudaStream_t st) {
 }
 
 static int check_common(const mask_plan* plan, int32_t M, int32_t K, int32_t N, const float* B, int64_t ldb,
-                        float* C, int64_t ldc, void* scratch, size_t scratch_bytes) {
+                        float* C, int64_t ldc, void* scratch, size_t scratch_bytes, int32_t scratch_columns) {
     MASK_REQUIRE(plan != nullptr, "plan is NULL");
     MASK_REQUIRE(M == plan->M, "M differs from the plan's");
     MASK_REQUIRE(M >= 1 && K >= 1 && N >= 0, "M, K must be positive and N non-negative");
@@ -442,7 +442,7 @@ static int check_common(const mask_plan* plan, int32_t M, int32_t K, int32_t N, 
     MASK_REQUIRE(ldb < ((int64_t)1 << 30), "ldb too large");
     MASK_REQUIRE((reinterpret_cast<uintptr_t>(B) & 15) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0,
                  "B and C must be 16-byte aligned");
-    const size_t need = mask_plan_scratch_bytes(plan, N);
+    const size_t need = mask_plan_scratch_bytes(plan, scratch_columns);
     if (need > 0) {
         if (scratch == nullptr || scratch_bytes < need) return fail(MASK_ERR_SCRATCH_TOO_SMALL, "scratch too small for the plan's split windows");
         MASK_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 15) == 0, "scratch must be 16-byte aligned");
@@ -543,18 +543,15 @@ static int fill_matrix_args(const mask_plan* plan, const mask_matrix* m, SpmmArg
 
 namespace mask {
 
-// Column blocks, and rows of partial tiles in the fix-up pass, are numbered in the y dimension of a grid (at most
-// 65 535), so wider products are taken in pieces of this many columns, one after the other.  Peers' copies of C are
-// written at the same offsets as C itself: such products stay whole.
-constexpr int32_t kPieceColumns = 1 << 21;
-
-static int launch_pieces(const mask_plan* plan, int format, const SpmmArgs& a, cudaStream_t st) {
-    const int32_t most = plan->n_peer_out ? a.N : kPieceColumns;
+// One after the other, products of at most `most` columns.  Column blocks, and rows of partial tiles in the fix-up pass,
+// are numbered in the y dimension of a grid (at most 65 535): that many columns are kPieceColumns.
+static int launch_pieces(const mask_plan* plan, int format, const SpmmArgs& a, int32_t most, cudaStream_t st) {
     for (int32_t c0 = 0, width; c0 < a.N; c0 += width) {
         SpmmArgs piece = a;
         width = std::min(most, a.N - c0);
         piece.B += c0;
         piece.C += c0;
+        piece.peer_col = c0;
         piece.N = width;
         piece.n_out = std::min(width, a.n_out - c0);
         const int rc = format == kFmtSrbcrs ? launch_spmm<kFmtSrbcrs>(plan, piece, st)
@@ -564,11 +561,9 @@ static int launch_pieces(const mask_plan* plan, int format, const SpmmArgs& a, c
     return MASK_OK;
 }
 
-}  // namespace mask
-
-extern "C" int mask_spmm(const mask_plan* plan, const mask_matrix* m, int32_t n, const float* d_B, int64_t ldb, float* d_C, int64_t ldc,
-                         float* d_pad, void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
-    using namespace mask;
+// mask_spmm with scratch for `scratch_columns` columns, in pieces of at most `most`
+static int spmm_in_pieces(const mask_plan* plan, const mask_matrix* m, int32_t n, const float* d_B, int64_t ldb, float* d_C, int64_t ldc,
+                          float* d_pad, void* d_scratch, size_t scratch_bytes, int epilogue, void* stream, int32_t most, int32_t scratch_columns) {
     MASK_REQUIRE(plan != nullptr && m != nullptr, "plan or matrix is NULL");
     MASK_REQUIRE(n >= 0 && n <= 0x7fffffff - 3, "bad column count");
     if (n == 0) return MASK_OK;
@@ -580,7 +575,8 @@ extern "C" int mask_spmm(const mask_plan* plan, const mask_matrix* m, int32_t n,
     MASK_REQUIRE(vec_out || plan->n_peer_out == 0, "peer outputs need N % 4 == 0, ldc % 4 == 0 and 16-byte aligned C");
     const float* B = pad ? d_pad : d_B;
     const int64_t ld = pad ? n4 : ldb;
-    int rc = check_common(plan, m->M, m->K, n4, B, ld, vec_out ? d_C : const_cast<float*>(B), vec_out ? ldc : n4, d_scratch, scratch_bytes);
+    int rc = check_common(plan, m->M, m->K, n4, B, ld, vec_out ? d_C : const_cast<float*>(B), vec_out ? ldc : n4, d_scratch, scratch_bytes,
+                          std::min(n4, scratch_columns));
     if (rc != MASK_OK) return rc;
     SpmmArgs a{};
     rc = fill_matrix_args(plan, m, a);
@@ -597,16 +593,23 @@ extern "C" int mask_spmm(const mask_plan* plan, const mask_matrix* m, int32_t n,
                                reinterpret_cast<float4*>(d_pad));
         if (rc != MASK_OK) return rc;
     }
-    return launch_pieces(plan, m->format, a, st);
+    return launch_pieces(plan, m->format, a, std::min(most, kPieceColumns), st);
+}
+
+}  // namespace mask
+
+extern "C" int mask_spmm(const mask_plan* plan, const mask_matrix* m, int32_t n, const float* d_B, int64_t ldb, float* d_C, int64_t ldc,
+                         float* d_pad, void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
+    return mask::spmm_in_pieces(plan, m, n, d_B, ldb, d_C, ldc, d_pad, d_scratch, scratch_bytes, epilogue, stream, mask::kPieceColumns, 0x7fffffff);
 }
 
 // The entry points that take a matrix array by array.
 namespace mask {
-static int spmm_arrays(const mask_plan* plan, const mask_matrix& m, int32_t N, const float* d_B, int64_t ldb, float* d_C, int64_t ldc,
-                       void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
-    const int rc = check_common(plan, m.M, m.K, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes);
+int spmm_arrays(const mask_plan* plan, const mask_matrix& m, int32_t N, const float* d_B, int64_t ldb, float* d_C, int64_t ldc, void* d_scratch,
+                size_t scratch_bytes, int epilogue, void* stream, int32_t most) {
+    const int rc = check_common(plan, m.M, m.K, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, std::min(N, most));
     if (rc != MASK_OK || N == 0) return rc;
-    return mask_spmm(plan, &m, N, d_B, ldb, d_C, ldc, nullptr, d_scratch, scratch_bytes, epilogue, stream);
+    return spmm_in_pieces(plan, &m, N, d_B, ldb, d_C, ldc, nullptr, d_scratch, scratch_bytes, epilogue, stream, most, most);
 }
 }  // namespace mask
 
@@ -616,7 +619,7 @@ extern "C" int mask_spmm_srbcrs(const mask_plan* plan, const int32_t* d_val_soff
                                 int epilogue, void* stream) {
     (void)d_val_soff;
     const mask_matrix m{mask::kFmtSrbcrs, M, K, 0, d_val_sidx, nullptr, nullptr, d_val_block_val};
-    return mask::spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, epilogue, stream);
+    return mask::spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, epilogue, stream, 0x7fffffff);
 }
 
 extern "C" int mask_spmm_metcf(const mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx,
@@ -625,7 +628,7 @@ extern "C" int mask_spmm_metcf(const mask_plan* plan, const int32_t* d_val_soff,
                                void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
     (void)d_val_soff;
     const mask_matrix m{mask::kFmtMetcf, M, K, 0, d_val_sidx, d_val_coo_off, d_val_coo_idx, d_val_coo_val};
-    return mask::spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, epilogue, stream);
+    return mask::spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, epilogue, stream, 0x7fffffff);
 }
 
 extern "C" int mask_spmm_mco(const mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx,
@@ -634,5 +637,5 @@ extern "C" int mask_spmm_mco(const mask_plan* plan, const int32_t* d_val_soff, c
                              void* d_scratch, size_t scratch_bytes, int epilogue, void* stream) {
     (void)d_val_soff;
     const mask_matrix m{mask::kFmtMco, M, K, 0, d_val_sidx, d_val_mco_off, d_val_mco_mask, d_val_mco_val};
-    return mask::spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, epilogue, stream);
+    return mask::spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, d_scratch, scratch_bytes, epilogue, stream, 0x7fffffff);
 }

@@ -11,7 +11,7 @@
 #include <mutex>
 
 #include "common.cuh"
-#include "plan.h"
+#include "spmm_common.cuh"
 
 namespace {
 
@@ -51,7 +51,12 @@ extern "C" int mask_spmm_srbcrs_static_scratch(const mask_plan* plan, const int3
     using namespace mask;
     MASK_REQUIRE(plan != nullptr, "plan is NULL");
     const size_t need = mask_plan_scratch_bytes(plan, N);
-    if (need > kStaticScratchBytes) {
+    // The pieces of a default plan may be shorter than its groups, for more blocks to work on them, and their partial
+    // tiles several times as many (power-law graph with 2^15 nodes: 1926 for 241).  That is no reason to refuse: the
+    // product then goes in pieces of columns whose partial tiles fit.
+    const size_t a_column = (size_t)plan->P * kWinRows * sizeof(float), in_groups = (size_t)plan->P_group * kWinRows * sizeof(float);
+    const int32_t most = need > kStaticScratchBytes ? (int32_t)(kStaticScratchBytes / a_column) & ~31 : N;
+    if (need > kStaticScratchBytes && (most == 0 || in_groups * (size_t)N > kStaticScratchBytes)) {
         set_error("this plan needs %zu bytes of partial tiles for N=%d but the built-in buffer holds %zu; use a plan "
                   "that splits fewer windows (policy row, or a larger group_tiles) or call mask_spmm_srbcrs with a "
                   "buffer of your own",
@@ -64,6 +69,7 @@ extern "C" int mask_spmm_srbcrs_static_scratch(const mask_plan* plan, const int3
     // Same kernels as mask_spmm_srbcrs; only where the partial tiles live differs.  Nothing in the
     // buffer has to start at zero: every partial tile the fix-up pass reads is written in full by
     // the main kernel of the same call.
-    return mask_spmm_srbcrs(plan, d_val_soff, d_val_sidx, d_val_block_val, M, K, N, d_B, ldb, d_C, ldc, scratch,
-                            kStaticScratchBytes, epilogue, stream);
+    (void)d_val_soff;
+    const mask_matrix m{kFmtSrbcrs, M, K, 0, d_val_sidx, nullptr, nullptr, d_val_block_val};
+    return spmm_arrays(plan, m, N, d_B, ldb, d_C, ldc, scratch, kStaticScratchBytes, epilogue, stream, most);
 }

@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kSweepThreads, 2) spmm_sweep_kernel(const Spmm
                 const int n_dst = slot < 0 ? 1 + p.n_peer_out : 1;
 #pragma unroll 1
                 for (int d = 0; d < n_dst; d++) {
-                    float* cb_ptr = slot >= 0 ? p.scratch + (int64_t)slot * kWinRows * p.N : (d == 0 ? p.C : p.peer_out[d - 1]);
+                    float* cb_ptr = slot >= 0 ? p.scratch + (int64_t)slot * kWinRows * p.N : (d == 0 ? p.C : p.peer_out[d - 1] + p.peer_col);
                     int row0 = w * kWinRows;
                     asm volatile("" : "+r"(row0));   // keeps the 16 row offsets from being hoisted out of this loop into registers
 #pragma unroll

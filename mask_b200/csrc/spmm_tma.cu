@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kTmaThreads, 2) spmm_tma_kernel(const SpmmArgs
                 for (int d = 0; d < n_dst; d++) {
                     int row0 = row00;
                     asm volatile("" : "+r"(row0));   // keeps the 16 row offsets from being hoisted out of this loop into registers
-                    float* dst = (slot >= 0 ? p.scratch + (int64_t)slot * kWinRows * p.N : (d == 0 ? p.C : p.peer_out[d - 1])) + col;
+                    float* dst = (slot >= 0 ? p.scratch + (int64_t)slot * kWinRows * p.N : (d == 0 ? p.C : p.peer_out[d - 1] + p.peer_col)) + col;
 #pragma unroll
                     for (int i = 0; i < 16; i++) {
                         const int r = i ^ (i >> 3);   // MMA-N index -> window row (SR-BCRS stores rows 8..15 swapped pairwise)

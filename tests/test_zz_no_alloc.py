@@ -128,3 +128,38 @@ def test_static_scratch_refuses_oversized_plans():
     assert b"built-in buffer" in L.mask_last_error()
     torch.cuda.synchronize()
     assert float(out.min()) == 7.0 and float(out.max()) == 7.0  # nothing was launched
+
+
+def test_static_scratch_of_default_plans_with_short_pieces(oracle_mod):
+    """A default plan may cut windows into pieces shorter than its groups.  What would fit if they were as long as the
+    groups is taken, in pieces of columns; peers' copies get every column; what would not fit is refused."""
+    import torch
+    from mask_b200 import _lib, engine, generators as G
+    L = _lib.lib()
+    m = G.rmat_gcn_normalised(scale=15, samples_per_node=16, seed=5)
+    p = engine.pack_srbcrs(*(torch.from_numpy(x).cuda() for x in (m.rowptr, m.colind, m.values)), m.M, m.K)
+    plan = engine.Plan(p.val_soff, m.M, p.T, "auto", 0)
+    tiles, group = np.diff(p.val_soff.cpu().numpy().astype(np.int64)), plan.info()["group_tiles"]
+    in_groups = int((-(-tiles // group))[tiles > group + group // 4].sum())
+    capacity = L.mask_static_scratch_capacity()
+    most = capacity // (64 * in_groups)
+    for N in (512, most // 4 * 4):
+        assert plan.scratch_bytes(N) > capacity >= 64 * in_groups * N
+        B = torch.randn(m.K, N, generator=torch.Generator(device="cuda").manual_seed(N), device="cuda")
+        want = engine.spmm(p, B, plan=plan)
+        peers = [torch.full((m.M, N), float("nan"), device="cuda") for _ in range(2)]
+        plan.set_peer_outputs(torch.tensor([t.data_ptr() for t in peers], dtype=torch.int64, device="cuda"))
+        out = torch.full((m.M, N), float("nan"), device="cuda")
+        _lib.check(_call_static(L, plan, p, B, out), "mask_spmm_srbcrs_static_scratch")
+        plan.set_peer_outputs(None)
+        absp = torch.sparse.mm(torch.sparse_csr_tensor(torch.from_numpy(m.rowptr).long(), torch.from_numpy(m.colind).long(),
+                                                       torch.from_numpy(np.abs(m.values)), size=(m.M, m.K)).cuda(), B.abs())
+        # both are within RTOL of the product: other pieces may take another kernel, which rounds B in another way
+        assert bool(((out - want).abs() <= 2 * RTOL * absp + ATOL).all())
+        for t in peers:
+            assert torch.equal(t, out)
+    N = most // 4 * 4 + 4
+    out = torch.full((m.M, N), 7.0, device="cuda")
+    assert _call_static(L, plan, p, torch.zeros((m.K, N), device="cuda"), out) == 4   # MASK_ERR_SCRATCH_TOO_SMALL
+    torch.cuda.synchronize()
+    assert float(out.min()) == 7.0 and float(out.max()) == 7.0
