@@ -2,8 +2,9 @@
  * mask_b200 -- C ABI of the B200 (sm_100a) SpMM engine for the SR-BCRS 16x8 and ME-TCF formats.
  *
  * C = A * B with A sparse FP32 packed into dense 16x8 tiles of window-condensed columns,
- * B dense FP32 row-major with N columns, TF32 tensor-core products (both operands rounded to
- * nearest, ties away, like cvt.rna.tf32.f32) and FP32 accumulation.
+ * B dense FP32 row-major with N columns, TF32 tensor-core products and FP32 accumulation.  The
+ * values of A are rounded to nearest, ties away, like cvt.rna.tf32.f32; those of B are rounded the
+ * same way or cut off to TF32, depending on the kernel: see the SpMM section.
  *
  * Conventions
  *   - every function returns a mask_status (0 = success); nothing throws or aborts;
@@ -271,8 +272,8 @@ int mask_peer_free(void* d_ptr);
  * 414-528).  Without this call a plan uses the widest block N fills.  Synchronises the stream.
  * mask_plan_column_features returns what was measured and chosen. */
 int mask_plan_autotune(mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t K, void* stream);
-/* mask_plan_create and mask_plan_autotune in one call: the device measures the columns while the host
- * builds the tables, and the stream is synchronised once less. */
+/* mask_plan_create and mask_plan_autotune in one call, the stream synchronised once less; the default
+ * policy's tables, too, are built from the column features on the device. */
 int mask_plan_create_tuned(const int32_t* d_val_soff, const int32_t* d_val_sidx, int32_t M, int32_t K, int64_t T,
                            int policy, int32_t group_tiles, void* stream, mask_plan** out);
 int mask_plan_column_features(const mask_plan* plan, mask_column_features* out, int32_t* nslab_wide);
@@ -301,6 +302,14 @@ int mask_plan_export(const mask_plan* plan, int32_t* frag_offset, int32_t* frag_
  * (examples/src_fp32/sr_bcrs/testbed/kernel.inc:1590-1700, kernel_lb.inc:62-381) and
  * dtc_spmm_kernel_fp32_val_idx_bind_stage2 (examples/src_fp32/dtc/testbed/kernel.inc:1982-2134).
  *
+ * Rounding of B.  The warp-level kernel rounds it to nearest, ties away; on the tcgen05 path the
+ * tensor core cuts it off (worst case per product 1.46e-3 of |a||b|, within the 2e-3 contract).
+ * Which one runs depends on the encoding, N, the plan's tile and group counts and its column
+ * features (mask_spmm_kernel_name tells), and a host-buffer session multiplies column chunks of a
+ * wider product with the kernel for the chunk's width.  So products of the same operands through
+ * another plan, another N or a session may differ in the fourth digit, each being within the
+ * contract; the same call gives the same bits.  MASK_NUMERICS_TF32X3 does not depend on it.
+ *
  * C[M,N] (leading dimension ldc) is fully overwritten -- no zero-fill by the caller and no
  * atomics: windows split across blocks are summed in tile order from per-fragment partial
  * tiles in d_scratch, so results are run-to-run deterministic.  B is [K,N] with leading
@@ -313,8 +322,8 @@ int mask_plan_export(const mask_plan* plan, int32_t* frag_offset, int32_t* frag_
 /* OR-able into `epilogue` (SR-BCRS only): three TF32 products per MMA -- hi(A)*hi(B) plus the
  * residual terms lo(A)*hi(B) and hi(A)*lo(B) -- which brings the result to FP32-level accuracy
  * (the reference compiler's compensated MMA, python/sparsene/op_gen/nvir/templates.py:53-76, on
- * by default in its Format-DSL bridge).  Runs on the warp-level kernel; 0.48 ms against 0.27 ms on
- * a 200 000-node power-law graph at N = 256. */
+ * by default in its Format-DSL bridge).  Runs on the warp-level kernel; 0.50 ms against 0.30 ms on
+ * a 200 000-node power-law graph at N = 256, 0.17 against 0.11 at N = 64. */
 #define MASK_NUMERICS_TF32X3 0x100
 
 int mask_spmm_srbcrs(const mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx,

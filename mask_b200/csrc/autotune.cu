@@ -4,9 +4,8 @@
 // featurizer (examples/src_fp32/dtc/testbed/featurize_mtx.cu:298-401: tiles per window, unique
 // columns, density, top-5 window share) and a catalogue of knobs (python/sparsene/op_gen/
 // strategy_agent.py:414-528: tile width, placement, stages); here they are a fixed rule over
-// measured features.  The window statistics (mask_features) come from val_soff, which the planner
-// has on the host anyway; what needs the device is the column side, from the 8 T entries of
-// val_sidx:
+// measured features.  The window statistics (mask_features) come from a host copy of val_soff; the
+// column side is measured on the device, from the 8 T entries of val_sidx:
 //   * band: how far the gathered rows of B lie from the diagonal position of their window (a stencil
 //     or banded matrix keeps them within a few thousand rows, so neighbouring windows share them and
 //     they stay in L2 whatever their width);

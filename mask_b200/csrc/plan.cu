@@ -1,4 +1,4 @@
-// Task planners (host) and the execution-plan handle.
+// Task planners and the execution-plan handle: the reference's mappings on the host, the default one on the device.
 #include "plan.h"
 
 #include <algorithm>

@@ -334,14 +334,21 @@ static int sweep_slabs(const mask_plan* plan, int N) {
 // through shared memory once to and once from, so it wins where full-width rows are gathered at the L2's or
 // shared memory's rate.  The warp kernel takes at most 128 columns at a time, has no minimum width, spreads small
 // matrices over up to 3256 blocks instead of 296, and re-reads (and rebuilds) the tiles for every block of columns.
-// Measured (us, tcgen05 / warp), SR-BCRS; power-law graphs of 20 000 / 300 000 / 2^20 / 2^22 nodes, stencils of
-// 27^3 / 100^3, uniform 700 / 4096 / 10^5 / 2 10^5 rows:
-//   N = 32     26 / 12,   -,         -,           -,               16 / 7,    -,           7.5 / 7.4,  9.1 / 9.3,  -,         -
-//   N = 128    28 / 23,   283 / 216, 1020 / 870,  -,               17 / 15,   586 / 517,   7.7 / 7.5,  9.6 / 11.6, 64 / 60,   132 / 136
-//   N = 192    32 / 28,   -,         1498 / 1362, -,               23 / 20,   880 / 929,   9.4 / 7.9,  12.0 / 12.9, 94 / 95,  206 / 209
-//   N = 256    32 / 33,   416 / 424, 1688 / 1681, -,               22 / 25,   945 / 1145,  9.4 / 8.2,  12.0 / 12.7, 108 / 116, 266 / 265
-//   N = 512    51 / 56,   798 / 813, 3363 / 3338, 28 500 / 26 900, 37 / 43,   1760 / 2050, 13.2 / 8.5, 17.2 / 19.1, 253 / 221, 599 / 512
-// ME-TCF and MCO, 20 000 nodes: N = 128 30 / 27, N = 256 33 / 39, N = 512 54 / 64; 4096 rows: 10 / 20, 13 / 21, 17 / 27.
+// It also rounds B where the tcgen05 kernel cuts it off: 2.1 to 3.0e-4 from the exact product (2-norm) against 4.2 to 4.7e-4.
+// Measured in turn (us, tcgen05 / warp), SR-BCRS; power-law graphs of 20 000 / 300 000 / 2^20 / 2^21 / 2^22 nodes:
+//   N = 32     27.8 / 13.0,  279 / 99,   975 / 293,   -,           -
+//   N = 128    29.9 / 24.8,  283 / 221,  1067 / 787,  -,           -
+//   N = 192    34.9 / 32.2,  415 / 336,  1615 / 1266, 3235 / 2784, 12 310 / 10 480
+//   N = 256    35.3 / 37.2,  426 / 420,  1761 / 1700, 3733 / 3642, 14 290 / 13 740
+//   N = 512    58.2 / 63.4,  839 / 843,  3403 / 3418, 7417 / 7350, 28 100 / 27 530
+// stencils of 27^3 / 100^3, uniform 700 / 4096 / 10^5 / 2 10^5 rows:
+//   N = 32     16.4 / 7.0,   556 / 186,    7.7 / 7.4,   9.0 / 9.2,    62.5 / 23.1,  121 / 45
+//   N = 128    16.9 / 14.5,  592 / 488,    8.0 / 7.5,   9.4 / 11.4,   64.7 / 53.4,  148 / 126
+//   N = 192    22.5 / 20.5,  958 / 796,    9.9 / 7.9,   11.8 / 12.7,  101 / 89,     224 / 197
+//   N = 256    22.1 / 24.2,  951 / 1037,   9.9 / 8.3,   11.7 / 12.7,  113 / 118,    278 / 257
+//   N = 512    36.5 / 42.3,  1701 / 2155,  14.2 / 8.7,  16.9 / 19.0,  260 / 230,    624 / 498
+// ME-TCF, 20 000 nodes: N = 128 31.8 / 29.7, N = 256 36.5 / 42.1, N = 512 63.2 / 70.4; 4096 rows: 10.2 / 18.9, 12.4 / 20.0,
+// 17.5 / 25.9.  MCO: 31.7 / 30.6, 36.8 / 45.8, 62.7 / 76.9; 10.4 / 16.2, 12.5 / 17.9, 17.6 / 25.2.
 static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, bool sidx_aligned) {
     if (tf32x3) return true;                    // compensated products: the warp kernel only
     if (!sidx_aligned || g_tune_sweep == 2) return false;
@@ -356,11 +363,20 @@ static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, 
     // rebuilds, a tcgen05 block an eighth.  With enough columns the warp kernel has more blocks to deal them to.
     if (plan->Gw < 4 * sm_count() && plan->T > (dense ? 24 : 16) * plan->Gw)
         return dense && (N > 128 ? plan->Gw * slabs <= (N > 256 ? 4 : 2) * sm_count() : N <= 64 && plan->Gw > 2 * sm_count());
-    if (N <= 128)   // a bitmap tile costs the warp kernel more to expand, and unaligned rows two passes a quarter-warp
-        return !(fmt == kFmtMco && N > 96 && N < 128 && !plan->hub_heavy && !plan->local);
+    // Bitmaps between 96 and 128 columns: the warp kernel pays for 128, for the expansion of every tile and for rows that
+    // do not start on whole lines (two passes a quarter-warp), and L2 serves either kernel if no column is hot.  N = 100 / 104 /
+    // 112 / 120 / 124, uniform 10^5 x 7 10^4: 72.3 / 76.2, 71.3 / 71.6, 71.5 / 70.5, 71.9 / 75.2, 75.7 / 85.1.  Not so up to 96 (N = 60
+    // 67.9 / 50.6, 92 70.3 / 67.8), at 128 (68.5 / 64.6), on a power-law graph of 300 000 nodes (330 / 317, 328 / 299, 328 / 294,
+    // 331 / 312, 340 / 350), a 60^3 stencil (150 / 149, 148 / 140, 148 / 138, 150 / 147, 156 / 170) and in SR-BCRS (64.5 / 58.8,
+    // N = 124 68.1 / 65.9).
+    if (N <= 128) return !(fmt == kFmtMco && N > 96 && N < 128 && !plan->hub_heavy && !plan->local);
     if (dense && work <= 150000 && (work <= 15000 || pads || (N <= 256 && !plan->local))) return true;   // too little work for long-lived blocks
     if (fmt == kFmtMco) return false;
-    if (plan->far_beyond_l2 && dense) return true;   // narrower rows of B: more of the hubs stay in L2
+    // Rows of B a quarter as wide: more of the hubs stay in L2 (2^22 nodes, N = 512: 141 GB through DRAM, the tcgen05 kernel
+    // 157).  24 turns each, quartiles of warp / tcgen05: N = 256 0.94-0.98 with 2^21 nodes, 0.94-0.95 with 3 10^6, 0.98-1.00 with
+    // 2^22; N = 512 0.98-1.00, 0.99-1.01, 1.01-1.02.  At full clocks the last is 24.8 / 26.7 ms; in a run of seconds the 1000 W limit
+    // brings the warp kernel to 1220 MHz and 28.4 ms, the tcgen05 kernel to 1430 MHz and 27.9.  Where it is a tie, the rounding of B decides.
+    if (plan->far_beyond_l2 && dense) return true;
     if (plan->slab_fits && N > 256) return true;
     return !plan->local && pads;
 }

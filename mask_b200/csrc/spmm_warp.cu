@@ -6,9 +6,11 @@
 // hands the next group to whichever SM has a free slot.  S = 3 ring slots of 4.5 KB leave room for 15 blocks per
 // SM, which also hide each other's dependent chains.  (Four-warp blocks, in which two warps of a block idled at
 // N = 64 and the blocks finished together, took 1.87 ms on a 2^21-node power-law graph at N = 64, now 1.28 ms; the
-// tcgen05 kernel took 0.32 ms at N = 128 on a 300 000-node graph in ME-TCF, here 0.24 ms.  At full width the
-// tcgen05 kernel moves fewer bytes per product and is the better one: see use_warp_kernel.)
-// 27-point stencil, N = 128: 16.7 TB/s from L2, 85 % of the gather alone.
+// tcgen05 kernel took 0.32 ms at N = 128 on a 300 000-node graph in ME-TCF, here 0.25 ms.  At full width the
+// tcgen05 kernel reads the tiles once instead of four times and is the better one where L2 serves the gathers: see
+// use_warp_kernel.)  27-point stencil, N = 128: 16.7 TB/s from L2, 85 % of the gather alone.  Power-law graph of 2^18 nodes,
+// N = 512 (profiled): 12.8 TB/s, 60 % of the sectors from L2, no unit above 60 % -- L1 58, issue slots 55, L2 54, DRAM 49,
+// tensor pipe 35: the latency of the gathers with 15 warps an SM, two steps each in flight.
 //
 // Each ring slot holds one step: KT tiles, for each the 8 gathered rows of B (32*NQ columns) and the tile
 // operand or what it is rebuilt from.  Gathered-row ids (and the value runs of the compact encodings) go
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
 // Tiles per step: one (two at 32 columns) where many blocks are resident, up to four times as many where few are.
 static constexpr int warp_step_tiles(int nq, int depth) { return (nq == 1 ? 2 : 1) << depth; }
 // Blocks per SM: as many as shared memory holds, except where the registers of the compensated products need
-// more room (N = 256, 200 000-node power-law graph: 12 blocks of 165 registers 475 us, 15 of 128 490 us).
+// more room (N = 256, 200 000-node power-law graph: 12 blocks of 165 registers 500 us, 14 blocks 508, 15 of 128 562).
 static constexpr int warp_blocks_per_sm(int nq, int depth, bool comp) {
     constexpr int blocks[4][3] = {{22, 12, 6}, {24, 13, 7}, {18, 10, 5}, {15, 8, 4}};
     constexpr int comp_blocks[4] = {22, 16, 14, 12};
