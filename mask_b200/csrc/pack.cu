@@ -83,10 +83,6 @@ constexpr int kHubThreads = 1024;
 constexpr int kBigBits = 1 << 19;                 // columns marked at a time: two blocks per SM
 constexpr int kHubBlocks = 8;
 constexpr int kHubBits = kMarkMax;                // most columns marked at a time by one block of a cluster
-constexpr int kBitmapBits = 1 << 20;              // columns a block marks at a time
-constexpr int kBitmapWords = kBitmapBits / 32;
-constexpr int kBitmapRuns = kBitmapWords / 128;
-constexpr int kBitmapSmem = kBitmapWords * 4 + kBitmapWords * 2;
 
 // One window of n <= 32 E entries: sorts (column, entry), numbers the distinct columns, writes every entry's
 // number to pos and the distinct columns to cols; returns how many there are.

@@ -15,9 +15,9 @@
 //                   (atomicMin), the children of a parent follow each other in (degree, id) order, and all
 //                   connected components advance together; components are then laid out by the rank of
 //                   their start node (the unvisited node of least (degree, id)) and each is reversed.
-//                   The traversal is one cooperative launch; a level costs about 10 us, which for meshes
-//                   and other graphs with tens to hundreds of levels is most of the time (64 000-node shuffled
-//                   27-point mesh, 40 levels: 0.44 of 0.8 ms; a launch
+//                   The traversal is one cooperative launch; a level costs about 9 us, which for meshes
+//                   and other graphs with tens to hundreds of levels is much of the time (64 000-node shuffled
+//                   27-point mesh, 41 levels: 0.38 of 0.93 ms with packing and plan; a launch
 //                   sequence with three radix sorts and a host read per level took 13 ms).
 // Applying an order -- gathering the rows of a device CSR matrix -- and undoing it are device work
 // too: the SpMM kernels take the order as a row map and write output row order[new_row] directly,

@@ -49,7 +49,6 @@ class Plan:
         self._address = h.value or 0
         self.policy = policy
         self.M, self.T = M, T
-        self._scratch = {}
         self._row_order = None
 
     def __del__(self):
@@ -101,18 +100,6 @@ class Plan:
         go = torch.zeros(i["groups"] + 1, dtype=torch.int32)
         check(lib().mask_plan_export(self._h, _ptr(fo), _ptr(fw), _ptr(go)), "mask_plan_export")
         return fo, fw[: i["fragments"]], go
-
-    def scratch(self, N: int, device) -> torch.Tensor | None:
-        """Partial-tile buffer for the current stream: products on different streams may overlap on
-        the GPU, so each stream gets its own buffer (products on one stream run in order and share it)."""
-        need = self.scratch_bytes(N)
-        if need == 0:
-            return None
-        key = (torch.cuda.current_stream().cuda_stream, device)
-        buf = self._scratch.get(key)
-        if buf is None or buf.numel() < need:
-            buf = self._scratch[key] = torch.empty(need, dtype=torch.uint8, device=device)
-        return buf
 
 
 @dataclass
