@@ -220,7 +220,7 @@ __global__ void row_lengths_kernel(const int32_t* __restrict__ ptr, int32_t M, i
 }
 
 // Takes diagonal and out-of-range entries off the degrees; *asymmetric is set if some other entry (r, c) has no
-// counterpart (c, r).
+// counterpart (c, r), or if a row is not strictly ascending: an entry listed twice would be queued twice.
 __global__ void __launch_bounds__(256) check_symmetry_kernel(const int32_t* __restrict__ ptr, const int32_t* __restrict__ col, int32_t M,
                                                              int64_t nnz, int32_t* __restrict__ deg, int32_t* __restrict__ asymmetric) {
     __shared__ int range[2];
@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(256) check_symmetry_kernel(const int32_t* __re
     const int r = row_of_entry(ptr, M, first, last, e < nnz ? e : last, range);
     if (e >= nnz) return;
     const int c = col[e];
+    if (e > ptr[r] && __ldg(col + e - 1) >= c) *asymmetric = 1;
     if (c < 0 || c >= M || c == r) {
         atomicSub(&deg[r], 1);
         return;

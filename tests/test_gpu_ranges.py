@@ -497,3 +497,21 @@ def test_overlapped_launches_keep_their_order(sweep, N, gt, scale):
             assert torch.equal(last, w)
     finally:
         engine.tune("sweep", 1)
+
+
+@pytest.mark.parametrize("name", ["path", "stars", "components", "many_edges"])
+@pytest.mark.parametrize("how", ["twice", "some_twice", "unsorted"])
+def test_rcm_of_rows_that_are_not_strictly_ascending(oracle_mod, name, how):
+    """Symmetric patterns with entries listed more than once, or out of order: the order is that of the pattern."""
+    from mask_b200 import engine
+    m = GRAPHS[name]()
+    rng = np.random.Generator(np.random.PCG64(3))
+    rows = [m.colind[m.rowptr[i]:m.rowptr[i + 1]] for i in range(m.M)]
+    if how == "unsorted":
+        rows = [rng.permutation(r) for r in rows]
+    else:
+        rows = [np.sort(np.concatenate([r, r if how == "twice" else r[rng.random(len(r)) < 0.1]])) for r in rows]
+    again = _rows_to_csr(rows, m.K, 1)
+    rp, ci, _ = _dev(again)
+    got = engine.reorder_rows(rp, ci, m.M, m.K, "row_rcm").cpu().numpy()
+    assert np.array_equal(got, oracle_mod.reorder_rows("row_rcm", m.M, m.K, m.rowptr, m.colind))
