@@ -444,6 +444,7 @@ struct FillArgs {
     int32_t skip_zero;         // MCO: entries with value 0 are not stored
     int32_t* sidx;
     float* block_val;          // SR-BCRS
+    int32_t whole_vectors;     // block_val is 16-byte aligned
     int32_t* edge_to_col;
     int32_t* edge_to_row;
     unsigned long long* tile_rows;   // ME-TCF: entries per row of a tile, 16 nibbles
@@ -658,7 +659,13 @@ __global__ void __launch_bounds__(kFillThreads, 10) fill_kernel(const FillArgs p
                 for (int i = 0; i < kSub; i++) {
                     if (i >= nt) break;
                     float4* from = reinterpret_cast<float4*>(tile) + i * 32 + lane;
-                    out[i * 32 + lane] = *from;
+                    const float4 v = *from;
+                    if (p.whole_vectors) {
+                        out[i * 32 + lane] = v;
+                    } else {
+                        float* at = p.block_val + (c + i) * kTileElems + 4 * lane;
+                        at[0] = v.x; at[1] = v.y; at[2] = v.z; at[3] = v.w;
+                    }
                     *from = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
             } else if (MODE == kCountMetcf) {
@@ -838,6 +845,7 @@ extern "C" int mask_srbcrs_fill(const int32_t* d_rowptr, const int32_t* d_colind
         FillArgs a = fill_args(s, M, d_values, d_val_soff, T);
         a.sidx = d_val_sidx;
         a.block_val = d_val_block_val;
+        a.whole_vectors = (reinterpret_cast<uintptr_t>(d_val_block_val) & 15) == 0;
         a.edge_to_col = d_edge_to_col;
         a.edge_to_row = d_edge_to_row;
         int rc = launch_fill<kFillSrbcrs>(a, st);

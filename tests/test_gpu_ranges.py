@@ -515,3 +515,22 @@ def test_rcm_of_rows_that_are_not_strictly_ascending(oracle_mod, name, how):
     rp, ci, _ = _dev(again)
     got = engine.reorder_rows(rp, ci, m.M, m.K, "row_rcm").cpu().numpy()
     assert np.array_equal(got, oracle_mod.reorder_rows("row_rcm", m.M, m.K, m.rowptr, m.colind))
+
+
+@pytest.mark.parametrize("by", [4, 8, 12])
+def test_pack_writes_tile_values_at_any_alignment(oracle_mod, by):
+    import torch
+    from mask_b200 import _lib, engine
+    from mask_b200.engine import _analyze, _ptr, _stream
+    m = _mixed_matrix()
+    rp, ci, va = _dev(m)
+    ws, soff, T, nnz = _analyze(rp, ci, m.M, m.K)
+    sidx = torch.empty(8 * T, dtype=torch.int32, device="cuda")
+    room = torch.full((128 * T + 8,), 7.0, device="cuda")
+    val = room[by // 4:by // 4 + 128 * T]
+    _lib.check(_lib.lib().mask_srbcrs_fill(_ptr(rp), _ptr(ci), _ptr(va), m.M, nnz, _ptr(ws), _ptr(soff), T, _ptr(sidx), _ptr(val), None, None, None,
+                                           _stream()), "mask_srbcrs_fill")
+    want = oracle_mod.pack_srbcrs(m.M, m.rowptr, m.colind, m.values)
+    assert np.array_equal(val.cpu().numpy().view(np.int32), want["val_block_val"].view(np.int32))
+    assert np.array_equal(sidx.cpu().numpy(), want["val_sidx"])
+    assert bool((room[:by // 4] == 7).all()) and bool((room[by // 4 + 128 * T:] == 7).all())
