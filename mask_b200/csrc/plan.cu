@@ -69,7 +69,7 @@ static void multi_bind(const int32_t* soff, int32_t W, std::vector<int32_t>& tas
 // with fewer than 128 tiles for every resident warp the pieces get shorter, so that all of them have work and
 // no long chain of tiles is left at the end.  Not below kMinPiece, where filling a block's pipeline costs more
 // than the balance gains, and not below the mean window: cutting every window adds a partial tile and a fix-up
-// for each (uniform 4096-node matrix, 42 tiles a window, N = 512: 23 us whole, 29 us in three pieces).
+// for each (uniform 4096-node matrix, 42 tiles a window, N = 512: 16.9 us whole, 23.8 us in three pieces).
 // With very many tiles the pieces get longer again: the partial tiles are then what counts (2^22-node power-law
 // graph, 15 M tiles, N = 512: pieces of 128 tiles write and read 5.6 GB of them, pieces of 512 0.6 GB).
 constexpr int32_t kMinPiece = 16;
