@@ -83,11 +83,11 @@ def test_srbcrs_spmm_policies(oracle_mod, name, policy, gt):
 @pytest.mark.parametrize("use_async,nq,knob", [(0, 1, 0), (0, 2, 0), (0, 2, 4), (0, 4, 0), (0, 4, 3),
                                                 (1, 1, 0), (1, 1, 4), (1, 2, 0), (1, 2, 3), (1, 2, 45), (1, 2, 5),
                                                 (1, 2, 6), (1, 2, 8), (1, 4, 0), (1, 4, 3), (1, 4, 43), (1, 4, 5),
-                                                (1, 4, 6), (1, 4, 8)])
+                                                (1, 4, 6), (1, 4, 8), (1, 3, 0)])
 @pytest.mark.parametrize("name,N", [("rmat12u", 512), ("hub_rows", 200), ("m33_empty_window", 64)])
 def test_srbcrs_spmm_kernel_variants(oracle_mod, name, N, use_async, nq, knob):
-    """Register-pipelined kernel (knob = occupancy target) and shared-memory ring kernel
-    (knob = ring slots per warp), every column-slab width."""
+    """Register-pipelined kernel (knob = occupancy target) and one-warp ring kernel (knob = "stages", accepted
+    without effect), every number of 32-column groups a warp takes."""
     import torch
     from mask_b200 import engine
     m = cases.SMALL[name]()
@@ -128,21 +128,26 @@ def test_metcf_spmm_matches_oracle(oracle_mod, name, N):
     out2 = engine.spmm(p, torch.from_numpy(B).cuda(), plan=plan2)
     _assert_close(oracle_mod, m, B, out2.cpu().numpy())
     assert plan2.status() == 0
-    try:  # and the mma.sync ME-TCF kernel
-        engine.tune("sweep", 0)
-        out3 = engine.spmm(p, torch.from_numpy(B).cuda(), plan=plan2)
-    finally:
-        engine.tune("sweep", 1)
-    _assert_close(oracle_mod, m, B, out3.cpu().numpy())
+    # and every kernel: tcgen05, one-warp ring, register-pipelined
+    for sweep, use_async in ((2, 1), (0, 1), (0, 0)):
+        try:
+            engine.tune("sweep", sweep)
+            engine.tune("async", use_async)
+            out3 = engine.spmm(p, torch.from_numpy(B).cuda(), plan=plan2)
+        finally:
+            engine.tune("sweep", 1)
+            engine.tune("async", 1)
+        _assert_close(oracle_mod, m, B, out3.cpu().numpy())
+    assert plan2.status() == 0
 
 
 @pytest.mark.parametrize("name", ["m1", "m17", "m33_empty_window", "hub_rows", "rmat10", "stencil8", "all_empty",
                                   "one_tile_windows", "uniform512"])
 @pytest.mark.parametrize("N", [40, 128, 256, 512])
 def test_mco_spmm_matches_oracle(oracle_mod, name, N):
-    """MCO / BIT-TCF (bitmap leaf): tcgen05 kernel in its slab variants, the register-pipelined
-    kernel, split windows, ReLU; and exactly the product the oracle
-    computes from the same arrays with both operands rounded."""
+    """MCO / BIT-TCF (bitmap leaf): tcgen05 kernel in its slab variants, the one-warp ring and the register-pipelined
+    kernel, split windows, ReLU; and, where B is rounded, the product the oracle computes from the same arrays with
+    both operands rounded, up to the rounding of the sums."""
     import torch
     from mask_b200 import engine
     m = cases.SMALL[name]()
@@ -159,18 +164,28 @@ def test_mco_spmm_matches_oracle(oracle_mod, name, N):
     assert plan2.status() == 0
     outs = []
     try:
-        for sweep, nslab in ((0, 0), (2, 1), (2, 2)):   # warp-level kernels; tcgen05 with 1 and 2 slabs
+        for sweep, nslab, use_async in ((0, 0, 1), (0, 0, 0), (2, 1, 1), (2, 2, 1)):   # warp-level kernels; tcgen05 with 1 and 2 slabs
             engine.tune("sweep", sweep)
             engine.tune("nslab", nslab)
+            engine.tune("async", use_async)
             o = torch.full((m.M, N), float("nan"), device="cuda")
             engine.spmm(p, Bd, out=o, plan=plan2)
             outs.append(o)
     finally:
         engine.tune("sweep", 1)
         engine.tune("nslab", 0)
+        engine.tune("async", 1)
     for o in outs:
         _assert_close(oracle_mod, m, B, o.cpu().numpy())
     assert plan2.status() == 0
+    # products of TF32 numbers are exact in FP32; n of them are summed with at most n roundings on each side, cut off
+    # (2^-23 of what is summed so far) where the tensor core adds
+    rounded = oracle_mod.spmm_from_mco(m.M, oracle_mod.pack_mco(m.M, m.rowptr, m.colind, m.values), B, round_tf32=True)
+    absp = oracle_mod.spmm_abs_f64(m.M, m.rowptr, m.colind, m.values, B)
+    n = int(np.diff(m.rowptr).max())
+    for o in outs[:2]:
+        bad, worst = oracle_mod.check_tolerance(o.cpu().numpy(), rounded, absp, max(n, 1) * 2.0**-22, 1e-30)
+        assert bad == 0, worst
 
 
 def test_relu_epilogue(oracle_mod):
@@ -279,9 +294,9 @@ def test_medium_rmat_against_oracle(oracle_mod):
 
 @pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
 def test_long_persistent_runs_every_encoding(oracle_mod, fmt):
-    """A 2^18-node power-law graph: every resident block walks its rings some two thousand times per
-    launch, for the 6-stage ring of SR-BCRS and the 5-stage ring of the compact encodings, at one and
-    two slabs per sweep, several launches each.  Hand-over faults that need many ring revolutions to
+    """A 2^18-node power-law graph: every resident block of the tcgen05 kernel walks its rings some two thousand
+    times per launch, for the 6-stage ring of SR-BCRS and the 5-stage ring of the compact encodings, at one
+    slab per sweep and more, several launches each.  Hand-over faults that need many ring revolutions to
     show (a waiter that misses a barrier phase) end in a bounded wait giving up, so the plan's status
     word is checked beside the sampled rows."""
     import torch
@@ -300,7 +315,12 @@ def test_long_persistent_runs_every_encoding(oracle_mod, fmt):
         out = torch.empty((m.M, N), device="cuda")
         for _ in range(4):
             out.fill_(float("nan"))
-            engine.spmm(p, Bd, out=out, plan=plan)
+            engine.tune("sweep", 2)
+            try:
+                assert engine.kernel_signature(p, N, plan)[0].startswith("spmm_sweep_kernel")
+                engine.spmm(p, Bd, out=out, plan=plan)
+            finally:
+                engine.tune("sweep", 1)
             assert plan.status() == 0
             bad, worst = oracle_mod.check_tolerance(out[rows_d].cpu().numpy(), ref, absp, RTOL, ATOL)
             assert bad == 0, (N, worst)
@@ -364,15 +384,16 @@ def test_srbcrs_spmm_tcgen05_kernel(oracle_mod, name, N, gt, nslab):
 
 
 @pytest.mark.parametrize("name,N,gt,umma,fmt,reorder", [
-    ("rmat12u", 64, 0, 1, "srbcrs", "none"),       # narrow N: cp.async ring kernel (warp-level MMA)
+    ("rmat12u", 64, 0, 1, "srbcrs", "none"),       # warp kernel
     ("hub_rows", 64, 3, 1, "srbcrs", "none"),      # split windows: fix-up kernel writes the rows
-    ("rmat12u", 512, 0, 1, "srbcrs", "none"),      # tcgen05 kernel, 4 slabs
-    ("hub_rows", 128, 3, 1, "srbcrs", "none"),     # tcgen05 kernel + fix-up
-    ("hub_rows", 64, 3, 2, "srbcrs", "none"),      # tcgen05 kernel forced at narrow N
+    ("rmat12u", 512, 0, 2, "srbcrs", "none"),      # tcgen05 kernel, 4 slabs
+    ("hub_rows", 128, 3, 2, "srbcrs", "none"),     # tcgen05 kernel + fix-up
+    ("hub_rows", 64, 3, 2, "srbcrs", "none"),      # tcgen05 kernel at narrow N
     ("m17", 40, 0, 0, "metcf", "none"),            # register kernel, ragged last window
-    ("m17", 40, 0, 1, "metcf", "none"),            # tcgen05 kernel, ME-TCF
+    ("m17", 40, 0, 1, "metcf", "none"),            # ME-TCF as the library routes it
+    ("m17", 40, 0, 2, "metcf", "none"),            # tcgen05 kernel, ME-TCF
     ("rmat10", 64, 0, 1, "srbcrs", "row_rcm"),     # rows scattered back through the row map
-    ("rmat10", 256, 0, 1, "srbcrs", "row_rcm"),    # the same through the tcgen05 epilogue
+    ("rmat10", 256, 0, 2, "srbcrs", "row_rcm"),    # the same through the tcgen05 epilogue
 ])
 def test_peer_outputs_receive_the_same_rows(oracle_mod, name, N, gt, umma, fmt, reorder):
     """mask_plan_set_peer_outputs: every extra output base gets exactly the rows C gets (here the
@@ -394,6 +415,9 @@ def test_peer_outputs_receive_the_same_rows(oracle_mod, name, N, gt, umma, fmt, 
     ptrs = torch.tensor([t.data_ptr() for t in peers], dtype=torch.int64, device="cuda")
     try:
         engine.tune("sweep", umma)
+        engine.tune("async", 0 if umma == 0 else 1)
+        kernel = engine.kernel_signature(p, N, plan)[0]
+        assert {0: "legacy routing", 1: "spmm_warp_kernel", 2: "spmm_sweep_kernel"}[umma] in kernel, kernel
         plan.set_peer_outputs(ptrs)
         engine.spmm(p, Bd, out=out, plan=plan, relu=True)
         plan.set_peer_outputs(None)
@@ -401,6 +425,7 @@ def test_peer_outputs_receive_the_same_rows(oracle_mod, name, N, gt, umma, fmt, 
         engine.spmm(p, Bd, out=plain, plan=plan, relu=True)
     finally:
         engine.tune("sweep", 1)
+        engine.tune("async", 1)
     assert plan.status() == 0
     assert torch.equal(out, plain)
     for t in peers:
@@ -453,7 +478,12 @@ def test_truncated_operand_worst_case(oracle_mod, N):
     B = np.abs(_dense(m.K, N, 47)) + np.float32(0.25)
     B = (B.view(np.uint32) | np.uint32(0x1FFF)).view(np.float32)
     plan = p.plan("auto")
-    out = engine.spmm(p, torch.from_numpy(B).cuda(), plan=plan).cpu().numpy()
+    engine.tune("sweep", 2)
+    try:
+        assert engine.kernel_signature(p, N, plan)[0].startswith("spmm_sweep_kernel")
+        out = engine.spmm(p, torch.from_numpy(B).cuda(), plan=plan).cpu().numpy()
+    finally:
+        engine.tune("sweep", 1)
     assert plan.status() == 0
     worst = _assert_close(oracle_mod, m, B, out)
     assert worst < 0.80, worst                            # 1.46e-3 / 2e-3 = 0.73 is the analytical ceiling
@@ -462,8 +492,9 @@ def test_truncated_operand_worst_case(oracle_mod, N):
     assert float(gate.max()) < 1.0, float(gate.max())     # the reference testbed's cuSPARSE gate
 
 
-def test_product_with_more_than_2_31_elements(oracle_mod):
-    """M * N = 2^31: output offsets need 64 bits.  A thin random matrix with 2^22 rows at N = 512;
+@pytest.mark.parametrize("sweep", [0, 2])
+def test_product_with_more_than_2_31_elements(oracle_mod, sweep):
+    """M * N = 2^31: output offsets need 64 bits, in both main kernels.  A thin random matrix with 2^22 rows at N = 512;
     sampled rows from the whole range, including the last windows, against the CPU oracle."""
     import torch
     from mask_b200 import engine, generators as G
@@ -483,7 +514,11 @@ def test_product_with_more_than_2_31_elements(oracle_mod):
     out = torch.full((M, N), float("nan"), device="cuda")
     assert out.numel() == 1 << 31
     plan = p.plan("auto")
-    engine.spmm(p, Bd, out=out, plan=plan)
+    engine.tune("sweep", sweep)
+    try:
+        engine.spmm(p, Bd, out=out, plan=plan)
+    finally:
+        engine.tune("sweep", 1)
     assert plan.status() == 0
     rows = np.unique(np.concatenate([rng.integers(0, M, size=4096), np.arange(M - 64, M), np.arange(0, 32),
                                      np.arange((1 << 21) - 32, (1 << 21) + 32)]))   # around offset 2^30 elements = 2^32 bytes
