@@ -398,7 +398,7 @@ static int launch_spmm(const mask_plan* plan, SpmmArgs a, cudaStream_t st) {
     if (plan->G == 0) return MASK_OK;
     // the register-pipelined kernel writes C 16 bytes at a time: rows that are not whole vectors go to the tcgen05 kernel
     const bool registers = g_tune_sweep == 0 && g_tune_async == 0 && !a.tf32x3 && a.vec_out;
-    if (!registers) {
+    if (!registers && plan->T > 0) {
         const int bad = check_packed_alignment(a);
         if (bad != MASK_OK) return bad;
     }

@@ -595,6 +595,17 @@ def test_packed_arrays_off_their_alignment(oracle_mod, fmt):
         assert call(_lib.NUMERICS_TF32X3)[0] == 0
     else:
         assert call(offsets=8)[0] == 0
+    # without tiles nothing is read
+    m, p = cases.SMALL["all_empty"](), None
+    p = {"srbcrs": engine.pack_srbcrs, "metcf": engine.pack_metcf, "mco": engine.pack_mco}[fmt](*_dev(m), m.M, m.K)
+    plan, sidx = p.new_plan(), torch.empty(4, dtype=torch.int32, device="cuda")
+    code, offsets, index, values = p._arrays()
+    index, values = torch.empty(8, dtype=torch.int64, device="cuda"), torch.empty(8, device="cuda")
+    p.val_sidx = sidx
+    B = _dense(m.K, N, 3)
+    Bd = torch.from_numpy(B).cuda()
+    rc, out = call(sidx=4, **({} if fmt == "mco" else dict(values=4)))
+    assert rc == 0 and bool((out == 0).all())
 
 
 @pytest.mark.parametrize("N,tf32x3,gt", [(65_535 * 128 + 132, True, 0), (4_194_304 + 36, False, 1), (2 * (1 << 21) + 3, False, 1)])
