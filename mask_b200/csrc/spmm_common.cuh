@@ -85,71 +85,60 @@ __device__ __forceinline__ float detach(float x) {
     return y;
 }
 
-// Writes (and clears) a warp's accumulators for fragment ff: straight to C when the fragment is
-// its whole window, else to the fragment's partial tile in scratch.  acc[q][j][i]: 32-column
-// group q, MMA j (column cb + 4n + j), accumulator register i.
-template <int NQ>
-__device__ __forceinline__ void flush_fragment(const SpmmArgs& p, int ff, int col_base, int g, int k,
-                                               float (&acc)[NQ][4][4]) {
-    const int w = p.frag_win[ff];
-    const int slot = p.frag_slot[ff];
-    float* dst;
-    int64_t ld;
-    int rows_ok;
-    if (slot < 0) {
-        dst = p.C + (int64_t)w * kWinRows * p.ldc;
-        ld = p.ldc;
-        rows_ok = p.M - w * kWinRows;
-    } else {
-        dst = p.scratch + (int64_t)slot * kWinRows * p.N;
-        ld = p.N;
-        rows_ok = kWinRows;
-    }
-    const bool relu = p.relu && slot < 0;
+// Writes (and clears) a warp's accumulators for a fragment of window `win`: straight to C when the fragment is
+// its whole window (part < 0), else to partial tile `part` in scratch.  acc[q][j][i]: 32-column group q, MMA j
+// (column cb + 4n + j), accumulator register i.  GUARD: there may be fewer than 32 NQ columns.
+template <int NQ, bool GUARD>
+__device__ __forceinline__ void write_fragment(const SpmmArgs& p, int win, int part, int col_base, int g, int k, float (&acc)[NQ][4][4]) {
+    const bool whole = part < 0;
+    const int64_t ld = whole ? p.ldc : p.N;
+    const int row = win * kWinRows + g, rows_ok = whole ? p.M - win * kWinRows : kWinRows;
+    const bool relu = p.relu && whole;
+    const bool plain = !whole || (p.vec_out && p.n_peer_out == 0);
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
-        const int c0 = col_base + 32 * q + 8 * k;
+    for (int h = 0; h < 2; h++) {
+        const bool in = g + 8 * h < rows_ok;
+        float* at = whole ? p.C + (int64_t)(p.row_map && in ? p.row_map[row + 8 * h] : row + 8 * h) * ld
+                          : p.scratch + ((int64_t)part * kWinRows + g + 8 * h) * ld;
+        at += col_base + 8 * k;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int r = g + 8 * h;
+        for (int q = 0; q < NQ; q++) {
             // A 128-bit store needs its four values in consecutive registers, and so does every
             // MMA accumulator quad -- with a different grouping.  detach() gives the store its own
             // registers, so the unavoidable moves happen here, once per fragment, instead of around
             // every MMA of the main loop.
-            float4 v0 = make_float4(detach(acc[q][0][2 * h]), detach(acc[q][1][2 * h]), detach(acc[q][2][2 * h]),
-                                    detach(acc[q][3][2 * h]));
-            float4 v1 = make_float4(detach(acc[q][0][2 * h + 1]), detach(acc[q][1][2 * h + 1]),
-                                    detach(acc[q][2][2 * h + 1]), detach(acc[q][3][2 * h + 1]));
+            float4 v0 = make_float4(detach(acc[q][0][2 * h]), detach(acc[q][1][2 * h]), detach(acc[q][2][2 * h]), detach(acc[q][3][2 * h]));
+            float4 v1 = make_float4(detach(acc[q][0][2 * h + 1]), detach(acc[q][1][2 * h + 1]), detach(acc[q][2][2 * h + 1]),
+                                    detach(acc[q][3][2 * h + 1]));
             if (relu) {
                 v0.x = fmaxf(v0.x, 0.f); v0.y = fmaxf(v0.y, 0.f); v0.z = fmaxf(v0.z, 0.f); v0.w = fmaxf(v0.w, 0.f);
                 v1.x = fmaxf(v1.x, 0.f); v1.y = fmaxf(v1.y, 0.f); v1.z = fmaxf(v1.z, 0.f); v1.w = fmaxf(v1.w, 0.f);
             }
-            if (r < rows_ok) {
-                float* row = (slot < 0 && p.row_map) ? p.C + (int64_t)p.row_map[w * kWinRows + r] * p.ldc : dst + (int64_t)r * ld;
-                if (slot < 0 && !p.vec_out) {   // C with an odd row length (never together with peers' copies)
-                    const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+            const int left = p.N - (col_base + 8 * k + 32 * q);   // columns from here on
+            if (plain) {
+                if (in && (!GUARD || left > 0)) *reinterpret_cast<float4*>(at + 32 * q) = v0;
+                if (in && (!GUARD || left > 4)) *reinterpret_cast<float4*>(at + 32 * q + 4) = v1;
+            } else if (in && !p.vec_out) {   // C with an odd row length (never together with peers' copies)
+                const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        if (c0 + i < p.n_out) row[c0 + i] = v[i];
-                    continue;
-                }
-                if (c0 < p.N) *reinterpret_cast<float4*>(row + c0) = v0;
-                if (c0 + 4 < p.N) *reinterpret_cast<float4*>(row + c0 + 4) = v1;
-                if (slot < 0) {  // the same row into every peer's copy of C (plain stores over NVLink)
-                    const int64_t off = row - p.C;
-                    for (int j = 0; j < p.n_peer_out; j++) {
-                        float* prow = p.peer_out[j] + p.peer_col + off;
-                        if (c0 < p.N) *reinterpret_cast<float4*>(prow + c0) = v0;
-                        if (c0 + 4 < p.N) *reinterpret_cast<float4*>(prow + c0 + 4) = v1;
-                    }
+                for (int i = 0; i < 8; i++)
+                    if (left + p.n_out - p.N > i) at[32 * q + i] = v[i];
+            } else if (in) {   // the same row into every peer's copy of C (plain stores over NVLink)
+                const int64_t off = at + 32 * q - p.C;
+                for (int j = -1; j < p.n_peer_out; j++) {
+                    float* to = (j < 0 ? p.C : p.peer_out[j] + p.peer_col) + off;
+                    if (left > 0) *reinterpret_cast<float4*>(to) = v0;
+                    if (left > 4) *reinterpret_cast<float4*>(to + 4) = v1;
                 }
             }
         }
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; q++)
 #pragma unroll
         for (int j = 0; j < 4; j++)
 #pragma unroll
             for (int i = 0; i < 4; i++) acc[q][j][i] = 0.f;
-    }
 }
 
 // spmm_mma.cu: the array entry points, in pieces of at most `most` columns.  Scratch for one piece.

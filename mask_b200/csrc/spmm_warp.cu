@@ -4,18 +4,21 @@
 // 19.5 TB/s over the GPU out of L2 and 7 TB/s out of DRAM, most of it with many warps and shallow rings.  So the
 // block is a single warp: no barrier, no idle partner when N does not fill four warps' columns, and the hardware
 // hands the next group to whichever SM has a free slot.  S = 3 ring slots of 4.5 KB leave room for 15 blocks per
-// SM, which also hide each other's dependent chains.  (Four-warp blocks, in which two warps of a block idled at
-// N = 64 and the blocks finished together, took 1.87 ms on a 2^21-node power-law graph at N = 64, now 1.28 ms; the
-// tcgen05 kernel took 0.32 ms at N = 128 on a 300 000-node graph in ME-TCF, here 0.25 ms.  At full width the
-// tcgen05 kernel reads the tiles once instead of four times and is the better one where L2 serves the gathers: see
-// use_warp_kernel.)  27-point stencil, N = 128: 16.7 TB/s from L2, 85 % of the gather alone.  Power-law graph of 2^18 nodes,
-// N = 512 (profiled): 12.8 TB/s, 60 % of the sectors from L2, no unit above 60 % -- L1 58, issue slots 55, L2 54, DRAM 49,
-// tensor pipe 35: the latency of the gathers with 15 warps an SM, two steps each in flight.
+// SM, which also hide each other's dependent chains.  At full width the tcgen05 kernel reads the tiles once instead
+// of four times: see use_warp_kernel.  27-point stencil of 60^3 nodes, N = 256 (profiled): 54 bytes per cycle and SM of the 69
+// of the bare gather, shared memory 61 %, tensor pipe 38 %, issue slots 38 %.
+//
+// The rest is the chain of one warp: 15 warps an SM do not hide it all.  With every gather taken out the loop still took
+// 78 % of its time when it spent 205 instructions on a tile and 128 columns; it now spends 128 (that stencil 195 -> 182 us, power-law
+// graph of 2^20 nodes at N = 512 3.14 -> 2.76 ms, of 2^21 nodes at N = 64 1.29 -> 1.19): ids are loaded
+// four tiles at a time into a register and handed out by shuffles instead of passing through a ring in shared memory, shared
+// addresses are 32-bit sums of a lane's constant and the slot, fragments are an outer loop, and what the end of a
+// fragment needs is loaded when it begins.
 //
 // Each ring slot holds one step: KT tiles, for each the 8 gathered rows of B (32*NQ columns) and the tile
-// operand or what it is rebuilt from.  Gathered-row ids (and the value runs of the compact encodings) go
-// through a ring of their own, S - 1 steps further ahead, so that they have landed when the copies that
-// need them as addresses are issued.  All synchronisation is cp.async.wait_group + __syncwarp.
+// operand.  What a tile of the compact encodings is rebuilt from is copied one step earlier, and the tile is rebuilt between the
+// products of the one before it (MCO, power-law graph of 2^20 nodes, N = 128: 880 -> 779 us; ME-TCF, uniform 10^5 rows: 58.8 -> 54.9).
+// All synchronisation is cp.async.wait_group + __syncwarp.
 //
 // Copy mapping and fragment mapping.  The load/store unit handles a 128-bit access one quarter-warp
 // (8 lanes) at a time and spends one pass per distinct 128-byte line, so the copy is issued with lane l ->
@@ -41,23 +44,49 @@ template <int NQ, int KT, int S, int FMT>
 struct WarpLayout {
     static constexpr bool kDense = FMT == kFmtSrbcrs;
     static constexpr int kBBytes = KT * NQ * 1024;   // gathered rows of one step
-    // per tile: the dense tile; ME-TCF 32 indices + 32 values of the run; MCO 16 B of mask + up to 128 values
-    static constexpr int kATile = kDense ? 512 : (FMT == kFmtMco ? 528 : 256);
-    static constexpr int kSlot = kBBytes + KT * kATile;
-    // per tile in the id ring: 8 ids, then (compact encodings) the [begin, end) of its run
-    static constexpr int kIdTile = kDense ? 32 : 48;
-    static constexpr int kIdRing = FMT == kFmtMetcf ? 8 : 4;   // steps; ME-TCF still needs a step's run when it consumes it
-    static constexpr int kIdStep = KT * kIdTile;
-    static constexpr int kIds = S * kSlot;
-    static constexpr int kTile = kIds + kIdRing * kIdStep;     // ME-TCF: the tile being rebuilt
+    // per tile: the dense tile; ME-TCF 32 indices + 32 values of the run, then [begin, end); MCO 16 B of mask + up to 128 values
+    static constexpr int kATile = kDense ? 512 : (FMT == kFmtMco ? 528 : 272);
+    static constexpr int kRunAt = 256;
+    static constexpr int kAStep = KT * kATile;
+    static constexpr int kARing = kDense || KT == 1 ? S : S + 1;
+    static constexpr int kA = S * kBBytes;
+    static constexpr int kTile = kA + kARing * kAStep;         // ME-TCF: the tile being rebuilt
     static constexpr int kBytes = kTile + (FMT == kFmtMetcf ? 512 : 0);
 };
+
+// Ids (and runs) are loaded a batch at a time, 32 ids in one coalesced load, and handed out by shuffles.
+template <int KT>
+struct WarpIds {
+    static constexpr int kTiles = KT > 4 ? KT : 4;   // tiles in a batch
+    static constexpr int kRegs = kTiles / 4;
+};
+
+__device__ __forceinline__ float4 lds128(uint32_t at) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    return v;
+}
+__device__ __forceinline__ float2 lds64(uint32_t at) {
+    float2 v;
+    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at));
+    return v;
+}
+__device__ __forceinline__ float lds32(uint32_t at) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at));
+    return v;
+}
+__device__ __forceinline__ void sts32(uint32_t at, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts64(uint32_t at, int x, int y) { asm volatile("st.shared.v2.s32 [%0], {%1,%2};" ::"r"(at), "r"(x), "r"(y) : "memory"); }
+__device__ __forceinline__ void sts128_zero(uint32_t at) { asm volatile("st.shared.v4.s32 [%0], {%1,%1,%1,%1};" ::"r"(at), "r"(0) : "memory"); }
 
 // COMP: three products per MMA (hi*hi and the two residual terms).
 template <int NQ, int KT, int S, int MINB, int FMT, bool GUARD, bool COMP>
 __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
     using L = WarpLayout<NQ, KT, S, FMT>;
-    constexpr bool METCF = FMT == kFmtMetcf, MCO = FMT == kFmtMco;
+    using I = WarpIds<KT>;
+    constexpr bool METCF = FMT == kFmtMetcf, MCO = FMT == kFmtMco, DENSE = L::kDense;
+    constexpr int kAhead = DENSE ? 0 : 1;   // steps by which the copies of the tiles are ahead of those of the gathered rows
     extern __shared__ __align__(128) unsigned char smem[];
 
     let_next_kernel_start();
@@ -70,7 +99,9 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
     const int n_tiles = p.group_tile[blockIdx.x + 1] - t0;   // indexed 0..n_tiles-1 below
     if (f >= f_end) return;
     int f_tend = p.frag_off[f + 1] - t0;
-    int f_next = p.frag_off[min((int64_t)f + 2, p.n_frag)] - t0;   // end of the following fragment, loaded ahead
+    // loaded ahead: the end of the following fragment, window and slot of the current one
+    int f_next = p.frag_off[min((int64_t)f + 2, p.n_frag)] - t0;
+    int win = p.frag_win[f], part = p.frag_slot[f];
 
     wait_for_previous_kernel();
 
@@ -78,17 +109,23 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
 
     // copy side: row lr (and lr + 4), chunk lc of every 32-column group
     const int lr = lane >> 3, lc = lane & 7;
-    const uint32_t cp0 = (uint32_t)(lr * 128 + ((lc ^ (lr & 6)) << 4));
-    const uint32_t cp1 = (uint32_t)((lr + 4) * 128 + ((lc ^ (lr & 6) ^ 4) << 4));
+    const uint32_t cp0 = ring + (uint32_t)(lr * 128 + ((lc ^ (lr & 6)) << 4));
+    const uint32_t cp1 = ring + (uint32_t)((lr + 4) * 128 + ((lc ^ (lr & 6) ^ 4) << 4));
+    const uint32_t cpa = ring + L::kA + lane * 16 + (MCO ? 16 : 0);
     bool qok[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; q++) qok[q] = !GUARD || (col_base + 32 * q + 4 * lc) < p.N;
     const char* Bcol = reinterpret_cast<const char*>(p.B + col_base + 4 * lc);
     const uint32_t ldb_bytes = (uint32_t)(p.ldb * 4);
+    // what this lane copies of a tile: 16 bytes of a dense one, 4 indices or values of a ME-TCF run, 4 values of a MCO run
+    const char* a_src = DENSE ? reinterpret_cast<const char*>(p.val_blk + (int64_t)t0 * kTileElems + lane * 4)
+                              : (METCF && lane < 8 ? reinterpret_cast<const char*>(p.coo_idx) : reinterpret_cast<const char*>(p.coo_val)) + (METCF ? lc : lane) * 16;
+    const unsigned long long* mask_src = MCO ? p.mco_mask + 2 * (int64_t)t0 : nullptr;
     // fragment side: chunk g of rows 2k and 2k + 1; tile columns 2k, 2k + 1 of rows g and g + 8
-    const int frag_off = 2 * k * 128 + ((g ^ (2 * k)) << 4);
+    const uint32_t fb = ring + 2 * k * 128 + ((g ^ (2 * k)) << 4);
     const int i0 = 8 * g + 2 * k;
-    const int ao0 = (L::kDense ? sw223(i0) : sw123(i0)) * 4, ao1 = (L::kDense ? sw223(i0 + 64) : sw123(i0 + 64)) * 4;
+    const int ao0 = DENSE ? sw223(i0) : sw123(i0), ao1 = DENSE ? sw223(i0 + 64) : sw123(i0 + 64);
+    const uint32_t fa0 = ring + (METCF ? L::kTile : L::kA) + ao0 * 4, fa1 = ring + (METCF ? L::kTile : L::kA) + ao1 * 4;
 
     float acc[NQ][4][4];
 #pragma unroll
@@ -98,174 +135,221 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
 #pragma unroll
             for (int i = 0; i < 4; i++) acc[q][j][i] = 0.f;
 
-    // ids (and runs) of step j -> id ring
-    auto issue_ids = [&](int j) {
-        const uint32_t dst = ring + L::kIds + (j & (L::kIdRing - 1)) * L::kIdStep;
-        const int u = lane >> 1, tt = j * KT + u;
-        if (lane < 2 * KT && tt < n_tiles)
-            cpa16(dst + u * L::kIdTile + (lane & 1) * 16, p.val_sidx + ((int64_t)t0 + tt) * kTileCols + (lane & 1) * 4);
-        if (METCF) {
-            const int v = lane - 16, tv = j * KT + v;
-            if (v >= 0 && v < KT && tv < n_tiles)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst + v * L::kIdTile + 32), "l"(p.coo_off + 2 * ((int64_t)t0 + tv)) : "memory");
-        } else if (MCO) {
-            const int v = (lane - 16) >> 1, tv = j * KT + v;
-            if (lane >= 16 && v < KT && tv < n_tiles)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + v * L::kIdTile + 32 + (lane & 1) * 4),
-                             "l"(p.coo_off + (int64_t)t0 + tv + (lane & 1)) : "memory");
-        }
+    // ---- copies ------------------------------------------------------------------------------------------
+    const int32_t* idp = p.val_sidx + (int64_t)t0 * kTileCols + lane;
+    auto load_ids = [&](int (&id)[I::kRegs], int tile) {
+#pragma unroll
+        for (int i = 0; i < I::kRegs; i++) id[i] = tile + 4 * i + (lane >> 3) < n_tiles ? __ldg(idp + (tile + 4 * i) * kTileCols) : 0;
     };
-    // operands of step j -> slot (byte offset); the step's ids are visible
-    auto issue_step = [&](int j, int slot) {
-        const unsigned char* idp = smem + L::kIds + (j & (L::kIdRing - 1)) * L::kIdStep;
+    auto load_runs = [&](int2& run, int tile) {
+        if (lane < I::kTiles && tile + lane < n_tiles)
+            run = METCF ? __ldg(reinterpret_cast<const int2*>(p.coo_off) + t0 + tile + lane)
+                        : make_int2(__ldg(p.coo_off + t0 + tile + lane), __ldg(p.coo_off + t0 + tile + lane + 1));
+    };
+    int id[I::kRegs], id_next[I::kRegs];
+    int2 run, run_next;
+    load_ids(id, 0);
+    if (!DENSE) load_runs(run, 0);
+    load_ids(id_next, I::kTiles);
+    if (!DENSE) load_runs(run_next, I::kTiles);
+
+    int b_tile = 0, a_tile = 0;   // first tiles whose rows, and whose own copies, have not been issued
+    auto issue_rows = [&](uint32_t slot) {   // gathered rows of the next step
 #pragma unroll
         for (int u = 0; u < KT; u++) {
-            const int tt = j * KT + u;
-            if (tt < n_tiles) {
-                const int* id = reinterpret_cast<const int*>(idp + u * L::kIdTile);
-                const uint32_t dst = ring + slot + u * NQ * 1024;
-                const char* r0 = Bcol + (uint64_t)(uint32_t)id[lr] * ldb_bytes;
-                const char* r1 = Bcol + (uint64_t)(uint32_t)id[lr + 4] * ldb_bytes;
+            if (b_tile + u < n_tiles) {
+                const int ids = id[u / 4], from = (KT < 4 ? (b_tile + u) & 3 : u & 3) * 8 + lr;
+                const uint32_t row0 = (uint32_t)__shfl_sync(0xffffffffu, ids, from), row1 = (uint32_t)__shfl_sync(0xffffffffu, ids, from + 4);
+                const char* r0 = Bcol + (uint64_t)row0 * ldb_bytes;
+                const char* r1 = Bcol + (uint64_t)row1 * ldb_bytes;
+                const uint32_t to = slot + u * NQ * 1024;
 #pragma unroll
                 for (int q = 0; q < NQ; q++) {
                     if (qok[q]) {
-                        cpa16(dst + cp0 + q * 1024, r0 + q * 128);
-                        cpa16(dst + cp1 + q * 1024, r1 + q * 128);
-                    }
-                }
-                const uint32_t at = ring + slot + L::kBBytes + u * L::kATile;
-                if (L::kDense) {
-                    cpa16(at + lane * 16, p.val_blk + ((int64_t)t0 + tt) * kTileElems + lane * 4);
-                } else {
-                    const int2 run = *reinterpret_cast<const int2*>(idp + u * L::kIdTile + 32);
-                    if (METCF) {   // the first 32 entries (runs start on multiples of 8 entries and are padded to 8)
-                        const int chunk = lane & 7;
-                        if (lane < 16 && run.x + 4 * chunk < ((run.y + 7) & ~7)) {
-                            const void* src = lane < 8 ? static_cast<const void*>(p.coo_idx + run.x + 4 * chunk)
-                                                       : static_cast<const void*>(p.coo_val + run.x + 4 * chunk);
-                            cpa16(at + lane * 16, src);
-                        }
-                    } else {       // mask, then the values (runs are multiples of 4 values)
-                        if (lane == 0) cpa16(at, p.mco_mask + 2 * ((int64_t)t0 + tt));
-                        if (run.x + 4 * lane < run.y) cpa16(at + 16 + lane * 16, p.coo_val + run.x + 4 * lane);
+                        cpa16(cp0 + to + q * 1024, r0 + q * 128);
+                        cpa16(cp1 + to + q * 1024, r1 + q * 128);
                     }
                 }
             }
+        }
+        b_tile += KT;
+        if (KT >= 4 || (b_tile & 3) == 0) {   // on to the next batch
+#pragma unroll
+            for (int i = 0; i < I::kRegs; i++) id[i] = id_next[i];
+            load_ids(id_next, b_tile + I::kTiles);
+        }
+    };
+    auto issue_tiles = [&](uint32_t slot) {   // the next step's tiles, or what they are rebuilt from
+#pragma unroll
+        for (int u = 0; u < KT; u++) {
+            if (a_tile + u < n_tiles) {
+                const uint32_t to = cpa + slot + u * L::kATile;
+                if (DENSE) {
+                    cpa16(to, a_src + u * (kTileElems * 4));
+                } else {
+                    const int src = KT < 4 ? (a_tile + u) & 3 : u;
+                    const int b = __shfl_sync(0xffffffffu, run.x, src), e = __shfl_sync(0xffffffffu, run.y, src);
+                    if (METCF) {   // the first 32 entries (runs start on multiples of 8 entries and are padded to 8)
+                        if (lane < 16 && b + 4 * lc < ((e + 7) & ~7)) cpa16(to, a_src + (int64_t)b * 4);
+                        if (lane == 16) sts64(to, b, e);   // 256 bytes from the tile's first copy
+                    } else {       // mask, then the values (runs are multiples of 4 values)
+                        if (lane == 0) cpa16(to - 16, mask_src + 2 * u);
+                        if (b + 4 * lane < e) cpa16(to, a_src + (int64_t)b * 4);
+                    }
+                }
+            }
+        }
+        a_tile += KT;
+        if (DENSE) a_src += KT * kTileElems * 4;
+        if (MCO) mask_src += 2 * KT;
+        if (!DENSE && (KT >= 4 || (a_tile & 3) == 0)) {
+            run = run_next;
+            load_runs(run_next, a_tile + I::kTiles);
         }
     };
 
-    // ---- prologue: ids of the first 2S - 2 steps, operands of the first S - 1 ------------------------
-#pragma unroll
-    for (int j = 0; j < 2 * S - 2; j++) issue_ids(j);
-    cpa_commit();
-    cpa_wait<0>();
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < S - 1; j++) {
-        issue_step(j, j * L::kSlot);
-        cpa_commit();
-    }
-
-    // ---- main loop: one trip per tile ------------------------------------------------------------------
-    int step = 0, next_slot = (S - 1) * L::kSlot, slot = -L::kSlot;
-    for (int t = 0;; t++) {
-        while (t == f_tend && f < f_end) {  // fragment finished (also: fragments without tiles)
-            flush_fragment<NQ>(p, f, col_base, g, k, acc);
-            f++;
-            f_tend = f < f_end ? f_next : -1;
-            f_next = p.frag_off[min((int64_t)f + 2, p.n_frag)] - t0;
+    // ---- operand of a tile: (g, 2k), (g + 8, 2k), (g, 2k + 1), (g + 8, 2k + 1) ------------------------------
+    // Dense tiles are read where they are used.  The others are rebuilt while the tile before them is multiplied, in
+    // three stages between the products, so that none of their chains of dependent accesses is waited for.
+    float af[4];
+    int2 rb_run;
+    float rb_idx, rb_val;
+    auto rebuild0 = [&](uint32_t at, int tile) {   // at: the tile's place in shared memory; behind the last tile: empty
+        if (METCF) {
+            const float2 r = lds64(ring + at + L::kRunAt);
+            rb_run = tile < n_tiles ? make_int2(__float_as_int(r.x), __float_as_int(r.y)) : make_int2(0, 0);
+            rb_idx = lds32(ring + at + lane * 4);   // behind the run: not used
+            rb_val = lds32(ring + at + 128 + lane * 4);
+            sts128_zero(ring + L::kTile + lane * 16);
         }
-        if (f >= f_end) break;
-        const int u = t & (KT - 1);
-        if (u == 0) {
-            cpa_wait<S - 2>();       // this step has landed (this thread's copies) ...
-            __syncwarp();            // ... and everybody's; also: all lanes are done with the slot refilled here
-            issue_step(step + S - 1, next_slot);
-            issue_ids(step + 2 * S - 2);
-            cpa_commit();
-            step++;
-            slot += L::kSlot;
-            if (slot == S * L::kSlot) slot = 0;
-            next_slot = slot;        // the slot consumed now is the next one to be refilled
+    };
+    auto rebuild1 = [&]() {
+        if (METCF) {
+            __syncwarp();
+            if (lane < rb_run.y - rb_run.x) sts32(ring + L::kTile + __float_as_int(rb_idx) * 4, rb_val);
+            for (int e = rb_run.x + 32 + lane; e < rb_run.y; e += 32) sts32(ring + L::kTile + __ldg(p.coo_idx + e) * 4, __ldg(p.coo_val + e));
         }
-        const unsigned char* bt = smem + slot + u * NQ * 1024 + frag_off;
-        // ME-TCF: the gathered rows before the tile is rebuilt, as many as registers hold, so that their loads overlap
-        // that chain (300 000-node power-law graph, N = 128: 275 us, now 252; all four groups of columns spill: 344).
-        constexpr int kEarly = METCF ? (NQ <= 2 ? NQ : (NQ == 4 ? 2 : 0)) : 0;
-        float4 early[kEarly > 0 ? kEarly : 1][2];
-#pragma unroll
-        for (int q = 0; q < kEarly; q++) {
-            early[q][0] = *reinterpret_cast<const float4*>(bt + q * 1024);
-            early[q][1] = *reinterpret_cast<const float4*>(bt + q * 1024 + 128);
-        }
-        const unsigned char* at = smem + slot + L::kBBytes + u * L::kATile;
-        float af[4];   // (g, 2k), (g + 8, 2k), (g, 2k + 1), (g + 8, 2k + 1)
+    };
+    auto rebuild2 = [&](uint32_t at) {
         if (MCO) {
             // values lie in ascending bit order: a value's place is the number of mask bits below its own.  Bits
             // 32i..32i+31 are rows 4i..4i+3.
-            const uint4 m = *reinterpret_cast<const uint4*>(at);
-            const float* vals = reinterpret_cast<const float*>(at + 16);
-            const int sh = (ao0 >> 2) & 31;
+            const float4 w = lds128(ring + at);
+            const uint32_t mx = __float_as_uint(w.x), my = __float_as_uint(w.y), mz = __float_as_uint(w.z), mw = __float_as_uint(w.w);
+            const int sh = ao0 & 31;
             const uint32_t below = (1u << sh) - 1u;
             const bool up = g >= 4;   // row g is in the second word of its half
-            const int n0 = __popc(m.x), n1 = n0 + __popc(m.y);
-            const uint32_t w0 = up ? m.y : m.x, w1 = up ? m.w : m.z;
-            const int c0 = (up ? n0 : 0) + __popc(w0 & below), c1 = n1 + (up ? __popc(m.z) : 0) + __popc(w1 & below);
+            const int n0 = __popc(mx), n1 = n0 + __popc(my);
+            const uint32_t w0 = up ? my : mx, w1 = up ? mw : mz;
+            const uint32_t c0 = ring + at + 16 + 4 * ((up ? n0 : 0) + __popc(w0 & below)), c1 = ring + at + 16 + 4 * (n1 + (up ? __popc(mz) : 0) + __popc(w1 & below));
             const uint32_t b0 = w0 >> sh, b1 = w1 >> sh;
-            af[0] = (b0 & 1u) ? vals[c0] : 0.f;
-            af[2] = (b0 & 2u) ? vals[c0 + (b0 & 1u)] : 0.f;
-            af[1] = (b1 & 1u) ? vals[c1] : 0.f;
-            af[3] = (b1 & 2u) ? vals[c1 + (b1 & 1u)] : 0.f;
+            af[0] = af[1] = af[2] = af[3] = 0.f;
+            if (b0 & 1u) af[0] = lds32(c0);
+            if (b0 & 2u) af[2] = lds32(c0 + (b0 & 1u) * 4);
+            if (b1 & 1u) af[1] = lds32(c1);
+            if (b1 & 2u) af[3] = lds32(c1 + (b1 & 1u) * 4);
         } else {
-            if (METCF) {   // rebuild the 16x8 tile: zero, then tile[idx] = value over the run
-                float* tile = reinterpret_cast<float*>(smem + L::kTile);
-                const int2 run = *reinterpret_cast<const int2*>(smem + L::kIds + ((step - 1) & (L::kIdRing - 1)) * L::kIdStep + u * L::kIdTile + 32);
-                const int rcnt = run.y - run.x;
-                const int idx = reinterpret_cast<const int*>(at)[lane];   // behind the run: not used
-                const float val = reinterpret_cast<const float*>(at + 128)[lane];
-                if (KT > 1 && u > 0) __syncwarp();   // the previous tile's fragments have been read
-                reinterpret_cast<float4*>(tile)[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-                __syncwarp();
-                if (lane < rcnt) tile[idx] = val;
-                for (int e = run.x + 32 + lane; e < run.y; e += 32) tile[__ldg(p.coo_idx + e)] = __ldg(p.coo_val + e);
-                __syncwarp();
-                at = smem + L::kTile;
-            }
-            const float2 v0 = *reinterpret_cast<const float2*>(at + ao0), v1 = *reinterpret_cast<const float2*>(at + ao1);
+            if (METCF) __syncwarp();
+            const float2 v0 = lds64(fa0 + (METCF ? 0 : at)), v1 = lds64(fa1 + (METCF ? 0 : at));
             af[0] = v0.x; af[1] = v1.x; af[2] = v0.y; af[3] = v1.y;
         }
-        if constexpr (COMP) {
+    };
+
+    // ---- prologue: operands of the first S - 1 steps ---------------------------------------------------
+    if (kAhead) issue_tiles(0);
+#pragma unroll
+    for (int j = 0; j < S - 1; j++) {
+        issue_rows(j * L::kBBytes);
+        issue_tiles((j + kAhead) * L::kAStep);
+        cpa_commit();
+    }
+    uint32_t b_slot = (S - 1) * L::kBBytes;                  // of the step before the current one: refilled next
+    uint32_t a_fill = (S - 1 + kAhead) % L::kARing * L::kAStep;  // the slot of tiles that is filled next
+    uint32_t a_slot = 0;                                     // the tile whose operand is read next
+    auto next_tile = [&]() { a_slot = a_slot == L::kARing * L::kAStep - L::kATile ? 0u : a_slot + L::kATile; };
+    if (!DENSE) {
+        cpa_wait<S - 2>();
+        __syncwarp();
+        rebuild0(L::kA + a_slot, 0);
+        rebuild1();
+        rebuild2(L::kA + a_slot);
+        next_tile();
+    }
+
+    // ---- main loop, fragment by fragment -----------------------------------------------------------------
+    int t = 0;
+    for (;;) {
+        for (; t < f_tend; t++) {
+            const int u = t & (KT - 1);
+            if (u == 0) {
+                cpa_wait<S - 2>();       // this step has landed (this thread's copies) ...
+                __syncwarp();            // ... and everybody's; also: all lanes are done with the slot refilled here
+                issue_rows(b_slot);
+                issue_tiles(a_fill);
+                cpa_commit();
+                a_fill = a_fill == (L::kARing - 1) * L::kAStep ? 0u : a_fill + L::kAStep;
+                b_slot = b_slot == (S - 1) * L::kBBytes ? 0u : b_slot + L::kBBytes;
+            } else if (METCF) {
+                __syncwarp();            // all lanes have read the rebuilt tile
+            }
+            const uint32_t bt = fb + b_slot + u * NQ * 1024;
+            if (DENSE) {
+                rebuild2(a_slot);
+                next_tile();
+            }
             uint32_t a[4], al[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) { a[i] = tf32_hi(af[i]); al[i] = tf32_lo(af[i], a[i]); }
-#pragma unroll
-            for (int q = 0; q < NQ; q++) {
-                const float4 v0 = *reinterpret_cast<const float4*>(bt + q * 1024);
-                const float4 v1 = *reinterpret_cast<const float4*>(bt + q * 1024 + 128);
-                const float b0[4] = {v0.x, v0.y, v0.z, v0.w}, b1[4] = {v1.x, v1.y, v1.z, v1.w};
-                uint32_t h0[4], h1[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) { h0[j] = tf32_hi(b0[j]); h1[j] = tf32_hi(b1[j]); }
-                // small terms first; four accumulators in turn, so that no product waits for the one before it
-#pragma unroll
-                for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], al, h0[j], h1[j]);
-#pragma unroll
-                for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], a, tf32_lo(b0[j], h0[j]), tf32_lo(b1[j], h1[j]));
-#pragma unroll
-                for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], a, h0[j], h1[j]);
+            for (int i = 0; i < 4; i++) {
+                a[i] = COMP ? tf32_hi(af[i]) : rna_bits(af[i]);
+                if (COMP) al[i] = tf32_lo(af[i], a[i]);
             }
-        } else {
-            const uint32_t a[4] = {rna_bits(af[0]), rna_bits(af[1]), rna_bits(af[2]), rna_bits(af[3])};
+            // Loads do not pass the rebuilding's stores: for ME-TCF two groups of columns are read before them, the others
+            // between its stages (each where it is used: uniform 10^5 rows, N = 128, 56.7 us, so 54.9).
+            float4 v[NQ][2];
+            auto read_rows = [&](int q) { v[q][0] = lds128(bt + q * 1024); v[q][1] = lds128(bt + q * 1024 + 128); };
+            if (METCF) {
+#pragma unroll
+                for (int q = 0; q < 2 && q < NQ; q++) read_rows(q);
+            }
+            if (!DENSE) rebuild0(L::kA + a_slot, t + 1);
 #pragma unroll
             for (int q = 0; q < NQ; q++) {
-                const float4 v0 = q < kEarly ? early[q][0] : *reinterpret_cast<const float4*>(bt + q * 1024);
-                const float4 v1 = q < kEarly ? early[q][1] : *reinterpret_cast<const float4*>(bt + q * 1024 + 128);
-                mma_tf32(acc[q][0], a, rna_bits(v0.x), rna_bits(v1.x));
-                mma_tf32(acc[q][1], a, rna_bits(v0.y), rna_bits(v1.y));
-                mma_tf32(acc[q][2], a, rna_bits(v0.z), rna_bits(v1.z));
-                mma_tf32(acc[q][3], a, rna_bits(v0.w), rna_bits(v1.w));
+                if (!METCF) read_rows(q);
+                const float b0[4] = {v[q][0].x, v[q][0].y, v[q][0].z, v[q][0].w}, b1[4] = {v[q][1].x, v[q][1].y, v[q][1].z, v[q][1].w};
+                if constexpr (COMP) {
+                    uint32_t h0[4], h1[4];
+#pragma unroll
+                    for (int j = 0; j < 4; j++) { h0[j] = tf32_hi(b0[j]); h1[j] = tf32_hi(b1[j]); }
+                    // small terms first; four accumulators in turn, so that no product waits for the one before it
+#pragma unroll
+                    for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], al, h0[j], h1[j]);
+#pragma unroll
+                    for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], a, tf32_lo(b0[j], h0[j]), tf32_lo(b1[j], h1[j]));
+#pragma unroll
+                    for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], a, h0[j], h1[j]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; j++) mma_tf32(acc[q][j], a, rna_bits(b0[j]), rna_bits(b1[j]));
+                }
+                if (!DENSE && q == 0) {
+                    rebuild1();
+                    if (METCF) {
+#pragma unroll
+                        for (int r = 2; r < NQ; r++) read_rows(r);
+                    }
+                }
+                if (!DENSE && q == (NQ > 1 ? 1 : 0)) {
+                    rebuild2(L::kA + a_slot);
+                    next_tile();
+                }
             }
         }
+        write_fragment<NQ, GUARD>(p, win, part, col_base, g, k, acc);
+        if (++f >= f_end) break;
+        f_tend = f_next;
+        f_next = p.frag_off[min((int64_t)f + 2, p.n_frag)] - t0;
+        win = p.frag_win[f];
+        part = p.frag_slot[f];
     }
     cpa_wait<0>();
 }

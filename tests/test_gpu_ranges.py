@@ -123,6 +123,33 @@ def test_warp_kernel_step_lengths(oracle_mod, fmt, N, windows):
         engine.tune("sweep", 1)
 
 
+# tiles with all 128 entries beside tiles with one, windows of 0, 1, 4, 5 and 9 tiles (batches of ids are 4 or 8 tiles), every step
+# length; gt: groups of single tiles, of a few, and as the plan has them
+@pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
+@pytest.mark.parametrize("N", [32, 64, 96, 260])
+@pytest.mark.parametrize("windows", [9, 900, 5000])
+@pytest.mark.parametrize("gt", [0, 1, 6])
+def test_warp_kernel_full_tiles_beside_single_entries(oracle_mod, fmt, N, windows, gt):
+    import torch
+    from mask_b200 import engine
+    rng = np.random.Generator(np.random.PCG64(windows + gt))
+    K, rows = 300, []
+    for w in range(windows):
+        tiles = (0, 1, 4, 5, 9)[w % 5]
+        full = np.sort(rng.choice(K, 8 * tiles, replace=False))
+        rows += [full if w % 3 else full[r::16] for r in range(16)]
+    m = _rows_to_csr(rows[:-3], K, 5)
+    p = {"srbcrs": engine.pack_srbcrs, "metcf": engine.pack_metcf, "mco": engine.pack_mco}[fmt](*_dev(m), m.M, m.K)
+    B = rng.standard_normal((K, N), dtype=np.float32)
+    out = torch.full((m.M, N), float("nan"), device="cuda")
+    engine.tune("sweep", 0)
+    try:
+        engine.spmm(p, torch.from_numpy(B).cuda(), out=out, plan=p.new_plan("auto", gt))
+    finally:
+        engine.tune("sweep", 1)
+    _assert_close(oracle_mod, m, B, out.cpu().numpy())
+
+
 @pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
 @pytest.mark.parametrize("N,offset,sweep", [(1, 0, 1), (3, 0, 1), (47, 0, 1), (47, 1, 2), (64, 3, 1), (129, 2, 1), (515, 0, 2)])
 def test_rows_that_are_not_whole_vectors(oracle_mod, fmt, N, offset, sweep):
