@@ -334,17 +334,20 @@ __global__ void __launch_bounds__(kChunkThreads) warp_group_jumps_kernel(const T
         groups[base + i] = cnt[i];
     }
 }
-// entry[c], first[c]: where the walk from fragment 0 enters chunk c, and how many groups begin before
+// entry[c], first[c]: where the walk from fragment 0 enters chunk c, and how many groups begin before.  A group is shorter than a
+// chunk, but not than what is left for the last one: that can be passed over, and is then entered behind its end.
 __global__ void warp_group_walk_kernel(const TableArgs a, const int32_t* __restrict__ exit_to, const int32_t* __restrict__ groups,
                                        int32_t* __restrict__ entry, int32_t* __restrict__ first) {
     const int32_t F = a.counts->frags;
     if (a.counts->bad) return;
     int32_t f = 0, g = 0;
-    for (int c = 0; f < F; c++) {   // a group is shorter than a chunk, so no chunk is passed over
+    for (int64_t c = 0; c * kChunk < F; c++) {
         entry[c] = f;
         first[c] = g;
-        g += groups[f];
-        f = exit_to[f];
+        if (f < F) {
+            g += groups[f];
+            f = exit_to[f];
+        }
     }
 }
 __global__ void __launch_bounds__(kChunkThreads) warp_group_write_kernel(const TableArgs a, const int32_t* __restrict__ entry, const int32_t* __restrict__ first) {

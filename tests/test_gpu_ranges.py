@@ -150,6 +150,26 @@ def test_warp_kernel_full_tiles_beside_single_entries(oracle_mod, fmt, N, window
     _assert_close(oracle_mod, m, B, out.cpu().numpy())
 
 
+# the groups of the warp kernel are found in chunks of 2048 fragments; the last chunk may be shorter than a group and have none of its own
+@pytest.mark.parametrize("windows", [2047, 2048, 2049, 2050, 2052, 4096, 4097, 4099])
+def test_plan_groups_at_the_edges_of_chunks(oracle_mod, windows):
+    import torch
+    from mask_b200 import engine
+    rng = np.random.Generator(np.random.PCG64(windows))
+    K = 2500
+    rows = [np.sort(rng.choice(K, n, replace=False)) for n in rng.integers(0, 3, 16 * windows - 5)]
+    m = _rows_to_csr(rows, K, 7)
+    p = engine.pack_srbcrs(*_dev(m), m.M, m.K)
+    B = rng.standard_normal((K, 64), dtype=np.float32)
+    out = torch.full((m.M, 64), float("nan"), device="cuda")
+    engine.tune("sweep", 0)
+    try:
+        engine.spmm(p, torch.from_numpy(B).cuda(), out=out)
+    finally:
+        engine.tune("sweep", 1)
+    _assert_close(oracle_mod, m, B, out.cpu().numpy())
+
+
 @pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
 @pytest.mark.parametrize("N,offset,sweep", [(1, 0, 1), (3, 0, 1), (47, 0, 1), (47, 1, 2), (64, 3, 1), (129, 2, 1), (515, 0, 2)])
 def test_rows_that_are_not_whole_vectors(oracle_mod, fmt, N, offset, sweep):
