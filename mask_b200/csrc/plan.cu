@@ -157,7 +157,7 @@ constexpr int32_t kFragCost = 4;
 constexpr int64_t kHigh = (int64_t)1 << 32;   // the scans carry two counts: one in each half
 
 struct PlanCounts {          // on the device in front of the tables, and on the host
-    int32_t frags, heads, groups, warp_groups, bad, group_pieces, pad[2];
+    int32_t frags, heads, groups, warp_groups, bad, group_pieces, warp_first, chunks_done;
     int32_t status[4];
 };
 
@@ -166,7 +166,8 @@ struct TableArgs {
     int32_t W, piece, group;
     int64_t T, max_frags;
     int32_t* frag_off; int32_t* frag_win; int32_t* frag_slot; int2* heads;
-    int32_t* group_off; int32_t* group_tile; int32_t* warp_off; int32_t* warp_tile;
+    int32_t* group_off; int32_t* group_tile;
+    int4* warp_group; int4* warp_first;
     PlanCounts* counts;
     PlanCounts* host;        // pinned: the counts for the host, `bad` until the kernels that know them write them
     const int32_t* local;    // NULL: not known to be
@@ -271,19 +272,25 @@ struct GroupsOut {
 // neighbours, short groups keep the band narrow (27-point stencil with 10^6 rows, N = 128: one window a group
 // 517 us, 128 tiles a group 585 us).
 //
+// A fragment that alone is far more than the target of its place would still run when everything else has ended: its warp
+// takes 0.6 to 1 us a tile, and 150 tiles begun 165 us into a product kept it going from 190 to 248 us.  Such groups are listed
+// a second time, to be taken before all others, and are empty in their place (power-law graphs, N = 128: 300 000 nodes 211 -> 171 us,
+// in ME-TCF 251 -> 201, 130 000 nodes 103 -> 84; N = 512 3 to 7 %).  The line at 3/2 of where a group ends: at twice that, 130 000 nodes
+// 88 us; shorter pieces instead cost more in the fix-up than they even out (two thirds of a piece: 86 us, 1 1/2: 94).
+//
 // Where a group ends depends on where it begins, so this is a walk; but from every fragment the end is known at
 // once.  Pointer doubling in shared memory finds for every fragment of a chunk where a walk that enters there leaves
 // the chunk and after how many groups; one thread then walks from chunk to chunk; and every chunk writes the groups of
 // the walk that enters it, itself cut into 32 parts in the same way.
 constexpr int kChunk = 2048, kChunkThreads = 1024, kPart = kChunk / 32;   // a group has at most 41 fragments: less than a part
 
+__device__ __forceinline__ int64_t warp_group_target(const TableArgs& a, int64_t c, int64_t total) {
+    if (a.local && *a.local) return kMinPiece;
+    const int64_t target = (total - c) / a.takers;
+    return target < kMinPiece ? kMinPiece : (target > 128 ? 128 : target);
+}
 __device__ __forceinline__ int64_t warp_group_end(const TableArgs& a, int64_t f, int64_t F, int64_t total) {
-    const int64_t c = cost_before(a, f);
-    int64_t target = kMinPiece;
-    if (!(a.local && *a.local)) {
-        target = (total - c) / a.takers;
-        target = target < kMinPiece ? kMinPiece : (target > 128 ? 128 : target);
-    }
+    const int64_t c = cost_before(a, f), target = warp_group_target(a, c, total);
     const int64_t limit = c + target * 5 / 4;
     int64_t lo = f + 1, hi = f + 2 + target * 5 / 4 / kFragCost;   // the end is in [lo, hi)
     if (hi > F + 1) hi = F + 1;
@@ -368,22 +375,38 @@ __global__ void __launch_bounds__(kChunkThreads) warp_group_write_kernel(const T
             part_first[p] = g;
             if (i < n) { g += cnt[i]; i = to[i]; }
         }
-        if (base + n == F) {
-            a.warp_off[g] = (int32_t)F;
-            a.warp_tile[g] = (int32_t)a.T;
-            a.host->warp_groups = g;
-        }
+        if (base + n == F) a.host->warp_groups = g;
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kChunkThreads) to[i] = -1;   // from here on: number of the group that begins here
     __syncthreads();
     if (threadIdx.x < 32) {
         const int end = min(n, ((int)threadIdx.x + 1) * kPart);
         int32_t g = part_first[threadIdx.x];
-        for (int32_t i = part_entry[threadIdx.x]; i < end; i = next[i], g++) {
-            a.warp_off[g] = (int32_t)base + i;
-            a.warp_tile[g] = a.frag_off[base + i];
+        for (int32_t i = part_entry[threadIdx.x]; i < end; i = next[i], g++) to[i] = g;
+    }
+    __syncthreads();
+    const bool local = a.local && *a.local;
+    for (int i = threadIdx.x; i < n; i += kChunkThreads) {
+        if (to[i] < 0) continue;
+        const int64_t f = base + i;
+        const int32_t t0 = a.frag_off[f];
+        int4 group = make_int4((int)f, (int)(base + next[i]), t0, a.frag_off[base + next[i]] - t0);
+        if (!local && next[i] == i + 1 && 2 * (group.w + kFragCost) > 3 * (warp_group_target(a, cost_before(a, f), total) * 5 / 4)) {
+            a.warp_first[atomicAdd(&a.counts->warp_first, 1)] = group;   // in any order: groups do not depend on one another
+            group.y = group.x;
         }
+        a.warp_group[to[i]] = group;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&a.counts->chunks_done, 1) == (F + kChunk - 1) / kChunk - 1) a.host->warp_first = *(volatile int32_t*)&a.counts->warp_first;
     }
 }
+
+// Groups listed first have more than 3/2 5/4 kMinPiece - kFragCost = 26 tiles.
+static int64_t warp_first_max(int64_t T) { return T / 26 + 1; }
 
 static int enqueue_warp_groups(const TableArgs& a, DevScratch& work, cudaStream_t st) {
     const int64_t chunks = (a.max_frags + kChunk - 1) / kChunk;
@@ -427,7 +450,7 @@ static int enqueue_auto_tables(mask_plan& p, const int32_t* d_val_soff, bool sam
     auto section = [&](int64_t n) { const size_t o = at; at += ((size_t)n + 3) & ~(size_t)3; return o; };
     const int64_t n = a.max_frags;
     const size_t o_fo = section(n + 1), o_fw = section(n), o_fs = section(n), o_go = section(n + 1), o_gt = section(n + 1),
-                 o_wo = section(n + 1), o_wt = section(n + 1), o_hd = section(2 * std::min<int64_t>(p.W, p.T / p.piece_tiles + 1));
+                 o_wg = section(4 * n), o_wf = section(4 * warp_first_max(p.T)), o_hd = section(2 * std::min<int64_t>(p.W, p.T / p.piece_tiles + 1));
     int rc = device_alloc(reinterpret_cast<void**>(&p.d_tables), at * sizeof(int32_t), st);
     if (rc == MASK_OK) rc = spine.alloc(scan_spine_words(n) * 8, st);
     if (rc != MASK_OK) return rc;
@@ -437,10 +460,10 @@ static int enqueue_auto_tables(mask_plan& p, const int32_t* d_val_soff, bool sam
     a.frag_slot = p.d_frag_slot = p.d_tables + o_fs;
     a.group_off = p.d_group_off = p.d_tables + o_go;
     a.group_tile = p.d_group_tile = p.d_tables + o_gt;
-    a.warp_off = p.d_tables + o_wo;
-    a.warp_tile = p.d_tables + o_wt;
-    p.d_warp_off = same_groups ? p.d_group_off : a.warp_off;
-    p.d_warp_tile = same_groups ? p.d_group_tile : a.warp_tile;
+    a.warp_group = reinterpret_cast<int4*>(p.d_tables + o_wg);
+    a.warp_first = reinterpret_cast<int4*>(p.d_tables + o_wf);
+    p.d_warp_group = same_groups ? nullptr : a.warp_group;
+    p.d_warp_first = a.warp_first;
     a.heads = reinterpret_cast<int2*>(p.d_tables + o_hd);
     p.d_heads = a.heads;
     p.d_status = p.d_tables + offsetof(PlanCounts, status) / 4;
@@ -491,8 +514,6 @@ static int upload_tables(mask_plan& p, const int32_t* soff, cudaStream_t st) {
     p.d_frag_slot = p.d_tables + o_fs;
     p.d_group_off = p.d_tables + o_go;
     p.d_group_tile = p.d_tables + o_gt;
-    p.d_warp_off = p.d_group_off;
-    p.d_warp_tile = p.d_group_tile;
     p.d_heads = reinterpret_cast<const int2*>(p.d_tables + o_hd);
     p.d_status = p.d_tables + o_st;
     cudaError_t e = cudaMemcpyAsync(p.d_tables, h, at * sizeof(int32_t), cudaMemcpyHostToDevice, st);
@@ -582,6 +603,7 @@ static int create_plan(const int32_t* d_val_soff, const int32_t* d_val_sidx, int
             p->P_group = c.group_pieces;
             p->G = c.groups;
             p->Gw = group_tiles > 0 ? p->G : c.warp_groups;
+            p->warp_first = group_tiles > 0 ? 0 : c.warp_first;
             return MASK_OK;
         }
         const int32_t* soff = stage.as<int32_t>();

@@ -13,7 +13,7 @@
 // fragments (their rows of C must still be written).  frag_slot[f] is -1 when the fragment is
 // its whole window (direct store to C) and otherwise the index of its 16xN partial tile in
 // scratch.  Thread block g processes fragments [group_off[g], group_off[g+1]); the blocks of the
-// warp-level kernel take [warp_off[g], warp_off[g+1]).  heads lists, for the fix-up pass, the first
+// warp-level kernel have groups of their own.  heads lists, for the fix-up pass, the first
 // fragment of every split window and the number of its pieces.
 struct mask_plan {
     int32_t M = 0;
@@ -37,8 +37,11 @@ struct mask_plan {
     int32_t* d_frag_slot = nullptr;
     int32_t* d_group_off = nullptr;
     int32_t* d_group_tile = nullptr;  // first tile of every group, then T
-    int32_t* d_warp_off = nullptr;
-    int32_t* d_warp_tile = nullptr;
+    // groups of the warp-level kernel: first fragment, end, first tile, tiles; NULL: it takes the plan's own groups.  The
+    // warp_first groups of d_warp_first are taken before the others, among which they are empty.
+    const int4* d_warp_group = nullptr;
+    const int4* d_warp_first = nullptr;
+    int32_t warp_first = 0;
     const int2* d_heads = nullptr;
     int32_t* d_status = nullptr;  // device status word: non-zero after a kernel gave up on a bounded wait
     const int32_t* d_row_map = nullptr;  // optional, not owned: output row of packed row i (a row reorder's order[])

@@ -13,6 +13,9 @@ struct SpmmArgs {
     const int32_t* frag_slot;
     const int32_t* group_off;
     const int32_t* group_tile;  // first tile of every group (+ closing entry): persistent kernel only
+    const int4* warp_group;     // warp-level kernel: the plan's d_warp_group and d_warp_first
+    const int4* warp_first;
+    int32_t n_warp_first;
     int64_t n_frag;             // fragments in the plan (frag_off has n_frag + 1 entries)
     int32_t n_groups;
     int32_t n_col_blocks;       // persistent kernel: column blocks of 128*NSLAB columns

@@ -93,10 +93,16 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
     const int lane = threadIdx.x;
     const int g = lane >> 2, k = lane & 3;
     const int col_base = blockIdx.y * (32 * NQ);
-    int f = p.group_off[blockIdx.x];
-    const int f_end = p.group_off[blockIdx.x + 1];
-    const int t0 = p.group_tile[blockIdx.x];
-    const int n_tiles = p.group_tile[blockIdx.x + 1] - t0;   // indexed 0..n_tiles-1 below
+    int4 group;
+    if (p.warp_group) {
+        const int b = (int)blockIdx.x - p.n_warp_first;
+        group = b < 0 ? p.warp_first[blockIdx.x] : p.warp_group[b];
+    } else {
+        const int f0 = p.group_off[blockIdx.x], f1 = p.group_off[blockIdx.x + 1], t = p.group_tile[blockIdx.x];
+        group = make_int4(f0, f1, t, p.group_tile[blockIdx.x + 1] - t);
+    }
+    int f = group.x;
+    const int f_end = group.y, t0 = group.z, n_tiles = group.w;   // tiles are indexed 0..n_tiles-1 below
     if (f >= f_end) return;
     int f_tend = p.frag_off[f + 1] - t0;
     // loaded ahead: the end of the following fragment, window and slot of the current one
@@ -398,7 +404,7 @@ static int launch_warp_variant(const mask_plan* plan, const SpmmArgs& a, cudaStr
     static std::atomic<uint64_t> opted_in;
     const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(kern), L::kBytes, opted_in);
     if (rc != MASK_OK) return rc;
-    dim3 grid((unsigned)plan->Gw, (unsigned)((a.N + 32 * NQ - 1) / (32 * NQ)));
+    dim3 grid((unsigned)(plan->Gw + a.n_warp_first), (unsigned)((a.N + 32 * NQ - 1) / (32 * NQ)));
     if (grid.y > 65535) return fail(MASK_ERR_INVALID_ARGUMENT, "N too large");
     return launch_overlapped(kern, grid, 32, L::kBytes, st, a);
 }
@@ -420,8 +426,10 @@ static int launch_warp_shape(const mask_plan* plan, const SpmmArgs& a, cudaStrea
 template <int FMT>
 int launch_spmm_warp(const mask_plan* plan, const SpmmArgs& a_in, cudaStream_t st, int tuned_nq) {
     SpmmArgs a = a_in;
-    a.group_off = plan->d_warp_off;
-    a.group_tile = plan->d_warp_tile;
+    a.group_tile = plan->d_group_tile;
+    a.warp_group = plan->d_warp_group;
+    a.warp_first = plan->d_warp_first;
+    a.n_warp_first = plan->warp_first;
     a.n_frag = plan->F;
     int nq, depth;
     choose_warp_shape(plan->Gw, plan->T, a.N, a.tf32x3, tuned_nq, &nq, &depth);

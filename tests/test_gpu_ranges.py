@@ -170,6 +170,31 @@ def test_plan_groups_at_the_edges_of_chunks(oracle_mod, windows):
     _assert_close(oracle_mod, m, B, out.cpu().numpy())
 
 
+# windows that are far longer than the groups around them are taken first: none, at the end, over the chunks of 2048 fragments in
+# which the groups are written; 26 tiles are too few, 27 enough, more than 5/4 of a piece are split
+@pytest.mark.parametrize("windows", [60, 2047, 2049, 6200])
+@pytest.mark.parametrize("long_tiles", [0, 26, 27, 100, 300])
+def test_long_windows_among_short_ones(oracle_mod, windows, long_tiles):
+    import torch
+    from mask_b200 import engine
+    rng = np.random.Generator(np.random.PCG64(windows + long_tiles))
+    K, rows = 2500, []
+    for w in range(windows):
+        long = long_tiles and (w % 97 == 50 or w >= windows - 3)
+        cols = np.sort(rng.choice(K, min(8 * long_tiles, K) if long else int(rng.integers(0, 20)), replace=False))
+        rows += [cols[r::16] for r in range(16)]
+    m = _rows_to_csr(rows[:-5], K, 7)
+    p = engine.pack_srbcrs(*_dev(m), m.M, m.K)
+    B = rng.standard_normal((K, 64), dtype=np.float32)
+    out = torch.full((m.M, 64), float("nan"), device="cuda")
+    engine.tune("sweep", 0)
+    try:
+        engine.spmm(p, torch.from_numpy(B).cuda(), out=out)
+    finally:
+        engine.tune("sweep", 1)
+    _assert_close(oracle_mod, m, B, out.cpu().numpy())
+
+
 @pytest.mark.parametrize("fmt", ["srbcrs", "metcf", "mco"])
 @pytest.mark.parametrize("N,offset,sweep", [(1, 0, 1), (3, 0, 1), (47, 0, 1), (47, 1, 2), (64, 3, 1), (129, 2, 1), (515, 0, 2)])
 def test_rows_that_are_not_whole_vectors(oracle_mod, fmt, N, offset, sweep):
