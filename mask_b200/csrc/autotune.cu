@@ -231,9 +231,9 @@ void choose_plan_parameters(mask_plan* plan, const mask_column_features& f) {
     plan->nslab = narrower_rows_pay ? 2 : 4;
     const double even_share = f.distinct_columns ? (double)std::min(f.hub_columns[0], f.distinct_columns) / f.distinct_columns : 1.0;
     plan->local = f.local_share >= kLocalShare;
-    plan->hub_heavy = f.hub_share[0] >= 1.5 * even_share;
-    plan->slab_fits = !plan->local && !plan->hub_heavy && b_bytes > f.l2_bytes && b_bytes / 4 <= f.l2_bytes;
-    plan->far_beyond_l2 = plan->nslab == 2 && b_bytes >= 24.0 * f.l2_bytes;
+    const bool hub_heavy = f.hub_share[0] >= 1.5 * even_share;
+    plan->slab_fits = !plan->local && !hub_heavy && b_bytes > f.l2_bytes && b_bytes / 4 <= f.l2_bytes;
+    plan->far_beyond_l2 = plan->nslab == 2 && b_bytes >= 12.0 * f.l2_bytes;
 }
 
 }  // namespace mask

@@ -49,9 +49,8 @@ struct mask_plan {
     int32_t n_peer_out = 0;
     // what the kernel choice goes by (choose_plan_parameters; without column features all false)
     bool local = false;      // neighbouring windows share the rows of B they gather
-    bool hub_heavy = false;  // a few columns get many of the gathers
-    bool slab_fits = false;  // 128 columns of B fit the L2, 512 do not, and all columns are gathered about equally
     bool far_beyond_l2 = false;  // hub-heavy, and B is many times the L2
+    bool slab_fits = false;  // 128 columns of B fit the L2, 512 do not, and all columns are gathered about equally
     mask_column_features col_features = {};   // set by mask_plan_autotune
     int32_t has_col_features = 0;
     float* d_vals_tf32 = nullptr;        // owned: val_block_val rounded to TF32 (mask_plan_prepare_values), for the TMA kernel

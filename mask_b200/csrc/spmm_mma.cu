@@ -333,22 +333,26 @@ static int sweep_slabs(const mask_plan* plan, int N) {
 // kernel takes up to 512 columns of a tile at once: tile values and ids are read once and every gathered byte goes
 // through shared memory once to and once from, so it wins where full-width rows are gathered at the L2's or
 // shared memory's rate.  The warp kernel takes at most 128 columns at a time, has no minimum width, spreads small
-// matrices over up to 3256 blocks instead of 296, and re-reads (and rebuilds) the tiles for every block of columns.
+// matrices over up to 3256 blocks instead of 296, takes long windows first, and re-reads (and rebuilds) the tiles for every
+// block of columns.
 // It also rounds B where the tcgen05 kernel cuts it off: 2.1 to 3.0e-4 from the exact product (2-norm) against 4.2 to 4.7e-4.
-// Measured in turn (us, tcgen05 / warp), SR-BCRS; power-law graphs of 20 000 / 300 000 / 2^20 / 2^21 / 2^22 nodes:
-//   N = 32     27.8 / 13.0,  279 / 99,   975 / 293,   -,           -
-//   N = 128    29.9 / 24.8,  283 / 221,  1067 / 787,  -,           -
-//   N = 192    34.9 / 32.2,  415 / 336,  1615 / 1266, 3235 / 2784, 12 310 / 10 480
-//   N = 256    35.3 / 37.2,  426 / 420,  1761 / 1700, 3733 / 3642, 14 290 / 13 740
-//   N = 512    58.2 / 63.4,  839 / 843,  3403 / 3418, 7417 / 7350, 28 100 / 27 530
-// stencils of 27^3 / 100^3, uniform 700 / 4096 / 10^5 / 2 10^5 rows:
-//   N = 32     16.4 / 7.0,   556 / 186,    7.7 / 7.4,   9.0 / 9.2,    62.5 / 23.1,  121 / 45
-//   N = 128    16.9 / 14.5,  592 / 488,    8.0 / 7.5,   9.4 / 11.4,   64.7 / 53.4,  148 / 126
-//   N = 192    22.5 / 20.5,  958 / 796,    9.9 / 7.9,   11.8 / 12.7,  101 / 89,     224 / 197
-//   N = 256    22.1 / 24.2,  951 / 1037,   9.9 / 8.3,   11.7 / 12.7,  113 / 118,    278 / 257
-//   N = 512    36.5 / 42.3,  1701 / 2155,  14.2 / 8.7,  16.9 / 19.0,  260 / 230,    624 / 498
-// ME-TCF, 20 000 nodes: N = 128 31.8 / 29.7, N = 256 36.5 / 42.1, N = 512 63.2 / 70.4; 4096 rows: 10.2 / 18.9, 12.4 / 20.0,
-// 17.5 / 25.9.  MCO: 31.7 / 30.6, 36.8 / 45.8, 62.7 / 76.9; 10.4 / 16.2, 12.5 / 17.9, 17.6 / 25.2.
+// Measured in turn (us, tcgen05 / warp), SR-BCRS; power-law graphs of 5000 / 20 000 / 130 000 / 300 000 / 2^20 / 2^21 nodes:
+//   N = 128    13 / 12,  29 / 21,  137 / 84,   274 / 171,  979 / 715,   2787 / 2082
+//   N = 192    16 / 14,  34 / 26,  184 / 124,  394 / 274,  1709 / 1138, 3929 / 3343
+//   N = 256    18 / 14,  35 / 31,  183 / 154,  395 / 335,  1803 / 1412, 4236 / 4145
+//   N = 512    23 / 21,  56 / 54,  308 / 293,  728 / 664,  3797 / 2985, -
+// stencils of 15^3 / 27^3 / 60^3 / 100^3, uniform 700 / 4096 / 20 000 / 10^5 / 2 10^5 rows:
+//   N = 128    7 / 5,    17 / 13,  126 / 94,   549 / 422,  8 / 6,   9 / 11,   21 / 18,  62 / 48,   122 / 116
+//   N = 192    8 / 7,    23 / 18,  184 / 148,  816 / 674,  10 / 6,  12 / 12,  29 / 18,  90 / 77,   194 / 178
+//   N = 256    8 / 6,    22 / 20,  184 / 184,  974 / 864,  10 / 7,  12 / 13,  29 / 25,  100 / 95,  267 / 229
+//   N = 512    10 / 9,   37 / 36,  327 / 365,  1724 / 2003, 13 / 7, 17 / 17,  47 / 42,  253 / 187, 600 / 451
+// ME-TCF (MCO like it, within a tenth), power-law and uniform:
+//   N = 128    16 / 16,  31 / 27,  151 / 99,   315 / 201,  1123 / 756,  2999 / 2183;   9 / 12, 10 / 17, 23 / 25, 69 / 55,   138 / 112
+//   N = 192    18 / 19,  35 / 32,  201 / 157,  434 / 334,  1658 / 1344, 3999 / 3522;  10 / 12, 12 / 19, 30 / 26, 99 / 89,   208 / 175
+//   N = 256    18 / 18,  36 / 37,  206 / 182,  446 / 386,  1884 / 1644, 4554 / 4232;  10 / 13, 12 / 19, 31 / 33, 106 / 106, 249 / 217
+//   N = 512    24 / 27,  60 / 62,  340 / 348,  822 / 754,  3615 / 3358, -;            14 / 13, 17 / 24, 50 / 53, 241 / 202, 577 / 429
+// stencils: N = 128 7 / 8, 18 / 18, 142 / 119, 619 / 509; 192 8 / 9, 26 / 27, 232 / 197, 1021 / 873; 256 8 / 8, 28 / 29, 261 / 227,
+// 1230 / 1059; 384 10 / 12, 38 / 37, 335 / 338, 1574 / 1674; 512 10 / 12, 42 / 48, 375 / 443, 1901 / 2379.
 static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, bool sidx_aligned) {
     if (tf32x3) return true;                    // compensated products: the warp kernel only
     if (!sidx_aligned || g_tune_sweep == 2) return false;
@@ -356,29 +360,29 @@ static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, 
     if (g_tune_sweep == 0) return true;
     if (g_tune_tma != 0 && fmt == kFmtSrbcrs && plan->d_vals_tf32 != nullptr) return false;
     const bool dense = fmt == kFmtSrbcrs;
-    const int64_t slabs = (N + 127) / 128, work = plan->T * slabs;
+    const int64_t slabs = (N + 127) / 128, T = plan->T, groups = plan->Gw;
     const int64_t block = 128 * sweep_slabs(plan, N), padded = (N + block - 1) / block * block;
     const bool pads = 4 * padded >= 5 * (int64_t)N;   // columns that the tcgen05 kernel's blocks would only pad: a quarter of N and more
-    // A handful of long groups: one warp takes a quarter of a microsecond per tile and twice that for one that it
-    // rebuilds, a tcgen05 block an eighth.  With enough columns the warp kernel has more blocks to deal them to.
-    if (plan->Gw < 4 * sm_count() && plan->T > (dense ? 24 : 16) * plan->Gw)
-        return dense && (N > 128 ? plan->Gw * slabs <= (N > 256 ? 4 : 2) * sm_count() : N <= 64 && plan->Gw > 2 * sm_count());
-    // Bitmaps between 96 and 128 columns: the warp kernel pays for 128, for the expansion of every tile and for rows that
-    // do not start on whole lines (two passes a quarter-warp), and L2 serves either kernel if no column is hot.  N = 100 / 104 /
-    // 112 / 120 / 124, uniform 10^5 x 7 10^4: 72.3 / 76.2, 71.3 / 71.6, 71.5 / 70.5, 71.9 / 75.2, 75.7 / 85.1.  Not so up to 96 (N = 60
-    // 67.9 / 50.6, 92 70.3 / 67.8), at 128 (68.5 / 64.6), on a power-law graph of 300 000 nodes (330 / 317, 328 / 299, 328 / 294,
-    // 331 / 312, 340 / 350), a 60^3 stencil (150 / 149, 148 / 140, 148 / 138, 150 / 147, 156 / 170) and in SR-BCRS (64.5 / 58.8,
-    // N = 124 68.1 / 65.9).
-    if (N <= 128) return !(fmt == kFmtMco && N > 96 && N < 128 && !plan->hub_heavy && !plan->local);
-    if (dense && work <= 150000 && (work <= 15000 || pads || (N <= 256 && !plan->local))) return true;   // too little work for long-lived blocks
-    if (fmt == kFmtMco) return false;
-    // Rows of B a quarter as wide: more of the hubs stay in L2 (2^22 nodes, N = 512: 141 GB through DRAM, the tcgen05 kernel
-    // 157).  24 turns each, quartiles of warp / tcgen05: N = 256 0.94-0.98 with 2^21 nodes, 0.94-0.95 with 3 10^6, 0.98-1.00 with
-    // 2^22; N = 512 0.98-1.00, 0.99-1.01, 1.01-1.02.  At full clocks the last is 24.8 / 26.7 ms; in a run of seconds the 1000 W limit
-    // brings the warp kernel to 1220 MHz and 28.4 ms, the tcgen05 kernel to 1430 MHz and 27.9.  Where it is a tie, the rounding of B decides.
-    if (plan->far_beyond_l2 && dense) return true;
-    if (plan->slab_fits && N > 256) return true;
-    return !plan->local && pads;
+    // A handful of long groups: one warp takes half a microsecond per tile and twice that for one that it
+    // rebuilds, a tcgen05 block an eighth.  With enough columns the warp kernel has more blocks to deal them to, and with very few
+    // groups (uniform 700 rows) neither fills the GPU.
+    if (groups < 4 * sm_count() && T > (dense ? 24 : 16) * groups) {
+        if (!dense) return false;
+        if (N > 128) return groups * slabs <= (N > 256 ? 4 : 2) * sm_count();
+        return N <= 64 ? groups > 2 * sm_count() : 2 * groups <= sm_count();
+    }
+    if (!dense && groups < 9 * sm_count() && T > 16 * groups && (N <= 128 || !pads)) return false;
+    if (N <= 128) return true;
+    const bool wide = N > 256 && !pads;
+    // Full-width rows pay where neighbouring windows share them (60^3 and 100^3 stencil), for tiles that are rebuilt also where the
+    // matrix is small; not where 128 columns of B stay in L2 and all of them do not (10^5 rows: 241 / 202; N = 416 196 / 208).
+    if (plan->local && wide) return dense && T * slabs <= 150000;
+    // Power-law graphs, N = 512, at full clocks and in a run of seconds (tcgen05 / warp, ms): 2^18 nodes 0.72 / 0.61 and 0.76 / 0.70,
+    // 2^19 1.39 / 1.28 and 1.53 / 1.48, 2^20 2.97 / 2.74 and 3.30 / 3.13, 2^22 26.7 / 24.2 and 27.9 / 27.2.  Two slabs of the tcgen05 kernel stay the
+    // plan table's answer between 4 and 12 times the L2, as its test has it.
+    if (dense && wide && plan->nslab == 2 && !plan->far_beyond_l2) return false;
+    if (dense || (plan->slab_fits && N > 448)) return true;
+    return T > (wide ? 250000 : (pads ? 20000 : 40000));
 }
 
 static bool aligned(const void* p, unsigned bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
