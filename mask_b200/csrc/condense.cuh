@@ -68,10 +68,11 @@ __device__ __forceinline__ int block_least(int x, int* word) {
     return __reduce_min_sync(0xffffffffu, lane < THREADS / 32 ? word[lane] : INT_MAX);
 }
 
-constexpr int kMarkMax = 1 << 20;   // most keys a MarkSet holds (its shared memory: 3/16 of a byte per key)
+constexpr int kMarkMax = 1 << 20;   // most keys a MarkSet holds
+constexpr int mark_set_bytes(int keys) { return keys / 8 + keys / 64; }   // bitmap, then `before`
 
-// A bitmap of columns (or other small numbers) in shared memory and what ranks them: 16-bit counts of the marks before every word within
-// its run of 128 words (4096 columns), and the marks before every run.
+// A bitmap of columns (or other small numbers) in shared memory and what ranks them: 16-bit counts of the marks before every four words
+// (128 columns) within their run of 128 words (4096 columns), and the marks before every run.
 struct MarkSet {
     uint32_t* bits;
     uint16_t* before;
@@ -95,7 +96,9 @@ struct MarkSet {
     }
     __device__ __forceinline__ void unmark(int d) { bits[d >> 5] = 0; }
     __device__ __forceinline__ int rank(int d) const {
-        return run_before[d >> 12] + before[d >> 5] + __popc(bits[d >> 5] & ((1u << (d & 31)) - 1u));
+        const ulonglong2 v = reinterpret_cast<const ulonglong2*>(bits)[d >> 7];
+        const unsigned long long below = (1ull << (d & 63)) - 1ull;
+        return run_before[d >> 12] + before[d >> 7] + (d & 64 ? __popcll(v.x) + __popcll(v.y & below) : __popcll(v.x & below));
     }
     // Counts the marks of the whole set (returned to every thread) and prepares rank(); called by all THREADS threads.
     template <int THREADS>
@@ -104,14 +107,13 @@ struct MarkSet {
         __syncthreads();
         for (int r = warp; r < n_runs; r += THREADS / 32) {   // four words a lane
             const uint4 v = reinterpret_cast<const uint4*>(bits)[r * 32 + lane];
-            const int a0 = __popc(v.x), a1 = a0 + __popc(v.y), a2 = a1 + __popc(v.z), c = a2 + __popc(v.w);
+            const int c = __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
             int x = c;
             for (int o = 1; o < 32; o <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, x, o);
                 if (lane >= o) x += y;
             }
-            const int s = x - c;
-            reinterpret_cast<ushort4*>(before)[r * 32 + lane] = make_ushort4((uint16_t)s, (uint16_t)(s + a0), (uint16_t)(s + a1), (uint16_t)(s + a2));
+            before[r * 32 + lane] = (uint16_t)(x - c);
             if (lane == 31) run_before[r] = x;
         }
         __syncthreads();

@@ -9,7 +9,7 @@
 //                  window are contiguous in the CSR.  Windows of up to 1024 entries: one warp sorts them in
 //                  registers (bitonic network over 1..32 keys a lane, key = column << 10 | entry) and
 //                  numbers the distinct ones.  Larger windows: one block marks the columns in a bitmap in
-//                  shared memory, 2^20 columns at a time, and ranks every entry by a prefix popcount, which
+//                  shared memory, 2^19 columns at a time, and ranks every entry by a prefix popcount, which
 //                  costs the same whatever the row lengths.  Rows that are not strictly ascending or columns
 //                  outside [0, K) raise an error flag.
 //   2. tiles       ceil(distinct / 8) per window, exclusive scan -> val_soff, total T; the scan also notes
@@ -21,7 +21,8 @@
 //                  histogram, 128-bit mask), scan the run lengths and place the entries.
 //
 // Measured on a power-law graph with 2^20 nodes (17.1 M entries, 1.97 M tiles; one read of the CSR and one
-// write of the packed arrays is 0.2 ms at copy speed): condense 0.37 ms, scan 0.01, SR-BCRS fill 0.32; a binary
+// write of the packed arrays is 0.2 ms at copy speed): condense 0.15 ms and, overlapping, 0.09 and 0.12 for large windows, scan 0.01,
+// SR-BCRS fill 0.32; a binary
 // search of every entry in its 15 sibling rows, two more scans and a scatter into cleared tiles took 2.3 ms.
 #include <algorithm>
 
@@ -79,10 +80,12 @@ constexpr int kSortIdxBits = 10;
 constexpr int kHubMin = 8192;                     // larger windows are shared by the blocks of a cluster
 constexpr int kBigThreads = 512;
 constexpr int kBigKeep = kHubMin / kBigThreads;
-constexpr int kHubThreads = 1024;
+constexpr int kHubThreads = 512;
+constexpr int kHubKeep = 8;                       // entries a thread of them keeps in registers
+static_assert(kHubThreads == 32 * kWinRows, "a warp for each row");
 constexpr int kBigBits = 1 << 19;                 // columns marked at a time: two blocks per SM
 constexpr int kHubBlocks = 8;
-constexpr int kHubBits = kMarkMax;                // most columns marked at a time by one block of a cluster
+constexpr int kHubBits = 1 << 19;                 // most columns marked at a time by one block of a cluster: two blocks per SM
 
 // One window of n <= 32 E entries: sorts (column, entry), numbers the distinct columns, writes every entry's
 // number to pos and the distinct columns to cols; returns how many there are.
@@ -133,6 +136,13 @@ __device__ __forceinline__ int entry_faults(const int32_t* __restrict__ colind, 
     return bad;
 }
 
+// Which of the 32 entries from e on begin a row, for a whole warp; bound: where row `lane` of the window begins (lanes 0..15).
+// (Comparing every entry with all 16 cost condense_big_kernel 139 us where this and no work behind a window's end cost 123.)
+__device__ __forceinline__ uint32_t row_starts(int bound, int e) {
+    const uint32_t at = (uint32_t)(bound - e);
+    return __reduce_or_sync(0xffffffffu, (threadIdx.x & 31) < kWinRows && at < 32u ? 1u << at : 0u);
+}
+
 // One warp per window; windows above kSortMax entries go to the list of the bitmap kernel.
 template <typename Key>
 __global__ void __launch_bounds__(128) condense_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
@@ -158,10 +168,8 @@ __global__ void __launch_bounds__(128) condense_kernel(const int32_t* __restrict
     int bad = 0;
     for (int j = 0; j < n; j += 32) {
         const int e = base + j + lane;
-        bool start = false;
-#pragma unroll
-        for (int i = 0; i < kWinRows; i++) start |= e == __shfl_sync(0xffffffffu, bound, i);
-        if (j + lane < n) bad |= entry_faults(colind, e, __ldg(colind + e), K, start);
+        const uint32_t starts = row_starts(bound, base + j);
+        if (j + lane < n) bad |= entry_faults(colind, e, __ldg(colind + e), K, starts >> lane & 1u);
     }
     if (bad) atomicOr(status, bad);
     int d = 0;
@@ -196,6 +204,7 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
         if (tid <= kWinRows) bound[tid] = (rowptr + w * kWinRows)[min(tid, M - w * kWinRows)];
         __syncthreads();
         const int e0 = bound[0], n = bound[kWinRows] - e0;
+        const int mine = bound[tid & (kWinRows - 1)];
         int total = 0, bad = 0;
         int c[kBigKeep];
 #pragma unroll
@@ -205,11 +214,10 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
         }
 #pragma unroll
         for (int i = 0; i < kBigKeep; i++) {
+            if (i * kBigThreads >= n) break;
             const int e = e0 + i * kBigThreads + tid;
-            bool start = false;
-#pragma unroll
-            for (int r = 0; r < kWinRows; r++) start |= e == bound[r];
-            if (e - e0 < n) bad |= entry_faults(colind, e, c[i], K, start);
+            const uint32_t starts = row_starts(mine, e - (tid & 31));
+            if (e - e0 < n) bad |= entry_faults(colind, e, c[i], K, starts >> (tid & 31) & 1u);
             if (c[i] >= K) c[i] = -1;
         }
         // the smallest column from `from` on, INT_MAX if there is none
@@ -224,20 +232,26 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
         for (int c0 = few ? 0 : least_from(0); c0 < K;) {
             const int span = min(kBigBits, K - c0);
 #pragma unroll
-            for (int i = 0; i < kBigKeep; i++)
+            for (int i = 0; i < kBigKeep; i++) {
+                if (i * kBigThreads >= n) break;
                 if (c[i] >= c0 && c[i] - c0 < span) marks.mark(c[i] - c0);
+            }
             const int all = marks.count<kBigThreads>(warp_sum);
 #pragma unroll
-            for (int i = 0; i < kBigKeep; i++)
+            for (int i = 0; i < kBigKeep; i++) {
+                if (i * kBigThreads >= n) break;
                 if (c[i] >= c0 && c[i] - c0 < span) {
                     const int q = total + marks.rank(c[i] - c0);
                     pos[e0 + i * kBigThreads + tid] = q;
                     cols[e0 + q] = c[i];
                 }
+            }
             __syncthreads();
 #pragma unroll
-            for (int i = 0; i < kBigKeep; i++)
+            for (int i = 0; i < kBigKeep; i++) {
+                if (i * kBigThreads >= n) break;
                 if (c[i] >= c0 && c[i] - c0 < span) marks.unmark(c[i] - c0);
+            }
             total += all;
             __syncthreads();
             if (span == K - c0) break;
@@ -253,10 +267,12 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
 // columns -- cut at the eighths of the window's longest row, so that the ranges hold about as many entries each --
 // which is a run of entries in each of the 16 rows, found by a 32-way search; the blocks exchange their counts
 // through distributed shared memory and rank what they marked themselves.  A range wider than kHubBits is taken in
-// parts (marked once to count, once more to rank), each from the smallest column that is left.  With one block per
-// window the 150 000 entries of the largest window of a power-law graph with 2^20 nodes took 0.3 ms while the rest of
-// the GPU had finished.
-__global__ void __cluster_dims__(kHubBlocks, 1, 1) __launch_bounds__(kHubThreads, 1)
+// parts (marked once to count, once more to rank), each from the smallest column that is left.  Up to kHubKeep entries a thread
+// are read once and kept.  A window takes 12 us, most of it waiting, whether a block has one entry a thread or five, so what
+// counts is how many clusters run at a time: with marks for 2^20 columns a block filled an SM, and ten clusters of 8 found
+// room (137 such windows of a power-law graph with 2^20 nodes: 165 us, with two blocks an SM 81 to 102; with marks for 2^18 most
+// ranges are taken in parts: 255).  With one block per window the 150 000 entries of the largest took 0.3 ms.
+__global__ void __cluster_dims__(kHubBlocks, 1, 1) __launch_bounds__(kHubThreads, 2)
 condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M, int32_t K, int32_t span,
                     int32_t* __restrict__ pos, int32_t* __restrict__ cols, int32_t* __restrict__ distinct,
                     const int32_t* __restrict__ hub_list, int32_t* __restrict__ status) {
@@ -283,12 +299,12 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
         __syncthreads();
         const int e0 = bound[0], n = bound[kWinRows] - e0;
         int bad = 0;
-        for (uint32_t j = me * kHubThreads + tid; j < (uint32_t)n; j += kHubBlocks * kHubThreads) {
-            const int e = e0 + (int)j;
-            bool start = false;
-#pragma unroll
-            for (int r = 0; r < kWinRows; r++) start |= e == bound[r];
-            bad |= entry_faults(colind, e, __ldg(colind + e), K, start);
+        const int row_begin = bound[lane & (kWinRows - 1)];
+#pragma unroll 4
+        for (uint32_t j0 = me * kHubThreads + warp * 32; j0 < (uint32_t)n; j0 += kHubBlocks * kHubThreads) {
+            const int e = e0 + (int)j0 + lane;
+            const uint32_t starts = row_starts(row_begin, e0 + (int)j0);
+            if (j0 + lane < (uint32_t)n) bad |= entry_faults(colind, e, __ldg(colind + e), K, starts >> lane & 1u);
         }
         if (bad) atomicOr(status, bad);
         int longest = 0;
@@ -300,18 +316,26 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
             return max(0, min(K, c));
         };
         const int c_lo = splitter(me), c_hi = max(c_lo, splitter(me + 1));
-        {   // warp: row warp % 16, lower or upper end
-            const int r = warp & (kWinRows - 1), hi = warp >> 4, key = hi ? c_hi : c_lo;
-            int p = bound[r], left = bound[r + 1] - p;
-            while (left > 0) {
-                const int stride = (left + 31) >> 5, probe = min((lane + 1) * stride, left);
-                const bool below = __ldg(colind + p + probe - 1) < key;
-                const int hits = __popc(__ballot_sync(0xffffffffu, below));   // the probes that hit come first
-                const int step = hits == 32 ? left : min(hits * stride, left);
-                p += step;
-                left = hits == 32 ? 0 : min(stride - 1, left - step);
+        {   // a row for each warp, both ends at once
+            int p[2] = {bound[warp], bound[warp]}, left[2] = {bound[warp + 1] - p[0], bound[warp + 1] - p[0]};
+            while (left[0] > 0 || left[1] > 0) {
+                int stride[2], probe[2];
+                bool below[2];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    stride[h] = (left[h] + 31) >> 5;
+                    probe[h] = min((lane + 1) * stride[h], left[h]);
+                    below[h] = left[h] > 0 && __ldg(colind + p[h] + probe[h] - 1) < (h ? c_hi : c_lo);
+                }
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int hits = __popc(__ballot_sync(0xffffffffu, below[h]));   // the probes that hit come first
+                    const int step = hits == 32 ? left[h] : min(hits * stride[h], left[h]);
+                    p[h] += step;
+                    left[h] = hits == 32 ? 0 : max(0, min(stride[h] - 1, left[h] - step));
+                }
             }
-            if (lane == 0) cut[hi][r] = p;
+            if (lane < 2) cut[lane][warp] = p[lane];
         }
         __syncthreads();
         if (tid == 0) {
@@ -334,9 +358,15 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
         // columns of [c0, c0 + part); others only occur in the list when rows are not ascending, which is an error anyway
         auto mark_part = [&](int c0, int part) {
             marks.n_runs = (part + 4095) / 4096;
-            for (int i0 = 0; i0 < m; i0 += kHubThreads) {
-                const int i = i0 + tid, c = i < m ? __ldg(colind + entry(i)) : -1;
-                marks.mark_ascending(c >= c0 && c - c0 < part ? c - c0 : -1);
+            for (int i0 = 0; i0 < m; i0 += 4 * kHubThreads) {
+                int c[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int i = i0 + k * kHubThreads + tid;
+                    c[k] = i < m ? __ldg(colind + entry(i)) : -1;
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) marks.mark_ascending(c[k] >= c0 && c[k] - c0 < part ? c[k] - c0 : -1);
             }
         };
         const bool whole = c_hi - c_lo <= span;
@@ -344,17 +374,42 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
         auto unmark_part = [&](int c0, int part) {
             int behind = INT_MAX;
             __syncthreads();
-            for (int i = tid; i < m; i += kHubThreads) {
-                const int c = __ldg(colind + entry(i));
-                if (c < c0) continue;
-                if (c - c0 < part) marks.unmark(c - c0);
-                else behind = min(behind, c);
+            if (whole) {   // every word that can be marked
+                for (int i = tid; i < marks.n_runs * 32; i += kHubThreads) reinterpret_cast<uint4*>(marks.bits)[i] = make_uint4(0u, 0u, 0u, 0u);
+            } else {
+#pragma unroll 4
+                for (int i = tid; i < m; i += kHubThreads) {
+                    const int c = __ldg(colind + entry(i));
+                    if (c < c0) continue;
+                    if (c - c0 < part) marks.unmark(c - c0);
+                    else behind = min(behind, c);
+                }
             }
             __syncthreads();
             return whole ? c_hi : block_least<kHubThreads>(behind, warp_sum);
         };
+        // Few entries, in one part: read once and kept.
+        const bool kept = whole && m <= kHubKeep * kHubThreads;
+        int ke[kHubKeep], kc[kHubKeep];
         int mine = 0;
-        for (int c0 = c_lo; c0 < c_hi;) {
+        if (kept) {
+#pragma unroll
+            for (int k = 0; k < kHubKeep; k++) {
+                const int i = k * kHubThreads + tid;
+                ke[k] = i < m ? entry(i) : -1;
+            }
+#pragma unroll
+            for (int k = 0; k < kHubKeep; k++) {
+                kc[k] = ke[k] >= 0 ? __ldg(colind + ke[k]) : -1;
+                if (kc[k] < c_lo || kc[k] >= c_hi) ke[k] = -1;
+            }
+            marks.n_runs = (c_hi - c_lo + 4095) / 4096;
+#pragma unroll
+            for (int k = 0; k < kHubKeep; k++)
+                if (k * kHubThreads < m) marks.mark_ascending(ke[k] >= 0 ? kc[k] - c_lo : -1);
+            mine = marks.count<kHubThreads>(warp_sum);
+        }
+        for (int c0 = kept ? c_hi : c_lo; c0 < c_hi;) {
             const int part = min(span, c_hi - c0);
             mark_part(c0, part);
             mine += marks.count<kHubThreads>(warp_sum);
@@ -368,21 +423,43 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
             total += v;
             if (i < me) ahead += v;
         }
-        for (int c0 = c_lo; c0 < c_hi;) {
+        if (kept) {
+#pragma unroll
+            for (int k = 0; k < kHubKeep; k++)
+                if (ke[k] >= 0) {
+                    const int q = ahead + marks.rank(kc[k] - c_lo);
+                    pos[ke[k]] = q;
+                    cols[e0 + q] = kc[k];
+                }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < kHubKeep; k++)
+                if (ke[k] >= 0) marks.unmark(kc[k] - c_lo);
+            __syncthreads();
+        }
+        for (int c0 = kept ? c_hi : c_lo; c0 < c_hi;) {
             const int part = min(span, c_hi - c0);
             int here = mine;
             if (!whole) {
                 mark_part(c0, part);
                 here = marks.count<kHubThreads>(warp_sum);
             }
-#pragma unroll 2
-            for (int i = tid; i < m; i += kHubThreads) {
-                const int e = entry(i), c = __ldg(colind + e);
-                if (c >= c0 && c - c0 < part) {
-                    const int q = ahead + marks.rank(c - c0);
-                    pos[e] = q;
-                    cols[e0 + q] = c;
+            for (int i0 = 0; i0 < m; i0 += 4 * kHubThreads) {
+                int e[4], c[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int i = i0 + k * kHubThreads + tid;
+                    e[k] = i < m ? entry(i) : -1;
                 }
+#pragma unroll
+                for (int k = 0; k < 4; k++) c[k] = e[k] >= 0 ? __ldg(colind + e[k]) : -1;
+#pragma unroll
+                for (int k = 0; k < 4; k++)
+                    if (c[k] >= c0 && c[k] - c0 < part) {
+                        const int q = ahead + marks.rank(c[k] - c0);
+                        pos[e[k]] = q;
+                        cols[e0 + q] = c[k];
+                    }
             }
             c0 = unmark_part(c0, part);
             ahead += here;
@@ -788,17 +865,17 @@ extern "C" int mask_pack_analyze(const int32_t* d_rowptr, const int32_t* d_colin
     MASK_CUDA_TRY(cudaGetLastError());
     if (nnz > kHubMin) {
         const int span = (int)std::min<int64_t>(((int64_t)K + 4095) / 4096 * 4096, kHubBits);   // columns a block marks at a time
-        const int smem = span / 8 + span / 16;
+        const int smem = mark_set_bytes(span);
         static std::atomic<uint64_t> opted_in;
-        const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(condense_hub_kernel), kHubBits / 8 + kHubBits / 16, opted_in);
+        const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(condense_hub_kernel), mark_set_bytes(kHubBits), opted_in);
         if (rc != MASK_OK) return rc;
         const int64_t most = std::min<int64_t>(W, nnz / kHubMin);
-        condense_hub_kernel<<<(unsigned)(kHubBlocks * std::min<int64_t>(most, std::max(1, sm_count() / kHubBlocks))), kHubThreads, smem, st>>>(
+        condense_hub_kernel<<<(unsigned)(kHubBlocks * std::min<int64_t>(most, std::max(1, 2 * sm_count() / kHubBlocks))), kHubThreads, smem, st>>>(
             d_rowptr, d_colind, M, K, span, s.pos, s.cols, s.distinct, s.hub_list, s.status);
         MASK_CUDA_TRY(cudaGetLastError());
     }
     if (nnz > kSortMax) {
-        constexpr int kSmem = kBigBits / 8 + kBigBits / 16;
+        constexpr int kSmem = mark_set_bytes(kBigBits);
         static std::atomic<uint64_t> opted_in;
         int rc = opt_in_shared_memory(reinterpret_cast<const void*>(condense_big_kernel), kSmem, opted_in);
         if (rc != MASK_OK) return rc;

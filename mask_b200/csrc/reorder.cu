@@ -817,7 +817,7 @@ int order_rcm_device(const int32_t* rowptr, const int32_t* colind, int32_t M, in
                                                                             flags + 1);
     MASK_CUDA_TRY(cudaGetLastError());
     if (n_edges > kAdjSortMax) {
-        constexpr int kSmem = kLongBits / 8 + kLongBits / 16;
+        constexpr int kSmem = mark_set_bytes(kLongBits);
         MASK_CUDA_TRY(cudaFuncSetAttribute(sort_long_adjacency_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
         const int64_t most = std::min<int64_t>(n_edges / kAdjSortMax, 2 * sm_count());
         sort_long_adjacency_kernel<<<(unsigned)most, 512, kSmem, st>>>(ptr, col, M, arr(kStarts), arr(kRank), arr(kOutPtr), adj, arr(kLong), flags + 1);
