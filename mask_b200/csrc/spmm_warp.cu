@@ -376,8 +376,13 @@ static constexpr int warp_blocks_per_sm(int nq, int depth, bool comp) {
 // round of long ones doubles the time).  The longest step that fits comes first, then the fewest columns that pad no
 // more than the widest block would.  us, one tile and all columns a step / as chosen here: uniform 16 384
 // rows, N = 64 18.6 / 9.1, N = 128 20.6 / 13.6; 15^3 stencil, N = 64 7.2 / 5.2, N = 256 10.7 / 6.8; power-law graph
-// of 20 000 nodes, N = 64 21.3 / 15.2.  With four times the resident blocks, long steps lose a quarter to a half.
-static void choose_warp_shape(int64_t groups, int64_t T, int N, bool comp, int tuned_nq, int* nq_out, int* depth_out) {
+// of 20 000 nodes, N = 64 21.3 / 15.2.  With four times the resident blocks, long steps lose a quarter to a half, but for blocks of
+// 64 columns: 13 of them with two tiles a step finish a long window sooner than 24 with one, and that is what a graph of
+// middling size waits for (SR-BCRS / ME-TCF / MCO, N = 64, us; one tile a step, two: 130 000 nodes 64 / 91 / 94, 58 / 73 / 69; 300 000 nodes
+// 123 / 162 / 161, 115 / 148 / 139; 600 000 nodes 228 / 296 / 296, 225 / 287 / 270; uniform 10^5 rows 35 / 43 / 41, 31 / 41 / 38; not with
+// more tiles, 2^20 nodes 413 / 528 in SR-BCRS and ME-TCF, 431 / 538, uniform 2 10^5 rows of 20 102, 111, nor with a stencil's short windows, 59, 62).
+static void choose_warp_shape(const mask_plan* plan, bool dense, int N, bool comp, int tuned_nq, int* nq_out, int* depth_out) {
+    const int64_t groups = plan->Gw, T = plan->T;
     const int slabs = (N + 127) / 128, widest = (N + 32 * slabs - 1) / (32 * slabs);
     const bool tuned = tuned_nq >= 1 && tuned_nq <= 4;
     for (int depth = 2; depth >= 0; depth--) {
@@ -393,7 +398,7 @@ static void choose_warp_shape(int64_t groups, int64_t T, int N, bool comp, int t
         }
     }
     *nq_out = tuned ? tuned_nq : widest;
-    *depth_out = 0;
+    *depth_out = *nq_out == 2 && !comp && !plan->local && T <= (dense ? 400000 : 1000000) ? 1 : 0;
 }
 
 template <int NQ, int DEPTH, int FMT, bool GUARD, bool COMP>
@@ -432,7 +437,7 @@ int launch_spmm_warp(const mask_plan* plan, const SpmmArgs& a_in, cudaStream_t s
     a.n_warp_first = plan->warp_first;
     a.n_frag = plan->F;
     int nq, depth;
-    choose_warp_shape(plan->Gw, plan->T, a.N, a.tf32x3, tuned_nq, &nq, &depth);
+    choose_warp_shape(plan, FMT == kFmtSrbcrs, a.N, a.tf32x3, tuned_nq, &nq, &depth);
     if constexpr (FMT == kFmtSrbcrs)
         if (a.tf32x3) return launch_warp_shape<FMT, true>(plan, a, st, nq, depth);
     return launch_warp_shape<FMT, false>(plan, a, st, nq, depth);
