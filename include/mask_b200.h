@@ -322,8 +322,8 @@ int mask_plan_export(const mask_plan* plan, int32_t* frag_offset, int32_t* frag_
 /* OR-able into `epilogue` (SR-BCRS only): three TF32 products per MMA -- hi(A)*hi(B) plus the
  * residual terms lo(A)*hi(B) and hi(A)*lo(B) -- which brings the result to FP32-level accuracy
  * (the reference compiler's compensated MMA, python/sparsene/op_gen/nvir/templates.py:53-76, on
- * by default in its Format-DSL bridge).  Runs on the warp-level kernel; 0.50 ms against 0.30 ms on
- * a 200 000-node power-law graph at N = 256, 0.17 against 0.11 at N = 64. */
+ * by default in its Format-DSL bridge).  Runs on the warp-level kernel; 0.59 ms against 0.33 ms on
+ * a 300 000-node power-law graph at N = 256, 0.18 against 0.12 at N = 64. */
 #define MASK_NUMERICS_TF32X3 0x100
 
 int mask_spmm_srbcrs(const mask_plan* plan, const int32_t* d_val_soff, const int32_t* d_val_sidx,
