@@ -21,7 +21,7 @@
 //                  histogram, 128-bit mask), scan the run lengths and place the entries.
 //
 // Measured on a power-law graph with 2^20 nodes (17.1 M entries, 1.97 M tiles; one read of the CSR and one
-// write of the packed arrays is 0.2 ms at copy speed): condense 0.15 ms and, overlapping, 0.09 and 0.12 for large windows, scan 0.01,
+// write of the packed arrays is 0.2 ms at copy speed): condense 0.13 ms and, overlapping, 0.09 and 0.12 for large windows, scan 0.01,
 // SR-BCRS fill 0.32; a binary
 // search of every entry in its 15 sibling rows, two more scans and a scatter into cleared tiles took 2.3 ms.
 #include <algorithm>
@@ -143,16 +143,18 @@ __device__ __forceinline__ uint32_t row_starts(int bound, int e) {
     return __reduce_or_sync(0xffffffffu, (threadIdx.x & 31) < kWinRows && at < 32u ? 1u << at : 0u);
 }
 
-// One warp per window; windows above kSortMax entries go to the list of the bitmap kernel.
+// One warp, which is a block, per window; windows above kSortMax entries go to the list of the bitmap kernel.  What bounds it is the
+// latency of a warp's loads and of its sort, so as many warps as registers allow (power-law graph with 2^20 nodes: four warps a
+// block, 20 of 96 registers an SM, 148 us; 24 single ones of 80 registers 135, 28 of 72 128; the 64-bit keys of more than 2^22
+// columns would spill).
 template <typename Key>
-__global__ void __launch_bounds__(128) condense_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
+__global__ void __launch_bounds__(32, sizeof(Key) == 4 ? 28 : 12) condense_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind,
                                                        int32_t M, int32_t K, int32_t W, int32_t* __restrict__ pos,
                                                        int32_t* __restrict__ cols, int32_t* __restrict__ rows,
                                                        int32_t* __restrict__ distinct, int32_t* __restrict__ big_list,
                                                        int32_t* __restrict__ hub_list, int32_t* __restrict__ status) {
-    __shared__ uint16_t slot_pos[4][kSortMax];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int w = blockIdx.x * 4 + warp;
+    __shared__ uint16_t slot_pos[kSortMax];
+    const int lane = threadIdx.x, w = blockIdx.x;
     if (w >= W) return;
     const int r0 = w * kWinRows;
     const int bound = __ldg(rowptr + r0 + min(min(lane, kWinRows), M - r0));   // lane i: where row i of the window begins
@@ -173,12 +175,12 @@ __global__ void __launch_bounds__(128) condense_kernel(const int32_t* __restrict
     }
     if (bad) atomicOr(status, bad);
     int d = 0;
-    if (n > 512) d = condense_warp<32, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
-    else if (n > 256) d = condense_warp<16, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
-    else if (n > 128) d = condense_warp<8, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
-    else if (n > 64) d = condense_warp<4, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
-    else if (n > 32) d = condense_warp<2, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
-    else if (n > 0) d = condense_warp<1, Key>(colind + base, n, lane, slot_pos[warp], pos + base, cols + base);
+    if (n > 512) d = condense_warp<32, Key>(colind + base, n, lane, slot_pos, pos + base, cols + base);
+    else if (n > 256) d = condense_warp<16, Key>(colind + base, n, lane, slot_pos, pos + base, cols + base);
+    else if (n > 128) d = condense_warp<8, Key>(colind + base, n, lane, slot_pos, pos + base, cols + base);
+    else if (n > 64) d = condense_warp<4, Key>(colind + base, n, lane, slot_pos, pos + base, cols + base);
+    else if (n > 32) d = condense_warp<2, Key>(colind + base, n, lane, slot_pos, pos + base, cols + base);
+    else if (n > 0) d = condense_warp<1, Key>(colind + base, n, lane, slot_pos, pos + base, cols + base);
     if (lane == 0) distinct[w] = d;
 }
 
@@ -859,9 +861,9 @@ extern "C" int mask_pack_analyze(const int32_t* d_rowptr, const int32_t* d_colin
     MASK_CUDA_TRY(cudaMemsetAsync(s.status, 0, 64, st));
     // a key is the column and the entry's index within the window
     if (K <= (1 << (32 - kSortIdxBits)))
-        condense_kernel<uint32_t><<<blocks_for(W, 4), 128, 0, st>>>(d_rowptr, d_colind, M, K, W, s.pos, s.cols, s.rows, s.distinct, s.big_list, s.hub_list, s.status);
+        condense_kernel<uint32_t><<<(unsigned)W, 32, 0, st>>>(d_rowptr, d_colind, M, K, W, s.pos, s.cols, s.rows, s.distinct, s.big_list, s.hub_list, s.status);
     else
-        condense_kernel<unsigned long long><<<blocks_for(W, 4), 128, 0, st>>>(d_rowptr, d_colind, M, K, W, s.pos, s.cols, s.rows, s.distinct, s.big_list, s.hub_list, s.status);
+        condense_kernel<unsigned long long><<<(unsigned)W, 32, 0, st>>>(d_rowptr, d_colind, M, K, W, s.pos, s.cols, s.rows, s.distinct, s.big_list, s.hub_list, s.status);
     MASK_CUDA_TRY(cudaGetLastError());
     if (nnz > kHubMin) {
         const int span = (int)std::min<int64_t>(((int64_t)K + 4095) / 4096 * 4096, kHubBits);   // columns a block marks at a time
