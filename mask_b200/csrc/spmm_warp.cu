@@ -30,6 +30,7 @@
 // it covers when rows do not start on 128-byte lines halves the passes, and cost more in instructions than it
 // saved: N = 100 84 -> 110 us.)
 #include "spmm_common.cuh"
+#include "tile_index.h"
 
 namespace mask {
 
@@ -142,10 +143,11 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
             for (int i = 0; i < 4; i++) acc[q][j][i] = 0.f;
 
     // ---- copies ------------------------------------------------------------------------------------------
+    static_assert(ids_before_tile(1) == kTileCols, "");
     const int32_t* idp = p.val_sidx + (int64_t)t0 * kTileCols + lane;
     auto load_ids = [&](int (&id)[I::kRegs], int tile) {
 #pragma unroll
-        for (int i = 0; i < I::kRegs; i++) id[i] = tile + 4 * i + (lane >> 3) < n_tiles ? __ldg(idp + (tile + 4 * i) * kTileCols) : 0;
+        for (int i = 0; i < I::kRegs; i++) id[i] = tile + 4 * i + (lane >> 3) < n_tiles ? __ldg(idp + ids_before_tile(tile + 4 * i)) : 0;
     };
     auto load_runs = [&](int2& run, int tile) {
         if (lane < I::kTiles && tile + lane < n_tiles)
