@@ -85,7 +85,9 @@ constexpr int kHubKeep = 8;                       // entries a thread of them ke
 static_assert(kHubThreads == 32 * kWinRows, "a warp for each row");
 constexpr int kBigBits = 1 << 19;                 // columns marked at a time: two blocks per SM
 constexpr int kHubBlocks = 8;
-constexpr int kHubBits = 1 << 19;                 // most columns marked at a time by one block of a cluster: two blocks per SM
+constexpr int kHubBits = 1 << 19;                 // columns marked at a time by one block of a cluster: two blocks per SM
+constexpr int kHubBitsWide = 1 << 20;             // the same where eight of those do not cover K: one block per SM
+static_assert(kHubBitsWide <= kMarkMax, "");
 
 // One window of n <= 32 E entries: sorts (column, entry), numbers the distinct columns, writes every entry's
 // number to pos and the distinct columns to cols; returns how many there are.
@@ -266,14 +268,18 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
 }
 
 // Windows of more than kHubMin entries, dealt to clusters of kHubBlocks blocks.  Every block takes a range of
-// columns -- cut at the eighths of the window's longest row, so that the ranges hold about as many entries each --
-// which is a run of entries in each of the 16 rows, found by a 32-way search; the blocks exchange their counts
-// through distributed shared memory and rank what they marked themselves.  A range wider than kHubBits is taken in
-// parts (marked once to count, once more to rank), each from the smallest column that is left.  Up to kHubKeep entries a thread
+// columns -- cut at the eighths of the window's longest row, so that the ranges hold about as many entries each, but no wider than
+// a block's marks where eight of those cover K -- which is a run of entries in each of the 16 rows, found by a 32-way search; the blocks
+// exchange their counts through distributed shared memory and rank what they marked themselves.  A range wider than the marks is taken
+// in parts (marked once to count, once more to rank), each from the smallest column that is left.  Up to kHubKeep entries a thread
 // are read once and kept.  A window takes 12 us, most of it waiting, whether a block has one entry a thread or five, so what
 // counts is how many clusters run at a time: with marks for 2^20 columns a block filled an SM, and ten clusters of 8 found
 // room (137 such windows of a power-law graph with 2^20 nodes: 165 us, with two blocks an SM 81 to 102; with marks for 2^18 most
 // ranges are taken in parts: 255).  With one block per window the 150 000 entries of the largest took 0.3 ms.
+// Where eight marks of 2^19 columns do not cover K, parts cost more than the second block is worth.  Condensing in all, ranges at the
+// eighths alone and 2^19 columns always / as here: power-law graphs of 2^20 nodes 369 / 374 us, 2^21 1600 / 1020, 2^22 4560 / 3030, 2^23
+// 13 800 / 10 200, 2^22 and twice the degree 12 000 / 6020; 200 windows of 12 000 / 30 000 / 100 000 entries spread over 2^20 columns
+// 122 / 130, 197 / 182, 502 / 505; over 2^22 262 / 140, 456 / 193, 1197 / 540; over 2^23 367 / 249, 652 / 341, 1675 / 977.
 __global__ void __cluster_dims__(kHubBlocks, 1, 1) __launch_bounds__(kHubThreads, 2)
 condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M, int32_t K, int32_t span,
                     int32_t* __restrict__ pos, int32_t* __restrict__ cols, int32_t* __restrict__ distinct,
@@ -281,7 +287,7 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int run_before[kHubBits / 4096];
+    __shared__ int run_before[kHubBitsWide / 4096];
     __shared__ int bound[kWinRows + 1];
     __shared__ int cut[2][kWinRows];           // first entry of the row in this block's columns, first behind them
     __shared__ int first[kWinRows + 1];        // list index of the row's first entry
@@ -313,11 +319,17 @@ condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restric
         for (int r = 1; r < kWinRows; r++)
             if (bound[r + 1] - bound[r] > bound[longest + 1] - bound[longest]) longest = r;
         const int at = bound[longest], len = bound[longest + 1] - at;   // len >= 512: the window has more than 8192 entries
-        auto splitter = [&](int i) {
-            const int c = i == 0 ? 0 : (i == kHubBlocks ? K : __ldg(colind + at + (int)((int64_t)len * i / kHubBlocks)));
-            return max(0, min(K, c));
-        };
-        const int c_lo = splitter(me), c_hi = max(c_lo, splitter(me + 1));
+        const bool cover = K <= kHubBlocks * span;   // then no range is wider than a span
+        int eighth[kHubBlocks];
+#pragma unroll
+        for (int i = 1; i <= kHubBlocks; i++) eighth[i - 1] = i == kHubBlocks ? K : min(K, __ldg(colind + at + (int)((int64_t)len * i / kHubBlocks)));
+        int c_lo = 0, c_hi = 0;
+#pragma unroll
+        for (int i = 1, c = 0; i <= kHubBlocks; i++) {
+            if (i == me + 1) c_lo = c;
+            c = max(c, cover ? max(K - (kHubBlocks - i) * span, min(eighth[i - 1], c + span)) : eighth[i - 1]);
+            if (i == me + 1) c_hi = c;
+        }
         {   // a row for each warp, both ends at once
             int p[2] = {bound[warp], bound[warp]}, left[2] = {bound[warp + 1] - p[0], bound[warp + 1] - p[0]};
             while (left[0] > 0 || left[1] > 0) {
@@ -866,13 +878,14 @@ extern "C" int mask_pack_analyze(const int32_t* d_rowptr, const int32_t* d_colin
         condense_kernel<unsigned long long><<<(unsigned)W, 32, 0, st>>>(d_rowptr, d_colind, M, K, W, s.pos, s.cols, s.rows, s.distinct, s.big_list, s.hub_list, s.status);
     MASK_CUDA_TRY(cudaGetLastError());
     if (nnz > kHubMin) {
-        const int span = (int)std::min<int64_t>(((int64_t)K + 4095) / 4096 * 4096, kHubBits);   // columns a block marks at a time
+        const int most_bits = K <= kHubBlocks * kHubBits ? kHubBits : kHubBitsWide;
+        const int span = (int)std::min<int64_t>(((int64_t)K + 4095) / 4096 * 4096, most_bits);   // columns a block marks at a time
         const int smem = mark_set_bytes(span);
         static std::atomic<uint64_t> opted_in;
-        const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(condense_hub_kernel), mark_set_bytes(kHubBits), opted_in);
+        const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(condense_hub_kernel), mark_set_bytes(kHubBitsWide), opted_in);
         if (rc != MASK_OK) return rc;
         const int64_t most = std::min<int64_t>(W, nnz / kHubMin);
-        condense_hub_kernel<<<(unsigned)(kHubBlocks * std::min<int64_t>(most, std::max(1, 2 * sm_count() / kHubBlocks))), kHubThreads, smem, st>>>(
+        condense_hub_kernel<<<(unsigned)(kHubBlocks * std::min<int64_t>(most, std::max(1, (most_bits == kHubBits ? 2 : 1) * sm_count() / kHubBlocks))), kHubThreads, smem, st>>>(
             d_rowptr, d_colind, M, K, span, s.pos, s.cols, s.distinct, s.hub_list, s.status);
         MASK_CUDA_TRY(cudaGetLastError());
     }

@@ -27,7 +27,7 @@ def _window(n, K, hub, seed):
 
 
 # sizes at which a window is sorted with more registers, ranked in one block's bitmap, shared by a cluster; key
-# width changes at 2^22 columns, bitmaps cover 2^19 (block) and 2^20 (block of a cluster) columns at a time
+# width changes at 2^22 columns, a block's bitmap covers 2^19 columns at a time (in a cluster 2^20 beyond 2^22 columns)
 @pytest.mark.parametrize("K", [3000, 600_000, 2_200_000, 4_300_000])
 @pytest.mark.parametrize("hub", [False, True])
 def test_pack_window_sizes(oracle_mod, K, hub):
@@ -42,6 +42,51 @@ def test_pack_window_sizes(oracle_mod, K, hub):
     _check_srbcrs(engine.pack_srbcrs(rp, ci, va, m.M, m.K), oracle_mod.pack_srbcrs(m.M, m.rowptr, m.colind, m.values))
     _check_metcf(engine.pack_metcf(rp, ci, va, m.M, m.K), oracle_mod.pack_metcf(m.M, m.rowptr, m.colind, m.values))
     _check_mco(engine.pack_mco(rp, ci, va, m.M, m.K), oracle_mod.pack_mco(m.M, m.rowptr, m.colind, m.values))
+
+
+# Windows shared by a cluster: up to 4096 entries a block are kept in registers, more are read again, and a block's range of
+# columns is taken in parts where eight bitmaps do not cover K (beyond 2^23); `skew`: most entries among the first columns, so that
+# the ranges differ in width
+@pytest.mark.parametrize("K", [1 << 18, 1 << 20, 1 << 21, 1 << 22, (1 << 22) + 1, 1 << 23, (1 << 23) + 1, 1 << 24])
+@pytest.mark.parametrize("skew", [False, True])
+def test_pack_hub_windows(oracle_mod, K, skew):
+    from mask_b200 import engine
+    rng = np.random.Generator(np.random.PCG64(K + skew))
+    rows = []
+    for n, longest in ((30_000, 1 / 16), (32_768, 0.6), (70_000, 1 / 16), (200_000, 1 / 16), (200_000, 0.6)):
+        for r in range(16):
+            u = rng.random(int(n * (longest if r == 5 else (1 - longest) / 15)))
+            rows.append(np.unique((K * (u ** 4 if skew else u)).astype(np.int32)))
+    m = _rows_to_csr(rows[:-2], K, 7)
+    rp, ci, va = _dev(m)
+    _check_srbcrs(engine.pack_srbcrs(rp, ci, va, m.M, m.K), oracle_mod.pack_srbcrs(m.M, m.rowptr, m.colind, m.values))
+    _check_metcf(engine.pack_metcf(rp, ci, va, m.M, m.K), oracle_mod.pack_metcf(m.M, m.rowptr, m.colind, m.values))
+
+
+def test_pack_time_of_hub_windows_does_not_jump_with_the_columns():
+    """200 windows of 100 000 entries spread over 2^22 columns cost about what they cost over 2^20.  With ranges taken in parts
+    they took 1.2 ms against 0.5; 1.6 times leaves room for noise."""
+    import torch
+    from mask_b200 import engine
+    windows, per = 200, 6250
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rowptr = torch.arange(16 * windows + 1, dtype=torch.int32, device="cuda") * per
+    ms = {}
+    for K in (1 << 20, 1 << 22):
+        step = K // per
+        colind = torch.arange(per, device="cuda") * step + torch.randint(0, step, (16 * windows, per), generator=gen, device="cuda")
+        colind = colind.to(torch.int32).reshape(-1)
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            a.record()
+            engine._analyze(rowptr, colind, 16 * windows, K)
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        ms[K] = sorted(times)[3]
+    assert ms[1 << 22] < 1.6 * ms[1 << 20], ms
 
 
 @pytest.mark.parametrize("n", [40, 1030, 9000])
