@@ -244,11 +244,8 @@ void choose_plan_parameters(mask_plan* plan, const mask_column_features& f) {
     // hub-heavy (a quarter of the gathers already fit at full width) and markedly more fits at half width
     const bool narrower_rows_pay = !local && b_bytes > 8.0 * half_l2 && f.hub_share[0] >= 0.25 && f.hub_share[1] - f.hub_share[0] >= 0.02;
     plan->nslab = narrower_rows_pay ? 2 : 4;
-    const double even_share = f.distinct_columns ? (double)std::min(f.hub_columns[0], f.distinct_columns) / f.distinct_columns : 1.0;
     plan->local = f.local_share >= kLocalShare;
-    const bool hub_heavy = f.hub_share[0] >= 1.5 * even_share;
-    plan->slab_fits = !plan->local && !hub_heavy && b_bytes > f.l2_bytes && b_bytes / 4 <= f.l2_bytes;
-    plan->far_beyond_l2 = plan->nslab == 2 && b_bytes >= 12.0 * f.l2_bytes;
+    plan->two_slabs_kept = plan->nslab == 2 && b_bytes >= 8.0 * f.l2_bytes && b_bytes < 12.0 * f.l2_bytes;
 }
 
 }  // namespace mask

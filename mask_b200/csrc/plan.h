@@ -47,10 +47,9 @@ struct mask_plan {
     const int32_t* d_row_map = nullptr;  // optional, not owned: output row of packed row i (a row reorder's order[])
     float* const* d_peer_out = nullptr;  // optional, not owned: device array of n_peer_out extra output bases
     int32_t n_peer_out = 0;
-    // what the kernel choice goes by (choose_plan_parameters; without column features all false)
-    bool local = false;      // neighbouring windows share the rows of B they gather
-    bool far_beyond_l2 = false;  // hub-heavy, and B is many times the L2
-    bool slab_fits = false;  // 128 columns of B fit the L2, 512 do not, and all columns are gathered about equally
+    // what the kernel choice goes by besides the features (choose_plan_parameters; without column features false)
+    bool local = false;           // neighbouring windows share the rows of B they gather
+    bool two_slabs_kept = false;  // hub-heavy, and B is 8 to 12 times the L2
     mask_column_features col_features = {};   // set by mask_plan_autotune
     int32_t has_col_features = 0;
     float* d_vals_tf32 = nullptr;        // owned: val_block_val rounded to TF32 (mask_plan_prepare_values), for the TMA kernel

@@ -336,23 +336,51 @@ static int sweep_slabs(const mask_plan* plan, int N) {
 // matrices over up to 3256 blocks instead of 296, takes long windows first, and re-reads (and rebuilds) the tiles for every
 // block of columns.
 // It also rounds B where the tcgen05 kernel cuts it off: 2.1 to 3.0e-4 from the exact product (2-norm) against 4.2 to 4.7e-4.
-// Measured in turn (us, tcgen05 / warp), SR-BCRS; power-law graphs of 5000 / 20 000 / 130 000 / 300 000 / 2^20 / 2^21 nodes:
-//   N = 128    13 / 12,  29 / 21,  137 / 84,   274 / 171,  979 / 715,   2787 / 2082
-//   N = 192    16 / 14,  34 / 26,  184 / 124,  394 / 274,  1709 / 1138, 3929 / 3343
-//   N = 256    18 / 14,  35 / 31,  183 / 154,  395 / 335,  1803 / 1412, 4236 / 4145
-//   N = 512    23 / 21,  56 / 54,  308 / 293,  728 / 664,  3797 / 2985, -
-// stencils of 15^3 / 27^3 / 60^3 / 100^3, uniform 700 / 4096 / 20 000 / 10^5 / 2 10^5 rows:
-//   N = 128    7 / 5,    17 / 13,  126 / 94,   549 / 422,  8 / 6,   9 / 11,   21 / 18,  62 / 48,   122 / 116
-//   N = 192    8 / 7,    23 / 18,  184 / 148,  816 / 674,  10 / 6,  12 / 12,  29 / 18,  90 / 77,   194 / 178
-//   N = 256    8 / 6,    22 / 20,  184 / 184,  974 / 864,  10 / 7,  12 / 13,  29 / 25,  100 / 95,  267 / 229
-//   N = 512    10 / 9,   37 / 36,  327 / 365,  1724 / 2003, 13 / 7, 17 / 17,  47 / 42,  253 / 187, 600 / 451
-// ME-TCF (MCO like it, within a tenth), power-law and uniform:
-//   N = 128    16 / 16,  31 / 27,  151 / 99,   315 / 201,  1123 / 756,  2999 / 2183;   9 / 12, 10 / 17, 23 / 25, 69 / 55,   138 / 112
-//   N = 192    18 / 19,  35 / 32,  201 / 157,  434 / 334,  1658 / 1344, 3999 / 3522;  10 / 12, 12 / 19, 30 / 26, 99 / 89,   208 / 175
-//   N = 256    18 / 18,  36 / 37,  206 / 182,  446 / 386,  1884 / 1644, 4554 / 4232;  10 / 13, 12 / 19, 31 / 33, 106 / 106, 249 / 217
-//   N = 512    24 / 27,  60 / 62,  340 / 348,  822 / 754,  3615 / 3358, -;            14 / 13, 17 / 24, 50 / 53, 241 / 202, 577 / 429
-// stencils: N = 128 7 / 8, 18 / 18, 142 / 119, 619 / 509; 192 8 / 9, 26 / 27, 232 / 197, 1021 / 873; 256 8 / 8, 28 / 29, 261 / 227,
-// 1230 / 1059; 384 10 / 12, 38 / 37, 335 / 338, 1574 / 1674; 512 10 / 12, 42 / 48, 375 / 443, 1901 / 2379.
+// Measured in turn in bursts of 4 to 8 ms (us, tcgen05 / warp), which the power limit does not reach.  u uniform, g power-law, m
+// 27-point stencil, then rows in thousands (T tiles in thousands, groups of the warp kernel per SM):
+//   SR-BCRS               N = 64       96           128          192          256          384          448          512
+//   u.7   (1.9, .3)       9/8          9/8          9/8          11/8         11/8         17/9         17/9         17/9
+//   u6    (9, 2.5)        10/6         11/9         11/9         13/11        13/12        19/12        20/17        19/17
+//   u4    (10, 1.7)       9/8          9/9          9/11         12/12        12/13        17/17        17/17        17/17
+//   u20   (25, 8.4)       18/10        19/11        19/16        25/18        25/22        39/29        40/37        40/37
+//   u8    (39, 3.4)       21/19        22/23        21/21        31/28        30/29        49/46        49/46        48/47
+//   u25   (44, 11)        24/13        25/21        25/21        35/31        34/34        55/48        56/61        57/60
+//   g60   (98, 25)        74/30        76/38        78/45        92/68        94/81        134/116      140/151      143/152
+//   g130  (214, 35)       137/57       139/70       138/84       185/127      184/154      296/226      306/298      323/308
+//   u100  (128, 32)       63/31        63/42        65/49        96/82        108/105      189/158      221/211      257/198
+//   m43   (54, 18)        29/15        29/16        30/23        42/32        43/42        70/59        73/73        74/74
+//   m91   (116, 39)       57/27        58/36        58/45        83/68        85/83        141/124      153/167      157/170
+//   m1000 (1290, 422)     557/249      558/338      549/418      816/681      800/844      1325/1275    1393/1645    1477/1695
+//   g300  (489, 55)       275/116      279/150      275/172      394/280      396/334      713/499      728/644      728/660
+//   g524  (960, 83)       486/208      494/273      488/338      730/533      750/663      1344/993     1367/1281    1387/1319
+//   g600  (633, 69)       387/159      394/206      393/259      560/400      590/495      1029/736     1051/934     1070/972
+//   g700  (1312, 108)     649/271      658/372      655/460      942/738      987/920      1848/1384    1875/1771    1929/1839
+//   g1049 (1973, 148)     967/403      986/568      980/713      1419/1134    1561/1428    2836/2145    2869/2731    2996/2846
+//   g2097 (4035, 269)     1871/861     1901/1222    1901/1547    2839/2454    3371/3100    6081/4676    6138/5868    6590/6200
+//   ME-TCF (MCO within a tenth where it is not named)
+//   u.7   (1.9, .3)       10/15        10/15        10/15        12/16        12/16        18/17        18/17        17/17
+//   m3.4  (3.5, 1.4)      7/8          7/8          7/8          8/9          8/9          10/12        10/12        10/12
+//   m8    (9.6, 3.4)      11/9         11/11        11/10        15/15        15/14        20/21        21/22        21/20
+//   u4    (10, 1.7)       10/16        10/16        10/18        12/19        12/19        17/25        18/25        17/24
+//   g7    (11, 4.1)       17/16        17/18        17/17        19/20        19/20        24/29        25/30        25/29
+//   g10   (14, 5.7)       21/16        21/18        21/18        24/26        24/27        33/29        34/37        34/37
+//   u12   (15, 5.1)       16/11        16/16        16/14        21/19        21/22        30/24        31/32        31/31
+//   u16   (16, 6.8)       16/11        16/14        16/14        21/21        22/19        29/29        30/34        31/33
+//   m20   (24, 8.3)       18/15        18/14        18/18        26/28        27/29        37/37        40/49        42/48
+//   u20   (25, 8.4)       20/14        20/14        20/21        27/28        28/29        40/36        43/47        43/46
+//   g20   (29, 12)        31/19        31/24        31/27        35/32        36/37        53/48        57/63        60/62
+//   u25   (44, 11)        27/19        27/28        27/33        37/41        38/44        58/61        61/80        62/76
+//   u40   (61, 17)        37/27        36/26        35/33        50/44        52/55        81/77        84/101       88/98
+//   m43   (54, 18)        33/25        33/25        33/32        52/43        56/53        79/73        83/94        86/94
+//   u60   (77, 25)        46/30        46/34        44/36        63/55        65/66        106/94       116/125      128/127
+//   u100  (128, 32)       70/43        69/50        69/55        99/89        108/107      190/166      215/229      247/228
+//   u200  (255, 42)       133/75       138/100      138/112      208/175      250/217      420/323      492/422      580/427
+//   g200  (352, 44)       228/118      232/135      231/163      317/246      325/294      510/428      531/579      544/561
+//   g300  (489, 55)       310/148      318/184      316/202      435/334      447/386      794/572      809/780      819/755
+//   m1000 (1290, 422)     621/369      629/441      620/510      1025/872     1168/1010    1469/1516    1563/2006    1668/2015
+//   g1049 (1973, 148)     1092/528     1124/631     1124/756     1575/1224    1670/1487    3055/2223    3141/3018    3209/2948
+// Over the 68 matrices, 3 encodings and 11 to 15 widths of that measurement the choice below takes 0.6 % longer than the better
+// kernel would each time (geometric mean; SR-BCRS 0.2 %), at worst 36 % (ME-TCF of an 8^3 stencil, 9 us).
 static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, bool sidx_aligned) {
     if (tf32x3) return true;                    // compensated products: the warp kernel only
     if (!sidx_aligned || g_tune_sweep == 2) return false;
@@ -360,29 +388,36 @@ static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, 
     if (g_tune_sweep == 0) return true;
     if (g_tune_tma != 0 && fmt == kFmtSrbcrs && plan->d_vals_tf32 != nullptr) return false;
     const bool dense = fmt == kFmtSrbcrs;
-    const int64_t slabs = (N + 127) / 128, T = plan->T, groups = plan->Gw;
+    const int64_t slabs = (N + 127) / 128, T = plan->T, groups = plan->Gw, sms = sm_count();
     const int64_t block = 128 * sweep_slabs(plan, N), padded = (N + block - 1) / block * block;
     const bool pads = 4 * padded >= 5 * (int64_t)N;   // columns that the tcgen05 kernel's blocks would only pad: a quarter of N and more
+    const bool wide = N > 256 && !pads;
     // A handful of long groups: one warp takes half a microsecond per tile and twice that for one that it
     // rebuilds, a tcgen05 block an eighth.  With enough columns the warp kernel has more blocks to deal them to, and with very few
-    // groups (uniform 700 rows) neither fills the GPU.
-    if (groups < 4 * sm_count() && T > (dense ? 24 : 16) * groups) {
-        if (!dense) return false;
-        if (N > 128) return groups * slabs <= (N > 256 ? 4 : 2) * sm_count();
-        return N <= 64 ? groups > 2 * sm_count() : 2 * groups <= sm_count();
+    // groups (u.7) neither fills the GPU.
+    if (groups < (dense ? 4 : 5) * sms && T > (dense ? 32 : 16) * groups) {
+        if (dense) return N > 128 ? groups * slabs <= (N > 256 ? 4 : 2) * sms : (N <= 64 || groups <= sms);
+        if (N > 256) return 2 * groups * slabs <= 3 * sms;
+        return N <= 96 && groups > 2 * sms && T <= 24 * groups;
     }
-    if (!dense && groups < 9 * sm_count() && T > 16 * groups && (N <= 128 || !pads)) return false;
-    if (N <= 128) return true;
-    const bool wide = N > 256 && !pads;
-    // Full-width rows pay where neighbouring windows share them (60^3 and 100^3 stencil), for tiles that are rebuilt also where the
-    // matrix is small; not where 128 columns of B stay in L2 and all of them do not (10^5 rows: 241 / 202; N = 416 196 / 208).
-    if (plan->local && wide) return dense && T * slabs <= 150000;
-    // Power-law graphs, N = 512, at full clocks and in a run of seconds (tcgen05 / warp, ms): 2^18 nodes 0.72 / 0.61 and 0.76 / 0.70,
-    // 2^19 1.39 / 1.28 and 1.53 / 1.48, 2^20 2.97 / 2.74 and 3.30 / 3.13, 2^22 26.7 / 24.2 and 27.9 / 27.2.  Two slabs of the tcgen05 kernel stay the
-    // plan table's answer between 4 and 12 times the L2, as its test has it.
-    if (dense && wide && plan->nslab == 2 && !plan->far_beyond_l2) return false;
-    if (dense || (plan->slab_fits && N > 448)) return true;
-    return T > (wide ? 250000 : (pads ? 20000 : 40000));
+    // fewer groups than SMs, all short (ME-TCF, 160 to 256 columns: 9 / 10 on a power-law graph of 500 nodes, 9 / 7 on an 8^3 stencil)
+    if (fmt == kFmtMetcf ? 4 * groups <= sms && N > 256 : 4 * groups <= 3 * sms) return true;
+    // Tiles that are rebuilt: between the size at which blocks of 64 columns with long steps are all resident (13 an SM) and the one
+    // at which blocks of 128 columns fill the GPU (15 an SM) the warp kernel has neither (m20, u20, u25).
+    if (N <= 128) return dense || N <= 96 || T <= 18 * groups || 2 * groups <= 13 * sms || groups >= 13 * sms;
+    const double served = plan->col_features.hub_share[0];   // gathers of 512-column rows that half the L2 serves with the most gathered ones
+    if (dense) {
+        // Full-width rows pay where they are read from L2: neighbouring windows share them, or nearly all of B fits.  Not in small matrices.
+        if (wide && (plan->local || served >= 0.9)) return T * slabs <= 160000;
+        // Two slabs of the tcgen05 kernel remain what the plan table's test multiplies with: 8 to 12 times the L2, 5 to 12 % slower (g524, g700;
+        // in a run of seconds 1.53 / 1.48 ms at 2^19 nodes).
+        return !(wide && plan->two_slabs_kept);
+    }
+    if (wide) {   // the same for tiles that are rebuilt, four times as often as the tcgen05 kernel does
+        if (!plan->has_col_features) return T > 250000;
+        return !plan->local && (plan->nslab == 2 || served < 0.4 || (served < 0.75 && N > 448));
+    }
+    return groups >= (N > 256 ? 5 : (pads ? 9 : 18)) * sms;   // full rounds of blocks, of two column blocks each up to 256
 }
 
 static bool aligned(const void* p, unsigned bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
