@@ -86,7 +86,7 @@ static_assert(kHubThreads == 32 * kWinRows, "a warp for each row");
 constexpr int kBigBits = 1 << 19;                 // columns marked at a time: two blocks per SM
 constexpr int kHubBlocks = 8;
 constexpr int kHubBits = 1 << 19;                 // columns marked at a time by one block of a cluster: two blocks per SM
-constexpr int kHubBitsWide = 1 << 20;             // the same where eight of those do not cover K: one block per SM
+constexpr int kHubBitsWide = 1 << 20;             // the same where eight of these cover K and eight of those do not: one block per SM
 static_assert(kHubBitsWide <= kMarkMax, "");
 
 // One window of n <= 32 E entries: sorts (column, entry), numbers the distinct columns, writes every entry's
@@ -279,7 +279,9 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
 // Where eight marks of 2^19 columns do not cover K, parts cost more than the second block is worth.  Condensing in all, ranges at the
 // eighths alone and 2^19 columns always / as here: power-law graphs of 2^20 nodes 369 / 374 us, 2^21 1600 / 1020, 2^22 4560 / 3030, 2^23
 // 13 800 / 10 200, 2^22 and twice the degree 12 000 / 6020; 200 windows of 12 000 / 30 000 / 100 000 entries spread over 2^20 columns
-// 122 / 130, 197 / 182, 502 / 505; over 2^22 262 / 140, 456 / 193, 1197 / 540; over 2^23 367 / 249, 652 / 341, 1675 / 977.
+// 122 / 130, 197 / 182, 502 / 505; over 2^22 262 / 140, 456 / 193, 1197 / 540; over 2^23 367 / 249, 652 / 341, 1675 / 977.  Beyond that there
+are parts either way, and two blocks an SM get through them sooner: 12 000 / 100 000 entries over 2^24 columns 570 / 2630 us, with marks for 2^20 773 /
+3300; over 2^26 1740 / 8360 and 2200 / 9160.
 __global__ void __cluster_dims__(kHubBlocks, 1, 1) __launch_bounds__(kHubThreads, 2)
 condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M, int32_t K, int32_t span,
                     int32_t* __restrict__ pos, int32_t* __restrict__ cols, int32_t* __restrict__ distinct,
@@ -878,7 +880,7 @@ extern "C" int mask_pack_analyze(const int32_t* d_rowptr, const int32_t* d_colin
         condense_kernel<unsigned long long><<<(unsigned)W, 32, 0, st>>>(d_rowptr, d_colind, M, K, W, s.pos, s.cols, s.rows, s.distinct, s.big_list, s.hub_list, s.status);
     MASK_CUDA_TRY(cudaGetLastError());
     if (nnz > kHubMin) {
-        const int most_bits = K <= kHubBlocks * kHubBits ? kHubBits : kHubBitsWide;
+        const int most_bits = K > kHubBlocks * kHubBits && K <= kHubBlocks * kHubBitsWide ? kHubBitsWide : kHubBits;
         const int span = (int)std::min<int64_t>(((int64_t)K + 4095) / 4096 * 4096, most_bits);   // columns a block marks at a time
         const int smem = mark_set_bytes(span);
         static std::atomic<uint64_t> opted_in;

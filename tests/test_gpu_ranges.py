@@ -27,7 +27,7 @@ def _window(n, K, hub, seed):
 
 
 # sizes at which a window is sorted with more registers, ranked in one block's bitmap, shared by a cluster; key
-# width changes at 2^22 columns, a block's bitmap covers 2^19 columns at a time (in a cluster 2^20 beyond 2^22 columns)
+# width changes at 2^22 columns, a block's bitmap covers 2^19 columns at a time (in a cluster 2^20 from 2^22 to 2^23 columns)
 @pytest.mark.parametrize("K", [3000, 600_000, 2_200_000, 4_300_000])
 @pytest.mark.parametrize("hub", [False, True])
 def test_pack_window_sizes(oracle_mod, K, hub):
