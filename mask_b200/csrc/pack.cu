@@ -280,8 +280,8 @@ __global__ void __launch_bounds__(kBigThreads, 2) condense_big_kernel(const int3
 // eighths alone and 2^19 columns always / as here: power-law graphs of 2^20 nodes 369 / 374 us, 2^21 1600 / 1020, 2^22 4560 / 3030, 2^23
 // 13 800 / 10 200, 2^22 and twice the degree 12 000 / 6020; 200 windows of 12 000 / 30 000 / 100 000 entries spread over 2^20 columns
 // 122 / 130, 197 / 182, 502 / 505; over 2^22 262 / 140, 456 / 193, 1197 / 540; over 2^23 367 / 249, 652 / 341, 1675 / 977.  Beyond that there
-are parts either way, and two blocks an SM get through them sooner: 12 000 / 100 000 entries over 2^24 columns 570 / 2630 us, with marks for 2^20 773 /
-3300; over 2^26 1740 / 8360 and 2200 / 9160.
+// are parts either way, and two blocks an SM get through them sooner: 12 000 / 100 000 entries over 2^24 columns 570 / 2630 us, with marks for 2^20 773 /
+// 3300; over 2^26 1740 / 8360 and 2200 / 9160.
 __global__ void __cluster_dims__(kHubBlocks, 1, 1) __launch_bounds__(kHubThreads, 2)
 condense_hub_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, int32_t M, int32_t K, int32_t span,
                     int32_t* __restrict__ pos, int32_t* __restrict__ cols, int32_t* __restrict__ distinct,
