@@ -31,6 +31,7 @@ struct SpmmArgs {
     const int32_t* row_map;    // optional: packed row i is output row row_map[i] (row reorder undone on the fly)
     const float* B;
     int64_t ldb;
+    uint32_t ldb_bytes;      // 4 ldb: warp-level kernel only
     float* C;
     int64_t ldc;
     float* scratch;

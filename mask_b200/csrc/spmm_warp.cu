@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
 #pragma unroll
     for (int q = 0; q < NQ; q++) qok[q] = !GUARD || (col_base + 32 * q + 4 * lc) < p.N;
     const char* Bcol = reinterpret_cast<const char*>(p.B + col_base + 4 * lc);
-    const uint32_t ldb_bytes = (uint32_t)(p.ldb * 4);
+    // from a register in the blocks that are faster so (see warp_blocks_per_sm)
+    const uint32_t ldb_bytes = NQ == 3 || (DENSE && NQ == 1) ? (uint32_t)(p.ldb * 4) : p.ldb_bytes;
     // what this lane copies of a tile: 16 bytes of a dense one, 4 indices or values of a ME-TCF run, 4 values of a MCO run
     const char* a_src = DENSE ? reinterpret_cast<const char*>(p.val_blk + (int64_t)t0 * kTileElems + lane * 4)
                               : (METCF && lane < 8 ? reinterpret_cast<const char*>(p.coo_idx) : reinterpret_cast<const char*>(p.coo_val)) + (METCF ? lc : lane) * 16;
@@ -147,7 +148,10 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
     const int32_t* idp = p.val_sidx + (int64_t)t0 * kTileCols + lane;
     auto load_ids = [&](int (&id)[I::kRegs], int tile) {
 #pragma unroll
-        for (int i = 0; i < I::kRegs; i++) id[i] = tile + 4 * i + (lane >> 3) < n_tiles ? __ldg(idp + ids_before_tile(tile + 4 * i)) : 0;
+        for (int i = 0; i < I::kRegs; i++) {
+            const bool in = NQ == 3 ? tile + 4 * i < n_tiles - (lane >> 3) : tile + 4 * i + (lane >> 3) < n_tiles;
+            id[i] = in ? __ldg(idp + ids_before_tile(tile + 4 * i)) : 0;
+        }
     };
     auto load_runs = [&](int2& run, int tile) {
         if (lane < I::kTiles && tile + lane < n_tiles)
@@ -366,6 +370,9 @@ __global__ void __launch_bounds__(32, MINB) spmm_warp_kernel(const SpmmArgs p) {
 static constexpr int warp_step_tiles(int nq, int depth) { return (nq == 1 ? 2 : 1) << depth; }
 // Blocks per SM: as many as shared memory holds, except where the registers of the compensated products need
 // more room (N = 256, 200 000-node power-law graph: 12 blocks of 165 registers 500 us, 14 blocks 508, 15 of 128 562).
+// The registers of 24 blocks of 64 columns (80) and of 18 blocks of 96 (96) are all in use, so that how an address is written decides what is
+// spilled: a row's length of B from the launch arguments instead of a register takes 64 and 128 columns 1 to 8 % less time, SR-BCRS
+// blocks of 32 columns 5 % more, blocks of 96 1 % more; the first form of the ids' bound costs blocks of 96 columns 1 to 2 %.
 static constexpr int warp_blocks_per_sm(int nq, int depth, bool comp) {
     constexpr int blocks[4][3] = {{22, 12, 6}, {24, 13, 7}, {18, 10, 5}, {15, 8, 4}};
     constexpr int comp_blocks[4] = {22, 16, 14, 12};
@@ -438,6 +445,7 @@ int launch_spmm_warp(const mask_plan* plan, const SpmmArgs& a_in, cudaStream_t s
     a.warp_first = plan->d_warp_first;
     a.n_warp_first = plan->warp_first;
     a.n_frag = plan->F;
+    a.ldb_bytes = (uint32_t)(a.ldb * 4);
     int nq, depth;
     choose_warp_shape(plan, FMT == kFmtSrbcrs, a.N, a.tf32x3, tuned_nq, &nq, &depth);
     if constexpr (FMT == kFmtSrbcrs)
