@@ -386,11 +386,19 @@ static constexpr int warp_blocks_per_sm(int nq, int depth, bool comp) {
 // more than the widest block would.  us, one tile and all columns a step / as chosen here: uniform 16 384
 // rows, N = 64 18.6 / 9.1, N = 128 20.6 / 13.6; 15^3 stencil, N = 64 7.2 / 5.2, N = 256 10.7 / 6.8; power-law graph
 // of 20 000 nodes, N = 64 21.3 / 15.2.  With four times the resident blocks, long steps lose a quarter to a half, but for blocks of
-// 64 columns: 13 of them with two tiles a step finish a long window sooner than 24 with one, and that is what a graph of
-// middling size waits for (SR-BCRS / ME-TCF / MCO, N = 64, us; one tile a step, two: 130 000 nodes 64 / 91 / 94, 58 / 73 / 69; 300 000 nodes
-// 123 / 162 / 161, 115 / 148 / 139; 600 000 nodes 228 / 296 / 296, 225 / 287 / 270; uniform 10^5 rows 35 / 43 / 41, 31 / 41 / 38; not with
-// more tiles, 2^20 nodes 413 / 528 in SR-BCRS and ME-TCF, 431 / 538, uniform 2 10^5 rows of 20 102, 111, nor with a stencil's short windows, 59, 62).
-static void choose_warp_shape(const mask_plan* plan, bool dense, int N, bool comp, int tuned_nq, int* nq_out, int* depth_out) {
+// 64 columns: 13 of them with two tiles a step finish a long window sooner than 24 with one, and that is what a power-law graph waits
+// for.  us, one tile a step / two, by thousands of tiles (power-law, then uniform matrices):
+//   N = 64     160 T       214        446        489        1003       1973        4890           128       505        1277
+//   SR-BCRS    49 / 44     58 / 56    104 / 104  115 / 114  218 / 224  404 / 429   1014 / 1055    33 / 31   100 / 111  429 / 427
+//   ME-TCF     71 / 55     89 / 69    147 / 130  161 / 142  294 / 273  522 / 513   1239 / 1208    43 / 39   131 / 128  362 / 356
+//   MCO        71 / 54     90 / 67    144 / 125  156 / 137  286 / 266  514 / 498   1226 / 1187    40 / 37   132 / 125  357 / 378
+//   N = 48
+//   SR-BCRS    54 / 45     63 / 56    107 / 104  116 / 113  214 / 222  384 / 420   961 / 1023     32 / 31   95 / 104   393 / 392
+//   ME-TCF     78 / 58     97 / 73    158 / 136  172 / 146  313 / 280  558 / 525   1338 / 1250    46 / 41   144 / 135  358 / 349
+//   MCO        79 / 55     99 / 68    157 / 126  170 / 138  313 / 266  562 / 496   1345 / 1187    44 / 38   146 / 126  357 / 362
+// So SR-BCRS takes two up to 400 000 tiles, tiles that are rebuilt always, but for bitmaps of large matrices without hubs.  Not with a
+// stencil's short windows (60^3, N = 64, SR-BCRS: 59 / 62).
+static void choose_warp_shape(const mask_plan* plan, int fmt, int N, bool comp, int tuned_nq, int* nq_out, int* depth_out) {
     const int64_t groups = plan->Gw, T = plan->T;
     const int slabs = (N + 127) / 128, widest = (N + 32 * slabs - 1) / (32 * slabs);
     const bool tuned = tuned_nq >= 1 && tuned_nq <= 4;
@@ -407,7 +415,9 @@ static void choose_warp_shape(const mask_plan* plan, bool dense, int N, bool com
         }
     }
     *nq_out = tuned ? tuned_nq : widest;
-    *depth_out = *nq_out == 2 && !comp && !plan->local && T <= (dense ? 400000 : 1000000) ? 1 : 0;
+    const bool hubs = plan->col_features.hub_share[0] >= 0.25;
+    const bool two = fmt == kFmtSrbcrs ? T <= 400000 : (fmt == kFmtMetcf || hubs || T <= 1000000);
+    *depth_out = *nq_out == 2 && !comp && !plan->local && two ? 1 : 0;
 }
 
 template <int NQ, int DEPTH, int FMT, bool GUARD, bool COMP>
@@ -447,7 +457,7 @@ int launch_spmm_warp(const mask_plan* plan, const SpmmArgs& a_in, cudaStream_t s
     a.n_frag = plan->F;
     a.ldb_bytes = (uint32_t)(a.ldb * 4);
     int nq, depth;
-    choose_warp_shape(plan, FMT == kFmtSrbcrs, a.N, a.tf32x3, tuned_nq, &nq, &depth);
+    choose_warp_shape(plan, FMT, a.N, a.tf32x3, tuned_nq, &nq, &depth);
     if constexpr (FMT == kFmtSrbcrs)
         if (a.tf32x3) return launch_warp_shape<FMT, true>(plan, a, st, nq, depth);
     return launch_warp_shape<FMT, false>(plan, a, st, nq, depth);
