@@ -31,7 +31,6 @@ struct SpmmArgs {
     const int32_t* row_map;    // optional: packed row i is output row row_map[i] (row reorder undone on the fly)
     const float* B;
     int64_t ldb;
-    uint32_t ldb_bytes;      // 4 ldb: warp-level kernel only
     float* C;
     int64_t ldc;
     float* scratch;
@@ -42,6 +41,7 @@ struct SpmmArgs {
     int32_t vec_out;         // rows of C can be written 16 bytes at a time
     int32_t relu;
     int32_t tf32x3;  // compensated products (MASK_NUMERICS_TF32X3)
+    uint32_t ldb_bytes;      // 4 ldb, warp-level kernel only; fills the padding (8 more bytes of arguments: 0.3 us more of the host's time a launch)
 };
 
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
