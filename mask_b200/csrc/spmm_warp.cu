@@ -62,19 +62,21 @@ struct WarpIds {
     static constexpr int kRegs = kTiles / 4;
 };
 
+// Shared memory by 32-bit address.  The loads name "memory" as the stores and copies do: they read what other lanes wrote, and
+// without it nothing keeps the compiler from moving them across the __syncwarp() between the two.
 __device__ __forceinline__ float4 lds128(uint32_t at) {
     float4 v;
-    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
     return v;
 }
 __device__ __forceinline__ float2 lds64(uint32_t at) {
     float2 v;
-    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at));
+    asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(at) : "memory");
     return v;
 }
 __device__ __forceinline__ float lds32(uint32_t at) {
     float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at));
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
     return v;
 }
 __device__ __forceinline__ void sts32(uint32_t at, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory"); }
