@@ -240,6 +240,10 @@ size_t mask_plan_scratch_bytes(const mask_plan* plan, int32_t N);
 /* Introspection for tests: numbers of fragments, groups, split fragments, and the group size. */
 int mask_plan_info(const mask_plan* plan, int64_t* n_frag, int64_t* n_groups, int64_t* n_partial,
                    int32_t* group_tiles);
+/* Introspection for tests: the groups of tiles that the blocks of the warp-level kernel take, as quadruples (first fragment, end,
+ * first tile, tiles) -- n_first that are taken before the others, then n_groups, among which those are empty.  h_groups may be NULL;
+ * with it the call waits for the device. */
+int mask_plan_warp_groups(const mask_plan* plan, int64_t* n_first, int64_t* n_groups, int32_t* h_groups);
 /* Makes every SpMM launched with this plan write packed row i to output row d_row_order[i]
  * (NULL = identity): a matrix packed from reordered rows then produces C in the original row
  * order with no separate pass.  Replaces the bridge's host-side unpack_output

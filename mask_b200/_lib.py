@@ -46,6 +46,7 @@ SIGNATURES = {
     "mask_plan_destroy": (None, [vp]),
     "mask_plan_scratch_bytes": (sz, [vp, i32]),
     "mask_plan_info": (C.c_int, [vp, C.POINTER(i64), C.POINTER(i64), C.POINTER(i64), C.POINTER(i32)]),
+    "mask_plan_warp_groups": (C.c_int, [vp, C.POINTER(i64), C.POINTER(i64), vp]),
     "mask_plan_export": (C.c_int, [vp, vp, vp, vp]),
     "mask_features_columns": (C.c_int, [vp, vp, i32, i32, i64, i32, vp, vp]),
     "mask_plan_autotune": (C.c_int, [vp, vp, vp, i32, vp]),

@@ -683,6 +683,30 @@ extern "C" int mask_plan_info(const mask_plan* p, int64_t* n_frag, int64_t* n_gr
     return MASK_OK;
 }
 
+extern "C" int mask_plan_warp_groups(const mask_plan* p, int64_t* n_first, int64_t* n_groups, int32_t* h_groups) {
+    using namespace mask;
+    MASK_REQUIRE(p != nullptr, "plan is NULL");
+    if (n_first) *n_first = p->warp_first;
+    if (n_groups) *n_groups = p->Gw;
+    if (!h_groups || p->Gw == 0) return MASK_OK;
+    if (p->warp_first) MASK_CUDA_TRY(cudaMemcpy(h_groups, p->d_warp_first, (size_t)p->warp_first * sizeof(int4), cudaMemcpyDeviceToHost));
+    h_groups += 4 * (size_t)p->warp_first;
+    if (p->d_warp_group) {
+        MASK_CUDA_TRY(cudaMemcpy(h_groups, p->d_warp_group, (size_t)p->Gw * sizeof(int4), cudaMemcpyDeviceToHost));
+        return MASK_OK;
+    }
+    std::vector<int32_t> off((size_t)p->Gw + 1), tile((size_t)p->Gw + 1);
+    MASK_CUDA_TRY(cudaMemcpy(off.data(), p->d_group_off, off.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
+    MASK_CUDA_TRY(cudaMemcpy(tile.data(), p->d_group_tile, tile.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
+    for (int64_t i = 0; i < p->Gw; i++, h_groups += 4) {
+        h_groups[0] = off[i];
+        h_groups[1] = off[i + 1];
+        h_groups[2] = tile[i];
+        h_groups[3] = tile[i + 1] - tile[i];
+    }
+    return MASK_OK;
+}
+
 extern "C" int mask_plan_set_row_map(mask_plan* p, const int32_t* d_row_order) {
     using namespace mask;
     MASK_REQUIRE(p != nullptr, "plan is NULL");

@@ -240,6 +240,62 @@ def test_long_windows_among_short_ones(oracle_mod, windows, long_tiles):
     _assert_close(oracle_mod, m, B, out.cpu().numpy())
 
 
+def _windows_of(tiles, K, seed):
+    """Windows of exactly tiles[w] tiles, columns spread over all K."""
+    rng = np.random.Generator(np.random.PCG64(seed))
+    rows = []
+    for t in tiles:
+        step = K // max(8 * t, 1)
+        cols = np.arange(8 * t) * step + rng.integers(0, step, 8 * t)
+        rows += [cols[r::16].astype(np.int32) for r in range(16)]
+    return _rows_to_csr(rows, K, seed)
+
+
+def _warp_groups(plan):
+    """The groups of the warp kernel: those taken first, the others; (first fragment, end, first tile, tiles) each."""
+    import ctypes as C
+    from mask_b200 import _lib
+    first, rest = C.c_int64(), C.c_int64()
+    _lib.check(_lib.lib().mask_plan_warp_groups(plan._h, C.byref(first), C.byref(rest), None), "mask_plan_warp_groups")
+    groups = np.full((first.value + rest.value, 4), -1, np.int32)
+    _lib.check(_lib.lib().mask_plan_warp_groups(plan._h, None, None, groups.ctypes.data), "mask_plan_warp_groups")
+    return groups[:first.value], groups[first.value:]
+
+
+# Windows long enough to be groups of their own, none of them cut (a piece is as long as the mean window): which are listed, by
+# their tiles and their place; 26 tiles are too few wherever they are, 27 enough where what is left is 16 tiles a resident warp
+@pytest.mark.parametrize("windows", [60, 2047, 2049, 6200])
+@pytest.mark.parametrize("long,short", [(26, 18), (27, 18), (100, 64)])
+def test_which_windows_are_taken_first(oracle_mod, windows, long, short):
+    import torch
+    from mask_b200 import engine
+    tiles = np.where(np.arange(windows) % 2 == 1, long, short)
+    K = 200_000
+    m = _windows_of(tiles, K, windows + long)
+    p = engine.pack_srbcrs(*_dev(m), m.M, m.K)
+    plan = p.new_plan()
+    first, rest = _warp_groups(plan)
+    assert p.T == tiles.sum() and plan.info()["partial"] == 0 and plan.column_features()["local_share"] < 0.9
+    before = np.cumsum(tiles) - tiles
+    takers = 15 * torch.cuda.get_device_properties(0).multi_processor_count
+    left = (tiles.sum() + 4 * windows - before - 4 * np.arange(windows)) // takers
+    target = np.clip(left, 16, 128)
+    listed = 2 * (tiles + 4) > 3 * (target * 5 // 4)
+    assert sorted(first[:, 0]) == list(np.flatnonzero(listed))
+    # every fragment in exactly one group, every group with the tiles of its fragments
+    groups = np.concatenate([first, rest[rest[:, 1] > rest[:, 0]]])
+    groups = groups[np.argsort(groups[:, 0])]
+    assert groups[0, 0] == 0 and groups[-1, 1] == windows and np.array_equal(groups[1:, 0], groups[:-1, 1])
+    assert np.array_equal(groups[:, 2], before[groups[:, 0]]) and np.array_equal(groups[:, 3], np.add.reduceat(tiles, groups[:, 0]))
+    B = np.random.Generator(np.random.PCG64(1)).standard_normal((K, 64), dtype=np.float32)
+    engine.tune("sweep", 0)
+    try:
+        out = engine.spmm(p, torch.from_numpy(B).cuda(), plan=plan)
+    finally:
+        engine.tune("sweep", 1)
+    _assert_close(oracle_mod, m, B, out.cpu().numpy())
+
+
 # The kernel that measured faster, on both sides of the lines of the choice: compact tiles by groups an SM (20 000 rows: 8.4, 4096:
 # 1.7) and columns, full-width SR-BCRS of power-law graphs whose B is 4 to 8 times the L2, short groups of 24 tiles
 @pytest.mark.parametrize("rows,cols,fmt,N,kernel", [
