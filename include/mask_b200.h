@@ -417,6 +417,8 @@ int mask_tune(const char* name, int value);
  * reference. */
 int mask_spmm_kernel_name(const mask_plan* plan, int format, int32_t N, int epilogue, char* out, size_t capacity);
 int mask_kernel_revision(void);
+/* Introspection for tests: columns of a block and tiles a step if the warp-level kernel runs; arguments as above. */
+int mask_spmm_warp_shape(const mask_plan* plan, int format, int32_t N, int epilogue, int32_t* columns, int32_t* step_tiles);
 
 /* cudaMemcpy2DAsync behind the C ABI, for hosts that drive their own upload / product / download
  * pipeline over column chunks of row-major host matrices (kind: 1 = host to device, 2 = device to

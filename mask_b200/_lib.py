@@ -61,6 +61,7 @@ SIGNATURES = {
     "mask_spmm_srbcrs_static_scratch": (C.c_int, [vp, vp, vp, vp, i32, i32, i32, vp, i64, vp, i64, C.c_int, vp]),
     "mask_tune": (C.c_int, [C.c_char_p, C.c_int]),
     "mask_spmm_kernel_name": (C.c_int, [vp, C.c_int, i32, C.c_int, C.c_char_p, sz]),
+    "mask_spmm_warp_shape": (C.c_int, [vp, C.c_int, i32, C.c_int, C.POINTER(i32), C.POINTER(i32)]),
     "mask_kernel_revision": (C.c_int, []),
     "mask_copy_2d_async": (C.c_int, [vp, sz, vp, sz, sz, sz, C.c_int, vp]),
     "mask_session_create_srbcrs": (C.c_int, [i32, i32, i64, vp, vp, vp, C.c_int, C.POINTER(vp)]),

@@ -162,5 +162,6 @@ int launch_spmm_tma(const mask_plan* plan, const SpmmArgs& a, int64_t K, cudaStr
 // spmm_warp.cu: one warp per block, every encoding.  nq = 32-column groups per warp (1..4; 0 = by N).
 template <int FMT>
 int launch_spmm_warp(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st, int nq);
+void warp_shape(const mask_plan* plan, int fmt, int N, bool comp, int tuned_nq, int* columns, int* step_tiles);   // what it would take
 
 }  // namespace mask

@@ -526,6 +526,14 @@ extern "C" int mask_spmm_kernel_name(const mask_plan* plan, int format, int32_t 
     return MASK_OK;
 }
 
+extern "C" int mask_spmm_warp_shape(const mask_plan* plan, int format, int32_t N, int epilogue, int32_t* columns, int32_t* step_tiles) {
+    using namespace mask;
+    MASK_REQUIRE(plan != nullptr && columns != nullptr && step_tiles != nullptr, "NULL argument");
+    MASK_REQUIRE(format >= kFmtSrbcrs && format <= kFmtMco && N > 0, "bad format or N");
+    warp_shape(plan, format, N, format == kFmtSrbcrs && (epilogue & MASK_NUMERICS_TF32X3), g_tune_nq, columns, step_tiles);
+    return MASK_OK;
+}
+
 extern "C" int mask_tune(const char* name, int value) {
     using namespace mask;
     MASK_REQUIRE(name != nullptr, "name is NULL");

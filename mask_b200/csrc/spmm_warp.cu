@@ -375,10 +375,13 @@ static constexpr int warp_step_tiles(int nq, int depth) { return (nq == 1 ? 2 : 
 // The registers of 24 blocks of 64 columns (80) and of 18 blocks of 96 (96) are all in use, so that how an address is written decides what is
 // spilled: a row's length of B from the launch arguments instead of a register takes 64 and 128 columns 1 to 8 % less time, SR-BCRS
 // blocks of 32 columns 5 % more, blocks of 96 1 % more; the first form of the ids' bound costs blocks of 96 columns 1 to 2 %.
-static constexpr int warp_blocks_per_sm(int nq, int depth, bool comp) {
+// Bitmaps take a tile's room more (WarpLayout), which costs some shapes a block.
+static constexpr int warp_blocks_per_sm(int fmt, int nq, int depth, bool comp) {
     constexpr int blocks[4][3] = {{22, 12, 6}, {24, 13, 7}, {18, 10, 5}, {15, 8, 4}};
+    constexpr int mco_blocks[4][3] = {{20, 10, 5}, {24, 13, 6}, {18, 9, 5}, {15, 7, 3}};
     constexpr int comp_blocks[4] = {22, 16, 14, 12};
-    return comp && depth == 0 ? comp_blocks[nq - 1] : blocks[nq - 1][depth];
+    if (comp && depth == 0) return comp_blocks[nq - 1];
+    return (fmt == kFmtMco ? mco_blocks : blocks)[nq - 1][depth];
 }
 
 // Columns per warp (32 nq) and tiles per step for `groups` groups of tiles.  With fewer blocks than an SM holds the
@@ -387,7 +390,10 @@ static constexpr int warp_blocks_per_sm(int nq, int depth, bool comp) {
 // round of long ones doubles the time).  The longest step that fits comes first, then the fewest columns that pad no
 // more than the widest block would.  us, one tile and all columns a step / as chosen here: uniform 16 384
 // rows, N = 64 18.6 / 9.1, N = 128 20.6 / 13.6; 15^3 stencil, N = 64 7.2 / 5.2, N = 256 10.7 / 6.8; power-law graph
-// of 20 000 nodes, N = 64 21.3 / 15.2.  With four times the resident blocks, long steps lose a quarter to a half, but for blocks of
+// of 20 000 nodes, N = 64 21.3 / 15.2.  Bitmaps by the blocks of the other encodings, more than are resident, / by their own: groups of 20
+// tiles, 870 of them at N = 32 12.0 / 7.9, 1600 12.4 / 11.9, 450 at N = 64 12.0 / 7.6, 1030 13.0 / 11.5, 590 at N = 128 15.3 / 11.6.  But at 128
+// columns and two tiles a step an eighth block begun late costs less than 64 columns and one tile: 1180 groups of 20 tiles 16.8 / 19.4, of 45
+// 31.4 / 40.1, of 8 9.3 / 9.4.  With four times the resident blocks, long steps lose a quarter to a half, but for blocks of
 // 64 columns: 13 of them with two tiles a step finish a long window sooner than 24 with one, and that is what a power-law graph waits
 // for.  us, one tile a step / two, by thousands of tiles (power-law, then uniform matrices):
 //   N = 64     160 T       214        446        489        1003       1973        4890           128       505        1277
@@ -408,8 +414,9 @@ static void choose_warp_shape(const mask_plan* plan, int fmt, int N, bool comp, 
         for (int nq = tuned ? tuned_nq : 1; nq <= (tuned ? tuned_nq : widest); nq++) {
             const int blocks = (N + 32 * nq - 1) / (32 * nq);
             if (blocks * nq > slabs * widest && !tuned) continue;
-            const int64_t resident = (int64_t)sm_count() * warp_blocks_per_sm(nq, depth, comp);
-            if (groups * blocks <= resident + (T <= 24 * groups ? resident / 16 : 0)) {
+            const int64_t resident = (int64_t)sm_count() * warp_blocks_per_sm(fmt, nq, depth, comp);
+            const int64_t second = fmt == kFmtMco && nq == 4 && depth == 1 ? resident / 7 : (T <= 24 * groups ? resident / 16 : 0);
+            if (groups * blocks <= resident + second) {
                 *nq_out = nq;
                 *depth_out = depth;
                 return;
@@ -422,11 +429,21 @@ static void choose_warp_shape(const mask_plan* plan, int fmt, int N, bool comp, 
     *depth_out = *nq_out == 2 && !comp && !plan->local && two ? 1 : 0;
 }
 
+void warp_shape(const mask_plan* plan, int fmt, int N, bool comp, int tuned_nq, int* columns, int* step_tiles) {
+    int nq, depth;
+    choose_warp_shape(plan, fmt, N, comp, tuned_nq, &nq, &depth);
+    *columns = 32 * nq;
+    *step_tiles = warp_step_tiles(nq, depth);
+}
+
 template <int NQ, int DEPTH, int FMT, bool GUARD, bool COMP>
 static int launch_warp_variant(const mask_plan* plan, const SpmmArgs& a, cudaStream_t st) {
     constexpr int KT = warp_step_tiles(NQ, DEPTH), S = 3;
     using L = WarpLayout<NQ, KT, S, FMT>;
-    auto kern = spmm_warp_kernel<NQ, KT, S, warp_blocks_per_sm(NQ, DEPTH, COMP), FMT, GUARD, COMP>;
+    constexpr int kBlocks = warp_blocks_per_sm(FMT, NQ, DEPTH, COMP);
+    // an SM has 228 KB, in units of 128 bytes, and keeps 1 KB a block for itself
+    static_assert(kBlocks * ((L::kBytes + 127) / 128 * 128 + 1024) <= 228 * 1024, "more blocks than an SM's shared memory holds");
+    auto kern = spmm_warp_kernel<NQ, KT, S, kBlocks, FMT, GUARD, COMP>;
     static std::atomic<uint64_t> opted_in;
     const int rc = opt_in_shared_memory(reinterpret_cast<const void*>(kern), L::kBytes, opted_in);
     if (rc != MASK_OK) return rc;

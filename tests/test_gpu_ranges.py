@@ -296,6 +296,36 @@ def test_which_windows_are_taken_first(oracle_mod, windows, long, short):
     _assert_close(oracle_mod, m, B, out.cpu().numpy())
 
 
+# Columns of a block and tiles a step by the number of groups (one a window up to 1700), on both sides of what an SM holds; bitmaps take
+# more room.  At 64 columns and more blocks than are resident, two tiles a step.
+@pytest.mark.parametrize("fmt,N,windows,shape", [
+    ("srbcrs", 32, 800, (32, 8)), ("metcf", 32, 800, (32, 8)), ("mco", 32, 740, (32, 8)), ("mco", 32, 800, (32, 4)),
+    ("srbcrs", 32, 1700, (32, 4)), ("mco", 32, 1480, (32, 4)), ("mco", 32, 1700, (32, 2)),
+    ("srbcrs", 64, 1000, (64, 4)), ("mco", 64, 880, (64, 4)), ("mco", 64, 1000, (64, 2)),
+    ("srbcrs", 128, 560, (128, 4)), ("mco", 128, 440, (64, 4)), ("mco", 128, 560, (64, 2)), ("mco", 128, 1180, (128, 2)), ("mco", 128, 1190, (64, 1)),
+    ("srbcrs", 64, 12_000, (64, 2)), ("metcf", 64, 12_000, (64, 2)), ("mco", 64, 12_000, (64, 2)), ("srbcrs", 96, 12_000, (96, 1)),
+    ("srbcrs", 64, 16_000, (64, 1)), ("mco", 64, 16_000, (64, 2))])
+def test_warp_kernel_shape(oracle_mod, fmt, N, windows, shape):
+    import ctypes as C
+    import torch
+    from mask_b200 import _lib, engine
+    K = 200_000
+    m = _windows_of(np.full(windows, 26), K, windows)
+    p = {"srbcrs": engine.pack_srbcrs, "metcf": engine.pack_metcf, "mco": engine.pack_mco}[fmt](*_dev(m), m.M, m.K)
+    plan = p.new_plan()
+    columns, step = C.c_int32(), C.c_int32()
+    code = {"srbcrs": 0, "metcf": 1, "mco": 2}[fmt]
+    _lib.check(_lib.lib().mask_spmm_warp_shape(plan._h, code, N, 0, C.byref(columns), C.byref(step)), "mask_spmm_warp_shape")
+    assert (columns.value, step.value) == shape, len(_warp_groups(plan)[1])
+    B = np.random.Generator(np.random.PCG64(N)).standard_normal((K, N), dtype=np.float32)
+    engine.tune("sweep", 0)
+    try:
+        out = engine.spmm(p, torch.from_numpy(B).cuda(), plan=plan)
+    finally:
+        engine.tune("sweep", 1)
+    _assert_close(oracle_mod, m, B, out.cpu().numpy())
+
+
 # The kernel that measured faster, on both sides of the lines of the choice: compact tiles by groups an SM (20 000 rows: 8.4, 4096:
 # 1.7) and columns, full-width SR-BCRS of power-law graphs whose B is 4 to 8 times the L2, short groups of 24 tiles
 @pytest.mark.parametrize("rows,cols,fmt,N,kernel", [
