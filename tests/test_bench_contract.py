@@ -28,6 +28,13 @@ def _check_base(d):
     assert d["higher_is_better"] is True and d["value"] > 0 and d["ms_per_step"] > 0
 
 
+def test_captured_traffic_is_of_the_kernels_that_run():
+    """A figure captured on another revision of the kernels is not reported."""
+    import bench
+    from mask_b200 import _lib
+    assert bench.NCU_TRAFFIC and {c["revision"] for c in bench.NCU_TRAFFIC.values()} == {_lib.lib().mask_kernel_revision()}
+
+
 def test_reference_arm_line():
     d = _run("--impl", "reference", "--scale", "12", "--steps", "2", "--warmup", "1")
     _check_base(d)
