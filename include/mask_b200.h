@@ -319,7 +319,8 @@ int mask_plan_export(const mask_plan* plan, int32_t* frag_offset, int32_t* frag_
  * tiles in d_scratch, so results are run-to-run deterministic.  B is [K,N] with leading
  * dimension ldb.  Requirements: N % 4 == 0, ldb % 4 == 0, ldc % 4 == 0, 16-byte aligned B and C.
  * The packed arrays must be 16-byte aligned too (MASK_ERR_INVALID_ARGUMENT), except that val_coo_off
- * needs 8 bytes, val_mco_off 4, and val_sidx 4 unless products are compensated.
+ * needs 8 bytes, val_mco_off 4, and val_sidx 4 unless products are compensated (at less than 16 they run on the
+ * tcgen05 kernel).
  * ------------------------------------------------------------------------------------------ */
 #define MASK_EPILOGUE_NONE 0
 #define MASK_EPILOGUE_RELU 1 /* C = max(A*B, 0), used between GCN layers */

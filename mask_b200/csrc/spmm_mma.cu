@@ -380,7 +380,9 @@ static int sweep_slabs(const mask_plan* plan, int N) {
 //   m1000 (1290, 422)     621/369      629/441      620/510      1025/872     1168/1010    1469/1516    1563/2006    1668/2015
 //   g1049 (1973, 148)     1092/528     1124/631     1124/756     1575/1224    1670/1487    3055/2223    3141/3018    3209/2948
 // Over the 68 matrices, 3 encodings and 11 to 15 widths of that measurement the choice below takes 0.6 % longer than the better
-// kernel would each time (geometric mean; SR-BCRS 0.2 %), at worst 36 % (ME-TCF of an 8^3 stencil, 9 us).
+// kernel would each time (geometric mean; SR-BCRS 0.2 %), at worst 36 % (ME-TCF of an 8^3 stencil, 9 us).  Small bitmap matrices have
+// become faster in the warp kernel since (choose_warp_shape): over 512 uniform ones of 60 to 5000 windows and widths 3.5 % longer, at worst
+// 75 % (700 windows of 5 tiles, N = 192, 10 us).
 static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, bool sidx_aligned) {
     if (tf32x3) return true;                    // compensated products: the warp kernel only
     if (!sidx_aligned || g_tune_sweep == 2) return false;
@@ -422,8 +424,9 @@ static bool use_warp_kernel(const mask_plan* plan, int fmt, int N, bool tf32x3, 
 
 static bool aligned(const void* p, unsigned bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
 
-// The packed arrays as the asynchronous copies read them: 16 bytes at a time, pairs of offsets 8.  Ids as well in the warp
-// kernel, which other products leave to the tcgen05 kernel when they are not aligned.
+// The packed arrays as the asynchronous copies read them: 16 bytes at a time, pairs of offsets 8.  Ids are read one by one by both
+// kernels; that off 16 bytes they go to the tcgen05 kernel, and compensated products refuse them, is from when the warp kernel
+// copied them, and is kept as what the call answers.
 static int check_packed_alignment(const SpmmArgs& a) {
     MASK_REQUIRE(aligned(a.val_blk, 16) && aligned(a.coo_idx, 16) && aligned(a.coo_val, 16) && aligned(a.mco_mask, 16),
                  "val_block_val, val_coo_idx, val_coo_val, val_mco_mask and val_mco_val must be 16-byte aligned");
