@@ -393,7 +393,8 @@ static constexpr int warp_blocks_per_sm(int fmt, int nq, int depth, bool comp) {
 // of 20 000 nodes, N = 64 21.3 / 15.2.  Bitmaps by the blocks of the other encodings, more than are resident, / by their own: groups of 20
 // tiles, 870 of them at N = 32 12.0 / 7.9, 1600 12.4 / 11.9, 450 at N = 64 12.0 / 7.6, 1030 13.0 / 11.5, 590 at N = 128 15.3 / 11.6.  But at 128
 // columns and two tiles a step an eighth block begun late costs less than 64 columns and one tile: 1180 groups of 20 tiles 16.8 / 19.4, of 45
-// 31.4 / 40.1, of 8 9.3 / 9.4.  With four times the resident blocks, long steps lose a quarter to a half, but for blocks of
+// 31.4 / 40.1, of 8 9.3 / 9.4.  So does a tenth of 96 columns for more than 9 1/2 an SM of more than 16 tiles: 1440 groups of 20 17.1 / 18.0, of 45
+// 32.7 / 37.7, but of 16 14.8 / 14.1, and 1400 of 45 32.0 / 25.8.  With four times the resident blocks, long steps lose a quarter to a half, but for blocks of
 // 64 columns: 13 of them with two tiles a step finish a long window sooner than 24 with one, and that is what a power-law graph waits
 // for.  us, one tile a step / two, by thousands of tiles (power-law, then uniform matrices):
 //   N = 64     160 T       214        446        489        1003       1973        4890           128       505        1277
@@ -407,16 +408,17 @@ static constexpr int warp_blocks_per_sm(int fmt, int nq, int depth, bool comp) {
 // So SR-BCRS takes two up to 400 000 tiles, tiles that are rebuilt always, but for bitmaps of large matrices without hubs.  Not with a
 // stencil's short windows (60^3, N = 64, SR-BCRS: 59 / 62).
 static void choose_warp_shape(const mask_plan* plan, int fmt, int N, bool comp, int tuned_nq, int* nq_out, int* depth_out) {
-    const int64_t groups = plan->Gw, T = plan->T;
+    const int64_t groups = plan->Gw, T = plan->T, sms = sm_count();
     const int slabs = (N + 127) / 128, widest = (N + 32 * slabs - 1) / (32 * slabs);
     const bool tuned = tuned_nq >= 1 && tuned_nq <= 4;
     for (int depth = 2; depth >= 0; depth--) {
         for (int nq = tuned ? tuned_nq : 1; nq <= (tuned ? tuned_nq : widest); nq++) {
             const int blocks = (N + 32 * nq - 1) / (32 * nq);
             if (blocks * nq > slabs * widest && !tuned) continue;
-            const int64_t resident = (int64_t)sm_count() * warp_blocks_per_sm(fmt, nq, depth, comp);
-            const int64_t second = fmt == kFmtMco && nq == 4 && depth == 1 ? resident / 7 : (T <= 24 * groups ? resident / 16 : 0);
-            if (groups * blocks <= resident + second) {
+            int per_sm = warp_blocks_per_sm(fmt, nq, depth, comp);
+            if (fmt == kFmtMco && depth == 1 && (nq == 4 || (nq == 3 && T > 16 * groups && 2 * groups * blocks > 19 * sms))) per_sm++;
+            const int64_t resident = sms * per_sm;
+            if (groups * blocks <= resident + (T <= 24 * groups ? resident / 16 : 0)) {
                 *nq_out = nq;
                 *depth_out = depth;
                 return;

@@ -303,6 +303,7 @@ def test_which_windows_are_taken_first(oracle_mod, windows, long, short):
     ("srbcrs", 32, 1700, (32, 4)), ("mco", 32, 1480, (32, 4)), ("mco", 32, 1700, (32, 2)),
     ("srbcrs", 64, 1000, (64, 4)), ("mco", 64, 880, (64, 4)), ("mco", 64, 1000, (64, 2)),
     ("srbcrs", 128, 560, (128, 4)), ("mco", 128, 440, (64, 4)), ("mco", 128, 560, (64, 2)), ("mco", 128, 1180, (128, 2)), ("mco", 128, 1190, (64, 1)),
+    ("srbcrs", 96, 1400, (96, 2)), ("mco", 96, 1330, (96, 2)), ("mco", 96, 1400, (96, 1)), ("mco", 96, 1440, (96, 2)), ("mco", 96, 1490, (96, 1)),
     ("srbcrs", 64, 12_000, (64, 2)), ("metcf", 64, 12_000, (64, 2)), ("mco", 64, 12_000, (64, 2)), ("srbcrs", 96, 12_000, (96, 1)),
     ("srbcrs", 64, 16_000, (64, 1)), ("mco", 64, 16_000, (64, 2))])
 def test_warp_kernel_shape(oracle_mod, fmt, N, windows, shape):
